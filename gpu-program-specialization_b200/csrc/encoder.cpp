@@ -5,7 +5,7 @@
  * and specializer (projects/secant/s_cpu.c:193-414, s_cubin_specialize.c:1203-1368), in their
  * order, expanding routine calls in place with their arguments bound once.  It builds an
  * expression DAG (a routine argument used several times becomes a shared node).
- * Stage 2 (classify) labels every node by what its value depends on: nothing (literals), the
+ * Stage 2 (label, as the nodes are made) notes for every node by what its value depends on: nothing (literals), the
  * coefficient bank, the row, or both.
  * Stage 3 (emit) linearises the DAG for a machine with one accumulator: a binary node whose
  * other operand is a leaf costs one instruction, a node with two computed operands spills the
@@ -44,9 +44,9 @@ struct Token {
     size_t width;
 };
 
-/* operations by opcode: {opcode, arity, SB_* code} */
+/* operations: {opcode, arity, SB_* code} */
 struct OperationRow { uint8_t opcode, arity, code; };
-const OperationRow kOperations[] = {
+constexpr OperationRow kOperations[] = {
     {SECANT_AST_INSTRUCTION_TYPE_ADD_F32, 2, SB_BIN_ADD},   {SECANT_AST_INSTRUCTION_TYPE_SUB_F32, 2, SB_BIN_SUB},
     {SECANT_AST_INSTRUCTION_TYPE_MUL_F32, 2, SB_BIN_MUL},   {SECANT_AST_INSTRUCTION_TYPE_DIV_F32, 2, SB_BIN_DIV},
     {SECANT_AST_INSTRUCTION_TYPE_MIN_F32, 2, SB_BIN_MIN},   {SECANT_AST_INSTRUCTION_TYPE_MAX_F32, 2, SB_BIN_MAX},
@@ -72,62 +72,71 @@ bool evaluable_opcode(unsigned op) {
     }
 }
 
+/* What the first byte of a token says, by opcode: every program is walked twice (preflight, parser)
+ * before its call can start, so the per-token work is one table row.  `status` comes before every
+ * other check; a row that is an operation with arity 0 (NONE) decodes but cannot be evaluated. */
+struct OpcodeTable {
+    struct Row { Token token; SecantResult status; } row[256];
+    OpcodeTable() {
+        for (unsigned op = 0; op < 256; ++op) {
+            const SecantAstInstruction first = (SecantAstInstruction)op;
+            Token t{TK_OPERATION, 0, 0, 0, 0, secant_ast_instruction_size_get(&first)};
+            SecantResult status = SECANT_SUCCESS;
+            if (!t.width) status = SECANT_ERROR_BAD_PROGRAM;
+            else if (!evaluable_opcode(op)) status = SECANT_ERROR_UNSUPPORTED_OP;
+            switch (op) {
+            case SECANT_AST_INSTRUCTION_TYPE_COLUMN_F32: t.kind = TK_COLUMN; break;
+            case SECANT_AST_INSTRUCTION_TYPE_BANK_CONSTANT_F32: t.kind = TK_BANK; break;
+            case SECANT_AST_INSTRUCTION_TYPE_AFFINE_BANK_F32: t.kind = TK_AFFINE; break;
+            case SECANT_AST_INSTRUCTION_TYPE_CONSTANT_BITS_F32: t.kind = TK_LITERAL; break;
+            case SECANT_AST_INSTRUCTION_TYPE_TOGGLE2_F32: t.kind = TK_TOGGLE; t.ways = 2; break;
+            case SECANT_AST_INSTRUCTION_TYPE_TOGGLE4_F32: t.kind = TK_TOGGLE; t.ways = 4; break;
+            case SECANT_AST_INSTRUCTION_TYPE_ROUTINE_ARG_F32: t.kind = TK_ARG; break;
+            case SECANT_AST_INSTRUCTION_TYPE_ROUTINE_F32: t.kind = TK_CALL; break;
+            case SECANT_AST_INSTRUCTION_TYPE_RETURN_F32: t.kind = TK_RETURN; break;
+            default:
+                for (const OperationRow& o : kOperations)
+                    if (o.opcode == op) { t.arity = t.node = o.arity; t.op = o.code; }
+            }
+            row[op] = Row{t, status};
+        }
+    }
+};
+const OpcodeTable kTable;
+
 /* Decodes one token and applies every check that needs no evaluation state: byte width, opcode
  * class, leaf index ranges, toggle bit ranges, finite affine payloads.  Both the runner's
  * preflight (projects/secant/s_cubin_runner.c:138-181) and the parser below start from it, so
  * the two cannot disagree on what a well-formed token is. */
-SecantResult read_token(const SecantAstInstruction* ins, const ProgramRules& rules, Token* t) {
-    const unsigned op = ins[0];
-    t->width = secant_ast_instruction_size_get(ins);
-    t->ways = t->arity = t->node = t->op = 0;
-    if (!t->width) return SECANT_ERROR_BAD_PROGRAM;
-    if (!evaluable_opcode(op)) return SECANT_ERROR_UNSUPPORTED_OP;
-    switch (op) {
-    case SECANT_AST_INSTRUCTION_TYPE_COLUMN_F32:
-        t->kind = TK_COLUMN;
-        return ins[1] < rules.num_columns ? SECANT_SUCCESS : SECANT_ERROR_BAD_PROGRAM;
-    case SECANT_AST_INSTRUCTION_TYPE_BANK_CONSTANT_F32:
-        t->kind = TK_BANK;
-        return rules.banks_allowed && ins[1] < rules.num_constants ? SECANT_SUCCESS : SECANT_ERROR_BAD_PROGRAM;
-    case SECANT_AST_INSTRUCTION_TYPE_AFFINE_BANK_F32:
-        t->kind = TK_AFFINE;
-        if (!rules.banks_allowed || ins[1] >= rules.num_constants) return SECANT_ERROR_BAD_PROGRAM;
-        return std::isfinite(secant_ast_affine_bank_scale_get(ins)) && std::isfinite(secant_ast_affine_bank_offset_get(ins))
-                   ? SECANT_SUCCESS : SECANT_ERROR_BAD_PROGRAM;
-    case SECANT_AST_INSTRUCTION_TYPE_CONSTANT_BITS_F32:
-        t->kind = TK_LITERAL;
-        return SECANT_SUCCESS;
-    case SECANT_AST_INSTRUCTION_TYPE_TOGGLE2_F32:
-    case SECANT_AST_INSTRUCTION_TYPE_TOGGLE4_F32:
-        t->kind = TK_TOGGLE;
-        t->ways = op == SECANT_AST_INSTRUCTION_TYPE_TOGGLE2_F32 ? 2 : 4;
-        if (!rules.banks_allowed || ins[1] >= rules.toggle_bits) return SECANT_ERROR_BAD_PROGRAM;
-        if (t->ways == 4 && (ins[2] >= rules.toggle_bits || ins[2] == ins[1])) return SECANT_ERROR_BAD_PROGRAM;
-        return SECANT_SUCCESS;
-    case SECANT_AST_INSTRUCTION_TYPE_ROUTINE_ARG_F32: t->kind = TK_ARG; return SECANT_SUCCESS;
-    case SECANT_AST_INSTRUCTION_TYPE_ROUTINE_F32: t->kind = TK_CALL; return SECANT_SUCCESS;
-    case SECANT_AST_INSTRUCTION_TYPE_RETURN_F32: t->kind = TK_RETURN; return SECANT_SUCCESS;
+inline SecantResult read_token(const SecantAstInstruction* ins, const ProgramRules& rules, Token* t) {
+    const OpcodeTable::Row& row = kTable.row[ins[0]];
+    *t = row.token;
+    if (row.status != SECANT_SUCCESS) return row.status;
+    bool good = true;
+    switch (row.token.kind) {
+    case TK_COLUMN: good = ins[1] < rules.num_columns; break;
+    case TK_BANK: good = rules.banks_allowed && ins[1] < rules.num_constants; break;
+    case TK_AFFINE:
+        good = rules.banks_allowed && ins[1] < rules.num_constants && std::isfinite(secant_ast_affine_bank_scale_get(ins)) &&
+               std::isfinite(secant_ast_affine_bank_offset_get(ins));
+        break;
+    case TK_TOGGLE:
+        good = rules.banks_allowed && ins[1] < rules.toggle_bits &&
+               (row.token.ways == 2 || (ins[2] < rules.toggle_bits && ins[2] != ins[1]));
+        break;
     default: break;
     }
-    t->kind = TK_OPERATION;
-    for (const OperationRow& row : kOperations)
-        if (row.opcode == op) {
-            t->arity = row.arity;
-            t->node = row.arity;
-            t->op = row.code;
-            return SECANT_SUCCESS;
-        }
-    return SECANT_SUCCESS; /* NONE: decodable, rejected when evaluated (arity 0) */
+    return good ? SECANT_SUCCESS : SECANT_ERROR_BAD_PROGRAM;
 }
 
-bool direct_leaf(TokenKind k) { return k == TK_COLUMN || k == TK_BANK || k == TK_AFFINE || k == TK_LITERAL; }
+inline bool direct_leaf(TokenKind k) { return k == TK_COLUMN || k == TK_BANK || k == TK_AFFINE || k == TK_LITERAL; }
 
 /* ---- expression DAG -------------------------------------------------------------------- */
 
 enum NodeType : uint8_t { N_COL, N_BANK, N_AFFINE, N_LIT, N_TOGGLE, N_UN, N_BIN, N_FMA };
 /* What a value depends on.  Joining two classes: a literal adopts the other class, bank and row
  * together make a mixed value. */
-enum ValueClass : int8_t { VC_UNKNOWN = -1, VC_LITERAL = 0, VC_BANK = 1, VC_ROW = 2, VC_MIXED = 3 };
+enum ValueClass : int8_t { VC_LITERAL = 0, VC_BANK = 1, VC_ROW = 2, VC_MIXED = 3 };
 
 ValueClass join(ValueClass a, ValueClass b) {
     if (a == b || b == VC_LITERAL) return a;
@@ -136,10 +145,13 @@ ValueClass join(ValueClass a, ValueClass b) {
 }
 
 struct Node {
-    NodeType type;
+    NodeType type = N_LIT;
     uint8_t op = 0;       /* SB_UN_* for N_UN, SB_BIN_{ADD,SUB,MUL,DIV,MIN,MAX} for N_BIN */
     uint8_t ways = 0;     /* toggle: 2 or 4 */
     uint8_t bit0 = 0, bit1 = 0xff;
+    ValueClass cls = VC_LITERAL;
+    bool toggled = false; /* a toggle lies somewhere below (or here): the value changes with the permutation */
+    uint8_t seen = 0;     /* marks of collect() */
     int32_t child[4] = {-1, -1, -1, -1};
     uint32_t index = 0;   /* column / bank slot / affine entry */
     uint32_t bits = 0;    /* literal */
@@ -147,13 +159,25 @@ struct Node {
     int32_t pending = 0;  /* uses not yet emitted */
     int32_t slot = -1;    /* spill slot holding the value, once computed */
     int32_t su = 0;       /* slots needed to compute the node into the accumulator */
-    ValueClass cls = VC_UNKNOWN;
     int32_t hoisted = -1; /* per-row value the prelude left */
     int32_t entry = -1;   /* constant-table entry the bank part left */
     int32_t weight = 0;   /* rough instruction cost of the sub-expression */
 };
 
 unsigned arity_of(const Node& n) { return n.type == N_UN ? 1 : n.type == N_BIN ? 2 : n.type == N_FMA ? 3 : 0; }
+
+/* rough executed-instruction weights used for scheduling (SbProgram::cost) and for choosing
+ * which row-only sub-expressions are worth a hoist slot */
+int unary_weight(unsigned op) {
+    switch (op) {
+    case SB_UN_NEG: case SB_UN_ABS: return 1;
+    case SB_UN_SIN: case SB_UN_COS: return 18;
+    case SB_UN_EXP: case SB_UN_EX2: return 9;
+    case SB_UN_LOG: return 14;
+    default: return 12;
+    }
+}
+int binary_weight(unsigned op) { return (op == SB_BIN_DIV || op == SB_BIN_RDIV) ? 11 : 1; }
 
 struct Parser {
     const SecantAstProgramList& routines;
@@ -163,7 +187,35 @@ struct Parser {
     std::vector<SbAffine>& affines; /* of this program */
     unsigned n_ops = 0;
 
-    int add(const Node& n) { nodes.push_back(n); return (int)nodes.size() - 1; }
+    Node& make(NodeType type) {
+        nodes.emplace_back();
+        nodes.back().type = type;
+        return nodes.back();
+    }
+    /* Labels the node just made with what its value depends on and what it costs, and returns its id.
+     * Children exist before their parents, so one look at them is enough. */
+    int label(Node& n) {
+        switch (n.type) {
+        case N_COL: n.cls = rules.columns_are_slots ? VC_MIXED : VC_ROW; break;
+        case N_BANK: case N_AFFINE: n.cls = VC_BANK; break;
+        case N_LIT: break;
+        case N_TOGGLE:
+            n.toggled = true;
+            for (unsigned i = 0; i < n.ways; ++i) n.cls = join(n.cls, nodes[(size_t)n.child[i]].cls);
+            break;
+        default: {
+            int64_t w = n.type == N_UN ? unary_weight(n.op) : n.type == N_BIN ? binary_weight(n.op) : 4;
+            for (unsigned i = 0; i < arity_of(n); ++i) {
+                const Node& c = nodes[(size_t)n.child[i]];
+                n.cls = join(n.cls, c.cls);
+                n.toggled = n.toggled || c.toggled;
+                w += c.weight;
+            }
+            n.weight = (int32_t)std::min<int64_t>(w, INT32_MAX); /* a shared value counts once per parent */
+        }
+        }
+        return (int)nodes.size() - 1;
+    }
 
     int affine_entry(uint32_t slot, float scale, float offset) {
         for (size_t i = 0; i < affines.size(); ++i)
@@ -188,23 +240,23 @@ struct Parser {
             if (t.kind == TK_ARG && (!args || ins[1] >= num_args)) return SECANT_ERROR_ROUTINE_ARG_IDX_OUT_OF_BOUNDS;
             if (pushes && top == SECANT_AST_MAX_STACK_DEPTH) return SECANT_ERROR_STACK_OVERFLOW;
             switch (t.kind) {
-            case TK_COLUMN: { Node nd{N_COL}; nd.index = ins[1]; stack[top++] = add(nd); break; }
-            case TK_BANK: { Node nd{N_BANK}; nd.index = ins[1]; stack[top++] = add(nd); break; }
+            case TK_COLUMN: { Node& nd = make(N_COL); nd.index = ins[1]; stack[top++] = label(nd); break; }
+            case TK_BANK: { Node& nd = make(N_BANK); nd.index = ins[1]; stack[top++] = label(nd); break; }
             case TK_AFFINE: {
-                Node nd{N_AFFINE};
+                Node& nd = make(N_AFFINE);
                 nd.index = (uint32_t)affine_entry(ins[1], secant_ast_affine_bank_scale_get(ins), secant_ast_affine_bank_offset_get(ins));
-                stack[top++] = add(nd);
+                stack[top++] = label(nd);
                 break;
             }
-            case TK_LITERAL: { Node nd{N_LIT}; nd.bits = secant_ast_constant_bits_get(ins); stack[top++] = add(nd); break; }
+            case TK_LITERAL: { Node& nd = make(N_LIT); nd.bits = secant_ast_constant_bits_get(ins); stack[top++] = label(nd); break; }
             case TK_ARG: stack[top++] = args[ins[1]]; break;
             case TK_TOGGLE: {
                 if (leaves_in_a_row < t.ways || top < t.ways) return SECANT_ERROR_BAD_PROGRAM;
-                Node nd{N_TOGGLE};
+                Node& nd = make(N_TOGGLE);
                 nd.ways = t.ways; nd.bit0 = ins[1]; nd.bit1 = t.ways == 4 ? ins[2] : 0xff;
                 for (size_t i = 0; i < t.ways; ++i) nd.child[i] = stack[top - t.ways + i];
                 top -= t.ways;
-                stack[top++] = add(nd);
+                stack[top++] = label(nd);
                 break;
             }
             case TK_CALL: {
@@ -226,11 +278,11 @@ struct Parser {
             case TK_OPERATION: {
                 if (!t.arity) return SECANT_ERROR_BAD_PROGRAM;
                 if (top < t.arity) return SECANT_ERROR_STACK_UNDERFLOW;
-                Node nd{t.node == 1 ? N_UN : t.node == 2 ? N_BIN : N_FMA};
+                Node& nd = make(t.node == 1 ? N_UN : t.node == 2 ? N_BIN : N_FMA);
                 nd.op = t.op;
                 for (unsigned i = 0; i < t.arity; ++i) nd.child[i] = stack[top - t.arity + i];
                 top -= t.arity;
-                stack[top++] = add(nd);
+                stack[top++] = label(nd);
                 ++n_ops;
                 break;
             }
@@ -251,18 +303,6 @@ struct Operand {
  * which an item that covers several permutations computes once, and values a toggle reaches. */
 enum Run { RUN_BANK = 0, RUN_SHARED = 1, RUN_ROW = 2, RUN_MAIN = 3, NUM_RUNS = 4 };
 
-/* rough executed-instruction weights used for scheduling (SbProgram::cost) and for choosing
- * which row-only sub-expressions are worth a hoist slot */
-int unary_weight(unsigned op) {
-    switch (op) {
-    case SB_UN_NEG: case SB_UN_ABS: return 1;
-    case SB_UN_SIN: case SB_UN_COS: return 18;
-    case SB_UN_EXP: case SB_UN_EX2: return 9;
-    case SB_UN_LOG: return 14;
-    default: return 12;
-    }
-}
-int binary_weight(unsigned op) { return (op == SB_BIN_DIV || op == SB_BIN_RDIV) ? 11 : 1; }
 int insn_weight(const SbInsn& ins) {
     const unsigned cs = ins.w0 & 0xffu;
     if (cs >= SB_CASE_BIN && cs < SB_CASE_UN) return 1 + binary_weight((cs - SB_CASE_BIN) / SB_NUM_KINDS);
@@ -271,29 +311,58 @@ int insn_weight(const SbInsn& ins) {
     return 2;
 }
 
+struct LeafEntry { NodeType type; uint32_t key; int entry; };
+
+/* Working storage of one encode_program() call.  Every thread keeps one: a program needs a dozen
+ * small arrays, and making them anew for each program cost as much as filling them (5.9 us per
+ * program of the 32-token, 16-slot kind on a 2.7 GHz Xeon; 3.7 us with the arrays kept, the nodes
+ * labelled as they are parsed and each phase resetting only the nodes it reached). */
+struct Scratch {
+    std::vector<Node> nodes;
+    std::vector<SbAffine> affines; /* of this program */
+    std::vector<SbInsn> code[NUM_RUNS];
+    std::vector<SbPatch> sites[NUM_RUNS]; /* SbPatch::insn is relative to the run until the record is assembled */
+    std::vector<uint8_t> slot_busy;
+    std::vector<int> touched;             /* nodes the phase being emitted reaches */
+    std::vector<LeafEntry> leaf_entries;
+    std::vector<int> bank_roots, row_roots, shared_roots, chosen;
+    std::vector<SbInsn> fused;
+    std::vector<uint8_t> is_site;
+    std::vector<uint32_t> moved;
+
+    void begin() {
+        if (nodes.capacity() > 8192) *this = Scratch(); /* an unusually large program's storage is not kept */
+        nodes.clear(); affines.clear(); slot_busy.clear(); touched.clear(); leaf_entries.clear();
+        bank_roots.clear(); row_roots.clear(); shared_roots.clear(); chosen.clear();
+        for (auto& c : code) c.clear();
+        for (auto& c : sites) c.clear();
+    }
+};
+
 /* Bookkeeping rule of the emitter: gen(id) leaves the value of node `id` in the accumulator and
  * never consumes a use; the instruction that reads a value (as its accumulator input or as its
  * operand) consumes one use of it.  A computed node with several parents is parked in a slot
  * right after it is computed; a slot is released when the last use of its node is consumed. */
 struct Emitter {
+    Scratch& mem;
     std::vector<Node>& nodes;
     const ProgramRules& rules;
     EncodedBatch& out;
     size_t lit_base;
     unsigned n_affine;
-    std::vector<SbInsn> code[NUM_RUNS];
-    std::vector<SbPatch> sites[NUM_RUNS]; /* SbPatch::insn is relative to the run until the record is assembled */
+    std::vector<SbInsn> (&code)[NUM_RUNS];
+    std::vector<SbPatch> (&sites)[NUM_RUNS];
     Run run = RUN_MAIN;
-    std::vector<uint8_t> slot_busy;
+    std::vector<uint8_t>& slot_busy;
     unsigned slots_high = 0, btmp_high = 0;
     unsigned n_entries = 0, n_hoisted = 0;
     bool uses_scratch = false;
     SecantResult error = SECANT_SUCCESS;
-    struct LeafEntry { NodeType type; uint32_t key; int entry; };
-    std::vector<LeafEntry> leaf_entries;
+    std::vector<LeafEntry>& leaf_entries;
 
-    Emitter(std::vector<Node>& nodes_, const ProgramRules& rules_, EncodedBatch& out_, unsigned n_affine_)
-        : nodes(nodes_), rules(rules_), out(out_), lit_base(out_.lits.size()), n_affine(n_affine_) {}
+    Emitter(Scratch& mem_, const ProgramRules& rules_, EncodedBatch& out_)
+        : mem(mem_), nodes(mem_.nodes), rules(rules_), out(out_), lit_base(out_.lits.size()), n_affine((unsigned)mem_.affines.size()),
+          code(mem_.code), sites(mem_.sites), slot_busy(mem_.slot_busy), leaf_entries(mem_.leaf_entries) {}
 
     static bool leaf_type(const Node& n) { return n.type <= N_TOGGLE; }
     /* a value that can be named as an operand without computing anything */
@@ -302,69 +371,34 @@ struct Emitter {
         return leaf_type(n) || n.slot >= 0 || (run != RUN_BANK && n.hoisted >= 0) || n.entry >= 0;
     }
 
-    ValueClass classify(int id) {
-        Node& n = nodes[id];
-        if (n.cls != VC_UNKNOWN) return n.cls;
-        ValueClass c = VC_LITERAL;
-        int w = 0;
-        switch (n.type) {
-        case N_COL: c = rules.columns_are_slots ? VC_MIXED : VC_ROW; break;
-        case N_BANK: case N_AFFINE: c = VC_BANK; break;
-        case N_LIT: break;
-        case N_TOGGLE:
-            for (unsigned i = 0; i < n.ways; ++i) c = join(c, classify(n.child[i]));
-            break;
-        default:
-            for (unsigned i = 0; i < arity_of(n); ++i) {
-                c = join(c, classify(nodes[id].child[i]));
-                w += nodes[nodes[id].child[i]].weight;
-            }
-            w += n.type == N_UN ? unary_weight(n.op) : n.type == N_BIN ? binary_weight(n.op) : 4;
-        }
-        nodes[id].cls = c;
-        nodes[id].weight = w;
-        return c;
-    }
-
     /* Sub-expressions to move out of the main part: maximal computed nodes whose value depends on
      * the bank only (or on nothing), and maximal computed nodes that depend on the row only.
      * Inside a row-only expression, literal-only computed nodes still go to the bank part. */
-    void collect(int id, bool inside_row, std::vector<int>& bank_roots, std::vector<int>& row_roots, std::vector<uint8_t>& seen) {
+    void collect(int id, bool inside_row, std::vector<int>& bank_roots, std::vector<int>& row_roots) {
+        Node& n = nodes[id];
         const unsigned mark = inside_row ? 2u : 1u;
-        if (seen[(size_t)id] & mark) return;
-        seen[(size_t)id] |= (uint8_t)mark;
-        const Node& n = nodes[id];
-        if (leaf_type(n)) return;
-        const ValueClass c = classify(id);
-        if (c <= VC_BANK && rules.hoist_bank) {
+        if (leaf_type(n) || (n.seen & mark)) return;
+        n.seen |= (uint8_t)mark;
+        if (n.cls <= VC_BANK && rules.hoist_bank) {
             if (std::find(bank_roots.begin(), bank_roots.end(), id) == bank_roots.end()) bank_roots.push_back(id);
             return;
         }
-        if (c == VC_ROW && rules.hoist_row && !inside_row) {
+        if (n.cls == VC_ROW && rules.hoist_row && !inside_row) {
             if (std::find(row_roots.begin(), row_roots.end(), id) == row_roots.end()) row_roots.push_back(id);
             inside_row = true;
         }
-        for (unsigned i = 0; i < arity_of(n); ++i) collect(nodes[id].child[i], inside_row, bank_roots, row_roots, seen);
+        for (unsigned i = 0; i < arity_of(n); ++i) collect(n.child[i], inside_row, bank_roots, row_roots);
     }
 
-    /* whether a toggle lies anywhere below the node: such a value changes with the permutation */
-    bool reaches_toggle(int id, std::vector<int8_t>& memo) {
-        if (memo[(size_t)id] >= 0) return memo[(size_t)id] != 0;
-        const Node& n = nodes[id];
-        bool any = n.type == N_TOGGLE;
-        for (unsigned i = 0; i < arity_of(n) && !any; ++i) any = reaches_toggle(nodes[id].child[i], memo);
-        memo[(size_t)id] = any ? 1 : 0;
-        return any;
-    }
     /* maximal computed row-only nodes below `id` that no toggle reaches */
-    void collect_shared(int id, std::vector<int>& shared, std::vector<int8_t>& memo) {
+    void collect_shared(int id, std::vector<int>& shared) {
         const Node& n = nodes[id];
         if (leaf_type(n)) return;
-        if (classify(id) == VC_ROW && !reaches_toggle(id, memo)) {
+        if (n.cls == VC_ROW && !n.toggled) {
             if (std::find(shared.begin(), shared.end(), id) == shared.end()) shared.push_back(id);
             return;
         }
-        for (unsigned i = 0; i < arity_of(n); ++i) collect_shared(nodes[id].child[i], shared, memo);
+        for (unsigned i = 0; i < arity_of(n); ++i) collect_shared(n.child[i], shared);
     }
 
     int alloc_slot() {
@@ -383,11 +417,12 @@ struct Emitter {
      * of the prelude could not be trusted by the main part of every bank group). */
     void begin_phase(Run r, int phase_root) {
         run = r;
-        for (auto& n : nodes) { n.uses = 0; n.pending = 0; n.slot = -1; }
+        for (int id : mem.touched) { Node& n = nodes[id]; n.uses = 0; n.pending = 0; n.slot = -1; } /* of the phase before */
+        mem.touched.clear();
         slot_busy.clear();
         if (r != RUN_BANK) slot_busy.assign(rules.reserved_slots, 1);
         prepare(phase_root);
-        for (auto& n : nodes) n.pending = n.uses;
+        for (int id : mem.touched) nodes[id].pending = nodes[id].uses;
     }
 
     /* Counts parent references of every reachable node and computes how many slots each needs
@@ -395,6 +430,7 @@ struct Emitter {
     void prepare(int id) {
         Node& n = nodes[id];
         if (n.uses++ > 0) return;
+        mem.touched.push_back(id);
         if (ready(id)) { n.su = 0; return; }
         const unsigned arity = arity_of(n);
         for (unsigned i = 0; i < arity; ++i) prepare(nodes[id].child[i]);
@@ -472,7 +508,7 @@ struct Emitter {
     void emit_reading(unsigned case_base, int id) {
         const Node& n = nodes[id];
         const bool open_toggle = n.type == N_TOGGLE && n.slot < 0 && n.entry < 0;
-        if (open_toggle && rules.split_parts && run != RUN_BANK && classify(id) <= VC_BANK) {
+        if (open_toggle && rules.split_parts && run != RUN_BANK && n.cls <= VC_BANK) {
             /* a toggle among constants is resolved once per bank in the bank part */
             const int e = entry_for(id);
             push(sb_w0(case_base + SB_KIND_CST, 0, (unsigned)e), 0);
@@ -553,10 +589,11 @@ struct Emitter {
             const bool table = run == RUN_BANK && nodes[id].entry >= 0 && nodes[id].slot < 0;
             if (!toggle && !hrow && !table) continue;
             emit_reading(SB_CASE_LOAD, id);
-            Node t{N_UN};
-            t.cls = VC_MIXED;
-            nodes.push_back(t);
+            nodes.emplace_back();
+            nodes.back().type = N_UN;
+            nodes.back().cls = VC_MIXED;
             const int temp = (int)nodes.size() - 1;
+            mem.touched.push_back(temp);
             park(temp);
             for (int j = i; j < 3; ++j)
                 if (ch[j] == id) { ch[j] = temp; ++nodes[temp].uses; ++nodes[temp].pending; consume(id); }
@@ -659,9 +696,10 @@ SecantResult preflight(const SecantAstInstruction* program, const ProgramRules& 
 
 SecantResult encode_program(const SecantAstInstruction* program, const SecantAstProgramList& routines,
                             const uint8_t* routine_arity, const ProgramRules& rules, EncodedBatch& out) {
-    std::vector<Node> nodes;
-    std::vector<SbAffine> affines;
-    nodes.reserve(64);
+    static thread_local Scratch mem;
+    mem.begin();
+    std::vector<Node>& nodes = mem.nodes;
+    std::vector<SbAffine>& affines = mem.affines;
     Parser parser{routines, routine_arity, rules, nodes, affines};
     int root = -1;
     SecantResult r = parser.frame(program, nullptr, 0, 0, &root);
@@ -674,35 +712,36 @@ SecantResult encode_program(const SecantAstInstruction* program, const SecantAst
     rec.affine_off = (uint32_t)out.affines.size();
     rec.lit_off = (uint32_t)out.lits.size();
 
-    Emitter em(nodes, rules, out, (unsigned)affines.size());
+    Emitter em(mem, rules, out);
     em.slots_high = rules.reserved_slots;
-    const ValueClass root_class = em.classify(root);
+    const ValueClass root_class = nodes[root].cls;
     if (rules.split_parts) { /* rollout records (columns_are_slots) have no row-only class: only bank roots turn up */
-        std::vector<int> bank_roots, row_roots;
-        std::vector<uint8_t> seen(nodes.size(), 0);
-        em.collect(root, false, bank_roots, row_roots, seen);
+        em.collect(root, false, mem.bank_roots, mem.row_roots);
         /* row-only expressions a toggle reaches change with the permutation; what lies below them and
          * does not is worth a value of its own, computed once for all permutations of an item */
-        std::vector<int8_t> memo(nodes.size(), -1);
-        std::vector<int> shared_roots, toggled_roots;
-        for (int id : row_roots) {
-            if (!em.reaches_toggle(id, memo)) { shared_roots.push_back(id); continue; }
-            if (rules.hoist_toggled) toggled_roots.push_back(id);
-            em.collect_shared(id, shared_roots, memo);
+        std::vector<int>& chosen = mem.chosen;
+        for (int id : mem.row_roots) {
+            if (nodes[id].toggled) {
+                if (rules.hoist_toggled) chosen.push_back(id);
+                em.collect_shared(id, mem.shared_roots);
+            } else {
+                mem.shared_roots.push_back(id);
+            }
         }
         /* keep the costliest values when there are more than the kernel has room for */
-        std::vector<int> chosen(shared_roots);
-        chosen.insert(chosen.end(), toggled_roots.begin(), toggled_roots.end());
-        std::stable_sort(chosen.begin(), chosen.end(), [&](int a, int b) { return nodes[a].weight > nodes[b].weight; });
-        if (chosen.size() > rules.max_hoisted) chosen.resize(rules.max_hoisted);
+        chosen.insert(chosen.begin(), mem.shared_roots.begin(), mem.shared_roots.end());
+        if (chosen.size() > rules.max_hoisted) {
+            std::stable_sort(chosen.begin(), chosen.end(), [&](int a, int b) { return nodes[a].weight > nodes[b].weight; });
+            chosen.resize(rules.max_hoisted);
+        }
         /* operands before the expressions that use them: children were created first */
-        std::sort(bank_roots.begin(), bank_roots.end());
+        std::sort(mem.bank_roots.begin(), mem.bank_roots.end());
         std::sort(chosen.begin(), chosen.end());
-        for (int id : bank_roots) em.hoist(RUN_BANK, id);
+        for (int id : mem.bank_roots) em.hoist(RUN_BANK, id);
         for (int id : chosen)
-            if (!em.reaches_toggle(id, memo)) em.hoist(RUN_SHARED, id);
+            if (!nodes[id].toggled) em.hoist(RUN_SHARED, id);
         for (int id : chosen)
-            if (em.reaches_toggle(id, memo)) em.hoist(RUN_ROW, id);
+            if (nodes[id].toggled) em.hoist(RUN_ROW, id);
         if (em.error != SECANT_SUCCESS) return em.error;
     }
     em.begin_phase(RUN_MAIN, root); /* counts the RETURN as the root's first use */
@@ -712,11 +751,13 @@ SecantResult encode_program(const SecantAstInstruction* program, const SecantAst
 
     if (rules.fuse_store_load) { /* a toggle site keeps its own instruction: its alternatives are whole instructions */
         std::vector<SbInsn>& code = em.code[RUN_MAIN];
-        std::vector<uint8_t> is_site(code.size(), 0);
+        std::vector<uint8_t>& is_site = mem.is_site;
+        is_site.assign(code.size(), 0);
         for (const SbPatch& p : em.sites[RUN_MAIN]) is_site[p.insn] = 1;
-        std::vector<SbInsn> fused;
-        std::vector<uint32_t> moved(code.size(), 0);
-        fused.reserve(code.size());
+        std::vector<SbInsn>& fused = mem.fused;
+        std::vector<uint32_t>& moved = mem.moved;
+        fused.clear();
+        moved.assign(code.size(), 0);
         for (size_t i = 0; i < code.size(); ++i) {
             const unsigned cs = code[i].w0 & 0xffu;
             moved[i] = (uint32_t)fused.size();

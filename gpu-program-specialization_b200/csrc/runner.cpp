@@ -9,6 +9,11 @@
  * the device through pinned memory on a copy stream, and the resident evaluator kernel
  * of batch k runs while batch k+1 is being encoded and uploaded.  Nothing is loaded or
  * unloaded, so the "module" counters of the statistics count program batches.
+ *
+ * A batch is encoded in pieces of 16 to 128 programs which the workers and the calling thread take
+ * in order, so the first launch of a call waits for its batch divided by the threads, not for one
+ * thread that encodes all of it (2,048 programs of 32 tokens: 7.3 ms before the first launch with
+ * one thread per batch, see kPiece below for the sizes).
  */
 #include "evaluator.cuh"
 #include "internal.h"
@@ -66,15 +71,22 @@ void* current_context(bool* ok) {
 
 size_t align256(size_t v) { return (v + 255) / 256 * 256; }
 
-enum SlotState { SLOT_FREE = 0, SLOT_ENCODING, SLOT_READY, SLOT_IN_FLIGHT };
+/* Programs per piece: enough pieces that the last ones do not leave threads idle, none so small that
+ * taking it costs as much as encoding it (a program takes about 2 us, a hand-over under 1 us). */
+constexpr size_t kPieceMin = 16, kPieceMax = 128, kPiecesPerThread = 4;
+constexpr size_t kSlots = 3; /* batches encoded, uploaded or running at a time */
+
+struct Piece {
+    EncodedBatch enc;
+    SecantResult status = SECANT_SUCCESS;
+};
 
 struct Slot {
-    EncodedBatch enc;
-    SlotState state = SLOT_FREE;
-    size_t batch = 0;              /* batch index held */
-    size_t first_program = 0;
-    SecantResult status = SECANT_SUCCESS;
-    double encode_seconds = 0;
+    std::vector<Piece> pieces;
+    size_t used_pieces = 0;         /* of the batch held */
+    size_t done_pieces = 0;         /* encoded, guarded by the runner's mutex */
+    std::vector<uint64_t> order, order_tmp; /* launch order of the batch's programs, see order_programs() */
+    std::vector<SbProgram> headers;
     void* pinned = nullptr;
     size_t pinned_cap = 0;
     void* device = nullptr;
@@ -101,7 +113,7 @@ struct SecantCubinRunnerImpl {
     std::vector<void*> scratch;      /* per compute stream: partial sums of the launch in flight */
     std::vector<size_t> scratch_cap;
     cudaStream_t copy_stream = nullptr;
-    cudaEvent_t ev_cleared = nullptr, ev_start = nullptr, ev_stop = nullptr;
+    cudaEvent_t ev_join = nullptr, ev_start = nullptr, ev_stop = nullptr;
     std::vector<Slot> slots;
     std::vector<std::thread> workers;
     std::vector<double> worker_seconds;
@@ -112,7 +124,10 @@ struct SecantCubinRunnerImpl {
     const SecantAstProgramSet* job_programs = nullptr;
     const uint8_t* job_arity = nullptr;
     ProgramRules job_rules;
-    size_t job_batch_size = 0, job_num_batches = 0, job_next_batch = 0;
+    size_t job_batch_size = 0, job_piece_size = 0, job_pieces_per_batch = 0, job_num_pieces = 0, job_next_piece = 0;
+    size_t job_open_batches = 0;   /* batches whose slot is free to be encoded into */
+    size_t job_encoding = 0;       /* pieces being encoded */
+    double job_encode_seconds = 0; /* summed over the pieces */
     bool job_abort = false;
     /* handle state */
     bool active = false, failed = false, shutdown = false;
@@ -139,50 +154,58 @@ struct SecantB200PopulationImpl {
 
 namespace {
 
+/* Takes the next piece of the job in order, SIZE_MAX when there is none to be had now; the caller
+ * holds the mutex. */
+size_t take_piece(SecantCubinRunnerImpl* r) {
+    if (!r->job_active || r->job_abort || r->job_next_piece >= r->job_num_pieces) return SIZE_MAX;
+    if (r->job_next_piece / r->job_pieces_per_batch >= r->job_open_batches) return SIZE_MAX;
+    ++r->job_encoding;
+    return r->job_next_piece++;
+}
+
+/* Encodes piece `index` into its slot; `lock` (held) is released meanwhile. */
+void encode_piece(SecantCubinRunnerImpl* r, std::unique_lock<std::mutex>& lock, size_t index, double* seconds) {
+    const SecantAstProgramSet* programs = r->job_programs;
+    const uint8_t* arity = r->job_arity;
+    const ProgramRules rules = r->job_rules;
+    const size_t batch = index / r->job_pieces_per_batch, within = index % r->job_pieces_per_batch;
+    Slot& slot = r->slots[batch % r->slots.size()];
+    Piece& piece = slot.pieces[within];
+    const size_t batch_first = batch * r->job_batch_size;
+    const size_t batch_end = std::min(programs->asts.count, batch_first + r->job_batch_size);
+    const size_t first = batch_first + within * r->job_piece_size;
+    const size_t end = std::min(batch_end, first + r->job_piece_size);
+    lock.unlock();
+
+    const double begin = now_seconds();
+    SecantResult status = SECANT_SUCCESS;
+    try { /* an allocation failure inside the encoder must reach the caller as a result code */
+        piece.enc.clear();
+        for (size_t i = first; i < end && status == SECANT_SUCCESS; ++i) {
+            status = encode_program(programs->asts.items[i], programs->routines, arity, rules, piece.enc);
+            if (status == SECANT_SUCCESS) piece.enc.programs.back().index = (uint32_t)i;
+        }
+    } catch (...) {
+        status = SECANT_ERROR_ALLOCATION_FAILED;
+    }
+    if (SB_FAULT("encode")) status = SECANT_ERROR_BAD_PROGRAM;
+    const double spent = now_seconds() - begin;
+
+    lock.lock();
+    piece.status = status;
+    *seconds += spent;
+    r->job_encode_seconds += spent;
+    --r->job_encoding;
+    if (++slot.done_pieces == slot.used_pieces || r->job_abort) r->cv_ready.notify_all();
+}
+
 void worker_main(SecantCubinRunnerImpl* r, size_t worker_index) {
     std::unique_lock<std::mutex> lock(r->mutex);
     for (;;) {
-        Slot* slot = nullptr;
-        r->cv_work.wait(lock, [&] {
-            if (r->shutdown) return true;
-            if (!r->job_active || r->job_abort || r->job_next_batch >= r->job_num_batches) return false;
-            for (auto& s : r->slots)
-                if (s.state == SLOT_FREE) { slot = &s; return true; }
-            return false;
-        });
-        if (r->shutdown) return;
-        const size_t batch = r->job_next_batch++;
-        slot->state = SLOT_ENCODING;
-        slot->batch = batch;
-        const SecantAstProgramSet* programs = r->job_programs;
-        const uint8_t* arity = r->job_arity;
-        const ProgramRules rules = r->job_rules;
-        const size_t first = batch * r->job_batch_size;
-        const size_t count = std::min(r->job_batch_size, programs->asts.count - first);
-        lock.unlock();
-
-        const double begin = now_seconds();
-        SecantResult status = SECANT_SUCCESS;
-        try { /* an allocation failure inside the encoder must reach the caller as a result code */
-            slot->enc.clear();
-            slot->enc.programs.reserve(count);
-            for (size_t i = 0; i < count && status == SECANT_SUCCESS; ++i) {
-                status = encode_program(programs->asts.items[first + i], programs->routines, arity, rules, slot->enc);
-                if (status == SECANT_SUCCESS) slot->enc.programs.back().index = (uint32_t)(first + i);
-            }
-        } catch (...) {
-            status = SECANT_ERROR_ALLOCATION_FAILED;
-        }
-        if (SB_FAULT("encode")) status = SECANT_ERROR_BAD_PROGRAM;
-        const double spent = now_seconds() - begin;
-
-        lock.lock();
-        slot->first_program = first;
-        slot->status = status;
-        slot->encode_seconds = spent;
-        slot->state = SLOT_READY;
-        r->worker_seconds[worker_index] += spent;
-        r->cv_ready.notify_all();
+        size_t piece = SIZE_MAX;
+        r->cv_work.wait(lock, [&] { return r->shutdown || (piece = take_piece(r)) != SIZE_MAX; });
+        if (r->shutdown) return; /* no job is active then */
+        encode_piece(r, lock, piece, &r->worker_seconds[worker_index]);
     }
 }
 
@@ -211,17 +234,17 @@ SecantResult runner_init(SecantCubinRunnerImpl* r, const SecantCubinRunnerOption
     r->scratch.assign(r->streams.size(), nullptr);
     r->scratch_cap.assign(r->streams.size(), 0);
     SB_CUDA(cudaStreamCreateWithFlags(&r->copy_stream, cudaStreamNonBlocking), "cudaStreamCreate");
-    SB_CUDA(cudaEventCreateWithFlags(&r->ev_cleared, cudaEventDisableTiming), "cudaEventCreate");
+    SB_CUDA(cudaEventCreateWithFlags(&r->ev_join, cudaEventDisableTiming), "cudaEventCreate");
     SB_CUDA(cudaEventCreate(&r->ev_start), "cudaEventCreate");
     SB_CUDA(cudaEventCreate(&r->ev_stop), "cudaEventCreate");
-    r->slots.resize(options->num_workers + 2); /* same slot budget as the reference: workers + 2 */
+    r->slots.resize(kSlots);
     for (auto& s : r->slots) {
         SB_CUDA(cudaEventCreateWithFlags(&s.uploaded, cudaEventDisableTiming), "cudaEventCreate");
         s.done.resize(r->streams.size());
         s.used.assign(r->streams.size(), 0);
         for (auto& e : s.done) SB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
     }
-    r->worker_seconds.assign(options->num_workers, 0.0);
+    r->worker_seconds.assign(options->num_workers + 1, 0.0); /* the calling thread's last */
     try {
         for (size_t i = 0; i < options->num_workers; ++i) {
             if (SB_FAULT("thread")) throw std::bad_alloc();
@@ -265,7 +288,7 @@ SecantResult runner_teardown(SecantCubinRunnerImpl* r) {
         if (r->scratch[k] && ok(cudaFree(r->scratch[k]))) { r->scratch[k] = nullptr; r->scratch_cap[k] = 0; }
     for (auto& s : r->streams) if (s && ok(cudaStreamDestroy(s))) s = nullptr;
     if (r->copy_stream && ok(cudaStreamDestroy(r->copy_stream))) r->copy_stream = nullptr;
-    if (r->ev_cleared && ok(cudaEventDestroy(r->ev_cleared))) r->ev_cleared = nullptr;
+    if (r->ev_join && ok(cudaEventDestroy(r->ev_join))) r->ev_join = nullptr;
     if (r->ev_start && ok(cudaEventDestroy(r->ev_start))) r->ev_start = nullptr;
     if (r->ev_stop && ok(cudaEventDestroy(r->ev_stop))) r->ev_stop = nullptr;
     return result;
@@ -308,25 +331,53 @@ uint64_t schedule_cost(const SbProgram& p) {
     return main_part * ((p.flags & SB_PROG_BANK_INDEPENDENT) ? 1u : 16u) + prelude;
 }
 
-/* Copies an encoded batch into the slot's pinned buffer, grows the device buffer when
- * needed, and enqueues the upload.  Layout: programs | insns | patches | affines | lits. */
+/* Puts the batch's programs in launch order: light programs first, heavy ones after them; inside each
+ * group the costly ones first, so that every CTA, which takes a strided subset, has a queue from its
+ * costliest item to its cheapest and its warps finish a tile close together; ties keep the run's order.
+ * order[i] = key << 32 | position in `headers`, sorted on the 22-bit key (1 heavy bit above 21 bits of
+ * inverted cost) by two counting passes. */
+void order_programs(Slot& s) {
+    constexpr unsigned kBits = 11, kBins = 1u << kBits;
+    const size_t n = s.headers.size();
+    s.order.resize(n);
+    for (size_t i = 0; i < n; ++i) {
+        const SbProgram& p = s.headers[i];
+        const uint64_t key = (is_light(p) ? 0u : 1u << 21) | (0x1fffffu - (uint32_t)schedule_cost(p));
+        s.order[i] = key << 32 | i;
+    }
+    if (n <= 512) { /* keys with the position below them are unique, so any sort gives the same order */
+        std::sort(s.order.begin(), s.order.end());
+        return;
+    }
+    s.order_tmp.resize(n);
+    for (unsigned pass = 0; pass < 2; ++pass) {
+        uint32_t at[kBins] = {0};
+        const unsigned shift = 32 + pass * kBits;
+        for (size_t i = 0; i < n; ++i) ++at[(s.order[i] >> shift) & (kBins - 1)];
+        uint32_t sum = 0;
+        for (uint32_t& a : at) { const uint32_t c = a; a = sum; sum += c; }
+        for (size_t i = 0; i < n; ++i) s.order_tmp[at[(s.order[i] >> shift) & (kBins - 1)]++] = s.order[i];
+        s.order.swap(s.order_tmp);
+    }
+}
+
+/* Joins the batch's encoded pieces in the slot's pinned buffer (a program's offsets move by what lies
+ * before its piece), grows the device buffer when needed, and enqueues the upload.
+ * Layout: programs | insns | patches | affines | lits. */
 SecantResult upload_batch(SecantCubinRunnerImpl* r, Slot& s, std::vector<DeviceBatch>* views) {
-    EncodedBatch& e = s.enc;
-    /* light programs first, heavy ones after them; SbProgram::index keeps their place in the run */
-    std::stable_partition(e.programs.begin(), e.programs.end(), is_light);
-    /* inside each group, costly programs first: every CTA takes a strided subset, so its queue runs
-     * from its costliest item to its cheapest and its warps finish a tile close together */
-    const auto light_end = std::find_if(e.programs.begin(), e.programs.end(), [](const SbProgram& p) { return !is_light(p); });
-    const auto by_cost = [](const SbProgram& a, const SbProgram& b) { return schedule_cost(a) > schedule_cost(b); };
-    std::stable_sort(e.programs.begin(), light_end, by_cost);
-    std::stable_sort(light_end, e.programs.end(), by_cost);
-    const size_t num_light = (size_t)(light_end - e.programs.begin());
+    size_t n_programs = 0, n_insns = 0, n_patches = 0, n_affines = 0, n_lits = 0;
+    for (size_t q = 0; q < s.used_pieces; ++q) {
+        const EncodedBatch& e = s.pieces[q].enc;
+        n_programs += e.programs.size(); n_insns += e.insns.size(); n_patches += e.patches.size();
+        n_affines += e.affines.size(); n_lits += e.lits.size();
+    }
+    if (n_insns > 0xffffffffull || n_patches > 0xffffffffull || n_affines > 0xffffffffull || n_lits > 0xffffffffull) return SECANT_ERROR_OVERFLOW;
     const size_t o_prog = 0;
-    const size_t o_insn = align256(o_prog + e.programs.size() * sizeof(SbProgram));
-    const size_t o_patch = align256(o_insn + e.insns.size() * sizeof(SbInsn));
-    const size_t o_aff = align256(o_patch + e.patches.size() * sizeof(SbPatch));
-    const size_t o_lit = align256(o_aff + e.affines.size() * sizeof(SbAffine));
-    const size_t total = align256(o_lit + e.lits.size() * sizeof(float) + 16);
+    const size_t o_insn = align256(o_prog + n_programs * sizeof(SbProgram));
+    const size_t o_patch = align256(o_insn + n_insns * sizeof(SbInsn));
+    const size_t o_aff = align256(o_patch + n_patches * sizeof(SbPatch));
+    const size_t o_lit = align256(o_aff + n_affines * sizeof(SbAffine));
+    const size_t total = align256(o_lit + n_lits * sizeof(float) + 16);
     if (s.pinned_cap < total) {
         if (s.pinned) SB_CUDA(cudaFreeHost(s.pinned), "cudaFreeHost");
         s.pinned = nullptr; s.pinned_cap = 0;
@@ -340,16 +391,33 @@ SecantResult upload_batch(SecantCubinRunnerImpl* r, Slot& s, std::vector<DeviceB
         s.device_cap = total + total / 2;
     }
     char* h = static_cast<char*>(s.pinned);
-    std::memcpy(h + o_prog, e.programs.data(), e.programs.size() * sizeof(SbProgram));
-    std::memcpy(h + o_insn, e.insns.data(), e.insns.size() * sizeof(SbInsn));
-    if (!e.patches.empty()) std::memcpy(h + o_patch, e.patches.data(), e.patches.size() * sizeof(SbPatch));
-    if (!e.affines.empty()) std::memcpy(h + o_aff, e.affines.data(), e.affines.size() * sizeof(SbAffine));
-    if (!e.lits.empty()) std::memcpy(h + o_lit, e.lits.data(), e.lits.size() * sizeof(float));
+    s.headers.clear();
+    size_t at_insn = 0, at_patch = 0, at_affine = 0, at_lit = 0;
+    for (size_t q = 0; q < s.used_pieces; ++q) {
+        const EncodedBatch& e = s.pieces[q].enc;
+        for (SbProgram p : e.programs) {
+            p.insn_off += (uint32_t)at_insn; p.patch_off += (uint32_t)at_patch;
+            p.affine_off += (uint32_t)at_affine; p.lit_off += (uint32_t)at_lit;
+            s.headers.push_back(p);
+        }
+        if (!e.insns.empty()) std::memcpy(h + o_insn + at_insn * sizeof(SbInsn), e.insns.data(), e.insns.size() * sizeof(SbInsn));
+        if (!e.patches.empty()) std::memcpy(h + o_patch + at_patch * sizeof(SbPatch), e.patches.data(), e.patches.size() * sizeof(SbPatch));
+        if (!e.affines.empty()) std::memcpy(h + o_aff + at_affine * sizeof(SbAffine), e.affines.data(), e.affines.size() * sizeof(SbAffine));
+        if (!e.lits.empty()) std::memcpy(h + o_lit + at_lit * sizeof(float), e.lits.data(), e.lits.size() * sizeof(float));
+        at_insn += e.insns.size(); at_patch += e.patches.size(); at_affine += e.affines.size(); at_lit += e.lits.size();
+    }
+    order_programs(s);
+    SbProgram* const out = reinterpret_cast<SbProgram*>(h + o_prog);
+    size_t num_light = 0;
+    for (size_t i = 0; i < n_programs; ++i) {
+        out[i] = s.headers[(uint32_t)s.order[i]];
+        num_light += (s.order[i] >> 53) == 0;
+    }
     SB_CUDA(cudaMemcpyAsync(s.device, s.pinned, total, cudaMemcpyHostToDevice, r->copy_stream), "program upload");
     SB_CUDA(cudaEventRecord(s.uploaded, r->copy_stream), "cudaEventRecord");
     const char* d = static_cast<const char*>(s.device);
     views->clear();
-    const size_t bounds[3] = {0, num_light, e.programs.size()};
+    const size_t bounds[3] = {0, num_light, n_programs};
     for (int k = 0; k < 2; ++k) {
         if (bounds[k] == bounds[k + 1]) continue;
         DeviceBatch db;
@@ -362,7 +430,7 @@ SecantResult upload_batch(SecantCubinRunnerImpl* r, Slot& s, std::vector<DeviceB
         db.num_programs = (uint32_t)(bounds[k + 1] - bounds[k]);
         db.max_insn = 1;
         for (size_t i = bounds[k]; i < bounds[k + 1]; ++i) {
-            const SbProgram& p = e.programs[i];
+            const SbProgram& p = out[i];
             db.max_insn = std::max<uint32_t>(db.max_insn, p.n_insn);
             db.max_extra = std::max<uint32_t>(db.max_extra, (uint32_t)p.n_affine + p.n_lits);
             db.max_slots = std::max<uint32_t>(db.max_slots, p.n_slots);
@@ -545,6 +613,37 @@ SecantResult retire_slot(SecantCubinRunnerImpl* r, Slot& s, bool* unknown) {
     return result;
 }
 
+/* Zeroes the output vectors of the programs from `first` on.  The evaluator writes every active bin of
+ * a program it was launched for, so only a call that fails half way has something to clear: the
+ * reference clears every vector before it starts (projects/secant/s_cubin_runner.c:243-286). */
+SecantResult clear_outputs(SecantCubinRunnerImpl* r, const std::vector<UnpackedRun>& runs, size_t first) {
+    for (const auto& run : runs) {
+        const size_t vectors = run.output_count / run.programs.asts.count; /* per program (targets) */
+        const size_t at = first * vectors;
+        if (at >= run.output_count) continue;
+        SB_CUDA(cudaMemset2DAsync(reinterpret_cast<float*>(run.output.address) + at * run.output.leading_dimension,
+                                  run.output.leading_dimension * sizeof(float), 0, run.output_width * sizeof(float),
+                                  run.output_count - at, r->streams[0]),
+                "clearing output");
+    }
+    return SECANT_SUCCESS;
+}
+
+/* Joins the compute streams that were used into stream 0, waits for it and reads the device time. */
+cudaError_t finish_streams(SecantCubinRunnerImpl* r, size_t streams_used, double* seconds) {
+    cudaError_t ce = cudaSuccess;
+    for (size_t k = 1; k < std::min(streams_used, r->streams.size()) && ce == cudaSuccess; ++k) {
+        ce = cudaEventRecord(r->ev_join, r->streams[k]);
+        if (ce == cudaSuccess) ce = cudaStreamWaitEvent(r->streams[0], r->ev_join, 0);
+    }
+    if (ce == cudaSuccess) ce = cudaEventRecord(r->ev_stop, r->streams[0]);
+    if (ce == cudaSuccess) ce = cudaEventSynchronize(r->ev_stop);
+    float ms = 0;
+    if (ce == cudaSuccess) ce = cudaEventElapsedTime(&ms, r->ev_start, r->ev_stop);
+    *seconds = ms * 1e-3;
+    return ce;
+}
+
 SecantResult execute(SecantCubinRunnerImpl* r, const std::vector<UnpackedRun>& runs, const ProgramRules& rules,
                      SecantRunnerStats* stats) {
     const SecantCubinPlan& plan = *r->plan;
@@ -564,30 +663,47 @@ SecantResult execute(SecantCubinRunnerImpl* r, const std::vector<UnpackedRun>& r
     const size_t num_batches = (P + batch_size - 1) / batch_size;
     const bool accumulate = plan.shape != SECANT_KERNEL_SHAPE_STATIC_MATERIALIZE_F32;
 
-    /* clear the active output bins only; padding between vectors is preserved */
+    const size_t threads = r->workers.size() + 1;
+    const size_t piece_size = std::min(kPieceMax, std::max(kPieceMin, batch_size / (threads * kPiecesPerThread)));
+    const size_t pieces_per_batch = (batch_size + piece_size - 1) / piece_size;
+    auto pieces_of = [&](size_t batch) { return (std::min(batch_size, P - batch * batch_size) + piece_size - 1) / piece_size; };
+    auto open_slot = [&](Slot& s, size_t batch) { /* under the mutex; grows the piece list only while no job runs on it */
+        s.used_pieces = pieces_of(batch);
+        s.done_pieces = 0;
+    };
+
     SB_CUDA(cudaEventRecord(r->ev_start, r->streams[0]), "cudaEventRecord");
-    if (accumulate)
-        for (const auto& run : runs)
-            SB_CUDA(cudaMemset2DAsync(reinterpret_cast<void*>(run.output.address), run.output.leading_dimension * sizeof(float), 0,
-                                      run.output_width * sizeof(float), run.output_count, r->streams[0]),
-                    "clearing output");
-    SB_CUDA(cudaEventRecord(r->ev_cleared, r->streams[0]), "cudaEventRecord");
-    for (size_t k = 1; k < r->streams.size(); ++k) SB_CUDA(cudaStreamWaitEvent(r->streams[k], r->ev_cleared, 0), "cudaStreamWaitEvent");
+    if (gram) { /* its statistics are added to range by range: the active entries start from zero */
+        result = clear_outputs(r, runs, 0);
+        if (result != SECANT_SUCCESS) return result;
+        SB_CUDA(cudaEventRecord(r->ev_join, r->streams[0]), "cudaEventRecord");
+        for (size_t k = 1; k < r->streams.size(); ++k) SB_CUDA(cudaStreamWaitEvent(r->streams[k], r->ev_join, 0), "cudaStreamWaitEvent");
+    }
 
     {
         std::lock_guard<std::mutex> lock(r->mutex);
-        for (auto& s : r->slots) { s.state = SLOT_FREE; std::fill(s.used.begin(), s.used.end(), 0); }
+        for (size_t k = 0; k < r->slots.size(); ++k) {
+            Slot& s = r->slots[k];
+            std::fill(s.used.begin(), s.used.end(), 0);
+            if (k >= num_batches) continue;
+            if (s.pieces.size() < pieces_per_batch) s.pieces.resize(pieces_per_batch);
+            open_slot(s, k);
+        }
         std::fill(r->worker_seconds.begin(), r->worker_seconds.end(), 0.0);
         r->job_programs = &programs;
         r->job_arity = arity;
         r->job_rules = rules;
         r->job_batch_size = batch_size;
-        r->job_num_batches = num_batches;
-        r->job_next_batch = 0;
+        r->job_piece_size = piece_size;
+        r->job_pieces_per_batch = pieces_per_batch;
+        r->job_num_pieces = (num_batches - 1) * pieces_per_batch + pieces_of(num_batches - 1);
+        r->job_next_piece = 0;
+        r->job_open_batches = std::min(num_batches, r->slots.size());
+        r->job_encode_seconds = 0;
         r->job_abort = false;
         r->job_active = true;
     }
-    r->cv_work.notify_all();
+    if (P > piece_size) r->cv_work.notify_all(); /* a single piece is the calling thread's own */
     /* Whatever way this function is left (a result code or an exception from a container), the
      * workers must be off this job first: they read `arity`, `programs` and `rules`, which live in
      * the caller's frames. */
@@ -595,105 +711,82 @@ SecantResult execute(SecantCubinRunnerImpl* r, const std::vector<UnpackedRun>& r
         SecantCubinRunnerImpl* r;
         ~JobGuard() {
             std::unique_lock<std::mutex> lock(r->mutex);
+            end(lock);
+        }
+        void end(std::unique_lock<std::mutex>& lock) {
             r->job_abort = true;
-            r->cv_ready.wait(lock, [&] {
-                for (auto& s : r->slots)
-                    if (s.state == SLOT_ENCODING) return false;
-                return true;
-            });
+            r->cv_ready.wait(lock, [&] { return r->job_encoding == 0; });
             r->job_active = false;
         }
     } job_guard{r};
 
     bool unknown = false;
-    size_t launched_batches = 0, stream_cursor = 0;
+    size_t launched_batches = 0, retired_batches = 0, stream_cursor = 0;
     double upload_seconds = 0, wait_seconds = 0, encode_sum = 0;
-    std::vector<Slot*> in_flight;
+    std::vector<DeviceBatch> views;
+    const auto retire = [&]() { /* the oldest batch in flight: wait for it and open its slot for the batch that comes next to it */
+        Slot& old = r->slots[retired_batches % r->slots.size()];
+        const double t_wait = now_seconds();
+        const SecantResult w = retire_slot(r, old, &unknown);
+        wait_seconds += now_seconds() - t_wait;
+        if (result == SECANT_SUCCESS) result = w;
+        const size_t next = retired_batches++ + r->slots.size();
+        if (next >= num_batches) return;
+        {
+            std::lock_guard<std::mutex> lock(r->mutex);
+            open_slot(old, next);
+            r->job_open_batches = next + 1;
+        }
+        r->cv_work.notify_all();
+    };
     for (size_t b = 0; b < num_batches && result == SECANT_SUCCESS; ++b) {
-        Slot* slot = nullptr;
+        Slot& slot = r->slots[b % r->slots.size()];
         {
             std::unique_lock<std::mutex> lock(r->mutex);
-            r->cv_ready.wait(lock, [&] {
-                for (auto& s : r->slots)
-                    if (s.state == SLOT_READY && s.batch == b) { slot = &s; return true; }
-                return false;
-            });
-            slot->state = SLOT_IN_FLIGHT;
+            while (slot.done_pieces < slot.used_pieces) {
+                const size_t piece = take_piece(r); /* nothing to launch yet: help */
+                if (piece != SIZE_MAX) encode_piece(r, lock, piece, &r->worker_seconds.back());
+                else r->cv_ready.wait(lock);
+            }
+            for (size_t q = 0; q < slot.used_pieces && result == SECANT_SUCCESS; ++q) result = slot.pieces[q].status; /* the first in program order */
         }
-        encode_sum += slot->encode_seconds;
-        result = slot->status;
         if (result != SECANT_SUCCESS) break;
-        std::vector<DeviceBatch> views;
         const double t_up = now_seconds();
-        result = upload_batch(r, *slot, &views);
+        result = upload_batch(r, slot, &views);
         upload_seconds += now_seconds() - t_up;
         if (result != SECANT_SUCCESS) break;
+        std::vector<cudaEvent_t>* done = num_batches > 2 ? &slot.done : nullptr; /* only a batch whose slot is used again is waited for by itself */
         if (gram) {
             const size_t first = b * batch_size;
-            result = launch_gram_batch(r, views, runs, first, std::min(batch_size, P - first), &stream_cursor, slot->uploaded, &slot->done,
-                                       &slot->used);
+            result = launch_gram_batch(r, views, runs, first, std::min(batch_size, P - first), &stream_cursor, slot.uploaded, done, &slot.used);
         } else {
             for (const DeviceBatch& db : views) {
-                result = launch_batch(r, db, runs, &stream_cursor, slot->uploaded, &slot->done, &slot->used);
+                result = launch_batch(r, db, runs, &stream_cursor, slot.uploaded, done, &slot.used);
                 if (result != SECANT_SUCCESS) break;
             }
         }
-        in_flight.push_back(slot);
+        if (result != SECANT_SUCCESS) break;
         ++launched_batches;
-        /* recycle the oldest batch once two are queued behind it, so workers always find a slot */
-        while (in_flight.size() > 2 || (result != SECANT_SUCCESS && !in_flight.empty())) {
-            Slot* old = in_flight.front();
-            in_flight.erase(in_flight.begin());
-            const double t_wait = now_seconds();
-            const SecantResult w = retire_slot(r, *old, &unknown);
-            wait_seconds += now_seconds() - t_wait;
-            if (result == SECANT_SUCCESS) result = w;
-            {
-                std::lock_guard<std::mutex> lock(r->mutex);
-                old->state = SLOT_FREE;
-            }
-            r->cv_work.notify_all();
-        }
+        /* recycle the oldest batch once two are queued behind it, so there is always a slot to encode into */
+        while (launched_batches - retired_batches > 2 && result == SECANT_SUCCESS) retire();
     }
     /* stop the workers' job, then drain what is still running */
     {
         std::unique_lock<std::mutex> lock(r->mutex);
-        r->job_abort = true;
-        r->cv_ready.wait(lock, [&] {
-            for (auto& s : r->slots)
-                if (s.state == SLOT_ENCODING) return false;
-            return true;
-        });
-        r->job_active = false;
+        job_guard.end(lock);
+        encode_sum = r->job_encode_seconds;
     }
     const double t_wait = now_seconds();
-    for (Slot* s : in_flight) {
-        const SecantResult w = retire_slot(r, *s, &unknown);
-        if (result == SECANT_SUCCESS) result = w;
+    if (result != SECANT_SUCCESS && !unknown) { /* nothing of the call stays in flight, and what was not scored reads zero */
+        if (!drain_streams(r)) unknown = true;
+        else if (accumulate) (void)clear_outputs(r, runs, launched_batches * batch_size);
     }
-    /* join all compute streams into stream 0 for the device-time interval */
     if (!unknown) {
-        cudaError_t ce = cudaSuccess;
-        for (size_t k = 1; k < r->streams.size() && ce == cudaSuccess; ++k) {
-            ce = cudaEventRecord(r->ev_cleared, r->streams[k]);
-            if (ce == cudaSuccess) ce = cudaStreamWaitEvent(r->streams[0], r->ev_cleared, 0);
-        }
-        if (ce == cudaSuccess) ce = cudaEventRecord(r->ev_stop, r->streams[0]);
-        if (ce == cudaSuccess) ce = cudaEventSynchronize(r->ev_stop);
-        if (ce == cudaSuccess) ce = cudaStreamSynchronize(r->copy_stream);
-        float ms = 0;
-        if (ce == cudaSuccess) ce = cudaEventElapsedTime(&ms, r->ev_start, r->ev_stop);
+        const cudaError_t ce = finish_streams(r, result == SECANT_SUCCESS ? stream_cursor : r->streams.size(), &stats->runtime_seconds);
         if (ce != cudaSuccess) { const SecantResult w = cuda_fail(r, ce, "completion"); unknown = true; if (result == SECANT_SUCCESS) result = w; }
-        stats->runtime_seconds = ms * 1e-3;
     }
     wait_seconds += now_seconds() - t_wait;
-    {
-        std::lock_guard<std::mutex> lock(r->mutex);
-        for (auto& s : r->slots) s.state = SLOT_FREE;
-        double critical = 0;
-        for (double w : r->worker_seconds) critical = w > critical ? w : critical;
-        stats->compile_critical_seconds = critical;
-    }
+    stats->compile_critical_seconds = *std::max_element(r->worker_seconds.begin(), r->worker_seconds.end());
     /* module counts in the reference's unit, a recipe-capacity worth of programs (callers such as
      * projects/secant/tests/toggle_cuda_test.c:245 check them); batches here are much larger */
     {
@@ -855,15 +948,7 @@ SecantResult copy_programs(const SecantAstProgramList& list, std::vector<uint8_t
 SecantResult execute_resident(SecantCubinRunnerImpl* r, SecantB200PopulationImpl* pop, const std::vector<UnpackedRun>& runs,
                               SecantRunnerStats* stats) {
     const SecantCubinPlan& plan = *r->plan;
-    const bool accumulate = plan.shape != SECANT_KERNEL_SHAPE_STATIC_MATERIALIZE_F32;
     SB_CUDA(cudaEventRecord(r->ev_start, r->streams[0]), "cudaEventRecord");
-    if (accumulate)
-        for (const auto& run : runs)
-            SB_CUDA(cudaMemset2DAsync(reinterpret_cast<void*>(run.output.address), run.output.leading_dimension * sizeof(float), 0,
-                                      run.output_width * sizeof(float), run.output_count, r->streams[0]),
-                    "clearing output");
-    SB_CUDA(cudaEventRecord(r->ev_cleared, r->streams[0]), "cudaEventRecord");
-    for (size_t k = 1; k < r->streams.size(); ++k) SB_CUDA(cudaStreamWaitEvent(r->streams[k], r->ev_cleared, 0), "cudaStreamWaitEvent");
     size_t cursor = 0;
     SecantResult result = SECANT_SUCCESS;
     for (auto& b : pop->batches) {
@@ -873,18 +958,10 @@ SecantResult execute_resident(SecantCubinRunnerImpl* r, SecantB200PopulationImpl
         }
         if (result != SECANT_SUCCESS) break;
     }
+    if (result != SECANT_SUCCESS && plan.shape != SECANT_KERNEL_SHAPE_STATIC_MATERIALIZE_F32 && drain_streams(r)) (void)clear_outputs(r, runs, 0);
     const double t_wait = now_seconds();
-    cudaError_t ce = cudaSuccess;
-    for (size_t k = 1; k < r->streams.size() && ce == cudaSuccess; ++k) {
-        ce = cudaEventRecord(r->ev_cleared, r->streams[k]);
-        if (ce == cudaSuccess) ce = cudaStreamWaitEvent(r->streams[0], r->ev_cleared, 0);
-    }
-    if (ce == cudaSuccess) ce = cudaEventRecord(r->ev_stop, r->streams[0]);
-    if (ce == cudaSuccess) ce = cudaEventSynchronize(r->ev_stop);
-    float ms = 0;
-    if (ce == cudaSuccess) ce = cudaEventElapsedTime(&ms, r->ev_start, r->ev_stop);
+    const cudaError_t ce = finish_streams(r, result == SECANT_SUCCESS ? cursor : r->streams.size(), &stats->runtime_seconds);
     stats->completion_wait_seconds = now_seconds() - t_wait;
-    stats->runtime_seconds = ms * 1e-3;
     {
         const size_t capacity = std::max<size_t>(1, r->plan->num_kernels * r->plan->asts_per_kernel);
         stats->num_modules = stats->modules_loaded = (pop->set.asts.count + capacity - 1) / capacity;
@@ -950,15 +1027,18 @@ SecantResult secant_b200_population_create(SecantCubinRunner r, const SecantAstP
         if (batch_size < 4096) batch_size = 4096;
         if (batch_size > P) batch_size = P;
         Slot staging; /* reuses the upload helper; its buffers are handed to the population */
+        staging.pieces.resize(1);
+        staging.used_pieces = 1;
         for (size_t first = 0; first < P && result == SECANT_SUCCESS; first += batch_size) {
             const size_t count = std::min(batch_size, P - first);
-            staging.enc.clear();
+            EncodedBatch& enc = staging.pieces[0].enc;
+            enc.clear();
             for (size_t i = 0; i < count && result == SECANT_SUCCESS; ++i) {
-                result = encode_program(programs->asts.items[first + i], programs->routines, arity, rules, staging.enc);
-                if (result == SECANT_SUCCESS) staging.enc.programs.back().index = (uint32_t)(first + i);
+                result = encode_program(programs->asts.items[first + i], programs->routines, arity, rules, enc);
+                if (result == SECANT_SUCCESS) enc.programs.back().index = (uint32_t)(first + i);
             }
             if (result != SECANT_SUCCESS) break;
-            for (const auto& p : staging.enc.programs) pop->total_ops += p.n_ops;
+            for (const auto& p : enc.programs) pop->total_ops += p.n_ops;
             if (!staging.uploaded && cudaEventCreateWithFlags(&staging.uploaded, cudaEventDisableTiming) != cudaSuccess) {
                 result = SECANT_ERROR_DRIVER_FAILED;
                 break;
