@@ -11,9 +11,15 @@
 #include <stddef.h>
 #include <stdint.h>
 
+struct CUmemPoolHandle_st;
+
 namespace sb {
 /* adds to the process-wide count reported by secant_b200_kernel_launch_count() */
 void note_kernel_launches(unsigned n);
+
+/* The library's memory pool of a device, null when there is none to be had (rk4.cpp); what it keeps
+ * goes back to the driver with secant_b200_release_cached_memory(). */
+::CUmemPoolHandle_st* record_pool(int device); /* a cudaMemPool_t */
 
 /* Grouped top-k of a [system][configuration] score grid (reduce.cu); scratch may be zero. */
 SecantResult grouped_topk(uintptr_t scores, size_t num_systems, size_t num_banks, uint32_t toggle_bits, uint32_t grouping, uint32_t k,

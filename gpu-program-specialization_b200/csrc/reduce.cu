@@ -70,9 +70,10 @@ best_config_kernel(const float* __restrict__ grid, unsigned long long configs, u
 /* ---- top-k --------------------------------------------------------------------------
  * Every score becomes a 64-bit key: high word = the float's bit pattern (monotonic for
  * non-negative floats; invalid scores map to 0xffffffff), low word = the index.  Smaller
- * key = better rank, and keys are unique.  A CTA sorts a tile of 4096 keys in shared memory
- * (bitonic network) and keeps the k smallest; rounds shrink the candidate list by
- * 4096 / k until one tile is left. */
+ * key = better rank, and keys are unique.  A CTA sorts a tile of up to 4096 keys in shared memory
+ * (bitonic network, the smallest power of two that holds the tile) and keeps the k smallest; rounds
+ * shrink the candidate list by 4096 / k until one tile is left, and the kernel that sorts the last
+ * tile writes the result: a population of up to 4096 programs is ranked by one launch and no scratch. */
 constexpr int kTile = 4096;
 constexpr int kSortThreads = 512;
 
@@ -82,11 +83,11 @@ __device__ __forceinline__ unsigned long long score_key(float v, unsigned long l
     return ((unsigned long long)hi << 32) | (index & 0xffffffffull);
 }
 
-__device__ void sort_tile(unsigned long long* keys) {
-    for (int size = 2; size <= kTile; size <<= 1)
+__device__ void sort_tile(unsigned long long* keys, int n) {
+    for (int size = 2; size <= n; size <<= 1)
         for (int stride = size >> 1; stride > 0; stride >>= 1) {
             __syncthreads();
-            for (int t = threadIdx.x; t < kTile / 2; t += kSortThreads) {
+            for (int t = threadIdx.x; t < n / 2; t += kSortThreads) {
                 const int lo = 2 * t - (t & (stride - 1));
                 const int hi = lo + stride;
                 const bool ascending = (lo & size) == 0;
@@ -97,38 +98,29 @@ __device__ void sort_tile(unsigned long long* keys) {
     __syncthreads();
 }
 
-/* first round: tiles of raw scores -> k best keys per tile */
+/* One round: tiles of candidate keys (`in`, or the raw scores in the first round) -> the k best keys
+ * of every tile, or, when `indices` is given (one tile left), the ranking itself. */
 __global__ void __launch_bounds__(kSortThreads)
-topk_first_kernel(const float* __restrict__ scores, unsigned long long count, unsigned int k, unsigned long long* out) {
+topk_round_kernel(const unsigned long long* __restrict__ in, const float* __restrict__ scores, unsigned long long count, unsigned int k,
+                  int sort_size, unsigned long long* out, unsigned long long* indices, float* values) {
     __shared__ unsigned long long keys[kTile];
     const unsigned long long base = (unsigned long long)blockIdx.x * kTile;
-    for (int t = threadIdx.x; t < kTile; t += kSortThreads) {
+    for (int t = threadIdx.x; t < sort_size; t += kSortThreads) {
         const unsigned long long i = base + t;
-        keys[t] = i < count ? score_key(scores[i], i) : ~0ull;
+        keys[t] = i >= count ? ~0ull : in ? in[i] : score_key(scores[i], i);
     }
-    sort_tile(keys);
-    for (unsigned int t = threadIdx.x; t < k; t += kSortThreads) out[(size_t)blockIdx.x * k + t] = keys[t];
-}
-
-/* later rounds: tiles of candidate keys -> k best keys per tile */
-__global__ void __launch_bounds__(kSortThreads)
-topk_merge_kernel(const unsigned long long* __restrict__ in, unsigned long long count, unsigned int k, unsigned long long* out) {
-    __shared__ unsigned long long keys[kTile];
-    const unsigned long long base = (unsigned long long)blockIdx.x * kTile;
-    for (int t = threadIdx.x; t < kTile; t += kSortThreads) keys[t] = base + t < count ? in[base + t] : ~0ull;
-    sort_tile(keys);
-    for (unsigned int t = threadIdx.x; t < k; t += kSortThreads) out[(size_t)blockIdx.x * k + t] = keys[t];
-}
-
-__global__ void topk_emit_kernel(const unsigned long long* __restrict__ keys, const float* __restrict__ scores,
-                                 unsigned long long count, unsigned int k, unsigned long long* indices, float* values) {
-    const unsigned int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= k) return;
-    const unsigned long long key = keys[t];
-    const bool present = t < count && key != ~0ull;
-    const unsigned long long index = key & 0xffffffffull;
-    indices[t] = present ? index : ~0ull;
-    if (values) values[t] = present ? scores[index] : CUDART_NAN_F;
+    sort_tile(keys, sort_size);
+    if (!indices) {
+        for (unsigned int t = threadIdx.x; t < k; t += kSortThreads) out[(size_t)blockIdx.x * k + t] = keys[t];
+        return;
+    }
+    for (unsigned int t = threadIdx.x; t < k; t += kSortThreads) {
+        const unsigned long long key = t < sort_size ? keys[t] : ~0ull;
+        const bool present = key != ~0ull; /* fewer than k scores: the rest of the ranks stay empty */
+        const unsigned long long index = key & 0xffffffffull;
+        indices[t] = present ? index : ~0ull;
+        if (values) values[t] = present ? scores[index] : CUDART_NAN_F;
+    }
 }
 
 size_t tiles_of(unsigned long long count) { return (size_t)((count + kTile - 1) / kTile); }
@@ -279,20 +271,20 @@ grouped_merge_kernel(const float* __restrict__ scores, unsigned long long config
  * 64-bit words.  Shared by the allocating and the caller-provided-scratch entry points. */
 static cudaError_t topk_rounds(const float* scores, unsigned long long count, unsigned int k, unsigned long long* scratch,
                                unsigned long long* indices, float* values, cudaStream_t stream) {
-    size_t tiles = tiles_of(count);
-    unsigned long long* cur = scratch;
-    unsigned long long* nxt = scratch + tiles * k;
-    topk_first_kernel<<<(unsigned)tiles, kSortThreads, 0, stream>>>(scores, count, k, cur);
-    unsigned launched = 2; /* first + emit */
-    unsigned long long have = (unsigned long long)tiles * k;
-    while (tiles > 1) {
-        tiles = tiles_of(have);
-        topk_merge_kernel<<<(unsigned)tiles, kSortThreads, 0, stream>>>(cur, have, k, nxt);
+    unsigned long long* out = scratch;
+    unsigned long long* other = scratch + tiles_of(count) * k;
+    const unsigned long long* in = nullptr;
+    unsigned launched = 0;
+    for (unsigned long long have = count;; in = out, out = other, other = const_cast<unsigned long long*>(in)) {
+        const size_t tiles = tiles_of(have);
+        const bool last = tiles == 1;
+        int sort_size = kTile;
+        while (last && sort_size / 2 >= 32 && (unsigned long long)sort_size / 2 >= have) sort_size /= 2;
+        topk_round_kernel<<<(unsigned)tiles, kSortThreads, 0, stream>>>(in, scores, have, k, sort_size, out, last ? indices : nullptr, values);
         ++launched;
+        if (last) break;
         have = (unsigned long long)tiles * k;
-        unsigned long long* t = cur; cur = nxt; nxt = t;
     }
-    topk_emit_kernel<<<(k + 255) / 256, 256, 0, stream>>>(cur, scores, count, k, indices, values);
     sb::note_kernel_launches(launched);
     return cudaGetLastError();
 }
@@ -401,13 +393,19 @@ SecantResult secant_b200_topk_static(uintptr_t scores, size_t count, size_t k, u
 SecantResult secant_b200_topk(uintptr_t scores, size_t count, size_t k, uintptr_t indices_out, uintptr_t scores_out, void* stream) {
     if (!scores || !indices_out || !count || !k || k > 2048 || count > 0xffffffffull || scores % 4 || indices_out % 8 || scores_out % 4)
         return SECANT_ERROR_INVALID_VALUE;
-    unsigned long long* scratch = nullptr;
-    const size_t words = secant_b200_topk_scratch_elements(count, k);
-    if (cudaMallocAsync(&scratch, words * sizeof(unsigned long long), (cudaStream_t)stream) != cudaSuccess) return SECANT_ERROR_ALLOCATION_FAILED;
+    unsigned long long* scratch = nullptr; /* one tile needs none */
+    if (count > kTile) { /* the library's own pool keeps the memory for the next call; the default pool gives it back at every synchronisation */
+        const size_t bytes = secant_b200_topk_scratch_elements(count, k) * sizeof(unsigned long long);
+        int device = 0;
+        const cudaMemPool_t pool = cudaGetDevice(&device) == cudaSuccess ? sb::record_pool(device) : nullptr;
+        const cudaError_t m = pool ? cudaMallocFromPoolAsync(reinterpret_cast<void**>(&scratch), bytes, pool, (cudaStream_t)stream)
+                                   : cudaMallocAsync(reinterpret_cast<void**>(&scratch), bytes, (cudaStream_t)stream);
+        if (m != cudaSuccess) return SECANT_ERROR_ALLOCATION_FAILED;
+    }
     cudaError_t e = topk_rounds(reinterpret_cast<const float*>(scores), count, (unsigned)k, scratch,
                                 reinterpret_cast<unsigned long long*>(indices_out), reinterpret_cast<float*>(scores_out),
                                 (cudaStream_t)stream);
-    const cudaError_t f = cudaFreeAsync(scratch, (cudaStream_t)stream);
+    const cudaError_t f = scratch ? cudaFreeAsync(scratch, (cudaStream_t)stream) : cudaSuccess;
     if (e == cudaSuccess) e = f;
     return e == cudaSuccess ? SECANT_SUCCESS : SECANT_ERROR_DRIVER_FAILED;
 }

@@ -30,12 +30,15 @@ using namespace sb;
 
 namespace {
 
-/* Record buffers live for one call; the pool keeps their memory between calls. */
+/* Buffers that live for one call (records here, the keys of the top-k reduction); the pool keeps their
+ * memory between calls. */
 constexpr int kMaxPoolDevices = 64;
 std::mutex g_pool_mutex;
 cudaMemPool_t g_pools[kMaxPoolDevices] = {};
 
-cudaMemPool_t record_pool(int device) {
+}  // namespace
+
+cudaMemPool_t sb::record_pool(int device) {
     if (device < 0 || device >= kMaxPoolDevices) return nullptr;
     std::lock_guard<std::mutex> lock(g_pool_mutex);
     if (!g_pools[device]) {
@@ -57,8 +60,6 @@ cudaMemPool_t record_pool(int device) {
     }
     return g_pools[device];
 }
-
-}  // namespace
 
 extern "C" SecantResult secant_b200_release_cached_memory(void) {
     std::lock_guard<std::mutex> lock(g_pool_mutex);

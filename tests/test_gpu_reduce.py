@@ -112,3 +112,13 @@ def test_grouped_topk_matches_the_reference_rule(cuda, grouping, systems, num_ba
     assert np.array_equal(idx.cpu().numpy().view(np.uint64), want_idx)
     assert np.array_equal(mse.cpu().numpy().view(np.uint32), want_mse.view(np.uint32))     # original bits, -0 included
     assert np.array_equal(counts.cpu().numpy().view(np.uint64), want_counts)
+
+
+@pytest.mark.parametrize("count,k", [(31, 31), (32, 7), (33, 64), (2048, 2048), (2049, 2048), (4095, 1), (8192, 2048), (8193, 2047)])
+def test_topk_at_the_edges_of_its_sort_sizes(cuda, count, k):
+    rng = np.random.default_rng(count * 3 + k)
+    scores = noisy_scores(rng, (count,))
+    idx, _ = R.topk(torch.tensor(scores, device="cuda"), k)
+    want = oracle_topk(scores, k)
+    idx = idx.cpu().numpy()
+    assert np.array_equal(idx[: len(want)].view(np.uint64), want) and np.all(idx[len(want):] == -1)
