@@ -64,6 +64,7 @@ struct DeviceBatch {
     uint32_t max_cst;     /* largest constant table */
     uint32_t max_btmp;    /* largest number of bank-part temporaries */
     uint32_t uses_scratch; /* some program needs the scratch spill slot */
+    uint64_t total_cst;   /* constant-table entries of all programs (an upper bound will do) */
 };
 
 struct EvalProblem {
@@ -102,6 +103,8 @@ struct LaunchPlan {
     size_t rows_per_split;
     size_t smem_bytes;
     size_t partial_elements;  /* floats of per-split partial sums the launch needs (0: materialize) */
+    size_t table_elements;    /* floats of constant tables, in the same buffer */
+    size_t table_offset;      /* where they begin in it: behind the partial sums, 16-byte aligned */
     uint32_t grid_x;
     bool ok;
     bool overflow;            /* !ok because a count does not fit the kernel's 32-bit indices */
@@ -124,6 +127,7 @@ struct Geom {
     uint32_t warp_bytes;
     uint32_t scratch_slot;    /* spill slot reserved for the element-by-element FMA */
     unsigned long long rows_per_split;
+    uint32_t direct;          /* rows are not split: sums go to the output, not to partial sums */
 };
 
 constexpr int kNumVariants = 3;
@@ -137,8 +141,8 @@ LaunchPlan plan_launch(const DeviceBatch& batch, const EvalProblem& problem, int
                        size_t scratch_limit);
 
 /* Enqueues the evaluation of one batch on `stream`: the evaluator kernel writes per-split partial
- * sums into `partial` (plan.partial_elements floats, private to the stream until the launch has
- * finished) and a second kernel adds them in a fixed order into the output, so a result does
+ * sums into `partial` (plan.table_offset + plan.table_elements floats, private to the stream until the
+ * launch has finished; the programs' constant tables are computed into its end first) and a second kernel adds them in a fixed order into the output, so a result does
  * not depend on the order CTAs ran in.  Returns the CUDA status of the launches. */
 cudaError_t launch_eval(const DeviceBatch& batch, const EvalProblem& problem, const LaunchPlan& plan, float* partial,
                         cudaStream_t stream, unsigned* launches);

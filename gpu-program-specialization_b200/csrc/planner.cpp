@@ -41,11 +41,12 @@ Geom make_geom(const DeviceBatch& batch, const EvalProblem& prob, const LaunchPl
     g.exec_bytes = round16(((size_t)batch.max_insn + 1) * sizeof(SbInsn));
     g.table_bytes = round16((size_t)std::max<uint32_t>(1u, ppi * gpi * batch.max_cst * rc) * 4);
     g.hoist_bytes = round16((size_t)batch.max_hoisted * 32u * rr * 4);
-    g.slot_bytes = round16(std::max<size_t>((size_t)slots * rr * rc * 128u, (size_t)batch.max_btmp * 128u));
+    g.slot_bytes = round16((size_t)slots * rr * rc * 128u);
     g.psum_bytes = round16((size_t)std::max<uint32_t>(1u, quantities(prob) * ppi * gpi * rc) * 4);
     g.warp_bytes = g.exec_bytes + g.table_bytes + g.hoist_bytes + g.slot_bytes + g.psum_bytes;
     g.scratch_slot = batch.max_slots; /* one slot beyond what the programs use */
     g.rows_per_split = plan.rows_per_split;
+    g.direct = 0;
     return g;
 }
 
@@ -174,6 +175,11 @@ LaunchPlan plan_with_tile(const DeviceBatch& batch, const EvalProblem& prob, int
         if (configs && n > (~0ull >> 3) / configs / nq) { plan.overflow = true; return plan; }
         plan.partial_elements = (size_t)(n * nq * configs);
     }
+    /* constant tables: one float per entry and (padded bank, permutation) */
+    const unsigned long long padded = materialize ? rc : ((unsigned long long)(prob.num_banks + rc - 1) / rc * rc) << prob.toggle_bits;
+    if (batch.total_cst > (~0ull >> 3) / padded) { plan.overflow = true; return plan; }
+    plan.table_elements = (size_t)(batch.total_cst * padded);
+    plan.table_offset = (plan.partial_elements + 3) / 4 * 4;
     plan.ok = true;
     return plan;
 }

@@ -128,6 +128,7 @@ typedef struct SbProgram {
     uint32_t cost;      /* scheduling weight: bits 0..15 main part per bank group, bits 16..31 row prelude */
     uint16_t mid_off;
     uint16_t reserved;
+    uint32_t cst_off;   /* constant-table entries of the programs before this one in launch order (set by the runner) */
 } SbProgram;
 
 #endif

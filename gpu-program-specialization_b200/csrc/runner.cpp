@@ -409,10 +409,14 @@ SecantResult upload_batch(SecantCubinRunnerImpl* r, Slot& s, std::vector<DeviceB
     order_programs(s);
     SbProgram* const out = reinterpret_cast<SbProgram*>(h + o_prog);
     size_t num_light = 0;
+    uint64_t entries = 0;
     for (size_t i = 0; i < n_programs; ++i) {
         out[i] = s.headers[(uint32_t)s.order[i]];
+        out[i].cst_off = (uint32_t)entries;
+        entries += out[i].n_cst;
         num_light += (s.order[i] >> 53) == 0;
     }
+    if (entries > 0xffffffffull) return SECANT_ERROR_OVERFLOW;
     SB_CUDA(cudaMemcpyAsync(s.device, s.pinned, total, cudaMemcpyHostToDevice, r->copy_stream), "program upload");
     SB_CUDA(cudaEventRecord(s.uploaded, r->copy_stream), "cudaEventRecord");
     const char* d = static_cast<const char*>(s.device);
@@ -436,6 +440,7 @@ SecantResult upload_batch(SecantCubinRunnerImpl* r, Slot& s, std::vector<DeviceB
             db.max_slots = std::max<uint32_t>(db.max_slots, p.n_slots);
             db.max_hoisted = std::max<uint32_t>(db.max_hoisted, p.n_hoisted);
             db.max_cst = std::max<uint32_t>(db.max_cst, p.n_cst);
+            db.total_cst += p.n_cst;
             db.max_btmp = std::max<uint32_t>(db.max_btmp, p.n_btmp);
             db.uses_scratch |= (p.flags & SB_PROG_USES_SCRATCH) ? 1u : 0u;
         }
@@ -515,23 +520,37 @@ SecantResult launch_batch(SecantCubinRunnerImpl* r, const DeviceBatch& db, const
         prob.fast_math = r->fast_math;
         if (runs[e].program_bank_stride)
             prob.banks = reinterpret_cast<const float*>(runs[e].banks.address) + runs[e].first_program_index * runs[e].program_bank_stride;
-        const LaunchPlan lp = plan_launch(db, prob, r->sm_count, r->smem_limit, r->scratch_limit);
-        if (!lp.ok) {
-            r->last_error = lp.overflow ? "configuration count beyond the evaluator's 32-bit item index" : "program batch does not fit shared memory";
-            return lp.overflow ? SECANT_ERROR_OVERFLOW : SECANT_ERROR_REGISTER_OVERFLOW;
-        }
-        float* partial = nullptr;
-        if (lp.partial_elements) {
-            const SecantResult a = stream_scratch(r, k, lp.partial_elements, &partial);
-            if (a != SECANT_SUCCESS) return a;
-        }
-        unsigned launches = 0;
         cudaError_t ce = after ? cudaStreamWaitEvent(stream, after, 0) : cudaSuccess;
-        if (ce == cudaSuccess) ce = launch_eval(db, prob, lp, partial, stream, &launches);
-        g_kernel_launches.fetch_add(launches);
-        if (launches)
-            g_row_stream_bytes.fetch_add((uint64_t)lp.num_groups * (prob.num_inputs + (prob.mode == EVAL_MATERIALIZE ? 0u : prob.num_targets)) *
-                                         (uint64_t)prob.num_rows * sizeof(float));
+        /* one launch, unless its constant tables (an entry per program constant and configuration) would
+         * take more than the scratch limit: then the programs in as many launches as it takes, and a
+         * program at a time at least */
+        const size_t per_program = std::max<size_t>(1, (size_t)db.max_cst * (size_t)((prob.num_banks + 3ull) << prob.toggle_bits));
+        const size_t fit = std::max<size_t>(1, r->scratch_limit / per_program);
+        const size_t step = db.total_cst <= r->scratch_limit / ((prob.num_banks + 3ull) << prob.toggle_bits) ? db.num_programs : fit;
+        for (size_t first = 0; first < db.num_programs && ce == cudaSuccess; first += step) {
+            DeviceBatch part = db;
+            if (step < db.num_programs) {
+                part.programs += first;
+                part.num_programs = (uint32_t)std::min<size_t>(step, db.num_programs - first);
+                part.total_cst = (uint64_t)part.num_programs * db.max_cst;
+            }
+            const LaunchPlan lp = plan_launch(part, prob, r->sm_count, r->smem_limit, r->scratch_limit);
+            if (!lp.ok) {
+                r->last_error = lp.overflow ? "configuration count beyond the evaluator's 32-bit item index" : "program batch does not fit shared memory";
+                return lp.overflow ? SECANT_ERROR_OVERFLOW : SECANT_ERROR_REGISTER_OVERFLOW;
+            }
+            float* partial = nullptr;
+            if (lp.partial_elements || lp.table_elements) {
+                const SecantResult a = stream_scratch(r, k, lp.table_offset + lp.table_elements, &partial);
+                if (a != SECANT_SUCCESS) return a;
+            }
+            unsigned launches = 0;
+            ce = launch_eval(part, prob, lp, partial, stream, &launches);
+            g_kernel_launches.fetch_add(launches);
+            if (launches)
+                g_row_stream_bytes.fetch_add((uint64_t)lp.num_groups * (prob.num_inputs + (prob.mode == EVAL_MATERIALIZE ? 0u : prob.num_targets)) *
+                                             (uint64_t)prob.num_rows * sizeof(float));
+        }
         if (ce == cudaSuccess && done) ce = cudaEventRecord((*done)[k], stream);
         if (ce != cudaSuccess) return cuda_fail(r, ce, "kernel launch");
         if (used) (*used)[k] = 1;
@@ -555,8 +574,12 @@ SecantResult launch_gram_batch(SecantCubinRunnerImpl* r, const std::vector<Devic
         /* rows per range: what the scratch limit leaves for this batch, between 128 and 16,384 */
         const size_t fit = r->scratch_limit / batch_programs;
         const size_t range = std::min<size_t>(run.rows, std::max<size_t>(128, std::min<size_t>(16384, fit)));
+        /* scratch: the range's predictions, then the constant tables of one view at a time (padded to four banks at most) */
+        size_t entries = 0;
+        for (const DeviceBatch& db : views) entries = std::max<size_t>(entries, db.total_cst);
+        const size_t predictions = (batch_programs * range + 3) / 4 * 4;
         float* scratch = nullptr;
-        const SecantResult a = stream_scratch(r, k, batch_programs * range, &scratch);
+        const SecantResult a = stream_scratch(r, k, predictions + 4 * entries, &scratch);
         if (a != SECANT_SUCCESS) return a;
         cudaError_t ce = after ? cudaStreamWaitEvent(stream, after, 0) : cudaSuccess;
         for (size_t r0 = 0; r0 < run.rows && ce == cudaSuccess; r0 += range) {
@@ -575,7 +598,7 @@ SecantResult launch_gram_batch(SecantCubinRunnerImpl* r, const std::vector<Devic
                     return lp.overflow ? SECANT_ERROR_OVERFLOW : SECANT_ERROR_REGISTER_OVERFLOW;
                 }
                 unsigned launches = 0;
-                ce = launch_eval(db, prob, lp, nullptr, stream, &launches);
+                ce = launch_eval(db, prob, lp, scratch + predictions, stream, &launches);
                 g_kernel_launches.fetch_add(launches);
                 if (ce != cudaSuccess) break;
             }
