@@ -5,6 +5,7 @@
 #define SECANT_B200_EVAL_KERNEL_CUH
 
 #include "evaluator.cuh"
+#include "pairs_ptx.cuh"
 #include "sbmath.cuh"
 
 #include <math_constants.h>
@@ -51,8 +52,9 @@ __device__ __noinline__ void fma_over_scratch(uint2 ins, const float* rowp, cons
 /* ---- the interpreter's core ------------------------------------------------------------------
  *
  * What a warp executes is its private copy of the program with every instruction of the row parts
- * rewritten once per item (rewrite() below): word 0 = a handler number, word 1 = the operand's byte
- * offset from one of four base addresses.  The handlers are PTX in one block so that three things hold
+ * rewritten once per item (rewrite() below): word 0 = the handler of the NEXT instruction (so that the
+ * indexed branch's table is read while this one works), word 1 = the operand's byte offset from one of
+ * four base addresses.  The handlers are PTX in one block so that three things hold
  * which the compiler does not give: the dispatch is one indexed branch that is known to be uniform (the
  * C++ switch became a tree of about ten compares and ten branches per instruction, with reconvergence
  * barriers around them), every handler leaves the tile in the registers the next one reads it from
@@ -121,11 +123,18 @@ __device__ __forceinline__ SbInsn rewrite(SbInsn ins, const OperandStrides& st) 
     return SbInsn{h, idx * stride};
 }
 
-/* asm operands: 0..7 the tile, 8..15 the operand, 16 the address of the next instruction, 17 and 18
- * the words of the instruction the block was left with; 19..22 the bases of dataset columns, hoisted
+/* into a warp's program copy, where an instruction's handler stands in the entry before it */
+__device__ __forceinline__ void put_insn(SbInsn* at, SbInsn ins) {
+    at[-1].w0 = ins.w0;
+    at->w1 = ins.w1;
+}
+
+/* asm operands: 0..7 the tile, 8..15 the operand, 16 the address of the next instruction, 17 the
+ * next handler and 18 word 1 of this instruction (at the end 17 says whether the run is over, 0, or an
+ * instruction was left, 1); 19..22 the bases of dataset columns, hoisted
  * values (less kHoistedOffset), constants and slots for this lane; 23 the pair (-1, -1), 24 the pair (-0, -0). */
-#define SB_NEXT "ld.shared.v2.u32 {%17, %18}, [%16];\n add.u32 %16, %16, 8;\n"
-#define SB_GO "brx.idx.uni %17, targets;\n"
+#define SB_NEXT "mov.u32 hb, %17;\n ld.shared.v2.u32 {%17, %18}, [%16];\n add.u32 %16, %16, 8;\n"
+#define SB_GO "brx.idx.uni hb, targets;\n"
 #define SB_AT(BASE) "add.u32 ad, %18, " BASE ";\n"
 #define SB_AT_ROW "setp.lt.s32 p, %18, 0;\n selp.b32 ad, %20, %19, p;\n add.u32 ad, ad, %18;\n"
 #define SB_ADD8(M0, M1, M2, M3, M4, M5, M6, M7) SB_TWO8("add.rn.f32x2", M0, M1, M2, M3, M4, M5, M6, M7)
@@ -201,83 +210,38 @@ __device__ __forceinline__ SbInsn rewrite(SbInsn ins, const OperandStrides& st) 
 #define SB_MAPQ_CST_8 SB_COPY("%2", "%0") SB_COPY("%4", "%0") SB_COPY("%6", "%0") SB_COPY("%3", "%1") SB_COPY("%5", "%1") SB_COPY("%7", "%1")
 #define SB_LOADQC_16 "ld.shared.b32 c0, [ad];\n mov.b64 %0, {c0, c0};\n"
 #define SB_MAPQ_CST_16 SB_COPY("%1", "%0") SB_COPY("%2", "%0") SB_COPY("%3", "%0") SB_COPY("%4", "%0") SB_COPY("%5", "%0") SB_COPY("%6", "%0") SB_COPY("%7", "%0")
-/* The accurate functions, on all eight pairs; the same steps, in the same order, as the scalar versions
- * of sbmath.cuh.  Each first makes sure that no lane has an argument outside the common range
- * (magnitudes compared three at a time, NaN wins) and leaves the block otherwise. */
+/* The accurate functions on all eight pairs (pairs_ptx.cuh). */
 #define SB_EACH(F) F("%0") F("%1") F("%2") F("%3") F("%4") F("%5") F("%6") F("%7")
-#define SB_PAIR_CONST(R, BITS) "mov.b64 " R ", " BITS ";\n"
-#define SB_TOP(A) "mov.b64 {f0, f1}, " A ";\n max.NaN.abs.f32 top, top, f0, f1;\n"
-#define SB_LOW(A) "mov.b64 {f0, f1}, " A ";\n min.NaN.f32 low, low, f0, f1;\n"
-#define SB_LOW_ABS(A) "mov.b64 {f0, f1}, " A ";\n min.NaN.abs.f32 low, low, f0, f1;\n"
-#define SB_ALL_OR_LEAVE "vote.sync.all.pred p, p, 0xffffffff;\n @!p bra.uni LEAVE;\n"
-#define SB_SIN_PAIR(A)                                                                                  \
-    "fma.rn.f32x2 t, " A ", k0, hf;\n add.rn.f32x2 t, t, k1;\n add.rn.f32x2 n, t, k2;\n add.rn.f32x2 n, n, nh;\n" \
-    "fma.rn.f32x2 r, n, k3, " A ";\n fma.rn.f32x2 r, n, k4, r;\n fma.rn.f32x2 r, n, k5, r;\n mul.rn.f32x2 z, r, r;\n" \
-    "fma.rn.f32x2 q, k6, z, k7;\n fma.rn.f32x2 q, q, z, k8;\n fma.rn.f32x2 q, q, z, k9;\n fma.rn.f32x2 q, q, z, k10;\n" \
-    "mul.rn.f32x2 z, r, z;\n fma.rn.f32x2 r, z, q, r;\n mov.b64 {c0, c1}, t;\n shl.b32 c0, c0, 31;\n shl.b32 c1, c1, 31;\n" \
-    "mov.b64 t, {c0, c1};\n xor.b64 " A ", r, t;\n"
-#define SB_EXP_PAIR(A)                                                                                  \
-    "fma.rn.f32x2 t, " A ", k0, k1;\n fma.rn.f32x2 n, t, %23, k1;\n fma.rn.f32x2 r, " A ", k0, n;\n fma.rn.f32x2 r, " A ", k2, r;\n" \
-    "mov.b64 {f0, f1}, r;\n ex2.approx.ftz.f32 f0, f0;\n ex2.approx.ftz.f32 f1, f1;\n mov.b64 {c0, c1}, t;\n" \
-    "shl.b32 c0, c0, 23;\n shl.b32 c1, c1, 23;\n mov.b32 c2, f0;\n mov.b32 c3, f1;\n add.u32 c0, c0, c2;\n add.u32 c1, c1, c3;\n" \
-    "mov.b64 " A ", {c0, c1};\n"
-/* the exponent becomes a float through the low bits of 1.5 * 2^23: exact, and off the conversion unit */
-#define SB_LOG_PAIR(A)                                                                                  \
-    "mov.b64 {c0, c1}, " A ";\n add.u32 c0, c0, 0xC0CAFB0D;\n add.u32 c1, c1, 0xC0CAFB0D;\n"             \
-    "shr.s32 c2, c0, 23;\n shr.s32 c3, c1, 23;\n add.u32 c2, c2, 0x4B400000;\n add.u32 c3, c3, 0x4B400000;\n mov.b64 n, {c2, c3};\n" \
-    "and.b32 c0, c0, 0x7fffff;\n and.b32 c1, c1, 0x7fffff;\n add.u32 c0, c0, 0x3F3504F3;\n add.u32 c1, c1, 0x3F3504F3;\n mov.b64 r, {c0, c1};\n" \
-    "add.rn.f32x2 n, n, k0;\n add.rn.f32x2 r, r, %23;\n fma.rn.f32x2 q, k1, r, k2;\n fma.rn.f32x2 q, q, r, k3;\n fma.rn.f32x2 q, q, r, k4;\n" \
-    "fma.rn.f32x2 q, q, r, k5;\n fma.rn.f32x2 q, q, r, k6;\n fma.rn.f32x2 q, q, r, k7;\n fma.rn.f32x2 q, q, r, k8;\n mul.rn.f32x2 z, r, r;\n" \
-    "mul.rn.f32x2 t, k9, z;\n mul.rn.f32x2 z, r, z;\n fma.rn.f32x2 t, z, q, t;\n fma.rn.f32x2 t, n, k10, t;\n add.rn.f32x2 r, r, t;\n" \
-    "fma.rn.f32x2 " A ", n, k11, r;\n"
-/* a / b, correctly rounded: Newton-Raphson from the hardware's reciprocal estimate and two residual
- * corrections (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000
- * processor", IBM J. Res. Dev. 34, 1990: with a reciprocal good to half an ulp and the residual
- * a - b q exact, the corrected quotient is the rounded one).  Works on -1/b and -q so that every step is
- * one fused multiply-add; the sign comes from the first product, since the corrections lose that of a
- * zero quotient. */
-#define SB_DIV_PAIR(A, B)                                                                               \
-    "mov.b64 {f0, f1}, " B ";\n neg.f32 f0, f0;\n neg.f32 f1, f1;\n rcp.approx.ftz.f32 f0, f0;\n rcp.approx.ftz.f32 f1, f1;\n mov.b64 r, {f0, f1};\n" \
-    "fma.rn.f32x2 t, " B ", r, k0;\n fma.rn.f32x2 r, r, t, r;\n mul.rn.f32x2 n, " A ", r;\n fma.rn.f32x2 t, " B ", n, " A ";\n"    \
-    "fma.rn.f32x2 q, t, r, n;\n fma.rn.f32x2 t, " B ", q, " A ";\n fma.rn.f32x2 q, t, r, q;\n"           \
-    "mov.b64 {c0, c1}, q;\n mov.b64 {c2, c3}, n;\n lop3.b32 c0, c0, c2, 0x80000000, 0x72;\n lop3.b32 c1, c1, c3, 0x80000000, 0x72;\n" \
-    "mov.b64 " A ", {c0, c1};\n"
-/* |b| within [2^-60, 2^60], |a| too or zero (2|a| - 1 in bits: zero wraps to the top): no step leaves the normal range */
-#define SB_LEAST(A) "mov.b64 {c0, c1}, " A ";\n shl.b32 c0, c0, 1;\n shl.b32 c1, c1, 1;\n sub.u32 c0, c0, 1;\n sub.u32 c1, c1, 1;\n min.u32 c2, c2, c0;\n min.u32 c2, c2, c1;\n"
 #define SB_FUNCTIONS                                                                                    \
-    "CO:\n mov.b64 hf, 0x3F0000003F000000;\n mov.b64 nh, 0xBF000000BF000000;\n bra.uni SC0;\n"          \
-    "SI:\n mov.b64 hf, 0;\n mov.b64 nh, %24;\n"                                                        \
+    "CO:\n" SB_COS_SHIFT "bra.uni SC0;\n SI:\n" SB_SIN_SHIFT                                            \
     "SC0:\n mov.f32 top, 0f00000000;\n" SB_EACH(SB_TOP) "setp.lt.f32 p, top, 0f45800000;\n" SB_ALL_OR_LEAVE SB_NEXT \
-    SB_PAIR_CONST("k0", "0x3EA2F9833EA2F983") SB_PAIR_CONST("k1", "0x4B4000004B400000") SB_PAIR_CONST("k2", "0xCB400000CB400000") SB_PAIR_CONST("k3", "0xC0490FDBC0490FDB") \
-    SB_PAIR_CONST("k4", "0x33BBBD2E33BBBD2E") SB_PAIR_CONST("k5", "0x27772CED27772CED") SB_PAIR_CONST("k6", "0xB2CD31C1B2CD31C1") SB_PAIR_CONST("k7", "0x3638B8243638B824") \
-    SB_PAIR_CONST("k8", "0xB9500BECB9500BEC") SB_PAIR_CONST("k9", "0x3C0888863C088886") SB_PAIR_CONST("k10", "0xBE2AAAABBE2AAAAB") SB_EACH(SB_SIN_PAIR) SB_GO \
+    SB_SIN_CONSTANTS SB_EACH(SB_SIN_PAIR) SB_GO                                                         \
     "EX:\n mov.f32 top, 0f00000000;\n" SB_EACH(SB_TOP) "setp.le.f32 p, top, 0f42AC0000;\n" SB_ALL_OR_LEAVE SB_NEXT \
-    SB_PAIR_CONST("k0", "0x3FB8AA3B3FB8AA3B") SB_PAIR_CONST("k1", "0x4B4000004B400000") SB_PAIR_CONST("k2", "0x32A5706032A57060") SB_EACH(SB_EXP_PAIR) SB_GO \
+    SB_EXP_CONSTANTS SB_MINUS_ONE SB_EACH(SB_EXP_PAIR) SB_GO                                            \
     "LG:\n mov.f32 top, 0f00000000;\n mov.f32 low, 0f7F800000;\n" SB_EACH(SB_TOP) SB_EACH(SB_LOW)       \
     "setp.lt.f32 p, top, 0f7F800000;\n setp.ge.and.f32 p, low, 0f00800000, p;\n" SB_ALL_OR_LEAVE SB_NEXT \
-    SB_PAIR_CONST("k0", "0xCB400000CB400000") SB_PAIR_CONST("k1", "0xBD9C5854BD9C5854") SB_PAIR_CONST("k2", "0x3E02AC143E02AC14") SB_PAIR_CONST("k3", "0xBE06C251BE06C251") \
-    SB_PAIR_CONST("k4", "0x3E116D423E116D42") SB_PAIR_CONST("k5", "0xBE2A392FBE2A392F") SB_PAIR_CONST("k6", "0x3E4CD0023E4CD002") SB_PAIR_CONST("k7", "0xBE800113BE800113") \
-    SB_PAIR_CONST("k8", "0x3EAAAAAA3EAAAAAA") SB_PAIR_CONST("k9", "0xBF000000BF000000") SB_PAIR_CONST("k10", "0x35BFBE8E35BFBE8E") SB_PAIR_CONST("k11", "0x3F3172003F317200") SB_EACH(SB_LOG_PAIR) SB_GO \
+    SB_LOG_CONSTANTS SB_MINUS_ONE SB_EACH(SB_LOG_PAIR) SB_GO                                            \
     "DV:\n mov.u32 c2, 0xffffffff;\n" SB_EACH(SB_LEAST) "mov.f32 top, 0f00000000;\n mov.f32 low, 0f7F800000;\n" \
     SB_EACH(SB_TOP) SB_TOP("%8") SB_TOP("%9") SB_TOP("%10") SB_TOP("%11") SB_TOP("%12") SB_TOP("%13") SB_TOP("%14") SB_TOP("%15") \
     SB_LOW_ABS("%8") SB_LOW_ABS("%9") SB_LOW_ABS("%10") SB_LOW_ABS("%11") SB_LOW_ABS("%12") SB_LOW_ABS("%13") SB_LOW_ABS("%14") SB_LOW_ABS("%15") \
-    "setp.le.f32 p, top, 0f5D800000;\n setp.ge.and.f32 p, low, 0f21800000, p;\n setp.ge.and.u32 p, c2, 0x42FFFFFF, p;\n" SB_ALL_OR_LEAVE SB_NEXT \
-    SB_PAIR_CONST("k0", "0x3F8000003F800000") SB_DIV_PAIR("%0", "%8") SB_DIV_PAIR("%1", "%9") SB_DIV_PAIR("%2", "%10") SB_DIV_PAIR("%3", "%11") \
+    SB_DIV_RANGE SB_ALL_OR_LEAVE SB_NEXT                                                                \
+    SB_DIV_CONSTANTS SB_DIV_PAIR("%0", "%8") SB_DIV_PAIR("%1", "%9") SB_DIV_PAIR("%2", "%10") SB_DIV_PAIR("%3", "%11") \
     SB_DIV_PAIR("%4", "%12") SB_DIV_PAIR("%5", "%13") SB_DIV_PAIR("%6", "%14") SB_DIV_PAIR("%7", "%15") SB_GO
+
 /* without the functions (approximate mathematics) they and the divisions leave the block */
 #define SB_NO_FUNCTIONS "SI:\n CO:\n EX:\n LG:\n DV:\n bra.uni LEAVE;\n"
 #define SB_CORE(N, FUNCTIONS)                                                                           \
-    "{\n .reg .u32 ad, c0, c1, c2, c3;\n .reg .f32 f0, f1, top, low;\n .reg .b64 m, t, n, r, z, q, hf, nh, k<12>;\n .reg .pred p;\n" \
-    "targets: .branchtargets LEAVE, LR, LC, LS, ST, SH, AR, AC, AS, SR, SC, SS, RR, RC, RS, MR, MC, MS, NG, AB, " \
+    "{\n" SB_PTX_REGISTERS                                                                             \
+    ".reg .u32 hb;\n targets: .branchtargets EN, LR, LC, LS, ST, SH, AR, AC, AS, SR, SC, SS, RR, RC, RS, MR, MC, MS, NG, AB, " \
     "DR, DC, DS, QR, QC, QS, SI, CO, EX, LG, LEAVE, LEAVE;\n"                                           \
-    SB_NEXT SB_GO                                                                                       \
+    "ld.shared.u32 %17, [%16+-8];\n" SB_NEXT SB_GO                                                       \
     SB_THREE(N, "L", SB_MOV8) SB_THREE(N, "A", SB_ADD8) SB_THREE(N, "S", SB_SUB8) SB_THREE(N, "R", SB_RSUB8) \
     SB_THREE(N, "M", SB_MUL8) SB_DIVISIONS(N)                                                           \
     "ST:\n" SB_AT("%22") SB_NEXT "st.shared.v2.b64 [ad], {%0, %1};\n st.shared.v2.b64 [ad+512], {%2, %3};\n st.shared.v2.b64 [ad+1024], {%4, %5};\n st.shared.v2.b64 [ad+1536], {%6, %7};\n" SB_GO \
     "SH:\n add.u32 ad, %18, %20;\n xor.b32 ad, ad, 0x80000000;\n" SB_NEXT SB_STOREH_##N SB_GO           \
     "NG:\n mov.b64 m, 0x8000000080000000;\n" SB_NEXT SB_NEG8 SB_GO                                       \
     "AB:\n mov.b64 m, 0x7fffffff7fffffff;\n" SB_NEXT SB_ABS8 SB_GO                                       \
-    FUNCTIONS "LEAVE:\n }"
+    FUNCTIONS "EN:\n mov.u32 %17, 0;\n bra.uni OUT;\n LEAVE:\n mov.u32 %17, 1;\n OUT:\n }"
 
 /* The tile is kept as pairs of rows (sbmath.cuh, f2): acc[h][c] holds rows 2h and 2h + 1 of bank column
  * c.  A ROW operand arrives as pairs straight from its 128-bit loads; a CST operand is doubled in
@@ -458,7 +422,8 @@ struct Machine {
             else if constexpr (RR == 8) SB_RUN_CORE(8, SB_FUNCTIONS);
             else if constexpr (FAST) SB_RUN_CORE(16, SB_NO_FUNCTIONS);
             else SB_RUN_CORE(16, SB_FUNCTIONS);
-            if (h == H_END) return;
+            if (h == 0u) return;
+            asm volatile("ld.shared.u32 %0, [%1+-16];" : "=r"(h) : "r"(ip) : "memory"); /* of the instruction the core stopped at */
             if (FAST && h < H_SIN) {
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
@@ -576,13 +541,13 @@ eval_kernel(const DeviceBatch batch, const EvalProblem prob, const Geom geom, fl
     float* const tiles = reinterpret_cast<float*>(smem);
     unsigned int* const queue = reinterpret_cast<unsigned int*>(smem + (size_t)geom.tile_bytes * geom.tile_buffers);
     unsigned char* const warea = smem + (size_t)geom.tile_bytes * geom.tile_buffers + 16 + (size_t)warp * geom.warp_bytes;
-    SbInsn* const exec = reinterpret_cast<SbInsn*>(warea);
+    SbInsn* const exec = reinterpret_cast<SbInsn*>(warea) + 1; /* the entry before the first holds the first handler */
     float* const table = reinterpret_cast<float*>(warea + geom.exec_bytes);
     float* const psum = reinterpret_cast<float*>(warea + geom.exec_bytes + geom.table_bytes + geom.hoist_bytes + geom.slot_bytes);
 
     typename M::Place place;
     place.exec = (uint32_t)__cvta_generic_to_shared(exec);
-    place.table = place.exec + geom.exec_bytes;
+    place.table = place.exec - 8u + geom.exec_bytes;
     place.hoist = place.table + geom.table_bytes + lane * 16u;
     place.slots = place.table + geom.table_bytes + geom.hoist_bytes + lane * 16u;
     place.tile_ld = geom.tile_rows;
@@ -655,8 +620,7 @@ eval_kernel(const DeviceBatch batch, const EvalProblem prob, const Geom geom, fl
             __syncwarp(); /* the previous item's reads of exec, table and psum are done */
             const SbInsn* const code = batch.insns + hp->insn_off + pre_off; /* the row parts; the bank part has run (bank_tables_kernel) */
 #pragma unroll 1
-            for (uint32_t i = lane; i < n_insn; i += 32) exec[i] = rewrite(code[i], strides);
-            if (lane == 0) exec[n_insn] = SbInsn{0u, 0u}; /* padding read by the instruction prefetch */
+            for (uint32_t i = lane; i < n_insn; i += 32) put_insn(exec + i, rewrite(code[i], strides));
             /* the item's permutations perm0 .. perm0 + ppi - 1 (one, unless the item holds every bank group) */
             const uint32_t block = materialize ? 0u : within / chunks;
             const uint32_t perm0 = block * ppi;
@@ -671,7 +635,7 @@ eval_kernel(const DeviceBatch batch, const EvalProblem prob, const Geom geom, fl
                     const SbPatch* p = patches + i;
                     unsigned choice = (perm >> p->bit0) & 1u;
                     if (p->bit1 != 0xffu) choice |= ((perm >> p->bit1) & 1u) << 1;
-                    if (p->insn >= pre_off) exec[p->insn - pre_off] = rewrite(p->alt[choice], strides);
+                    if (p->insn >= pre_off) put_insn(exec + (p->insn - pre_off), rewrite(p->alt[choice], strides));
                 }
                 __syncwarp();
             };

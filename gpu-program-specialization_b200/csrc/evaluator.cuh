@@ -170,10 +170,12 @@ struct Rk4Problem {
     const uint32_t* order;          /* optional [num_systems]: the system whose items are taken k-th (costliest first) */
     unsigned long long* integrated; /* optional device counter: (trajectory, observation interval) pairs integrated */
 };
+/* Scans the times and reference values once per call and raises *problem.invalid_flag; every launch_rk4()
+ * of the call has to come after it. */
+cudaError_t launch_rk4_validation(const Rk4Problem& problem, cudaStream_t stream);
 /* batch.programs holds num_systems * num_states records, system-major, encoded with
- * columns_are_slots, 4 * num_states reserved slots and a bank part.  `concurrent` = how many such
- * launches share the device at a time (the launch takes that share of the resident CTAs). */
-cudaError_t launch_rk4(const DeviceBatch& batch, const Rk4Problem& problem, size_t smem_limit, unsigned concurrent, cudaStream_t stream);
+ * columns_are_slots, 4 * num_states reserved slots and a bank part. */
+cudaError_t launch_rk4(const DeviceBatch& batch, const Rk4Problem& problem, size_t smem_limit, cudaStream_t stream);
 
 /* Adds the statistics of the static Gram shape for a batch of cohorts over `rows` rows of
  * materialized predictions [program of the batch][prediction_ld] (gram.cu); statistics points at

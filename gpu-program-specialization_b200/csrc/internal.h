@@ -38,6 +38,9 @@ struct UnpackedRun {
     size_t output_count = 0, output_width = 0; /* cleared region: count vectors of width elements */
 };
 
+/* cuCtxGetCurrent; *ok is false when the driver cannot be asked (runner.cpp). */
+void* current_context(bool* ok);
+
 SecantResult recipe_header_validate(const SecantCubinRecipeHeader* recipe);
 SecantResult recipe_validate(const SecantCubinRecipeHeader* recipe);
 void plan_fill(SecantCubinPlan* plan, const SecantCubinRecipeHeader* recipe, size_t cubin_size);

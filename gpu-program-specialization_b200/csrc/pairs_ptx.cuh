@@ -1,0 +1,76 @@
+/*
+ * pairs_ptx.cuh - the accurate functions and the division on pairs of floats, as PTX text for the
+ * interpreters' cores (eval_kernel.cuh, rollout.cu).
+ *
+ * The same steps, in the same order, as the scalar versions of sbmath.cuh, so a value has the same bits
+ * whichever computed it.  They work on named registers the cores declare (SB_PTX_REGISTERS), take the
+ * pair to be replaced as their argument, and hold for the common range of arguments only: a core
+ * compares the magnitudes first (SB_TOP, SB_LOW: three at a time, NaN wins) and leaves its block with
+ * the whole warp when an argument is outside (SB_ALL_OR_LEAVE, a label LEAVE).
+ */
+#ifndef SECANT_B200_PAIRS_PTX_CUH
+#define SECANT_B200_PAIRS_PTX_CUH
+
+#define SB_PTX_REGISTERS ".reg .u32 ad, c0, c1, c2, c3;\n .reg .f32 f0, f1, top, low;\n .reg .b64 m, t, n, r, z, q, hf, nh, mone, k<12>;\n .reg .pred p;\n"
+#define SB_PAIR_CONST(R, BITS) "mov.b64 " R ", " BITS ";\n"
+#define SB_TOP(A) "mov.b64 {f0, f1}, " A ";\n max.NaN.abs.f32 top, top, f0, f1;\n"
+#define SB_LOW(A) "mov.b64 {f0, f1}, " A ";\n min.NaN.f32 low, low, f0, f1;\n"
+#define SB_LOW_ABS(A) "mov.b64 {f0, f1}, " A ";\n min.NaN.abs.f32 low, low, f0, f1;\n"
+#define SB_ALL_OR_LEAVE "vote.sync.all.pred p, p, 0xffffffff;\n @!p bra.uni LEAVE;\n"
+/* constants of the steps below */
+#define SB_SIN_CONSTANTS \
+    SB_PAIR_CONST("k0", "0x3EA2F9833EA2F983") SB_PAIR_CONST("k1", "0x4B4000004B400000") SB_PAIR_CONST("k2", "0xCB400000CB400000") \
+    SB_PAIR_CONST("k3", "0xC0490FDBC0490FDB") SB_PAIR_CONST("k4", "0x33BBBD2E33BBBD2E") SB_PAIR_CONST("k5", "0x27772CED27772CED") \
+    SB_PAIR_CONST("k6", "0xB2CD31C1B2CD31C1") SB_PAIR_CONST("k7", "0x3638B8243638B824") SB_PAIR_CONST("k8", "0xB9500BECB9500BEC") \
+    SB_PAIR_CONST("k9", "0x3C0888863C088886") SB_PAIR_CONST("k10", "0xBE2AAAABBE2AAAAB")
+#define SB_EXP_CONSTANTS \
+    SB_PAIR_CONST("k0", "0x3FB8AA3B3FB8AA3B") SB_PAIR_CONST("k1", "0x4B4000004B400000") SB_PAIR_CONST("k2", "0x32A5706032A57060")
+#define SB_LOG_CONSTANTS \
+    SB_PAIR_CONST("k0", "0xCB400000CB400000") SB_PAIR_CONST("k1", "0xBD9C5854BD9C5854") SB_PAIR_CONST("k2", "0x3E02AC143E02AC14") \
+    SB_PAIR_CONST("k3", "0xBE06C251BE06C251") SB_PAIR_CONST("k4", "0x3E116D423E116D42") SB_PAIR_CONST("k5", "0xBE2A392FBE2A392F") \
+    SB_PAIR_CONST("k6", "0x3E4CD0023E4CD002") SB_PAIR_CONST("k7", "0xBE800113BE800113") SB_PAIR_CONST("k8", "0x3EAAAAAA3EAAAAAA") \
+    SB_PAIR_CONST("k9", "0xBF000000BF000000") SB_PAIR_CONST("k10", "0x35BFBE8E35BFBE8E") SB_PAIR_CONST("k11", "0x3F3172003F317200")
+#define SB_DIV_CONSTANTS \
+    SB_PAIR_CONST("k0", "0x3F8000003F800000")
+#define SB_MINUS_ONE "mov.b64 mone, 0xBF800000BF800000;\n"
+/* sin and cos differ in the shift by half a turn, taken off again after the rounding */
+#define SB_SIN_SHIFT "mov.b64 hf, 0;\n mov.b64 nh, 0x8000000080000000;\n"
+#define SB_COS_SHIFT "mov.b64 hf, 0x3F0000003F000000;\n mov.b64 nh, 0xBF000000BF000000;\n"
+#define SB_SIN_PAIR(A)                                                                                  \
+    "fma.rn.f32x2 t, " A ", k0, hf;\n add.rn.f32x2 t, t, k1;\n add.rn.f32x2 n, t, k2;\n add.rn.f32x2 n, n, nh;\n" \
+    "fma.rn.f32x2 r, n, k3, " A ";\n fma.rn.f32x2 r, n, k4, r;\n fma.rn.f32x2 r, n, k5, r;\n mul.rn.f32x2 z, r, r;\n" \
+    "fma.rn.f32x2 q, k6, z, k7;\n fma.rn.f32x2 q, q, z, k8;\n fma.rn.f32x2 q, q, z, k9;\n fma.rn.f32x2 q, q, z, k10;\n" \
+    "mul.rn.f32x2 z, r, z;\n fma.rn.f32x2 r, z, q, r;\n mov.b64 {c0, c1}, t;\n shl.b32 c0, c0, 31;\n shl.b32 c1, c1, 31;\n" \
+    "mov.b64 t, {c0, c1};\n xor.b64 " A ", r, t;\n"
+#define SB_EXP_PAIR(A)                                                                                  \
+    "fma.rn.f32x2 t, " A ", k0, k1;\n fma.rn.f32x2 n, t, mone, k1;\n fma.rn.f32x2 r, " A ", k0, n;\n fma.rn.f32x2 r, " A ", k2, r;\n" \
+    "mov.b64 {f0, f1}, r;\n ex2.approx.ftz.f32 f0, f0;\n ex2.approx.ftz.f32 f1, f1;\n mov.b64 {c0, c1}, t;\n" \
+    "shl.b32 c0, c0, 23;\n shl.b32 c1, c1, 23;\n mov.b32 c2, f0;\n mov.b32 c3, f1;\n add.u32 c0, c0, c2;\n add.u32 c1, c1, c3;\n" \
+    "mov.b64 " A ", {c0, c1};\n"
+/* the exponent becomes a float through the low bits of 1.5 * 2^23: exact, and off the conversion unit */
+#define SB_LOG_PAIR(A)                                                                                  \
+    "mov.b64 {c0, c1}, " A ";\n add.u32 c0, c0, 0xC0CAFB0D;\n add.u32 c1, c1, 0xC0CAFB0D;\n"             \
+    "shr.s32 c2, c0, 23;\n shr.s32 c3, c1, 23;\n add.u32 c2, c2, 0x4B400000;\n add.u32 c3, c3, 0x4B400000;\n mov.b64 n, {c2, c3};\n" \
+    "and.b32 c0, c0, 0x7fffff;\n and.b32 c1, c1, 0x7fffff;\n add.u32 c0, c0, 0x3F3504F3;\n add.u32 c1, c1, 0x3F3504F3;\n mov.b64 r, {c0, c1};\n" \
+    "add.rn.f32x2 n, n, k0;\n add.rn.f32x2 r, r, mone;\n fma.rn.f32x2 q, k1, r, k2;\n fma.rn.f32x2 q, q, r, k3;\n fma.rn.f32x2 q, q, r, k4;\n" \
+    "fma.rn.f32x2 q, q, r, k5;\n fma.rn.f32x2 q, q, r, k6;\n fma.rn.f32x2 q, q, r, k7;\n fma.rn.f32x2 q, q, r, k8;\n mul.rn.f32x2 z, r, r;\n" \
+    "mul.rn.f32x2 t, k9, z;\n mul.rn.f32x2 z, r, z;\n fma.rn.f32x2 t, z, q, t;\n fma.rn.f32x2 t, n, k10, t;\n add.rn.f32x2 r, r, t;\n" \
+    "fma.rn.f32x2 " A ", n, k11, r;\n"
+/* a / b, correctly rounded: Newton-Raphson from the hardware's reciprocal estimate and two residual
+ * corrections (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000
+ * processor", IBM J. Res. Dev. 34, 1990: with a reciprocal good to half an ulp and the residual
+ * a - b q exact, the corrected quotient is the rounded one).  Works on -1/b and -q so that every step is
+ * one fused multiply-add; the sign comes from the first product, since the corrections lose that of a
+ * zero quotient. */
+#define SB_DIV_PAIR(A, B)                                                                               \
+    "mov.b64 {f0, f1}, " B ";\n neg.f32 f0, f0;\n neg.f32 f1, f1;\n rcp.approx.ftz.f32 f0, f0;\n rcp.approx.ftz.f32 f1, f1;\n mov.b64 r, {f0, f1};\n" \
+    "fma.rn.f32x2 t, " B ", r, k0;\n fma.rn.f32x2 r, r, t, r;\n mul.rn.f32x2 n, " A ", r;\n fma.rn.f32x2 t, " B ", n, " A ";\n"    \
+    "fma.rn.f32x2 q, t, r, n;\n fma.rn.f32x2 t, " B ", q, " A ";\n fma.rn.f32x2 q, t, r, q;\n"           \
+    "mov.b64 {c0, c1}, q;\n mov.b64 {c2, c3}, n;\n lop3.b32 c0, c0, c2, 0x80000000, 0x72;\n lop3.b32 c1, c1, c3, 0x80000000, 0x72;\n" \
+    "mov.b64 " A ", {c0, c1};\n"
+/* |b| within [2^-60, 2^60], |a| too or zero (2|a| - 1 in bits: zero wraps to the top): no step leaves the normal range */
+#define SB_LEAST(A) "mov.b64 {c0, c1}, " A ";\n shl.b32 c0, c0, 1;\n shl.b32 c1, c1, 1;\n sub.u32 c0, c0, 1;\n sub.u32 c1, c1, 1;\n min.u32 c2, c2, c0;\n min.u32 c2, c2, c1;\n"
+/* after SB_LEAST over the dividends, SB_TOP over both, SB_LOW_ABS over the divisors (c2 = ~0, top = 0, low = inf before) */
+#define SB_DIV_RANGE "setp.le.f32 p, top, 0f5D800000;\n setp.ge.and.f32 p, low, 0f21800000, p;\n setp.ge.and.u32 p, c2, 0x42FFFFFF, p;\n"
+
+#endif

@@ -21,6 +21,8 @@
 #include <cstddef>
 #include <cstring>
 #include <exception>
+#include <functional>
+#include <new>
 #include <mutex>
 #include <system_error>
 #include <thread>
@@ -35,6 +37,165 @@ namespace {
 constexpr int kMaxPoolDevices = 64;
 std::mutex g_pool_mutex;
 cudaMemPool_t g_pools[kMaxPoolDevices] = {};
+
+/* What a call needs on the device besides its records: streams, an event and pinned staging buffers.
+ * Making and destroying them took as long as scoring a few hundred systems (measured: 0.9 ms of a 2.4 ms
+ * call), so finished calls leave them for later ones of the same context: at most kKeptCalls sets, each
+ * used by one call at a time, given back by secant_b200_release_cached_memory(). */
+constexpr int kComputeStreams = 2; /* the next launch takes the SMs that the one before it leaves */
+constexpr size_t kKeptCalls = 4, kKeptStaging = 16, kKeptStagingBytes = (size_t)64 << 20;
+struct Staging { void* host = nullptr; size_t bytes = 0; };
+struct CallResources {
+    int device = 0;
+    void* context = nullptr;
+    cudaStream_t compute[kComputeStreams] = {}, copies = nullptr;
+    cudaEvent_t uploaded = nullptr, validated = nullptr;
+    std::vector<Staging> staging; /* by launch of a call */
+};
+std::mutex g_calls_mutex;
+std::vector<CallResources*> g_calls;
+
+cudaError_t destroy_resources(CallResources* r) {
+    cudaError_t e = cudaSuccess;
+    auto keep = [&](cudaError_t f) { if (e == cudaSuccess) e = f; };
+    for (Staging& s : r->staging) if (s.host) keep(cudaFreeHost(s.host));
+    for (cudaStream_t q : r->compute) if (q) keep(cudaStreamDestroy(q));
+    if (r->copies) keep(cudaStreamDestroy(r->copies));
+    if (r->uploaded) keep(cudaEventDestroy(r->uploaded));
+    if (r->validated) keep(cudaEventDestroy(r->validated));
+    delete r;
+    return e;
+}
+
+/* A set for the current context, kept or new; null with *e set when one cannot be made. */
+CallResources* take_resources(int device, cudaError_t* e) {
+    bool known = false;
+    void* context = current_context(&known);
+    {
+        std::lock_guard<std::mutex> lock(g_calls_mutex);
+        for (size_t i = 0; i < g_calls.size(); ++i)
+            if (known && g_calls[i]->device == device && g_calls[i]->context == context) {
+                CallResources* r = g_calls[i];
+                g_calls.erase(g_calls.begin() + (ptrdiff_t)i);
+                return r;
+            }
+    }
+    CallResources* r = new (std::nothrow) CallResources();
+    if (!r) { *e = cudaErrorMemoryAllocation; return nullptr; }
+    r->device = device;
+    r->context = known ? context : nullptr;
+    *e = cudaStreamCreateWithFlags(&r->copies, cudaStreamNonBlocking);
+    if (*e == cudaSuccess) *e = cudaEventCreateWithFlags(&r->uploaded, cudaEventDisableTiming);
+    if (*e == cudaSuccess) *e = cudaEventCreateWithFlags(&r->validated, cudaEventDisableTiming);
+    for (int i = 0; i < kComputeStreams && *e == cudaSuccess; ++i) *e = cudaStreamCreateWithFlags(&r->compute[i], cudaStreamNonBlocking);
+    if (*e == cudaSuccess) return r;
+    destroy_resources(r);
+    return nullptr;
+}
+/* `clean`: every stream is idle and nothing failed */
+cudaError_t leave_resources(CallResources* r, bool clean) {
+    size_t bytes = 0;
+    for (const Staging& s : r->staging) bytes += s.bytes;
+    if (clean && r->context && bytes <= kKeptStagingBytes) {
+        std::lock_guard<std::mutex> lock(g_calls_mutex);
+        if (g_calls.size() < kKeptCalls) {
+            try {
+                g_calls.push_back(r);
+                return cudaSuccess;
+            } catch (const std::bad_alloc&) {
+            }
+        }
+    }
+    return destroy_resources(r);
+}
+/* Pinned memory for the records of launch `c`, null when there is none to be had (pageable memory will do). */
+char* staging_for(CallResources* r, size_t c, size_t bytes) {
+    if (c >= kKeptStaging) return nullptr;
+    try {
+        if (r->staging.size() <= c) r->staging.resize(c + 1);
+    } catch (const std::bad_alloc&) {
+        return nullptr;
+    }
+    Staging& s = r->staging[c];
+    if (s.bytes < bytes) {
+        if (s.host) cudaFreeHost(s.host);
+        s = Staging();
+        if (cudaHostAlloc(&s.host, bytes + bytes / 4, cudaHostAllocDefault) != cudaSuccess) {
+            cudaGetLastError();
+            s = Staging();
+            return nullptr;
+        }
+        s.bytes = bytes + bytes / 4;
+    }
+    return static_cast<char*>(s.host);
+}
+
+/* Threads that help calls with their host work.  They are started when first wanted (a call of 600
+ * systems spent 0.3 ms of 2.4 starting and joining its own), at most kMostHelpers for the process, wait
+ * between calls, and are joined by secant_b200_release_cached_memory().  A call never depends on them:
+ * it does whatever no helper has taken. */
+constexpr size_t kMostHelpers = 15;
+class Helpers {
+public:
+    struct Job {
+        std::function<void()> work;
+        size_t tickets = 0, active = 0;
+    };
+    void start(Job* job, size_t wanted) {
+        std::lock_guard<std::mutex> lock(mutex_);
+        job->tickets = std::min(wanted, kMostHelpers);
+        if (!job->tickets) return;
+        jobs_.push_back(job);
+        try {
+            while (threads_.size() < job->tickets) threads_.emplace_back([this, now = generation_] { serve(now); });
+        } catch (const std::exception&) {
+            /* no memory or no thread to be had: fewer helpers, or none */
+        }
+        wake_.notify_all();
+    }
+    /* after this no helper is on the job or will be */
+    void finish(Job* job) {
+        std::unique_lock<std::mutex> lock(mutex_);
+        job->tickets = 0;
+        jobs_.erase(std::remove(jobs_.begin(), jobs_.end(), job), jobs_.end());
+        done_.wait(lock, [&] { return job->active == 0; });
+    }
+    void stop() {
+        std::vector<std::thread> threads;
+        {
+            std::lock_guard<std::mutex> lock(mutex_);
+            ++generation_;
+            threads.swap(threads_);
+        }
+        wake_.notify_all();
+        for (std::thread& t : threads) t.join();
+    }
+
+private:
+    void serve(const unsigned generation) {
+        std::unique_lock<std::mutex> lock(mutex_);
+        for (;;) {
+            wake_.wait(lock, [&] { return generation != generation_ || !jobs_.empty(); });
+            if (generation != generation_) return;
+            Job* job = jobs_.front();
+            if (--job->tickets == 0) jobs_.erase(jobs_.begin());
+            ++job->active;
+            lock.unlock();
+            job->work();
+            lock.lock();
+            if (--job->active == 0) done_.notify_all();
+        }
+    }
+    std::mutex mutex_;
+    std::condition_variable wake_, done_;
+    std::vector<Job*> jobs_;
+    std::vector<std::thread> threads_;
+    unsigned generation_ = 0;
+};
+Helpers& helpers() {
+    static Helpers* const all = new Helpers(); /* never destroyed: its threads may wait until the process ends */
+    return *all;
+}
 
 }  // namespace
 
@@ -66,6 +227,14 @@ extern "C" SecantResult secant_b200_release_cached_memory(void) {
     SecantResult result = SECANT_SUCCESS;
     for (cudaMemPool_t pool : g_pools)
         if (pool && cudaMemPoolTrimTo(pool, 0) != cudaSuccess) result = SECANT_ERROR_DRIVER_FAILED;
+    helpers().stop();
+    std::vector<CallResources*> idle;
+    {
+        std::lock_guard<std::mutex> calls(g_calls_mutex);
+        idle.swap(g_calls);
+    }
+    for (CallResources* r : idle)
+        if (destroy_resources(r) != cudaSuccess) result = SECANT_ERROR_DRIVER_FAILED;
     return result;
 }
 
@@ -130,27 +299,35 @@ extern "C" SecantResult secant_b200_rk4_score(const SecantB200Rk4Run* given) {
     SecantResult result = routine_arities(programs.routines, arity);
     if (result != SECANT_SUCCESS) return result;
 
-    /* Host threads work on pieces of 128 systems: first every piece is scanned (nothing is launched
-     * before every program has passed the scan, and the first failing program in order decides the
-     * result), then the pieces are encoded while the calling thread joins sixteen encoded pieces into
-     * one launch, uploads it and starts its kernels, so encoding overlaps the kernels of earlier
-     * launches.  A structural error found while encoding a later piece ends the call with that
-     * code; scores of earlier launches may already have been written. */
-    constexpr size_t kPieceSystems = 128, kPiecesPerLaunch = 16;
-    const size_t num_pieces = (run->num_systems + kPieceSystems - 1) / kPieceSystems;
-    const size_t num_chunks = (num_pieces + kPiecesPerLaunch - 1) / kPiecesPerLaunch;
+    /* Host threads work on pieces of 128 systems, or of 16 at least when that gives every thread a few:
+     * first every piece is scanned (nothing is launched before every program has passed the scan, and
+     * the first failing program in order decides the result), then the pieces are encoded while the
+     * calling thread joins encoded pieces into launches, uploads them and starts their kernels, so
+     * encoding overlaps the kernels of earlier launches.  A structural error found while encoding a
+     * later piece ends the call with that code; scores of earlier launches may already have been
+     * written.
+     * The first launch takes 4,096 systems, each later one twice as many as the one before, up to
+     * 16,384: few and large launches, because warps of two launches on one SM slow each other down
+     * (4,096 systems of three states, 64 trajectories, 1,000 steps: 37.2 ms as two launches side by
+     * side, 25.7 as one; the same number of warps on every SM, an item takes 16.9 ms instead of 9.8)
+     * and because a launch's last items leave groups of warps idle.  Encoding takes a tenth of the
+     * time of the kernels, so each launch is ready long before its predecessor ends. */
+    constexpr size_t kFirstLaunch = 4096, kLargestLaunch = 16384;
+    const size_t piece_systems = std::min<size_t>(128, std::max<size_t>(16, (run->num_systems + 63) / 64 + 15) / 16 * 16);
+    const size_t num_pieces = (run->num_systems + piece_systems - 1) / piece_systems;
     struct Piece {
         EncodedBatch enc;
-        std::vector<uint32_t> cost; /* per system: its main parts' instructions, weighted as the rollout machine executes them */
+        std::vector<uint32_t> cost; /* per system: its longest main part's instructions, weighted as the rollout machine executes them */
         SecantResult status = SECANT_SUCCESS;
     };
     struct Chunk {
-        std::vector<char> host;
+        std::vector<char> pageable; /* where no pinned memory is to be had */
         char* device = nullptr;
         bool pooled = false;
     };
     std::vector<Piece> pieces;
     std::vector<Chunk> chunks;
+    std::vector<size_t> bounds; /* the first piece of every launch, and the end */
     std::mutex mutex;
     std::condition_variable ready;
     std::vector<char> done;          /* piece encoded */
@@ -160,14 +337,18 @@ extern "C" SecantResult secant_b200_rk4_score(const SecantB200Rk4Run* given) {
     std::atomic<bool> stop{false};
     try {
         pieces.resize(num_pieces);
-        chunks.resize(num_chunks);
+        for (size_t at = 0, size = kFirstLaunch / piece_systems; at < num_pieces; at += size, size = std::min(2 * size, kLargestLaunch / piece_systems))
+            bounds.push_back(at);
+        bounds.push_back(num_pieces);
+        chunks.resize(bounds.size() - 1);
         done.assign(num_pieces, 0);
     } catch (const std::bad_alloc&) {
         return SECANT_ERROR_ALLOCATION_FAILED;
     }
+    const size_t num_chunks = chunks.size();
     auto piece_range = [&](size_t c, size_t* first, size_t* count) {
-        *first = c * kPieceSystems * S;
-        *count = std::min(kPieceSystems, run->num_systems - c * kPieceSystems) * S;
+        *first = c * piece_systems * S;
+        *count = std::min(piece_systems, run->num_systems - c * piece_systems) * S;
     };
     auto scan_one = [&](size_t c) {
         size_t first, count;
@@ -198,7 +379,7 @@ extern "C" SecantResult secant_b200_rk4_score(const SecantB200Rk4Run* given) {
                         const bool function = cs >= SB_CASE_UN && cs < SB_CASE_FMA && cs != SB_CASE_UN + SB_UN_NEG && cs != SB_CASE_UN + SB_UN_ABS;
                         cost += division || function ? 70u : 25u;
                     }
-                    piece.cost[i / S] += cost;
+                    piece.cost[i / S] = std::max(piece.cost[i / S], cost); /* a warp per state: the longest decides */
                 }
             }
         } catch (const std::bad_alloc&) {
@@ -229,15 +410,24 @@ extern "C" SecantResult secant_b200_rk4_score(const SecantB200Rk4Run* given) {
             encode_one(c);
         }
     };
-    std::vector<std::thread> workers;
     const unsigned hardware = std::thread::hardware_concurrency();
-    const size_t want_workers = std::min<size_t>(num_pieces > 1 ? num_pieces - 1 : 0, std::min<unsigned>(hardware ? hardware : 1u, 16u) - 1u);
-    try {
-        workers.reserve(want_workers);
-        for (size_t w = 0; w < want_workers; ++w) workers.emplace_back(worker);
-    } catch (const std::exception&) {
-        /* no memory or no thread to be had: fewer helpers, or none; the calling thread does whatever is left */
-    }
+    struct Help { /* whatever way the call ends, no helper is left on its locals */
+        Helpers::Job job;
+        std::function<void()> before;
+        ~Help() {
+            before();
+            helpers().finish(&job);
+        }
+    } help;
+    help.before = [&] {
+        {
+            std::lock_guard<std::mutex> lock(mutex);
+            stop.store(true);
+        }
+        ready.notify_all();
+    };
+    help.job.work = worker;
+    helpers().start(&help.job, std::min<size_t>(num_pieces - 1, (hardware ? hardware : 1u) - 1u));
     scan_pieces();
     {
         std::unique_lock<std::mutex> lock(mutex);
@@ -254,38 +444,27 @@ extern "C" SecantResult secant_b200_rk4_score(const SecantB200Rk4Run* given) {
                                      cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess)) {
         cudaGetLastError();
         result = SECANT_ERROR_DRIVER_FAILED;
-        {
-            std::lock_guard<std::mutex> lock(mutex);
-            stop.store(true);
-        }
-        ready.notify_all();
     }
-    if (result != SECANT_SUCCESS) {
-        for (std::thread& t : workers) t.join();
-        return result;
-    }
+    if (result != SECANT_SUCCESS) return result;
     const cudaMemPool_t pool = record_pool(device); /* null: plain allocations */
 
-    /* records travel on their own stream, so an upload never waits for the kernels of earlier chunks;
-     * the chunks' kernels go round the compute streams, so a chunk smaller than the GPU shares it
-     * with its neighbours */
-    constexpr int kComputeStreams = 8;
-    cudaStream_t compute[kComputeStreams] = {}, copies = nullptr;
-    const unsigned concurrent = (unsigned)std::min<size_t>(num_chunks, kComputeStreams);
-    cudaEvent_t uploaded = nullptr;
-    cudaError_t e = cudaStreamCreateWithFlags(&copies, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&uploaded, cudaEventDisableTiming);
+    /* records travel on their own stream, so an upload never waits for the kernels of earlier launches;
+     * these take turns on the compute streams */
+    const unsigned streams = (unsigned)std::min<size_t>(num_chunks, kComputeStreams);
+    cudaError_t e = cudaSuccess;
+    CallResources* const res = take_resources(device, &e);
+    if (!res) return e == cudaErrorMemoryAllocation ? SECANT_ERROR_ALLOCATION_FAILED : SECANT_ERROR_DRIVER_FAILED;
+    cudaStream_t const copies = res->copies;
+    cudaEvent_t const uploaded = res->uploaded;
     /* what the caller queued on the default stream before this call (fills, copies, an event wait)
      * comes first, as it did when the kernels themselves ran on that stream */
-    if (e == cudaSuccess) e = cudaEventRecord(uploaded, nullptr);
-    for (int i = 0; i < kComputeStreams && e == cudaSuccess; ++i) {
-        e = cudaStreamCreateWithFlags(&compute[i], cudaStreamNonBlocking);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(compute[i], uploaded, 0);
-    }
+    e = cudaEventRecord(uploaded, nullptr);
+    for (unsigned i = 0; i < streams && e == cudaSuccess; ++i) e = cudaStreamWaitEvent(res->compute[i], uploaded, 0);
     auto align256 = [](size_t v) { return (v + 255) / 256 * 256; };
     unsigned launches = 0;
+    size_t flag_offset = 0;
     for (size_t c = 0; c < num_chunks && e == cudaSuccess && result == SECANT_SUCCESS; ++c) {
-        const size_t piece0 = c * kPiecesPerLaunch, piece1 = std::min(num_pieces, piece0 + kPiecesPerLaunch);
+        const size_t piece0 = bounds[c], piece1 = bounds[c + 1];
         for (size_t q = piece0; q < piece1; ++q)
             for (;;) { /* wait for piece q; while it is in other hands, encode pieces nobody has taken */
                 {
@@ -320,15 +499,20 @@ extern "C" SecantResult secant_b200_rk4_score(const SecantB200Rk4Run* given) {
         const size_t o_aff = align256(o_patch + n_patches * sizeof(SbPatch));
         const size_t o_lit = align256(o_aff + n_affines * sizeof(SbAffine));
         const size_t o_flag = align256(o_lit + n_lits * sizeof(float) + 16); /* one word raised by the data validation */
+        if (c == 0) flag_offset = o_flag;
         const size_t o_order = o_flag + 256;
         const size_t total = align256(o_order + n_programs / S * sizeof(uint32_t));
-        try {
-            chunk.host.assign(total, 0);
-        } catch (const std::bad_alloc&) {
-            result = SECANT_ERROR_ALLOCATION_FAILED;
-            break;
+        char* host = staging_for(res, c, total);
+        if (!host) {
+            try {
+                chunk.pageable.resize(total);
+            } catch (const std::bad_alloc&) {
+                result = SECANT_ERROR_ALLOCATION_FAILED;
+                break;
+            }
+            host = chunk.pageable.data();
         }
-        char* host = chunk.host.data();
+        std::memset(host + o_flag, 0, o_order - o_flag); /* the flag and the queue's counter start from zero */
         {
             size_t at_program = 0, at_insn = 0, at_patch = 0, at_affine = 0, at_lit = 0;
             for (size_t q = piece0; q < piece1; ++q) {
@@ -373,10 +557,10 @@ extern "C" SecantResult secant_b200_rk4_score(const SecantB200Rk4Run* given) {
         char* d = chunk.device;
         e = cudaMemcpyAsync(d, host, total, cudaMemcpyHostToDevice, copies);
         if (e == cudaSuccess) e = cudaEventRecord(uploaded, copies);
-        cudaStream_t stream = compute[c % kComputeStreams];
+        cudaStream_t stream = res->compute[c % kComputeStreams];
         if (e == cudaSuccess) e = cudaStreamWaitEvent(stream, uploaded, 0);
         if (e != cudaSuccess) break;
-        const size_t first_system = piece0 * kPieceSystems;
+        const size_t first_system = piece0 * piece_systems;
         const size_t systems = n_programs / S;
         DeviceBatch db;
         std::memset(&db, 0, sizeof(db));
@@ -406,7 +590,6 @@ extern "C" SecantResult secant_b200_rk4_score(const SecantB200Rk4Run* given) {
         p.offsets = reinterpret_cast<const uint32_t*>(run->trajectory_offsets);
         p.total_points = (uint32_t)total_points;
         p.allow_missing = run->allow_missing_observations;
-        p.invalid_flag = reinterpret_cast<int*>(d + o_flag);
         p.queue = reinterpret_cast<unsigned long long*>(d + o_flag + 8); /* uploaded as zeros with the records */
         p.order = reinterpret_cast<const uint32_t*>(d + o_order);
         p.sampled = sampled ? reinterpret_cast<const SecantB200SampledParameter*>(run->sampled_parameters) + first_system * K : nullptr;
@@ -416,35 +599,34 @@ extern "C" SecantResult secant_b200_rk4_score(const SecantB200Rk4Run* given) {
         p.output = reinterpret_cast<float*>(run->output.address) + first_system * run->output.leading_dimension;
         p.output_ld = run->output.leading_dimension;
         p.integrated = reinterpret_cast<unsigned long long*>(run->integrated_intervals);
-        e = launch_rk4(db, p, (size_t)limit, concurrent, stream);
+        p.invalid_flag = reinterpret_cast<int*>(chunks[0].device + flag_offset); /* one scan of the data for all launches */
+        if (c == 0) {
+            e = launch_rk4_validation(p, stream);
+            ++launches;
+            if (e == cudaSuccess) e = cudaEventRecord(res->validated, stream);
+        } else if (c < streams) {
+            e = cudaStreamWaitEvent(stream, res->validated, 0);
+        }
+        if (e == cudaSuccess) e = launch_rk4(db, p, (size_t)limit, stream);
         if (e == cudaErrorInvalidConfiguration) { result = SECANT_ERROR_REGISTER_OVERFLOW; e = cudaSuccess; break; }
-        if (e == cudaSuccess) launches += 2;
+        if (e == cudaSuccess) ++launches;
     }
     stop.store(true);
-    for (std::thread& t : workers) t.join();
-    cudaStream_t all_streams[kComputeStreams + 1];
-    for (int i = 0; i < kComputeStreams; ++i) all_streams[i] = compute[i];
-    all_streams[kComputeStreams] = copies;
-    for (cudaStream_t q : all_streams) /* also on failure: nothing of this call stays in flight */
-        if (q) {
-            const cudaError_t f = cudaStreamSynchronize(q);
-            if (e == cudaSuccess) e = f;
-        }
+    helpers().finish(&help.job);
+    const cudaError_t launched = e;
+    for (unsigned i = 0; i <= streams; ++i) { /* also on failure: nothing of this call stays in flight */
+        const cudaError_t f = cudaStreamSynchronize(i < streams ? res->compute[i] : copies);
+        if (e == cudaSuccess) e = f;
+    }
     for (Chunk& chunk : chunks) /* every stream has been waited for: nothing reads the buffers any more */
         if (chunk.device) {
             const cudaError_t f = chunk.pooled ? cudaFreeAsync(chunk.device, copies) : cudaFree(chunk.device);
             if (e == cudaSuccess) e = f;
         }
-    if (copies) { /* the pool may hand the memory to the next call once the frees have been reached */
-        const cudaError_t f = cudaStreamSynchronize(copies);
+    {
+        const cudaError_t f = leave_resources(res, e == cudaSuccess && launched == cudaSuccess);
         if (e == cudaSuccess) e = f;
     }
-    if (uploaded) cudaEventDestroy(uploaded);
-    for (cudaStream_t q : all_streams)
-        if (q) {
-            const cudaError_t f = cudaStreamDestroy(q);
-            if (e == cudaSuccess) e = f;
-        }
     if (launches) note_kernel_launches(launches);
     if (result != SECANT_SUCCESS) return result;
     return e == cudaSuccess ? SECANT_SUCCESS : SECANT_ERROR_DRIVER_FAILED;

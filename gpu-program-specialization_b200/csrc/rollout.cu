@@ -9,16 +9,14 @@
  * sq = fma(err, err, sq).  Score = sq / residuals, or FLT_MAX when anything was not finite.
  *
  * Mapping (different from the reference, which gives a thread one configuration and loops all
- * trajectories inside it): one warp per (system, configuration), lanes = trajectories, RR per
+ * trajectories inside it): one warp per (system, configuration, state), lanes = trajectories, RR per
  * lane.  RR is chosen from the trajectory count so that a pass of 32 * RR trajectories keeps all
- * lanes busy: 1 up to 32 trajectories, 2 up to 64, 4 beyond.  The integrator's vectors live in
- * the warp's slots: slot s = stage state s (what COLUMN s of a right-hand side reads), then
- * next-stage, sum and state vectors (the state is not touched during a step, so it doubles as the
- * step's base).  A right-hand side is a flat record (record.h) whose operands are constants of
- * the program (CST) and slots (SLOT); the machine below knows only those two kinds, so its
- * dispatch is an operand fetch followed by a switch over the operation.
+ * lanes busy: 1 up to 32 trajectories, 2 up to 64, 4 beyond.  A right-hand side is a flat record
+ * (record.h) whose operands are constants of the program, stage values (what COLUMN s reads) and
+ * temporaries of the warp.
  */
 #include "evaluator.cuh"
+#include "pairs_ptx.cuh"
 #include "sbmath.cuh"
 
 #include <algorithm>
@@ -27,101 +25,21 @@ namespace sb {
 
 namespace {
 
+using sbm::f2;
+
 constexpr int kRolloutMaxWarps = 16;
 constexpr float kFltMax = 3.402823466e+38f;
 
-template <int RR>
-__device__ __forceinline__ void load_lanes(const float* p, float (&x)[RR]) {
-    if constexpr (RR == 4) {
-        const float4 v = *reinterpret_cast<const float4*>(p);
-        x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
-    } else if constexpr (RR == 2) {
-        const float2 v = *reinterpret_cast<const float2*>(p);
-        x[0] = v.x; x[1] = v.y;
-    } else {
-        x[0] = *p;
-    }
-}
-template <int RR>
-__device__ __forceinline__ void store_lanes(float* p, const float (&x)[RR]) {
-    if constexpr (RR == 4) *reinterpret_cast<float4*>(p) = make_float4(x[0], x[1], x[2], x[3]);
-    else if constexpr (RR == 2) *reinterpret_cast<float2*>(p) = make_float2(x[0], x[1]);
-    else *p = x[0];
-}
-
-/* One element through the same pieces as the four-element functions of sbmath.cuh (common-range
- * body, then the general version where the argument asks for it), so a value has the same bits
- * whichever width computed it.  The narrow machines call these instead of padding a four-element
- * call. */
-__device__ __noinline__ float unary1(float x, unsigned op) {
+/* Two elements behind one call, any argument: what the core leaves to others.  The whole warp is here. */
+__device__ __noinline__ f2 unary_pair(f2 v, unsigned op) {
     switch (op) {
-    case SB_UN_SIN: case SB_UN_COS: {
-        const int shift = op == SB_UN_COS ? 1 : 0;
-        return fabsf(x) < 4096.0f ? sbm::sincos_small(x, 0.5f * (float)shift) : sbm::sincos_any(x, shift);
-    }
-    case SB_UN_EXP: {
-        float r = sbm::exp_mid(x);
-        if (!(fabsf(x) <= 86.0f)) {
-            bool hard = false;
-            r = sbm::exp_repair(x, r, hard);
-            if (hard) r = sbm::exp_any(x);
-        }
-        return r;
-    }
-    case SB_UN_LOG: return sbm::log_is_special(x) ? sbm::log_any(x) : sbm::log_normal(x);
-    case SB_UN_EX2: return fabsf(x) <= 124.0f ? sbm::exp2_mid(x) : sbm::exp2f_(x);
-    case SB_UN_SQRT: return __fsqrt_rn(x);
-    case SB_UN_RCP: return __frcp_rn(x);
-    case SB_UN_RSQRT: return __frcp_rn(__fsqrt_rn(x));
-    case SB_UN_LG2: return log2f(x);
-    default: return tanhf(x);
+    case SB_UN_SIN: case SB_UN_COS: return sbm::sincos_pair(v, op == SB_UN_COS ? 1 : 0);
+    case SB_UN_EXP: return sbm::exp_pair(v);
+    case SB_UN_LOG: return sbm::log_pair(v);
+    default: return sbm::pack2(sbm::any1(sbm::lo2(v), op), sbm::any1(sbm::hi2(v), op));
     }
 }
-__device__ __noinline__ float div1(float a, float b) { return __fdiv_rn(a, b); }
-
-/* The same for two elements behind one call: their dependency chains interleave. */
-__device__ __noinline__ float2 unary2(float2 v, unsigned op) {
-    float2 o;
-    switch (op) {
-    case SB_UN_SIN: case SB_UN_COS: {
-        const int shift = op == SB_UN_COS ? 1 : 0;
-        const float half = 0.5f * (float)shift;
-        o.x = sbm::sincos_small(v.x, half); o.y = sbm::sincos_small(v.y, half);
-        if (!(fabsf(v.x) < 4096.0f && fabsf(v.y) < 4096.0f)) {
-            if (!(fabsf(v.x) < 4096.0f)) o.x = sbm::sincos_any(v.x, shift);
-            if (!(fabsf(v.y) < 4096.0f)) o.y = sbm::sincos_any(v.y, shift);
-        }
-        return o;
-    }
-    case SB_UN_EXP: {
-        o.x = sbm::exp_mid(v.x); o.y = sbm::exp_mid(v.y);
-        if (!(fabsf(v.x) <= 86.0f && fabsf(v.y) <= 86.0f)) {
-            bool hard = false;
-            o.x = sbm::exp_repair(v.x, o.x, hard); o.y = sbm::exp_repair(v.y, o.y, hard);
-            if (hard) {
-                if (fabsf(v.x) > 86.0f) o.x = sbm::exp_any(v.x);
-                if (fabsf(v.y) > 86.0f) o.y = sbm::exp_any(v.y);
-            }
-        }
-        return o;
-    }
-    case SB_UN_LOG:
-        o.x = sbm::log_normal(v.x); o.y = sbm::log_normal(v.y);
-        if (sbm::log_is_special(v.x)) o.x = sbm::log_any(v.x);
-        if (sbm::log_is_special(v.y)) o.y = sbm::log_any(v.y);
-        return o;
-    case SB_UN_EX2:
-        o.x = fabsf(v.x) <= 124.0f ? sbm::exp2_mid(v.x) : sbm::exp2f_(v.x);
-        o.y = fabsf(v.y) <= 124.0f ? sbm::exp2_mid(v.y) : sbm::exp2f_(v.y);
-        return o;
-    case SB_UN_SQRT: return make_float2(__fsqrt_rn(v.x), __fsqrt_rn(v.y));
-    case SB_UN_RCP: return make_float2(__frcp_rn(v.x), __frcp_rn(v.y));
-    case SB_UN_RSQRT: return make_float2(__frcp_rn(__fsqrt_rn(v.x)), __frcp_rn(__fsqrt_rn(v.y)));
-    case SB_UN_LG2: return make_float2(log2f(v.x), log2f(v.y));
-    default: return make_float2(tanhf(v.x), tanhf(v.y));
-    }
-}
-__device__ __noinline__ float2 div2(float2 a, float2 b) { return make_float2(__fdiv_rn(a.x, b.x), __fdiv_rn(a.y, b.y)); }
+__device__ __noinline__ f2 div_pair(f2 a, f2 b) { return sbm::pack2(sbm::div1(sbm::lo2(a), sbm::lo2(b)), sbm::div1(sbm::hi2(a), sbm::hi2(b))); }
 
 /* ---- shared memory by 32-bit shared-window address ------------------------------------------
  * The interpreter's operands, the integrator's vectors and the instruction stream itself are read
@@ -134,139 +52,222 @@ __device__ __forceinline__ void lds(uint32_t a, float (&x)[RR]) {
     else if constexpr (RR == 2) asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(x[0]), "=f"(x[1]) : "r"(a));
     else asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x[0]) : "r"(a));
 }
+__device__ __forceinline__ uint32_t lds_word(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
 template <int RR>
 __device__ __forceinline__ void sts(uint32_t a, const float (&x)[RR]) {
     if constexpr (RR == 4) asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(x[0]), "f"(x[1]), "f"(x[2]), "f"(x[3]) : "memory");
     else if constexpr (RR == 2) asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(a), "f"(x[0]), "f"(x[1]) : "memory");
     else asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(x[0]) : "memory");
 }
-__device__ __forceinline__ void lds_pair(uint32_t a, uint32_t& lo, uint32_t& hi) {
-    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(lo), "=r"(hi) : "r"(a));
-}
-__device__ __forceinline__ uint32_t lds_word(uint32_t a) {
-    uint32_t v;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
-    return v;
-}
 
 /* Handlers of the rollout machine.  A warp rewrites the main part of its private copy of a record
- * once per item into this form: word 0 = handler (bits 0..7) and, for H_UNARY, the function (bits
- * 8..15); word 1 = the operand's shared-window address, with bit 31 set when every lane reads its own
- * RR floats of a slot (the lane's offset is added) and clear when all lanes read one table entry.
- * H_STORE_LOAD (slot = acc, then acc = operand) carries the slot's address in bits 8..31 of word 0.
- * H_FMA keeps the record's form (operand kinds in bits 8..13 of word 0, three 10-bit indices in
- * word 1).  One item runs its right-hand sides states x 4 stages x steps times, so the rewrite is free
- * and the dispatch per instruction is an address add, one load and one dense switch. */
-enum { H_END = 0, H_STORE, H_LOAD, H_ADD, H_SUB, H_RSUB, H_MUL, H_DIV, H_RDIV, H_MIN, H_MAX, H_NEG, H_ABS, H_UNARY, H_STORE_LOAD, H_FMA };
-constexpr uint32_t kPerLane = 0x80000000u;
+ * once per item into this form: word 0 = the handler of the NEXT instruction (so that the indexed branch's
+ * table is read while this one works), word 1 = where the operand is (C: the shared address of a
+ * constant-table entry, one for all lanes; V: the offset of a state in the vector of stage values; T: the
+ * offset of one of the warp's temporaries) or, for the functions, SB_UN_*.  H_STLOAD (temporary = acc,
+ * then acc = operand) keeps the temporary's offset, in units of 128 bytes, above the operand's 18 bits.
+ * One item runs its right-hand sides 4 stages x steps times, so the rewrite is free.
+ *
+ * The machine is one block of PTX for the reasons given in eval_kernel.cuh, and here for one more: an
+ * item is one chain of dependent instructions, so what an interpreted instruction costs decides how long
+ * a call takes (two values per lane share it, where the population evaluator's sixteen do).  With the
+ * C++ machine it cost 50 issued instructions, of which dispatch was half; here it costs 22, the
+ * integrator's part included.  In a chain of them one takes 75 cycles for an addition with any operand,
+ * 110 for an exponential, 200 for a sine or a division (one warp alone on its SM). */
+enum { H_END = 0, H_LOAD = 1, H_STORE = 4, H_STLOAD = 5, H_ADD = 8, H_SUB = 11, H_RSUB = 14, H_MUL = 17, H_DIV = 20, H_RDIV = 23, /* + kind */
+       H_MIN = 26, H_MAX = 29, H_NEG = 32, H_ABS = 33, H_SIN = 34, H_COS, H_EXP, H_LOG, H_UNARY, H_FMA };
+enum { RK_CST = 0, RK_STATE = 1, RK_TEMP = 2 };
+constexpr uint32_t kStoredShift = 18, kStoredUnit = 128;
+
+/* the constants of the functions by pairs, read two at a time: moves would cost as much as the
+ * arithmetic of a single pair (pairs_ptx.cuh has the same numbers as text) */
+__constant__ __align__(16) unsigned long long kPairConstants[] = {
+    0x3EA2F9833EA2F983ull, 0x4B4000004B400000ull, 0xCB400000CB400000ull, 0xC0490FDBC0490FDBull, 0x33BBBD2E33BBBD2Eull, 0x27772CED27772CEDull,
+    0xB2CD31C1B2CD31C1ull, 0x3638B8243638B824ull, 0xB9500BECB9500BECull, 0x3C0888863C088886ull, 0xBE2AAAABBE2AAAABull, 0ull,
+    0x3FB8AA3B3FB8AA3Bull, 0x4B4000004B400000ull, 0x32A5706032A57060ull, 0ull,
+    0xCB400000CB400000ull, 0xBD9C5854BD9C5854ull, 0x3E02AC143E02AC14ull, 0xBE06C251BE06C251ull, 0x3E116D423E116D42ull, 0xBE2A392FBE2A392Full,
+    0x3E4CD0023E4CD002ull, 0xBE800113BE800113ull, 0x3EAAAAAA3EAAAAAAull, 0xBF000000BF000000ull, 0x35BFBE8E35BFBE8Eull, 0x3F3172003F317200ull};
+
+/* The block carries a whole observation interval: the instruction that ends a right-hand side goes on with
+ * the integrator's part of the stage (E0 to E3: sum += weight * rhs, the next stage's value of this
+ * warp's state from the step's base), meets the other warps of the item at their barrier and starts the
+ * next stage, until the interval's steps are done.
+ *
+ * asm operands: 0 the address of the next instruction, 1 the next handler and 2 word 1 of this
+ * instruction (at the end 1 says whether the interval is done, 0, or an instruction was left, 1), 3 and 4
+ * the accumulator (RR = 1: both halves of 3 hold the value), 5 and 6 the stage sum, 7 and 8 the state (base of the step), 9 and 10 the addresses of this stage's values and of the next
+ * stage's for this lane, 11 the stage, 12 the steps left; 13 the address of the temporaries for this lane,
+ * 14 the pair (-1, -1), 15 the constants, 16 to 21 h / 2, h and h / 6, 22 the first instruction, 23 the
+ * offset of this warp's state, 24 and 25 the barrier and its threads (0: no barrier), 26 the first handler. */
+#define RK_NEXT "mov.u32 hb, %1;\n ld.shared.v2.u32 {%1, %2}, [%0];\n add.u32 %0, %0, 8;\n"
+#define RK_GO "brx.idx.uni hb, targets;\n"
+#define RK_FETCH_1(A) "ld.shared.b32 c0, [" A "];\n mov.b64 x0, {c0, c0};\n"
+#define RK_FETCH_2(A) "ld.shared.b64 x0, [" A "];\n"
+#define RK_FETCH_4(A) "ld.shared.v2.b64 {x0, x1}, [" A "];\n"
+#define RK_KEEP_1(A, P, Q) "mov.b64 {c0, c1}, " P ";\n st.shared.b32 [" A "], c0;\n"
+#define RK_KEEP_2(A, P, Q) "st.shared.b64 [" A "], " P ";\n"
+#define RK_KEEP_4(A, P, Q) "st.shared.v2.b64 [" A "], {" P ", " Q "};\n"
+#define RK_BOTH_1(F) F("%3", "x0")
+#define RK_BOTH_2(F) F("%3", "x0")
+#define RK_BOTH_4(F) F("%3", "x0") F("%4", "x1")
+#define RK_EACH_1(F) F("%3")
+#define RK_EACH_2(F) F("%3")
+#define RK_EACH_4(F) F("%3") F("%4")
+#define RK_EACHX_1(F) F("x0")
+#define RK_EACHX_2(F) F("x0")
+#define RK_EACHX_4(F) F("x0") F("x1")
+#define RK_MOV(A, X) "mov.b64 " A ", " X ";\n"
+#define RK_ADD(A, X) "add.rn.f32x2 " A ", " A ", " X ";\n"
+#define RK_SUB(A, X) "fma.rn.f32x2 " A ", " X ", mone, " A ";\n"
+#define RK_RSUB(A, X) "fma.rn.f32x2 " A ", " A ", mone, " X ";\n"
+#define RK_MUL(A, X) "mul.rn.f32x2 " A ", " A ", " X ";\n"
+#define RK_MIN(A, X) "mov.b64 {f0, f1}, " A ";\n mov.b64 {top, low}, " X ";\n min.f32 f0, f0, top;\n min.f32 f1, f1, low;\n mov.b64 " A ", {f0, f1};\n"
+#define RK_MAX(A, X) "mov.b64 {f0, f1}, " A ";\n mov.b64 {top, low}, " X ";\n max.f32 f0, f0, top;\n max.f32 f1, f1, low;\n mov.b64 " A ", {f0, f1};\n"
+#define RK_NEG(A) "xor.b64 " A ", " A ", 0x8000000080000000;\n"
+#define RK_ABS(A) "and.b64 " A ", " A ", 0x7fffffff7fffffff;\n"
+#define RK_SWAP(A, X) "mov.b64 m, " A ";\n mov.b64 " A ", " X ";\n mov.b64 " X ", m;\n"
+/* an operation with a constant (label NAME C), a state (NAME V) and a temporary (NAME T) */
+#define RK_THREE(N, NAME, F)                                                                            \
+    NAME "C:\n" RK_FETCH_##N("%2") RK_NEXT RK_BOTH_##N(F) RK_GO                                          \
+    NAME "V:\n add.u32 ad, %2, %9;\n" RK_FETCH_##N("ad") RK_NEXT RK_BOTH_##N(F) RK_GO                    \
+    NAME "T:\n add.u32 ad, %2, %13;\n" RK_FETCH_##N("ad") RK_NEXT RK_BOTH_##N(F) RK_GO
+#define RK_STLOAD(N, NAME, BASE)                                                                        \
+    NAME ":\n shr.u32 c2, %2, 18;\n shl.b32 c2, c2, 7;\n add.u32 c2, c2, %13;\n" RK_KEEP_##N("c2", "%3", "%4")       \
+    "and.b32 ad, %2, 0x3ffff;\n" BASE RK_FETCH_##N("ad") RK_NEXT RK_BOTH_##N(RK_MOV) RK_GO
+#define RK_FETCH_THEN(N, NAME, WHERE)                                                                   \
+    NAME "C:\n" RK_FETCH_##N("%2") "bra.uni " WHERE ";\n"                                               \
+    NAME "V:\n add.u32 ad, %2, %9;\n" RK_FETCH_##N("ad") "bra.uni " WHERE ";\n"                         \
+    NAME "T:\n add.u32 ad, %2, %13;\n" RK_FETCH_##N("ad") "bra.uni " WHERE ";\n"
+#define RK_K2(A, B, OFF) "ld.const.v2.u64 {" A ", " B "}, [%15+" OFF "];\n"
+#define RK_CORE(N)                                                                                      \
+    "{\n" SB_PTX_REGISTERS ".reg .b64 x0, x1;\n .reg .pred meet;\n .reg .u32 hb;\n"                                                        \
+    "stages: .branchtargets E0, E1, E2, E3;\n targets: .branchtargets EN, LC, LV, LT, ST, KC, KV, KT, AC, AV, AT, SC, SV, STT, RC, RV, RT, MC, MV, MT, DC, DV, DT, QC, QV, QT, " \
+    "NC, NV, NT, XC, XV, XT, NG, AB, SI, CO, EX, LG, LEAVE, LEAVE;\n mov.b64 mone, %14;\n setp.ne.u32 meet, %25, 0;\n"               \
+    "ld.shared.u32 %1, [%0+-8];\n" RK_NEXT RK_GO                                                         \
+    RK_THREE(N, "L", RK_MOV) RK_THREE(N, "A", RK_ADD) RK_THREE(N, "R", RK_RSUB)                         \
+    "SC:\n" RK_FETCH_##N("%2") RK_NEXT RK_BOTH_##N(RK_SUB) RK_GO                                         \
+    "SV:\n add.u32 ad, %2, %9;\n" RK_FETCH_##N("ad") RK_NEXT RK_BOTH_##N(RK_SUB) RK_GO                   \
+    "STT:\n add.u32 ad, %2, %13;\n" RK_FETCH_##N("ad") RK_NEXT RK_BOTH_##N(RK_SUB) RK_GO                  \
+    RK_THREE(N, "M", RK_MUL) RK_THREE(N, "N", RK_MIN) RK_THREE(N, "X", RK_MAX)                          \
+    "ST:\n add.u32 ad, %2, %13;\n" RK_NEXT RK_KEEP_##N("ad", "%3", "%4") RK_GO                                       \
+    RK_STLOAD(N, "KC", "") RK_STLOAD(N, "KV", "add.u32 ad, ad, %9;\n") RK_STLOAD(N, "KT", "add.u32 ad, ad, %13;\n") \
+    "NG:\n" RK_NEXT RK_EACH_##N(RK_NEG) RK_GO "AB:\n" RK_NEXT RK_EACH_##N(RK_ABS) RK_GO                  \
+    "CO:\n" SB_COS_SHIFT "bra.uni SC0;\n SI:\n" SB_SIN_SHIFT                                            \
+    "SC0:\n" RK_K2("k0", "k1", "0") RK_K2("k2", "k3", "16") RK_K2("k4", "k5", "32") RK_K2("k6", "k7", "48") RK_K2("k8", "k9", "64") \
+    RK_K2("k10", "m", "80") "mov.f32 top, 0f00000000;\n" RK_EACH_##N(SB_TOP) "setp.lt.f32 p, top, 0f45800000;\n" SB_ALL_OR_LEAVE RK_NEXT \
+    RK_EACH_##N(SB_SIN_PAIR) RK_GO                                                                      \
+    "EX:\n" RK_K2("k0", "k1", "96") RK_K2("k2", "m", "112") "mov.f32 top, 0f00000000;\n" RK_EACH_##N(SB_TOP) \
+    "setp.le.f32 p, top, 0f42AC0000;\n" SB_ALL_OR_LEAVE RK_NEXT RK_EACH_##N(SB_EXP_PAIR) RK_GO          \
+    "LG:\n" RK_K2("k0", "k1", "128") RK_K2("k2", "k3", "144") RK_K2("k4", "k5", "160") RK_K2("k6", "k7", "176") RK_K2("k8", "k9", "192") \
+    RK_K2("k10", "k11", "208") "mov.f32 top, 0f00000000;\n mov.f32 low, 0f7F800000;\n" RK_EACH_##N(SB_TOP) RK_EACH_##N(SB_LOW) \
+    "setp.lt.f32 p, top, 0f7F800000;\n setp.ge.and.f32 p, low, 0f00800000, p;\n" SB_ALL_OR_LEAVE RK_NEXT RK_EACH_##N(SB_LOG_PAIR) RK_GO \
+    RK_FETCH_THEN(N, "D", "DIV") RK_FETCH_THEN(N, "Q", "RDIV")                                          \
+    /* operand / acc; what leaves for an unusual argument takes the accumulator along as it was */      \
+    "RDIV:\n mov.u32 c2, 0xffffffff;\n mov.f32 top, 0f00000000;\n mov.f32 low, 0f7F800000;\n" RK_EACHX_##N(SB_LEAST) \
+    RK_EACH_##N(SB_TOP) RK_EACHX_##N(SB_TOP) RK_EACH_##N(SB_LOW_ABS) SB_DIV_RANGE SB_ALL_OR_LEAVE       \
+    RK_BOTH_##N(RK_SWAP) "bra.uni DW;\n"                                                                \
+    "DIV:\n mov.u32 c2, 0xffffffff;\n mov.f32 top, 0f00000000;\n mov.f32 low, 0f7F800000;\n" RK_EACH_##N(SB_LEAST) \
+    RK_EACH_##N(SB_TOP) RK_EACHX_##N(SB_TOP) RK_EACHX_##N(SB_LOW_ABS) SB_DIV_RANGE SB_ALL_OR_LEAVE      \
+    "DW:\n" RK_NEXT SB_DIV_CONSTANTS RK_BOTH_##N(SB_DIV_PAIR) RK_GO                                      \
+    "EN:\n brx.idx.uni %11, stages;\n"                                                                   \
+    "E0:\n mov.b64 k0, 0;\n" RK_STAGE_##N(RK_FIRST, "%16", "%17") "bra.uni SWAP;\n"                    \
+    "E1:\n mov.b64 k0, 0x4000000040000000;\n" RK_STAGE_##N(RK_TWICE, "%16", "%17") "bra.uni SWAP;\n"   \
+    "E2:\n mov.b64 k0, 0x4000000040000000;\n" RK_STAGE_##N(RK_TWICE, "%18", "%19") "bra.uni SWAP;\n"   \
+    "E3:\n" RK_LAST_##N "add.u32 ad, %10, %23;\n" RK_KEEP_##N("ad", "%7", "%8")                         \
+    "mov.u32 c0, %9;\n mov.u32 %9, %10;\n mov.u32 %10, c0;\n mov.u32 %11, 0;\n mov.u32 %0, %22;\n"    \
+    "sub.u32 %12, %12, 1;\n setp.eq.u32 p, %12, 0;\n @p bra.uni DONE;\n bra.uni MEET;\n"              \
+    "SWAP:\n add.u32 ad, %10, %23;\n" RK_KEEP_##N("ad", "x0", "x1")                                     \
+    "mov.u32 c0, %9;\n mov.u32 %9, %10;\n mov.u32 %10, c0;\n add.u32 %11, %11, 1;\n mov.u32 %0, %22;\n" \
+    "MEET:\n mov.u32 %1, %26;\n" RK_NEXT "@meet barrier.cta.sync %24, %25;\n" RK_GO                                          \
+    "DONE:\n mov.u32 %1, 0;\n bra.uni OUT;\n LEAVE:\n mov.u32 %1, 1;\n OUT:\n }"
+/* the weights of the stages are 1, 2, 2, 1; the first sum is rhs + 0, as fma(1, rhs, 0) rounds */
+#define RK_FIRST(SUM, A) "add.rn.f32x2 " SUM ", " A ", k0;\n"
+#define RK_TWICE(SUM, A) "fma.rn.f32x2 " SUM ", " A ", k0, " SUM ";\n"
+#define RK_STAGE_1(SUM, H0, H1) SUM("%5", "%3") "fma.rn.f32x2 x0, " H0 ", %3, %7;\n"
+#define RK_STAGE_2(SUM, H0, H1) RK_STAGE_1(SUM, H0, H1)
+#define RK_STAGE_4(SUM, H0, H1) RK_STAGE_1(SUM, H0, H1) SUM("%6", "%4") "fma.rn.f32x2 x1, " H1 ", %4, %8;\n"
+#define RK_LAST_1 "add.rn.f32x2 %5, %3, %5;\n fma.rn.f32x2 %7, %20, %5, %7;\n"
+#define RK_LAST_2 RK_LAST_1
+#define RK_LAST_4 RK_LAST_1 "add.rn.f32x2 %6, %4, %6;\n fma.rn.f32x2 %8, %21, %6, %8;\n"
 
 template <int RR>
 struct Rollout {
-    float acc[RR];
-    uint32_t lane_off; /* byte offset of this lane's RR floats inside a slot */
-    uint32_t slot0;    /* shared address of slot 0; slot s lies s * 32 * RR floats further */
+    uint32_t temps; /* shared address of this lane's part of the warp's first temporary; the next lie 32 * RR floats further each */
 
-    __device__ __forceinline__ uint32_t slot_address(uint32_t s) const { return slot0 + s * (uint32_t)(RR * 128) + lane_off; }
-    __device__ __forceinline__ void get(uint32_t s, float (&x)[RR]) const { lds<RR>(slot_address(s), x); }
-    __device__ __forceinline__ void put(uint32_t s, const float (&x)[RR]) const { sts<RR>(slot_address(s), x); }
+    /* What stays the same for a warp while it integrates an item. */
+    struct Item {
+        uint32_t start, first;     /* shared address of the rewritten main part; its first handler */
+        uint32_t own;              /* offset of this warp's state in the vector of stage values */
+        uint32_t barrier, threads; /* of the item's warps; threads = 0: one warp, no barrier */
+        uint32_t program, first_temp, table; /* the record's number; its first temporary slot; its constant table (RR copies of every entry) */
+    };
+    static __device__ __forceinline__ f2 pair(const float (&v)[RR], int i) { return sbm::pack2(v[RR > 2 ? 2 * i : 0], v[RR > 2 ? 2 * i + 1 : RR - 1]); }
 
-    __device__ __forceinline__ void apply_unary(unsigned op) {
-        if constexpr (RR == 4) {
-            const float4 o = sbm::unary4(make_float4(acc[0], acc[1], acc[2], acc[3]), op);
-            acc[0] = o.x; acc[1] = o.y; acc[2] = o.z; acc[3] = o.w;
-        } else if constexpr (RR == 2) {
-            const float2 o = unary2(make_float2(acc[0], acc[1]), op);
-            acc[0] = o.x; acc[1] = o.y;
-        } else {
-            acc[0] = unary1(acc[0], op);
-        }
-    }
-    /* acc = a / b */
-    __device__ __forceinline__ void divide(const float (&a)[RR], const float (&b)[RR]) {
-        if constexpr (RR == 4) {
-            const float4 o = sbm::div4(make_float4(a[0], a[1], a[2], a[3]), make_float4(b[0], b[1], b[2], b[3]));
-            acc[0] = o.x; acc[1] = o.y; acc[2] = o.z; acc[3] = o.w;
-        } else if constexpr (RR == 2) {
-            const float2 o = div2(make_float2(a[0], a[1]), make_float2(b[0], b[1]));
-            acc[0] = o.x; acc[1] = o.y;
-        } else {
-            acc[0] = div1(a[0], b[0]);
-        }
-    }
-
-    /* acc = value of the rewritten main part: `count` instructions (the closing END not counted)
-     * starting at shared address `ip`; `table` is the shared address of the program's constant
-     * table (RR copies of every entry) */
-    __device__ __forceinline__ void run(uint32_t ip, uint32_t count, uint32_t table) {
-        uint32_t n0, n1;
-        lds_pair(ip, n0, n1); /* the record ends with END and one padding entry, so reading ahead is safe */
-        ip += 8;
+    /* Integrates `steps` steps of this warp's state, whose base is `state`; now and other are the shared
+     * addresses of the two vectors of stage values for this lane, and at the end `now` holds the new states
+     * of all warps that have come this far. */
+    __device__ __forceinline__ void interval(const Item& item, const DeviceBatch& batch, uint32_t steps, float (&state)[RR], const float (&half)[RR],
+                                             const float (&h)[RR], const float (&sixth)[RR], uint32_t& now, uint32_t& other) {
+        constexpr int W = RR > 2 ? 1 : 0; /* the second pair, where there is one */
+        f2 a0 = 0ull, a1 = 0ull, sum0 = 0ull, sum1 = 0ull, st0 = pair(state, 0), st1 = pair(state, W);
+        uint32_t ip = item.start, stage = 0u, handler, w;
+#define RK_RUN(N)                                                                                                          \
+        asm volatile(RK_CORE(N)                                                                                            \
+                     : "+r"(ip), "=&r"(handler), "=&r"(w), "+l"(a0), "+l"(a1), "+l"(sum0), "+l"(sum1), "+l"(st0), "+l"(st1), "+r"(now), "+r"(other), \
+                       "+r"(stage), "+r"(steps)                                                                             \
+                     : "r"(temps), "l"(sbm::both2(-1.0f)), "l"(__cvta_generic_to_constant(kPairConstants)), "l"(pair(half, 0)), "l"(pair(half, W)), \
+                       "l"(pair(h, 0)), "l"(pair(h, W)), "l"(pair(sixth, 0)), "l"(pair(sixth, W)), "r"(item.start), "r"(item.own),         \
+                       "r"(item.barrier), "r"(item.threads), "r"(item.first)                                                                 \
+                     : "memory")
 #pragma unroll 1
-        for (; count; --count) {
-            const uint32_t w0 = n0, w1 = n1;
-            lds_pair(ip, n0, n1);
-            ip += 8;
-            const unsigned handler = w0 & 0xffu;
-            float x[RR];
-            if (handler != H_FMA) lds<RR>((w1 & 0x00ffffffu) + ((uint32_t)((int32_t)w1 >> 31) & lane_off), x);
-            if (handler == H_MUL) {
-#pragma unroll
-                for (int q = 0; q < RR; ++q) acc[q] = __fmul_rn(acc[q], x[q]);
-                continue;
-            }
-            if (handler == H_ADD) {
-#pragma unroll
-                for (int q = 0; q < RR; ++q) acc[q] = __fadd_rn(acc[q], x[q]);
-                continue;
-            }
-            if (handler == H_LOAD) {
-#pragma unroll
-                for (int q = 0; q < RR; ++q) acc[q] = x[q];
-                continue;
-            }
-            if (handler == H_STORE_LOAD) {
-                sts<RR>((w0 >> 8) + lane_off, acc);
-#pragma unroll
-                for (int q = 0; q < RR; ++q) acc[q] = x[q];
-                continue;
-            }
-            switch (handler) {
-            case H_STORE: sts<RR>((w1 & 0x00ffffffu) + lane_off, acc); break;
-            case H_SUB:
-#pragma unroll
-                for (int q = 0; q < RR; ++q) acc[q] = __fsub_rn(acc[q], x[q]);
-                break;
-            case H_RSUB:
-#pragma unroll
-                for (int q = 0; q < RR; ++q) acc[q] = __fsub_rn(x[q], acc[q]);
-                break;
-            case H_DIV: divide(acc, x); break;
-            case H_RDIV: divide(x, acc); break;
-            case H_MIN:
-#pragma unroll
-                for (int q = 0; q < RR; ++q) acc[q] = fminf(acc[q], x[q]);
-                break;
-            case H_MAX:
-#pragma unroll
-                for (int q = 0; q < RR; ++q) acc[q] = fmaxf(acc[q], x[q]);
-                break;
-            case H_NEG:
-#pragma unroll
-                for (int q = 0; q < RR; ++q) acc[q] = -acc[q];
-                break;
-            case H_ABS:
-#pragma unroll
-                for (int q = 0; q < RR; ++q) acc[q] = fabsf(acc[q]);
-                break;
-            case H_UNARY: apply_unary((w0 >> 8) & 0xffu); break;
-            case H_FMA: fused(w0, w1, table); break;
-            default: break; /* H_END inside the counted range: unreachable for records produced by the encoder */
-            }
+        for (;;) {
+            if constexpr (RR == 1) RK_RUN(1);
+            else if constexpr (RR == 2) RK_RUN(2);
+            else RK_RUN(4);
+            if (handler == 0u) break;
+            handler = lds_word(ip - 16u); /* of the instruction the core stopped at */
+            slow(a0, a1, handler, w, now, batch, item.program, item.first_temp, (ip - item.start) / (uint32_t)sizeof(SbInsn) - 1u, item.table);
         }
+#undef RK_RUN
+        state[0] = sbm::lo2(st0);
+        if constexpr (RR > 1) state[1] = sbm::hi2(st0);
+        if constexpr (RR > 2) { state[2] = sbm::lo2(st1); state[3] = sbm::hi2(st1); }
+    }
+    /* what the core leaves to others: unusual arguments, the rarer functions, fused multiply-adds */
+    __device__ __forceinline__ void slow(f2& a0, f2& a1, uint32_t h, uint32_t w, uint32_t states, const DeviceBatch& batch, uint32_t program,
+                                         uint32_t first_temp, uint32_t at, uint32_t table) {
+        if (h == H_FMA) { /* its three operands need the record's own words */
+            const SbProgram* const pr = batch.programs + program;
+            const SbInsn ins = batch.insns[pr->insn_off + pr->main_off + at];
+            float acc[RR];
+            acc[0] = sbm::lo2(a0);
+            if constexpr (RR > 1) acc[1] = sbm::hi2(a0);
+            if constexpr (RR > 2) { acc[2] = sbm::lo2(a1); acc[3] = sbm::hi2(a1); }
+            fused(acc, ins.w0, ins.w1, states, first_temp, table);
+            a0 = pair(acc, 0);
+            a1 = pair(acc, RR > 2 ? 1 : 0);
+            return;
+        }
+        if (h >= H_SIN) {
+            a0 = unary_pair(a0, w);
+            if constexpr (RR > 2) a1 = unary_pair(a1, w);
+            return;
+        }
+        const uint32_t kind = (h - H_DIV) % 3u;
+        float x[RR];
+        lds<RR>(w + (kind == RK_STATE ? states : kind == RK_TEMP ? temps : 0u), x);
+        const f2 x0 = pair(x, 0), x1 = pair(x, RR > 2 ? 1 : 0);
+        const bool reverse = h >= H_RDIV;
+        a0 = reverse ? div_pair(x0, a0) : div_pair(a0, x0);
+        if constexpr (RR > 2) a1 = reverse ? div_pair(x1, a1) : div_pair(a1, x1);
     }
 
     /* FMA_F32 over three operands of any kind (table entry, slot, or the accumulator) */
-    __device__ __forceinline__ void fused(uint32_t w0, uint32_t w1, uint32_t table) {
+    __device__ __forceinline__ void fused(float (&acc)[RR], uint32_t w0, uint32_t w1, uint32_t states, uint32_t first_temp, uint32_t table) {
         const unsigned kinds = (w0 >> 8) & 0x3fu;
         float v[3][RR];
 #pragma unroll
@@ -277,37 +278,42 @@ struct Rollout {
 #pragma unroll
                 for (int q = 0; q < RR; ++q) v[i][q] = acc[q];
             } else if (kind == SB_KIND_CST) lds<RR>(table + index * (uint32_t)(RR * 4), v[i]);
-            else get(index, v[i]);
+            else lds<RR>(index < first_temp ? states + index * (uint32_t)(RR * 128) : temps + (index - first_temp) * (uint32_t)(RR * 128), v[i]);
         }
 #pragma unroll
         for (int q = 0; q < RR; ++q) acc[q] = __fmaf_rn(v[0][q], v[1][q], v[2][q]);
     }
 };
 
-/* Rewrites instruction `in` of a record's main part for the machine above. */
+/* Rewrites instruction `in` of a record's main part for the machine above; `table` is the shared address
+ * of the record's constant table, `first_temp` the first slot that is a temporary (the ones before it are
+ * the states). */
 template <int RR>
-__device__ __forceinline__ SbInsn rewritten(SbInsn in, uint32_t table, uint32_t slot0) {
+__device__ __forceinline__ SbInsn rewritten(SbInsn in, uint32_t table, uint32_t first_temp) {
     const unsigned cs = in.w0 & 0xffu;
     const uint32_t idx = in.w0 >> 16;
-    unsigned handler = H_END, aux = 0, kind = SB_NUM_KINDS; /* SB_NUM_KINDS: no operand */
-    if (cs >= SB_CASE_LOAD && cs < SB_CASE_STORE) { handler = H_LOAD; kind = cs - SB_CASE_LOAD; }
-    else if (cs == SB_CASE_STORE && (in.w1 & SB_STORE_THEN_LOAD)) {
-        const unsigned loaded = (in.w1 >> 16) & 3u;
-        const uint32_t from = in.w1 & 0xffffu;
-        if (loaded == SB_KIND_ROW) return SbInsn{H_END, table};
-        const uint32_t operand = loaded == SB_KIND_CST ? table + from * (uint32_t)(RR * 4) : ((slot0 + from * (uint32_t)(RR * 128)) | kPerLane);
-        return SbInsn{H_STORE_LOAD | ((slot0 + idx * (uint32_t)(RR * 128)) << 8), operand};
-    } else if (cs == SB_CASE_STORE) { handler = H_STORE; kind = SB_KIND_SLOT; }
-    else if (cs >= SB_CASE_BIN && cs < SB_CASE_UN) { handler = H_ADD + (cs - SB_CASE_BIN) / SB_NUM_KINDS; kind = (cs - SB_CASE_BIN) % SB_NUM_KINDS; }
-    else if (cs >= SB_CASE_UN && cs < SB_CASE_FMA) {
-        aux = cs - SB_CASE_UN;
-        handler = aux == SB_UN_NEG ? H_NEG : aux == SB_UN_ABS ? H_ABS : H_UNARY;
-    } else if (cs == SB_CASE_FMA) return SbInsn{(in.w0 & 0xffffff00u) | H_FMA, in.w1};
-    if (kind == SB_KIND_ROW) handler = H_END; /* rollout records have no per-row operands */
-    uint32_t operand = table; /* instructions without an operand read (and ignore) the table's first entry */
-    if (kind == SB_KIND_CST) operand = table + idx * (uint32_t)(RR * 4);
-    if (kind == SB_KIND_SLOT) operand = (slot0 + idx * (uint32_t)(RR * 128)) | kPerLane;
-    return SbInsn{handler | (aux << 8), operand};
+    const auto made = [&](unsigned handler, unsigned kind, uint32_t i) {
+        if (kind == SB_KIND_CST) return SbInsn{handler + RK_CST, table + i * (uint32_t)(RR * 4)};
+        if (i < first_temp) return SbInsn{handler + RK_STATE, i * (uint32_t)(RR * 128)};
+        return SbInsn{handler + RK_TEMP, (i - first_temp) * (uint32_t)(RR * 128)};
+    };
+    if (cs >= SB_CASE_LOAD && cs < SB_CASE_STORE) return made(H_LOAD, cs - SB_CASE_LOAD, idx);
+    if (cs == SB_CASE_STORE && (in.w1 & SB_STORE_THEN_LOAD)) {
+        SbInsn both = made(H_STLOAD, (in.w1 >> 16) & 3u, in.w1 & 0xffffu);
+        both.w1 |= ((idx - first_temp) * (RR * 128u / kStoredUnit)) << kStoredShift;
+        return both;
+    }
+    if (cs == SB_CASE_STORE) return SbInsn{H_STORE, (idx - first_temp) * (uint32_t)(RR * 128)};
+    if (cs >= SB_CASE_BIN && cs < SB_CASE_UN) /* in the record's order of operations */
+        return made(H_ADD + 3u * ((cs - SB_CASE_BIN) / SB_NUM_KINDS), (cs - SB_CASE_BIN) % SB_NUM_KINDS, idx);
+    if (cs >= SB_CASE_UN && cs < SB_CASE_FMA) {
+        const unsigned un = cs - SB_CASE_UN;
+        const unsigned h = un == SB_UN_NEG ? H_NEG : un == SB_UN_ABS ? H_ABS : un == SB_UN_SIN ? H_SIN : un == SB_UN_COS ? H_COS
+                         : un == SB_UN_EXP ? H_EXP : un == SB_UN_LOG ? H_LOG : H_UNARY;
+        return SbInsn{h, un};
+    }
+    if (cs == SB_CASE_FMA) return SbInsn{H_FMA, 0u};
+    return SbInsn{H_END, 0u};
 }
 
 /* The bank part of a record (record.h): sub-expressions that depend on the candidate's constants
@@ -339,14 +345,14 @@ __device__ __noinline__ void rollout_bank_part(const SbInsn* code, const float* 
             case SB_BIN_SUB: acc = __fsub_rn(acc, x); break;
             case SB_BIN_RSUB: acc = __fsub_rn(x, acc); break;
             case SB_BIN_MUL: acc = __fmul_rn(acc, x); break;
-            case SB_BIN_DIV: acc = div1(acc, x); break;
-            case SB_BIN_RDIV: acc = div1(x, acc); break;
+            case SB_BIN_DIV: acc = __fdiv_rn(acc, x); break;
+            case SB_BIN_RDIV: acc = __fdiv_rn(x, acc); break;
             case SB_BIN_MIN: acc = fminf(acc, x); break;
             default: acc = fmaxf(acc, x); break;
             }
         } else if (cs < SB_CASE_FMA) {
             const unsigned op = cs - SB_CASE_UN;
-            acc = op == SB_UN_NEG ? -acc : op == SB_UN_ABS ? fabsf(acc) : unary1(acc, op);
+            acc = op == SB_UN_NEG ? -acc : op == SB_UN_ABS ? fabsf(acc) : sbm::any1(acc, op);
         } else {
             const unsigned kinds = (ins.w0 >> 8) & 0x3fu;
             float v[3];
@@ -372,222 +378,233 @@ __device__ __forceinline__ float sampled_constant(const Rk4Problem& prob, unsign
     return fminf(p.upper, fmaxf(p.lower, value));
 }
 
-/* Shared memory of one warp, in this order: per state the record (exec_bytes) and the constant
- * table (table_bytes); then one area for the source constants of the record being set up and the
- * bank part's temporaries (source_bytes), the main parts' start addresses (16 words), the slots. */
+/* h / 6 rounded to nearest, for h >= 0: the quotient's estimate and one correction (Markstein) give the
+ * rounded quotient for every significand (checked for all 2^24), as long as nothing underflows. */
+__device__ __forceinline__ float sixth_of(float h) {
+    if (h != 0.0f && !(h > 1e-30f)) return h / 6.0f;
+    const float c = 1.0f / 6.0f, q = __fmul_rn(h, c);
+    return __fmaf_rn(__fmaf_rn(-6.0f, q, h), c, q);
+}
+
+/* Shared memory of one group (the S warps of an item): the two vectors of stage values, S states each,
+ * and one word for the item's number; then per warp the record of its right-hand side (exec_bytes), its
+ * constant table (table_bytes), its source constants and bank-part temporaries (source_bytes), its
+ * temporaries (temp_bytes). */
 struct RolloutLayout {
-    uint32_t exec_bytes, table_bytes, source_bytes, warp_bytes;
+    uint32_t exec_bytes, table_bytes, source_bytes, temp_bytes, warp_bytes, group_bytes;
 };
 
+/* The S warps of a group meet at a named barrier of their own; a group of one warp needs none. */
+__device__ __forceinline__ void group_sync(uint32_t barrier, uint32_t threads) {
+    if (threads == 32u) __syncwarp();
+    else asm volatile("barrier.cta.sync %0, %1;" ::"r"(barrier), "r"(threads) : "memory");
+}
+__device__ __forceinline__ bool group_all(uint32_t barrier, uint32_t threads, bool ok) { /* also a barrier */
+    if (threads == 32u) return __all_sync(0xffffffffu, ok);
+    uint32_t all;
+    asm volatile("{ .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n barrier.cta.red.and.pred q, %2, %3, p;\n selp.u32 %0, 1, 0, q;\n }"
+                 : "=r"(all) : "r"((uint32_t)ok), "r"(barrier), "r"(threads) : "memory");
+    return all != 0u;
+}
+
+/* An item (system, configuration) is integrated by S warps, one per state: the right-hand sides of a stage
+ * are independent, so the chain of dependent instructions that decides how long an item takes is that of
+ * the longest right-hand side and not that of all of them.  A warp keeps its own state, stage sum and step
+ * sizes in registers; the stage values are in shared memory twice, so one barrier per stage is enough
+ * (a warp writes the next stage's value of its state while others still read this stage's).
+ * 4,096 systems of three states, 64 trajectories, 1,000 steps: 71.8 ms with one warp per item and the
+ * machine in C++, 25.6 now; the warps that are resident (30 of an SM's 64, by their registers) issue in
+ * 44 % of the cycles, and wait for one another at the barriers for a third of their time. */
 template <int RR>
 __global__ void __launch_bounds__(kRolloutMaxWarps * 32, RR == 4 ? 1 : 2)
 rk4_kernel(const DeviceBatch batch, const Rk4Problem prob, const RolloutLayout lay) {
     constexpr uint32_t PASS = 32 * RR; /* trajectories of one pass */
     extern __shared__ __align__(16) unsigned char smem[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t S = prob.num_states, K = prob.num_constants;
-    unsigned char* const warea = smem + (size_t)warp * lay.warp_bytes;
-    unsigned char* const tables = warea + (size_t)S * lay.exec_bytes;
-    float* const source = reinterpret_cast<float*>(tables + (size_t)S * lay.table_bytes);
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, group = warp / S, s = warp - group * S;
+    const uint32_t barrier = group + 1u, threads = S * 32u;
+    unsigned char* const garea = smem + (size_t)group * lay.group_bytes;
+    const uint32_t stage_bytes = S * (uint32_t)(RR * 128);
+    const uint32_t stage0 = shared_address(garea) + lane * (uint32_t)(RR * 4); /* this lane's part of the first vector; the second follows it */
+    volatile unsigned long long* const item_word = reinterpret_cast<volatile unsigned long long*>(garea + 2u * stage_bytes);
+    unsigned char* const warea = garea + 2u * stage_bytes + 16u + (size_t)s * lay.warp_bytes;
+    SbInsn* const exec = reinterpret_cast<SbInsn*>(warea) + 1; /* the entry before the first holds the first handler */
+    float* const table = reinterpret_cast<float*>(warea + lay.exec_bytes);
+    float* const source = reinterpret_cast<float*>(warea + lay.exec_bytes + lay.table_bytes);
     float* const tmp = source + K + batch.max_extra;
-    uint32_t* const starts = reinterpret_cast<uint32_t*>(reinterpret_cast<unsigned char*>(source) + lay.source_bytes);
-    float* const slot_area = reinterpret_cast<float*>(starts + 16);
-    const uint32_t slot0 = shared_address(slot_area);
+    const uint32_t table_address = shared_address(table), first_temp = 4u * S; /* the records' reserved slots */
+    Rollout<RR> m;
+    m.temps = shared_address(warea + lay.exec_bytes + lay.table_bytes + lay.source_bytes) + lane * (uint32_t)(RR * 4);
     const unsigned long long configs = (unsigned long long)prob.num_banks << prob.toggle_bits;
     const unsigned long long num_items = configs * prob.num_systems;
     unsigned int integrated = 0; /* (trajectory, observation interval) pairs this lane carried out */
-    /* Items are drawn from a device-wide counter: a warp whose candidate went invalid early takes
+    /* Items are drawn from a device-wide counter: a group whose candidate went invalid early takes
      * the next one at once, and no warp slot idles behind the longest item of its CTA. */
+#pragma unroll 1
     for (;;) {
     unsigned long long item = 0;
-    if (lane == 0) item = atomicAdd(prob.queue, 1ull);
-    item = __shfl_sync(0xffffffffu, item, 0);
+    if (s == 0 && lane == 0) item = atomicAdd(prob.queue, 1ull);
+    if (S > 1) {
+        if (s == 0 && lane == 0) *item_word = item;
+        group_sync(barrier, threads);
+        item = *item_word;
+    } else {
+        item = __shfl_sync(0xffffffffu, item, 0);
+    }
     if (item >= num_items) break;
     const uint32_t turn = (uint32_t)(item / configs);
     const uint32_t sys = prob.order ? prob.order[turn] : turn;
-    const unsigned long long cfg = item % configs;
+    const unsigned long long cfg = item - turn * configs;
     const unsigned long long perm = cfg & ((1ull << prob.toggle_bits) - 1ull);
     const uint32_t bank = (uint32_t)(cfg >> prob.toggle_bits);
     const float* bank_ptr = prob.banks ? prob.banks + (size_t)sys * prob.system_bank_stride + (size_t)bank * prob.bank_stride : nullptr;
 
-    /* private copy of every right-hand side: toggles resolved, the bank part run once, the main
-     * part rewritten for the machine */
-    for (uint32_t s = 0; s < S; ++s) {
-        const SbProgram pr = batch.programs[sys * S + s];
-        SbInsn* exec = reinterpret_cast<SbInsn*>(warea + (size_t)s * lay.exec_bytes);
-        float* table = reinterpret_cast<float*>(tables + (size_t)s * lay.table_bytes);
-        for (uint32_t i = lane; i < pr.n_insn; i += 32) exec[i] = batch.insns[pr.insn_off + i];
-        if (lane == 0) exec[pr.n_insn] = SbInsn{0u, 0u};
+    /* private copy of the right-hand side: toggles resolved, the bank part run once, the main part
+     * rewritten for the machine */
+    const SbProgram* const pr = batch.programs + sys * S + s;
+    const uint32_t n_insn = pr->n_insn, main_off = pr->main_off;
+    {
+        const uint32_t n_patch = pr->n_patch, n_affine = pr->n_affine, n_source = K + n_affine + pr->n_lits;
+#pragma unroll 1
+        for (uint32_t i = lane; i < n_insn; i += 32) exec[i] = batch.insns[pr->insn_off + i];
         __syncwarp();
-        for (uint32_t i = lane; i < pr.n_patch; i += 32) {
-            const SbPatch* p = batch.patches + pr.patch_off + i;
+#pragma unroll 1
+        for (uint32_t i = lane; i < n_patch; i += 32) {
+            const SbPatch* p = batch.patches + pr->patch_off + i;
             unsigned choice = (unsigned)(perm >> p->bit0) & 1u;
             if (p->bit1 != 0xffu) choice |= ((unsigned)(perm >> p->bit1) & 1u) << 1;
             exec[p->insn] = p->alt[choice];
         }
-        for (uint32_t e = lane; e < K + pr.n_affine + pr.n_lits; e += 32) {
+#pragma unroll 1
+        for (uint32_t e = lane; e < n_source; e += 32) {
             float v;
             if (e < K) v = prob.sampled ? sampled_constant(prob, (unsigned long long)sys * K + e, bank) : bank_ptr[e];
-            else if (e < K + pr.n_affine) {
-                const SbAffine a = batch.affines[pr.affine_off + e - K];
+            else if (e < K + n_affine) {
+                const SbAffine a = batch.affines[pr->affine_off + e - K];
                 const float slot = prob.sampled ? sampled_constant(prob, (unsigned long long)sys * K + a.slot, bank) : bank_ptr[a.slot];
                 v = __fadd_rn(__fmul_rn(slot, a.scale), a.offset);
-            } else v = batch.lits[pr.lit_off + e - K - pr.n_affine];
+            } else v = batch.lits[pr->lit_off + e - K - n_affine];
             source[e] = v;
         }
         __syncwarp();
-        if (pr.main_off) rollout_bank_part(exec, source, tmp, table, RR);
-        __syncwarp(); /* the next record's constants overwrite `source` */
-        const uint32_t table_address = shared_address(table);
-        for (uint32_t i = pr.main_off + lane; i < pr.n_insn; i += 32) exec[i] = rewritten<RR>(exec[i], table_address, slot0);
-        /* start address and length of the main part in one word (shared addresses fit 18 bits) */
-        if (lane == 0) starts[s] = shared_address(exec + pr.main_off) | ((uint32_t)(pr.n_insn - pr.main_off - 1u) << 18);
+        if (main_off) rollout_bank_part(exec, source, tmp, table, RR);
+        __syncwarp();
+#pragma unroll 1
+        for (uint32_t i0 = main_off; i0 < n_insn; i0 += 32) { /* in place: every lane reads before any writes */
+            const uint32_t i = i0 + lane;
+            const SbInsn made = i < n_insn ? rewritten<RR>(exec[i], table_address, first_temp) : SbInsn{H_END, 0u};
+            __syncwarp();
+            if (i < n_insn) {
+                (exec + i)[-1].w0 = made.w0;
+                exec[i].w1 = made.w1;
+            }
+            __syncwarp();
+        }
     }
-    __syncwarp();
+    const typename Rollout<RR>::Item place{shared_address(exec + main_off), lds_word(shared_address(exec + main_off) - 8u), s * (uint32_t)(RR * 128), barrier, S > 1 ? threads : 0u,
+                                           sys * S + s, first_temp, table_address};
 
-    const uint32_t STAGE = 0, NEXT = S, SUM = 2 * S, STATE = 3 * S, BASE = STATE;
     const bool ragged = prob.offsets != nullptr;
-    Rollout<RR> m;
-    m.slot0 = slot0;
-    m.lane_off = (uint32_t)lane * (uint32_t)(RR * 4);
-    const uint32_t starts_address = shared_address(starts), tables_address = shared_address(tables);
     float sq = 0.0f;
     unsigned long long residuals = 0;
     /* any non-finite time or reference value (NaN excepted where it means "unobserved"), found
      * by the validation kernel, invalidates every score; so do offsets that do not span the data */
     bool ok = *prob.invalid_flag == 0;
     if (ragged) ok = ok && prob.offsets[0] == 0u && prob.offsets[prob.num_trajectories] == prob.total_points;
-    /* a candidate that is already invalid scores FLT_MAX whatever follows: the warp stops integrating it */
-    bool alive = __all_sync(0xffffffffu, ok);
+    /* a candidate that is already invalid scores FLT_MAX whatever follows: the group stops integrating it */
+    bool alive = group_all(barrier, threads, ok);
+    uint32_t now = stage0, other = stage0 + stage_bytes; /* the vectors of this stage's values and of the next stage's */
+#pragma unroll 1
     for (uint32_t t0 = 0; t0 < prob.num_trajectories && alive; t0 += PASS) {
-        uint32_t begin[RR], npts[RR], longest = 0;
+        uint32_t at[RR], npts[RR], longest = 0; /* the point a trajectory has reached; its number of points */
+        float state[RR], reached[RR], next[RR]; /* the times of that point and of the one after it */
+        const float* const reference = prob.reference + (size_t)s * prob.reference_ld; /* of this warp's state */
 #pragma unroll
         for (int q = 0; q < RR; ++q) {
             const uint32_t traj = t0 + lane * RR + q;
             const bool live = traj < prob.num_trajectories;
-            begin[q] = 0; npts[q] = 0;
+            at[q] = 0; npts[q] = 0;
             if (live && ragged) {
                 const uint32_t b = prob.offsets[traj], e = prob.offsets[traj + 1];
                 const bool sane = e > b && e <= prob.total_points;
                 ok = ok && sane;
-                if (sane) { begin[q] = b; npts[q] = e - b; }
+                if (sane) { at[q] = b; npts[q] = e - b; }
             } else if (live) {
-                begin[q] = traj * prob.points_per_trajectory; npts[q] = prob.points_per_trajectory;
+                at[q] = traj * prob.points_per_trajectory; npts[q] = prob.points_per_trajectory;
             }
             longest = max(longest, npts[q]);
+            state[q] = npts[q] ? reference[at[q]] : 0.0f;
+            reached[q] = npts[q] ? prob.times[ragged ? at[q] : 0u] : 0.0f;
+            next[q] = npts[q] > 1u ? prob.times[ragged ? at[q] + 1u : 1u] : 0.0f;
+            ok = ok && (fabsf(state[q]) <= kFltMax); /* initial states must be complete and finite */
         }
-#pragma unroll
-        for (int d = 16; d; d >>= 1) longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, d));
-        for (uint32_t s = 0; s < S; ++s) {
-            float v[RR];
-#pragma unroll
-            for (int q = 0; q < RR; ++q) {
-                v[q] = npts[q] ? prob.reference[(size_t)s * prob.reference_ld + begin[q]] : 0.0f;
-                ok = ok && (fabsf(v[q]) <= kFltMax); /* initial states must be complete and finite */
-            }
-            m.put(STATE + s, v);
-        }
-        alive = __all_sync(0xffffffffu, ok);
+        longest = __reduce_max_sync(0xffffffffu, longest);
+        sts<RR>(now + s * (uint32_t)(RR * 128), state);
+        alive = group_all(barrier, threads, ok);
+#pragma unroll 1
         for (uint32_t k = 1; k < longest && alive; ++k) {
             /* per trajectory step size; a trajectory that has ended keeps integrating with h = 0
-             * and is left out of every check and sum */
-            float h[RR], sixth[RR];
-            bool act[RR];
+             * and is left out of every check and sum.  What memory holds for the end of this interval
+             * and for the next one is asked for here and used after the interval's stages. */
+            float h[RR], half[RR], sixth[RR], expected[RR];
 #pragma unroll
             for (int q = 0; q < RR; ++q) {
-                act[q] = k < npts[q];
-                const uint32_t at = ragged ? begin[q] + k : k;
-                const float interval = act[q] ? prob.times[at] - prob.times[at - 1] : 0.0f;
-                const float step = interval / (float)prob.substeps;
-                ok = ok && (!act[q] || ((fabsf(interval) <= kFltMax) && interval > 0.0f && step > 0.0f));
-                h[q] = act[q] ? step : 0.0f;
-                sixth[q] = h[q] / 6.0f;
+                const bool act = k < npts[q];
+                const float interval = act ? next[q] - reached[q] : 0.0f;
+                const float step = prob.substeps == 1u ? interval : interval / (float)prob.substeps;
+                ok = ok && (!act || ((fabsf(interval) <= kFltMax) && interval > 0.0f && step > 0.0f));
+                h[q] = act ? step : 0.0f;
+                half[q] = __fmul_rn(0.5f, h[q]);
+                sixth[q] = sixth_of(h[q]);
+                integrated += act ? 1u : 0u;
+                reached[q] = next[q];
+                ++at[q];
+                expected[q] = act ? reference[at[q]] : 0.0f;
+                if (k + 1u < npts[q]) next[q] = prob.times[ragged ? at[q] + 1u : k + 1u];
             }
-            for (uint32_t sub = 0; sub < prob.substeps; ++sub) {
-                for (uint32_t s = 0; s < S; ++s) {
-                    float v[RR], zero[RR];
-                    m.get(STATE + s, v);
-                    m.put(STAGE + s, v);
+            m.interval(place, batch, prob.substeps, state, half, h, sixth, now, other);
 #pragma unroll
-                    for (int q = 0; q < RR; ++q) zero[q] = 0.0f;
-                    m.put(SUM + s, zero);
+            for (int q = 0; q < RR; ++q)
+                if (k < npts[q]) {
+                    ok = ok && fabsf(state[q]) <= kFltMax; /* one state that is not finite and no residual counts */
+                    if (prob.allow_missing && expected[q] != expected[q]) continue; /* unobserved */
+                    const float err = __fsub_rn(state[q], expected[q]);
+                    sq = __fmaf_rn(err, err, sq);
+                    ++residuals;
                 }
-#pragma unroll 1
-                for (int stage = 0; stage < 4; ++stage) {
-                    const float weight = (stage == 0 || stage == 3) ? 1.0f : 2.0f;
-                    for (uint32_t s = 0; s < S; ++s) {
-                        const uint32_t start = lds_word(starts_address + 4u * s);
-                        m.run(start & 0x3ffffu, start >> 18, tables_address + s * lay.table_bytes); /* acc = rhs of state s at the stage values */
-                        float v[RR];
-                        m.get(SUM + s, v);
-#pragma unroll
-                        for (int q = 0; q < RR; ++q) v[q] = __fmaf_rn(weight, m.acc[q], v[q]);
-                        m.put(SUM + s, v);
-                        if (stage != 3) {
-                            m.get(BASE + s, v);
-#pragma unroll
-                            for (int q = 0; q < RR; ++q) v[q] = __fmaf_rn(stage == 2 ? h[q] : __fmul_rn(0.5f, h[q]), m.acc[q], v[q]);
-                            m.put(NEXT + s, v);
-                        }
-                    }
-                    if (stage != 3)
-                        for (uint32_t s = 0; s < S; ++s) {
-                            float v[RR];
-                            m.get(NEXT + s, v);
-                            m.put(STAGE + s, v);
-                        }
-                }
-                for (uint32_t s = 0; s < S; ++s) {
-                    float sum[RR], base[RR];
-                    m.get(SUM + s, sum);
-                    m.get(BASE + s, base);
-#pragma unroll
-                    for (int q = 0; q < RR; ++q) base[q] = __fmaf_rn(sixth[q], sum[q], base[q]);
-                    m.put(STATE + s, base);
-                }
-            }
-            for (uint32_t s = 0; s < S; ++s) { /* all states must be finite before any residual counts */
-                float v[RR];
-                m.get(STATE + s, v);
-#pragma unroll
-                for (int q = 0; q < RR; ++q) ok = ok && (!act[q] || fabsf(v[q]) <= kFltMax);
-            }
-#pragma unroll
-            for (int q = 0; q < RR; ++q) integrated += act[q] ? 1u : 0u;
-            alive = __all_sync(0xffffffffu, ok);
-            for (uint32_t s = 0; s < S; ++s) {
-                float v[RR];
-                m.get(STATE + s, v);
-#pragma unroll
-                for (int q = 0; q < RR; ++q)
-                    if (act[q]) {
-                        const float ref = prob.reference[(size_t)s * prob.reference_ld + begin[q] + k];
-                        if (prob.allow_missing && ref != ref) continue; /* unobserved */
-                        const float err = __fsub_rn(v[q], ref);
-                        sq = __fmaf_rn(err, err, sq);
-                        ++residuals;
-                    }
-            }
+            alive = group_all(barrier, threads, ok);
         }
     }
-    float total = sq;
+    /* the warps' sums meet in their source areas, which the next item fills only after another barrier */
 #pragma unroll
-    for (int d = 16; d; d >>= 1) total += __shfl_xor_sync(0xffffffffu, total, d);
-    uint32_t lo = (uint32_t)residuals, hi = (uint32_t)(residuals >> 32);
+    for (int d = 16; d; d >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, d);
+    {
+        uint32_t lo = (uint32_t)residuals, hi = (uint32_t)(residuals >> 32);
 #pragma unroll
-    for (int d = 16; d; d >>= 1) {
-        const unsigned long long other = ((unsigned long long)__shfl_xor_sync(0xffffffffu, hi, d) << 32) | __shfl_xor_sync(0xffffffffu, lo, d);
-        residuals += other;
-        lo = (uint32_t)residuals; hi = (uint32_t)(residuals >> 32);
+        for (int d = 16; d; d >>= 1) {
+            residuals += ((unsigned long long)__shfl_xor_sync(0xffffffffu, hi, d) << 32) | __shfl_xor_sync(0xffffffffu, lo, d);
+            lo = (uint32_t)residuals; hi = (uint32_t)(residuals >> 32);
+        }
     }
-    const bool all_ok = __all_sync(0xffffffffu, ok);
     if (lane == 0) {
+        source[0] = sq;
+        source[1] = __uint_as_float((uint32_t)residuals);
+        source[2] = __uint_as_float((uint32_t)(residuals >> 32));
+    }
+    group_sync(barrier, threads);
+    if (s == 0 && lane == 0) {
+        float total = sq;
+        for (uint32_t c = 1; c < S; ++c) {
+            const float* other_source = source + (size_t)c * (lay.warp_bytes / 4u);
+            total += other_source[0];
+            residuals += ((unsigned long long)__float_as_uint(other_source[2]) << 32) | __float_as_uint(other_source[1]);
+        }
         const bool finite = fabsf(total) <= kFltMax;
-        prob.output[(size_t)sys * prob.output_ld + cfg] = (all_ok && residuals && finite) ? total / (float)residuals : kFltMax;
+        prob.output[(size_t)sys * prob.output_ld + cfg] = (alive && residuals && finite) ? total / (float)residuals : kFltMax;
     }
-    __syncwarp(); /* the next item overwrites the warp's program and slot areas */
+    if (S == 1) __syncwarp(); /* a group of several meets again before anything is overwritten */
     }
-    if (prob.integrated) {
+    if (prob.integrated && s == 0) {
 #pragma unroll
         for (int d = 16; d; d >>= 1) integrated += __shfl_xor_sync(0xffffffffu, integrated, d);
         if (lane == 0) atomicAdd(prob.integrated, (unsigned long long)integrated);
@@ -615,32 +632,35 @@ __global__ void rk4_validate_kernel(const Rk4Problem prob) {
 uint32_t round16(size_t v) { return (uint32_t)((v + 15) / 16 * 16); }
 
 template <int RR>
-cudaError_t launch_width(const DeviceBatch& batch, const Rk4Problem& prob, size_t smem_limit, unsigned concurrent, cudaStream_t stream) {
+cudaError_t launch_width(const DeviceBatch& batch, const Rk4Problem& prob, size_t smem_limit, cudaStream_t stream) {
     RolloutLayout lay;
+    const uint32_t S = prob.num_states;
     lay.exec_bytes = round16(((size_t)batch.max_insn + 1) * sizeof(SbInsn));
-    lay.table_bytes = round16(((size_t)batch.max_cst + 1) * RR * 4); /* one entry at least: instructions without an operand read it */
+    lay.table_bytes = round16(((size_t)batch.max_cst + 1) * RR * 4);
     lay.source_bytes = round16(((size_t)prob.num_constants + batch.max_extra + batch.max_btmp) * 4 + 16);
-    /* max_slots already includes the integrator's reserved slots */
-    lay.warp_bytes = prob.num_states * (lay.exec_bytes + lay.table_bytes) + lay.source_bytes + 64u + batch.max_slots * (uint32_t)RR * 128u;
-    const uint32_t warp_bytes = lay.warp_bytes;
-    /* warps per CTA: the count that puts most warps on an SM (shared memory per SM is the CTA limit
+    /* max_slots includes the four reserved per state that the records leave before their temporaries */
+    lay.temp_bytes = (batch.max_slots > 4u * S ? batch.max_slots - 4u * S : 0u) * (uint32_t)RR * 128u;
+    lay.warp_bytes = lay.exec_bytes + lay.table_bytes + lay.source_bytes + lay.temp_bytes;
+    lay.group_bytes = 2u * S * (uint32_t)(RR * 128) + 16u + S * lay.warp_bytes;
+    /* groups per CTA: the count that puts most warps on an SM (shared memory per SM is the CTA limit
      * plus 1 KB reserved per resident CTA; the register file holds 64 K registers, allocated per warp
-     * in units of 256) */
+     * in units of 256; a CTA has fifteen barriers to give to groups) */
     cudaFuncAttributes attributes;
     cudaError_t e = cudaFuncGetAttributes(&attributes, rk4_kernel<RR>);
     if (e != cudaSuccess) return e;
     const int warp_registers = (attributes.numRegs * 32 + 255) / 256 * 256;
     const int register_warps = std::min(64, 65536 / std::max(256, warp_registers));
-    int warps = 0, best = 0;
-    for (int w = 2; w <= kRolloutMaxWarps; ++w) {
-        const size_t cta = (size_t)warp_bytes * w;
+    int groups = 0, best = 0;
+    for (int g = 1; g <= 15 && g * (int)S <= kRolloutMaxWarps; ++g) {
+        const size_t cta = (size_t)lay.group_bytes * g;
         if (cta > smem_limit) break;
-        const int ctas = std::min((int)((smem_limit + 1024) / (cta + 1024)), register_warps / w);
-        if (ctas && ctas * w >= best) { best = ctas * w; warps = w; }
+        const int ctas = std::min((int)((smem_limit + 1024) / (cta + 1024)), register_warps / (g * (int)S));
+        if (ctas && ctas * g >= best) { best = ctas * g; groups = g; }
     }
-    /* a main part's length travels in 14 bits; the start words of the states' main parts have 16 places */
-    if (!warps || batch.max_insn > 16383u || prob.num_states > 16u) return cudaErrorInvalidConfiguration;
-    const size_t smem = (size_t)warp_bytes * warps;
+    const int warps = groups * (int)S;
+    /* a parked temporary's offset has 14 bits, a state's 18 with the rest of the word */
+    if (!groups || batch.max_slots * (uint32_t)RR > 16383u) return cudaErrorInvalidConfiguration;
+    const size_t smem = (size_t)lay.group_bytes * groups;
     e = cudaFuncSetAttribute(rk4_kernel<RR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_limit);
     if (e != cudaSuccess) return e;
     /* the largest shared-memory carve-out, always: left to itself the driver gave a CTA that fits the
@@ -652,24 +672,24 @@ cudaError_t launch_width(const DeviceBatch& batch, const Rk4Problem& prob, size_
     /* warps draw items from the queue until it is empty, so the grid only has to fill the device */
     int device = 0, sms = 0;
     if ((e = cudaGetDevice(&device)) != cudaSuccess || (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess) return e;
-    /* a launch that shares the device with `concurrent` - 1 others takes its share of the resident
-     * CTAs: its warps then work through several items each, and one that drew a short item (an
-     * invalid candidate) goes on with the next instead of idling until its CTA's longest item ends */
-    const unsigned long long resident = (unsigned long long)sms * (unsigned)std::max(1, best / warps);
-    const unsigned long long share = std::max<unsigned long long>(1, (resident + concurrent - 1) / std::max(1u, concurrent));
-    const unsigned long long blocks = std::min<unsigned long long>((items + warps - 1) / warps, share);
-    const size_t values = (size_t)prob.total_points * (prob.num_states + 1);
-    rk4_validate_kernel<<<(unsigned)std::min<size_t>(1024, (values + 255) / 256), 256, 0, stream>>>(prob);
+    const unsigned long long resident = (unsigned long long)sms * (unsigned)std::max(1, best / groups);
+    const unsigned long long blocks = std::min<unsigned long long>((items + groups - 1) / groups, resident);
     rk4_kernel<RR><<<(unsigned)blocks, warps * 32, smem, stream>>>(batch, prob, lay);
     return cudaGetLastError();
 }
 
 }  // namespace
 
-cudaError_t launch_rk4(const DeviceBatch& batch, const Rk4Problem& prob, size_t smem_limit, unsigned concurrent, cudaStream_t stream) {
-    if (prob.num_trajectories <= 32) return launch_width<1>(batch, prob, smem_limit, concurrent, stream);
-    if (prob.num_trajectories <= 64) return launch_width<2>(batch, prob, smem_limit, concurrent, stream);
-    return launch_width<4>(batch, prob, smem_limit, concurrent, stream);
+cudaError_t launch_rk4_validation(const Rk4Problem& prob, cudaStream_t stream) {
+    const size_t values = (size_t)prob.total_points * (prob.num_states + 1);
+    rk4_validate_kernel<<<(unsigned)std::min<size_t>(1024, (values + 255) / 256), 256, 0, stream>>>(prob);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_rk4(const DeviceBatch& batch, const Rk4Problem& prob, size_t smem_limit, cudaStream_t stream) {
+    if (prob.num_trajectories <= 32) return launch_width<1>(batch, prob, smem_limit, stream);
+    if (prob.num_trajectories <= 64) return launch_width<2>(batch, prob, smem_limit, stream);
+    return launch_width<4>(batch, prob, smem_limit, stream);
 }
 
 }  // namespace sb

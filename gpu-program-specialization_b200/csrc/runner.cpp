@@ -44,29 +44,26 @@ std::atomic<uint64_t> g_kernel_launches{0};
 std::atomic<uint64_t> g_row_stream_bytes{0};
 void note_kernel_launches(unsigned n) { g_kernel_launches.fetch_add(n); }
 
-namespace {
-
-double now_seconds() {
-    return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
-}
-
 /* cuCtxGetCurrent without linking the driver library: the library must load on machines
  * that have no GPU driver at all. */
 void* current_context(bool* ok) {
     typedef int (*GetCurrentFn)(void**);
-    static GetCurrentFn fn = nullptr;
-    static bool resolved = false;
-    if (!resolved) {
+    static const GetCurrentFn fn = [] {
         void* entry = nullptr;
         cudaDriverEntryPointQueryResult status;
-        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &entry, cudaEnableDefault, &status) == cudaSuccess &&
-            status == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<GetCurrentFn>(entry);
-        resolved = true;
-    }
+        return cudaGetDriverEntryPoint("cuCtxGetCurrent", &entry, cudaEnableDefault, &status) == cudaSuccess &&
+                       status == cudaDriverEntryPointSuccess
+                   ? reinterpret_cast<GetCurrentFn>(entry) : nullptr;
+    }();
     void* ctx = nullptr;
     *ok = fn && fn(&ctx) == 0;
     return ctx;
+}
+
+namespace {
+
+double now_seconds() {
+    return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
 }
 
 size_t align256(size_t v) { return (v + 255) / 256 * 256; }
