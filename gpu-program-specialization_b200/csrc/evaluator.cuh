@@ -65,6 +65,7 @@ struct DeviceBatch {
     uint32_t max_btmp;    /* largest number of bank-part temporaries */
     uint32_t uses_scratch; /* some program needs the scratch spill slot */
     uint64_t total_cst;   /* constant-table entries of all programs (an upper bound will do) */
+    uint64_t total_cost;  /* scheduling weights of all programs */
 };
 
 struct EvalProblem {
@@ -136,9 +137,10 @@ constexpr int kVariantBanks[kNumVariants] = {4, 2, 1};
 
 Geom make_geom(const DeviceBatch& batch, const EvalProblem& problem, const LaunchPlan& plan);
 
-/* scratch_limit: most floats of per-split partial sums a launch may use (row splits are reduced to fit). */
+/* scratch_limit: most floats of per-split partial sums a launch may use (row splits are reduced to fit).
+ * share: the part of the machine a small launch should count on (another one runs beside it). */
 LaunchPlan plan_launch(const DeviceBatch& batch, const EvalProblem& problem, int sm_count, size_t smem_limit,
-                       size_t scratch_limit);
+                       size_t scratch_limit, double share = 1.0);
 
 /* Enqueues the evaluation of one batch on `stream`: the evaluator kernel writes per-split partial
  * sums into `partial` (plan.table_offset + plan.table_elements floats, private to the stream until the

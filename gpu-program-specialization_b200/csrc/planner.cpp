@@ -52,8 +52,72 @@ Geom make_geom(const DeviceBatch& batch, const EvalProblem& prob, const LaunchPl
 
 namespace {
 
+size_t smem_needed(const Geom& g, uint32_t warps) { return (size_t)g.tile_bytes * g.tile_buffers + 16 + (size_t)g.warp_bytes * warps; }
+
+/* How a launch is cut into queue items and CTAs when it is small: the sums do not depend on it (they
+ * depend on the tiles and the row splits, which stay as they are), so it may follow the machine.
+ *
+ * The rules above it aim at large launches, whose grid is many waves deep.  With few programs or rows
+ * they gave grids of 150 CTAs on 148 SMs (two waves for one), a dozen items for twenty warps, or half
+ * the warps because a second tile buffer was reserved that a CTA of one tile does not use.  Here the cut
+ * with the shortest estimated time is taken: the grid's waves times a CTA's rounds of items.  The
+ * constants are issue slots, measured on the 64-set population: 330 for one pass of the main part with
+ * its loss, about 900 to set an item up, and a warp that issues every seventh cycle when alone; an SM
+ * issues 2.6 per cycle at best. */
+struct Cut { uint32_t gpi, ppi; unsigned long long groups; };
+
+double cut_cycles(const LaunchPlan& plan, const Cut& cut, unsigned long long programs, unsigned long long items_per_program, uint32_t passes, size_t tiles,
+                  bool hoists, int sms) {
+    const unsigned long long items = (programs + cut.groups - 1) / cut.groups * items_per_program;
+    const double active = (double)std::min<unsigned long long>(plan.warps, items);
+    const double rate = std::min(0.14, 2.6 / active);
+    const double item = 900.0 + passes * ((hoists ? 120.0 : 0.0) + 330.0 * cut.gpi * cut.ppi);
+    const double rounds = std::max((double)((items + plan.warps - 1) / plan.warps), (double)items / plan.warps + 0.5);
+    const double cta = 3000.0 + tiles * (1500.0 + rounds * item / rate);
+    const unsigned long long grid = cut.groups * plan.row_splits;
+    return (double)((grid + sms - 1) / sms) * cta;
+}
+
+/* `sms`: the part of the machine this launch has when another runs beside it. */
+void balance_small(LaunchPlan* plan, const DeviceBatch& batch, const EvalProblem& prob, int sms, size_t smem_limit) {
+    const bool materialize = prob.mode == EVAL_MATERIALIZE;
+    const uint32_t rr = (uint32_t)kVariantRows[plan->variant], rc = (uint32_t)kVariantBanks[plan->variant], pass = 32u * rr;
+    const unsigned long long P = batch.num_programs, bank_groups = materialize ? 1 : (prob.num_banks + rc - 1) / rc;
+    const size_t tiles = (plan->rows_per_split + plan->tile_rows - 1) / plan->tile_rows;
+    /* as many warps as fit beside the tile buffers that are used */
+    const auto refit = [&](LaunchPlan* p) {
+        const Geom g = make_geom(batch, prob, *p);
+        while (p->warps < 20 && smem_needed(g, p->warps + 1) <= smem_limit) ++p->warps;
+        p->smem_bytes = smem_needed(g, p->warps);
+    };
+    if (plan->tile_buffers == 1) refit(plan);
+    if ((unsigned long long)plan->num_groups * plan->row_splits >= 8ull * (unsigned long long)sms) return; /* deep enough */
+    const uint32_t passes = (uint32_t)((std::min<size_t>(plan->tile_rows, prob.num_rows) + pass - 1) / pass);
+    const auto items_of = [&](const Cut& c) { return materialize ? 1ull : ((bank_groups / c.gpi) << prob.toggle_bits) / c.ppi; };
+    Cut best{plan->groups_per_item, plan->perms_per_item, plan->num_groups};
+    double least = 0.97 * cut_cycles(*plan, best, P, items_of(best), passes, tiles, batch.max_hoisted != 0, sms);
+    const Cut widest = best;
+    for (uint32_t gpi = widest.gpi; gpi >= 1; --gpi) {
+        if (bank_groups % gpi) continue;
+        for (uint32_t ppi = gpi == bank_groups ? widest.ppi : 1u; ppi >= 1; ppi /= 2)
+            for (unsigned waves = 0; waves <= 8; ++waves) {
+                Cut c{gpi, ppi, waves ? (unsigned long long)waves * sms / plan->row_splits : widest.groups};
+                c.groups = std::max<unsigned long long>(1, std::min(c.groups, P));
+                const unsigned long long items = items_of(c);
+                if (items > 0xffffff00ull / ((P + c.groups - 1) / c.groups)) continue;
+                const double t = cut_cycles(*plan, c, P, items, passes, tiles, batch.max_hoisted != 0, sms);
+                if (t < least) { least = t; best = c; }
+            }
+    }
+    plan->groups_per_item = best.gpi;
+    plan->perms_per_item = best.ppi;
+    plan->num_groups = (uint32_t)best.groups;
+    plan->grid_x = plan->num_groups * plan->row_splits;
+    refit(plan);
+}
+
 LaunchPlan plan_with_tile(const DeviceBatch& batch, const EvalProblem& prob, int sm_count, size_t smem_limit, size_t scratch_limit,
-                          int variant) {
+                          int variant, double share) {
     LaunchPlan plan{};
     plan.ok = false;
     plan.overflow = false;
@@ -117,7 +181,7 @@ LaunchPlan plan_with_tile(const DeviceBatch& batch, const EvalProblem& prob, int
                 trial.row_splits = 1;
                 trial.rows_per_split = prob.num_rows;
                 const Geom g = make_geom(batch, prob, trial);
-                const size_t need = (size_t)g.tile_bytes * g.tile_buffers + 16 + (size_t)g.warp_bytes * trial.warps;
+                const size_t need = smem_needed(g, trial.warps);
                 if (need > smem_limit) continue;
                 plan = trial;
                 plan.smem_bytes = need;
@@ -164,7 +228,7 @@ LaunchPlan plan_with_tile(const DeviceBatch& batch, const EvalProblem& prob, int
     const size_t tiles_per_split = (tiles + splits - 1) / splits;
     plan.rows_per_split = tiles_per_split * plan.tile_rows;
     plan.row_splits = (uint32_t)((prob.num_rows + plan.rows_per_split - 1) / plan.rows_per_split);
-    if (tiles_per_split == 1) plan.tile_buffers = 1; /* smem_bytes stays an upper bound */
+    if (tiles_per_split == 1) plan.tile_buffers = 1;
     const unsigned long long grid = groups * plan.row_splits;
     if (grid > 0x7fffffffull) { plan.overflow = true; return plan; }
     plan.grid_x = (uint32_t)grid;
@@ -180,13 +244,14 @@ LaunchPlan plan_with_tile(const DeviceBatch& batch, const EvalProblem& prob, int
     if (batch.total_cst > (~0ull >> 3) / padded) { plan.overflow = true; return plan; }
     plan.table_elements = (size_t)(batch.total_cst * padded);
     plan.table_offset = (plan.partial_elements + 3) / 4 * 4;
+    balance_small(&plan, batch, prob, std::max(1, (int)(sm_count * share)), smem_limit);
     plan.ok = true;
     return plan;
 }
 
 }  // namespace
 
-LaunchPlan plan_launch(const DeviceBatch& batch, const EvalProblem& prob, int sm_count, size_t smem_limit, size_t scratch_limit) {
+LaunchPlan plan_launch(const DeviceBatch& batch, const EvalProblem& prob, int sm_count, size_t smem_limit, size_t scratch_limit, double share) {
     /* register tile: 4 rows x 4 banks per thread, or 8 x 2 / 16 x 1 when there are fewer banks.  Up
      * to four banks take the 8 x 2 tile: three or four banks are then two bank groups, so the row
      * prelude serves two runs of the main part and computes each row's value twice instead of four
@@ -198,7 +263,7 @@ LaunchPlan plan_launch(const DeviceBatch& batch, const EvalProblem& prob, int sm
     if (prob.mode == EVAL_MATERIALIZE) variant = 2;
     LaunchPlan plan{};
     for (; variant >= 0; --variant) {
-        plan = plan_with_tile(batch, prob, sm_count, smem_limit, scratch_limit, variant);
+        plan = plan_with_tile(batch, prob, sm_count, smem_limit, scratch_limit, variant, share);
         if (plan.ok || plan.overflow) break;
     }
     return plan;

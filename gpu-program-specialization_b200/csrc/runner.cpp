@@ -438,6 +438,7 @@ SecantResult upload_batch(SecantCubinRunnerImpl* r, Slot& s, std::vector<DeviceB
             db.max_hoisted = std::max<uint32_t>(db.max_hoisted, p.n_hoisted);
             db.max_cst = std::max<uint32_t>(db.max_cst, p.n_cst);
             db.total_cst += p.n_cst;
+            db.total_cost += schedule_cost(p);
             db.max_btmp = std::max<uint32_t>(db.max_btmp, p.n_btmp);
             db.uses_scratch |= (p.flags & SB_PROG_USES_SCRATCH) ? 1u : 0u;
         }
@@ -504,10 +505,19 @@ SecantResult stream_scratch(SecantCubinRunnerImpl* r, size_t k, size_t elements,
     return SECANT_SUCCESS;
 }
 
+/* The part of the machine a view's launch should count on: with two views of one run entry on two streams
+ * both are on the device at a time, and when neither fills it they share it by their work. */
+double view_share(const SecantCubinRunnerImpl* r, const std::vector<DeviceBatch>& views, const DeviceBatch& db, size_t entries) {
+    if (r->streams.size() < 2 || entries != 1 || views.size() < 2) return 1.0;
+    double all = 0.0;
+    for (const DeviceBatch& v : views) all += (double)v.total_cost;
+    return std::min(0.95, std::max(0.05, (double)db.total_cost / std::max(1.0, all)));
+}
+
 /* Enqueues the evaluation of one device-resident batch for every run entry, spreading
  * entries over the compute streams.  `after` (optional) is an event each stream waits on
  * first; `done`/`used` (optional) receive one completion event per touched stream. */
-SecantResult launch_batch(SecantCubinRunnerImpl* r, const DeviceBatch& db, const std::vector<UnpackedRun>& runs,
+SecantResult launch_batch(SecantCubinRunnerImpl* r, const DeviceBatch& db, double share, const std::vector<UnpackedRun>& runs,
                           size_t* stream_cursor, cudaEvent_t after, std::vector<cudaEvent_t>* done, std::vector<char>* used) {
     const SecantCubinPlan& plan = *r->plan;
     for (size_t e = 0; e < runs.size(); ++e) {
@@ -531,7 +541,7 @@ SecantResult launch_batch(SecantCubinRunnerImpl* r, const DeviceBatch& db, const
                 part.num_programs = (uint32_t)std::min<size_t>(step, db.num_programs - first);
                 part.total_cst = (uint64_t)part.num_programs * db.max_cst;
             }
-            const LaunchPlan lp = plan_launch(part, prob, r->sm_count, r->smem_limit, r->scratch_limit);
+            const LaunchPlan lp = plan_launch(part, prob, r->sm_count, r->smem_limit, r->scratch_limit, share);
             if (!lp.ok) {
                 r->last_error = lp.overflow ? "configuration count beyond the evaluator's 32-bit item index" : "program batch does not fit shared memory";
                 return lp.overflow ? SECANT_ERROR_OVERFLOW : SECANT_ERROR_REGISTER_OVERFLOW;
@@ -781,7 +791,7 @@ SecantResult execute(SecantCubinRunnerImpl* r, const std::vector<UnpackedRun>& r
             result = launch_gram_batch(r, views, runs, first, std::min(batch_size, P - first), &stream_cursor, slot.uploaded, done, &slot.used);
         } else {
             for (const DeviceBatch& db : views) {
-                result = launch_batch(r, db, runs, &stream_cursor, slot.uploaded, done, &slot.used);
+                result = launch_batch(r, db, view_share(r, views, db, runs.size()), runs, &stream_cursor, slot.uploaded, done, &slot.used);
                 if (result != SECANT_SUCCESS) break;
             }
         }
@@ -973,7 +983,7 @@ SecantResult execute_resident(SecantCubinRunnerImpl* r, SecantB200PopulationImpl
     SecantResult result = SECANT_SUCCESS;
     for (auto& b : pop->batches) {
         for (const DeviceBatch& db : b.views) {
-            result = launch_batch(r, db, runs, &cursor, nullptr, nullptr, nullptr);
+            result = launch_batch(r, db, view_share(r, b.views, db, runs.size()), runs, &cursor, nullptr, nullptr, nullptr);
             if (result != SECANT_SUCCESS) break;
         }
         if (result != SECANT_SUCCESS) break;
