@@ -49,8 +49,11 @@ void plan_fill(SecantCubinPlan* plan, const SecantCubinRecipeHeader* recipe, siz
 SecantResult run_unpack(const SecantCubinPlan& plan, const SecantCubinRunHeader* header, UnpackedRun* out);
 /* Restates s_runs_validate (projects/secant/s_cubin_runner.c:195-241): identical program
  * arrays, address ranges, overlap inside and across entries, program preflight. */
+enum PreflightScan { SCAN_EVERYTHING, SCAN_ROUTINES /* the caller sees to the programs */, SCAN_NOTHING };
 SecantResult runs_validate(const SecantCubinPlan& plan, const UnpackedRun* runs, size_t count, ProgramRules* rules_ret,
-                           bool skip_preflight = false);
+                           PreflightScan scan = SCAN_EVERYTHING);
+/* preflight() of every program of a list, the first failure in order. */
+SecantResult preflight_all(const SecantAstProgramList& list, const ProgramRules& rules);
 
 }  // namespace sb
 

@@ -159,8 +159,7 @@ SecantResult run_unpack(const SecantCubinPlan& plan, const SecantCubinRunHeader*
  * the same program arrays; inside an entry the four device ranges are disjoint; no entry's output
  * touches anything another entry reads or writes; then the program preflight with the smallest
  * toggle_bits of the batch. */
-SecantResult runs_validate(const SecantCubinPlan& plan, const UnpackedRun* runs, size_t count, ProgramRules* rules_ret,
-                           bool skip_preflight) {
+SecantResult runs_validate(const SecantCubinPlan& plan, const UnpackedRun* runs, size_t count, ProgramRules* rules_ret, PreflightScan scan) {
     const SecantAstProgramSet& programs = runs[0].programs;
     unsigned smallest_bits = 32;
     for (size_t i = 0; i < count; ++i) {
@@ -204,15 +203,18 @@ SecantResult runs_validate(const SecantCubinPlan& plan, const UnpackedRun* runs,
     if (rules.banks_allowed)
         for (size_t i = 0; i < count; ++i) rules.hoist_toggled = rules.hoist_toggled || runs[i].num_banks > 2;
     rules.hoist_row = rules.hoist_toggled || rules.toggle_bits > 0;
-    if (!skip_preflight) {
-        const SecantAstProgramList* lists[2] = {&programs.routines, &programs.asts};
-        for (const SecantAstProgramList* list : lists)
-            for (size_t i = 0; i < list->count; ++i) {
-                const SecantResult s = preflight(list->items[i], rules);
-                if (s != SECANT_SUCCESS) return s;
-            }
-    }
     *rules_ret = rules;
+    SecantResult s = SECANT_SUCCESS;
+    if (scan != SCAN_NOTHING) s = preflight_all(programs.routines, rules);
+    if (s == SECANT_SUCCESS && scan == SCAN_EVERYTHING) s = preflight_all(programs.asts, rules);
+    return s;
+}
+
+SecantResult preflight_all(const SecantAstProgramList& list, const ProgramRules& rules) {
+    for (size_t i = 0; i < list.count; ++i) {
+        const SecantResult s = preflight(list.items[i], rules);
+        if (s != SECANT_SUCCESS) return s;
+    }
     return SECANT_SUCCESS;
 }
 
