@@ -228,8 +228,31 @@ __device__ __forceinline__ void put_insn(SbInsn* at, SbInsn ins) {
     SB_DIV_CONSTANTS SB_DIV_PAIR("%0", "%8") SB_DIV_PAIR("%1", "%9") SB_DIV_PAIR("%2", "%10") SB_DIV_PAIR("%3", "%11") \
     SB_DIV_PAIR("%4", "%12") SB_DIV_PAIR("%5", "%13") SB_DIV_PAIR("%6", "%14") SB_DIV_PAIR("%7", "%15") SB_GO
 
-/* without the functions (approximate mathematics) they and the divisions leave the block */
-#define SB_NO_FUNCTIONS "SI:\n CO:\n EX:\n LG:\n DV:\n bra.uni LEAVE;\n"
+/* The approximate functions: the hardware's, in the forms that flush subnormal numbers where the
+ * arguments show that there are none to flush (the other forms scale before and after: 5 to 8
+ * instructions per element instead of 1 or 2; both forms give the same bits there, tried for every
+ * argument).  The rest leaves the block as above.  1,024 programs x 16 sets x 1,048,583 rows: 27.6 ms with
+ * these functions outside the block, 22.2 inside it. */
+#define SB_FAST_TWO(OP, A) "mov.b64 {f0, f1}, " A ";\n " OP " f0, f0;\n " OP " f1, f1;\n mov.b64 " A ", {f0, f1};\n"
+#define SB_FAST_SIN(A) SB_FAST_TWO("sin.approx.f32", A)
+#define SB_FAST_COS(A) SB_FAST_TWO("cos.approx.f32", A)
+#define SB_FAST_EXP(A) "mul.rn.f32x2 " A ", " A ", k0;\n" SB_FAST_TWO("ex2.approx.ftz.f32", A)
+#define SB_FAST_LOG(A) SB_FAST_TWO("lg2.approx.ftz.f32", A) "mul.rn.f32x2 " A ", " A ", k0;\n"
+#define SB_FAST_DIV(A, B) SB_FAST_TWO("rcp.approx.ftz.f32", B) "mul.rn.f32x2 " A ", " A ", " B ";\n"
+#define SB_FAST_FUNCTIONS                                                                               \
+    "CO:\n" SB_NEXT SB_EACH(SB_FAST_COS) SB_GO                                                          \
+    "SI:\n" SB_NEXT SB_EACH(SB_FAST_SIN) SB_GO                                                          \
+    "EX:\n mov.f32 top, 0f00000000;\n" SB_EACH(SB_TOP) "setp.le.f32 p, top, 0f42AE0000;\n" SB_ALL_OR_LEAVE SB_NEXT \
+    SB_PAIR_CONST("k0", "0x3FB8AA3B3FB8AA3B") SB_EACH(SB_FAST_EXP) SB_GO                                \
+    "LG:\n mov.f32 low, 0f7F800000;\n" SB_EACH(SB_LOW) "setp.ge.f32 p, low, 0f00800000;\n" SB_ALL_OR_LEAVE SB_NEXT \
+    SB_PAIR_CONST("k0", "0x3F3172183F317218") SB_EACH(SB_FAST_LOG) SB_GO                                \
+    "DV:\n mov.f32 top, 0f00000000;\n mov.f32 low, 0f7F800000;\n" \
+    SB_TOP("%8") SB_TOP("%9") SB_TOP("%10") SB_TOP("%11") SB_TOP("%12") SB_TOP("%13") SB_TOP("%14") SB_TOP("%15") \
+    SB_LOW_ABS("%8") SB_LOW_ABS("%9") SB_LOW_ABS("%10") SB_LOW_ABS("%11") SB_LOW_ABS("%12") SB_LOW_ABS("%13") SB_LOW_ABS("%14") SB_LOW_ABS("%15") \
+    "setp.le.f32 p, top, 0f7E800000;\n setp.ge.and.f32 p, low, 0f00800000, p;\n" SB_ALL_OR_LEAVE SB_NEXT \
+    SB_FAST_DIV("%0", "%8") SB_FAST_DIV("%1", "%9") SB_FAST_DIV("%2", "%10") SB_FAST_DIV("%3", "%11")   \
+    SB_FAST_DIV("%4", "%12") SB_FAST_DIV("%5", "%13") SB_FAST_DIV("%6", "%14") SB_FAST_DIV("%7", "%15") SB_GO
+
 #define SB_CORE(N, FUNCTIONS)                                                                           \
     "{\n" SB_PTX_REGISTERS                                                                             \
     ".reg .u32 hb;\n targets: .branchtargets EN, LR, LC, LS, ST, SH, AR, AC, AS, SR, SC, SS, RR, RC, RS, MR, MC, MS, NG, AB, " \
@@ -416,11 +439,11 @@ struct Machine {
                      : "memory")
 #pragma unroll 1
         for (;;) {
-            if constexpr (RR == 4 && FAST) SB_RUN_CORE(4, SB_NO_FUNCTIONS);
+            if constexpr (RR == 4 && FAST) SB_RUN_CORE(4, SB_FAST_FUNCTIONS);
             else if constexpr (RR == 4) SB_RUN_CORE(4, SB_FUNCTIONS);
-            else if constexpr (RR == 8 && FAST) SB_RUN_CORE(8, SB_NO_FUNCTIONS);
+            else if constexpr (RR == 8 && FAST) SB_RUN_CORE(8, SB_FAST_FUNCTIONS);
             else if constexpr (RR == 8) SB_RUN_CORE(8, SB_FUNCTIONS);
-            else if constexpr (FAST) SB_RUN_CORE(16, SB_NO_FUNCTIONS);
+            else if constexpr (FAST) SB_RUN_CORE(16, SB_FAST_FUNCTIONS);
             else SB_RUN_CORE(16, SB_FUNCTIONS);
             if (h == 0u) return;
             asm volatile("ld.shared.u32 %0, [%1+-16];" : "=r"(h) : "r"(ip) : "memory"); /* of the instruction the core stopped at */
