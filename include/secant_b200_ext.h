@@ -171,8 +171,10 @@ typedef struct SecantB200Rk4Run {
 SECANT_DEC SecantResult secant_b200_rk4_score(const SecantB200Rk4Run* run);
 /* The call's record buffers come from a stream-ordered memory pool of the library's own (one per
  * device, created on first use), which keeps what the largest call so far needed: allocating and
- * freeing them with cudaMalloc/cudaFree cost 2 to 300 ms per call.  This returns the cached memory of
- * every device to the driver; buffers of calls in flight are not touched. */
+ * freeing them with cudaMalloc/cudaFree cost 2 to 300 ms per call.  Up to four sets of streams, events and
+ * pinned buffers (64 MiB a set) and up to fifteen helper threads are kept between calls too.  This returns
+ * the cached memory of every device to the driver, destroys the idle sets and joins the threads; what
+ * calls in flight use is not touched. */
 SECANT_DEC SecantResult secant_b200_release_cached_memory(void);
 
 /*
