@@ -75,7 +75,7 @@ enum Handler : uint32_t {
     H_ADD = 6, H_SUB = 9, H_RSUB = 12, H_MUL = 15, /* + kind */
     H_NEG = 18, H_ABS = 19,
     H_DIV = 20, H_RDIV = 23,                       /* + kind: X is fetched, then the block is left */
-    H_SIN = 26, H_COS, H_EXP, H_LOG,               /* the block is left; word 1 = SB_UN_* */
+    H_SIN = 26, H_COS, H_EXP, H_LOG, H_TANH,       /* unusual arguments leave the block; word 1 = SB_UN_* */
     H_UNARY,                                       /* any other function, word 1 = SB_UN_* */
     H_RARE,                                        /* word 1 = the record's word 0 */
     H_COUNT
@@ -105,7 +105,7 @@ struct HandlerTable {
             else if (cs >= SB_CASE_UN && cs < SB_CASE_FMA) {
                 const unsigned un = cs - SB_CASE_UN;
                 const unsigned h = un == SB_UN_NEG ? H_NEG : un == SB_UN_ABS ? H_ABS : un == SB_UN_SIN ? H_SIN : un == SB_UN_COS ? H_COS
-                                 : un == SB_UN_EXP ? H_EXP : un == SB_UN_LOG ? H_LOG : H_UNARY;
+                                 : un == SB_UN_EXP ? H_EXP : un == SB_UN_LOG ? H_LOG : un == SB_UN_TANH ? H_TANH : H_UNARY;
                 e = h | un << 16;
             }
             entry[cs] = e;
@@ -218,6 +218,7 @@ __device__ __forceinline__ void put_insn(SbInsn* at, SbInsn ins) {
     SB_SIN_CONSTANTS SB_EACH(SB_SIN_PAIR) SB_GO                                                         \
     "EX:\n mov.f32 top, 0f00000000;\n" SB_EACH(SB_TOP) "setp.le.f32 p, top, 0f42AC0000;\n" SB_ALL_OR_LEAVE SB_NEXT \
     SB_EXP_CONSTANTS SB_MINUS_ONE SB_EACH(SB_EXP_PAIR) SB_GO                                            \
+    "TH:\n" SB_NEXT SB_TANH_CONSTANTS SB_MINUS_ONE SB_EACH(SB_TANH_PAIR) SB_GO                          \
     "LG:\n mov.f32 top, 0f00000000;\n mov.f32 low, 0f7F800000;\n" SB_EACH(SB_TOP) SB_EACH(SB_LOW)       \
     "setp.lt.f32 p, top, 0f7F800000;\n setp.ge.and.f32 p, low, 0f00800000, p;\n" SB_ALL_OR_LEAVE SB_NEXT \
     SB_LOG_CONSTANTS SB_MINUS_ONE SB_EACH(SB_LOG_PAIR) SB_GO                                            \
@@ -236,11 +237,13 @@ __device__ __forceinline__ void put_insn(SbInsn* at, SbInsn ins) {
 #define SB_FAST_TWO(OP, A) "mov.b64 {f0, f1}, " A ";\n " OP " f0, f0;\n " OP " f1, f1;\n mov.b64 " A ", {f0, f1};\n"
 #define SB_FAST_SIN(A) SB_FAST_TWO("sin.approx.f32", A)
 #define SB_FAST_COS(A) SB_FAST_TWO("cos.approx.f32", A)
+#define SB_FAST_TANH(A) SB_FAST_TWO("tanh.approx.f32", A)
 #define SB_FAST_EXP(A) "mul.rn.f32x2 " A ", " A ", k0;\n" SB_FAST_TWO("ex2.approx.ftz.f32", A)
 #define SB_FAST_LOG(A) SB_FAST_TWO("lg2.approx.ftz.f32", A) "mul.rn.f32x2 " A ", " A ", k0;\n"
 #define SB_FAST_DIV(A, B) SB_FAST_TWO("rcp.approx.ftz.f32", B) "mul.rn.f32x2 " A ", " A ", " B ";\n"
 #define SB_FAST_FUNCTIONS                                                                               \
     "CO:\n" SB_NEXT SB_EACH(SB_FAST_COS) SB_GO                                                          \
+    "TH:\n" SB_NEXT SB_EACH(SB_FAST_TANH) SB_GO                                                         \
     "SI:\n" SB_NEXT SB_EACH(SB_FAST_SIN) SB_GO                                                          \
     "EX:\n mov.f32 top, 0f00000000;\n" SB_EACH(SB_TOP) "setp.le.f32 p, top, 0f42AE0000;\n" SB_ALL_OR_LEAVE SB_NEXT \
     SB_PAIR_CONST("k0", "0x3FB8AA3B3FB8AA3B") SB_EACH(SB_FAST_EXP) SB_GO                                \
@@ -256,7 +259,7 @@ __device__ __forceinline__ void put_insn(SbInsn* at, SbInsn ins) {
 #define SB_CORE(N, FUNCTIONS)                                                                           \
     "{\n" SB_PTX_REGISTERS                                                                             \
     ".reg .u32 hb;\n targets: .branchtargets EN, LR, LC, LS, ST, SH, AR, AC, AS, SR, SC, SS, RR, RC, RS, MR, MC, MS, NG, AB, " \
-    "DR, DC, DS, QR, QC, QS, SI, CO, EX, LG, LEAVE, LEAVE;\n"                                           \
+    "DR, DC, DS, QR, QC, QS, SI, CO, EX, LG, TH, LEAVE, LEAVE;\n"                                           \
     "ld.shared.u32 %17, [%16+-8];\n" SB_NEXT SB_GO                                                       \
     SB_THREE(N, "L", SB_MOV8) SB_THREE(N, "A", SB_ADD8) SB_THREE(N, "S", SB_SUB8) SB_THREE(N, "R", SB_RSUB8) \
     SB_THREE(N, "M", SB_MUL8) SB_DIVISIONS(N)                                                           \

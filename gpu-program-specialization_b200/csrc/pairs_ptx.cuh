@@ -11,7 +11,7 @@
 #ifndef SECANT_B200_PAIRS_PTX_CUH
 #define SECANT_B200_PAIRS_PTX_CUH
 
-#define SB_PTX_REGISTERS ".reg .u32 ad, c0, c1, c2, c3;\n .reg .f32 f0, f1, top, low;\n .reg .b64 m, t, n, r, z, q, hf, nh, mone, k<12>;\n .reg .pred p;\n"
+#define SB_PTX_REGISTERS ".reg .u32 ad, c0, c1, c2, c3, c4, c5;\n .reg .f32 f0, f1, top, low;\n .reg .b64 m, t, n, r, z, q, hf, nh, mone, k<12>;\n .reg .pred p;\n"
 #define SB_PAIR_CONST(R, BITS) "mov.b64 " R ", " BITS ";\n"
 #define SB_TOP(A) "mov.b64 {f0, f1}, " A ";\n max.NaN.abs.f32 top, top, f0, f1;\n"
 #define SB_LOW(A) "mov.b64 {f0, f1}, " A ";\n min.NaN.f32 low, low, f0, f1;\n"
@@ -68,6 +68,28 @@
     "fma.rn.f32x2 q, t, r, n;\n fma.rn.f32x2 t, " B ", q, " A ";\n fma.rn.f32x2 q, t, r, q;\n"           \
     "mov.b64 {c0, c1}, q;\n mov.b64 {c2, c3}, n;\n lop3.b32 c0, c0, c2, 0x80000000, 0x72;\n lop3.b32 c1, c1, c3, 0x80000000, 0x72;\n" \
     "mov.b64 " A ", {c0, c1};\n"
+/* tanh of anything.  Below 0.9 an odd polynomial (relative error 2^-29.8 before rounding, fitted by weighted
+ * least squares), from there on 1 - 2 / (e^2|x| + 1) with the exponential's steps and one Newton step on
+ * the reciprocal, |x| cut at 10 where the result is 1; both are computed and one is chosen.  NaN takes the
+ * polynomial's side.  At most 1.3 ulp off (all float32 arguments; CUDA's function: 1.8). */
+#define SB_TANH_CONSTANTS \
+    SB_PAIR_CONST("k0", "0xB9EECA99B9EECA99") SB_PAIR_CONST("k1", "0x3B2941E73B2941E7") SB_PAIR_CONST("k2", "0xBC0767FDBC0767FD") \
+    SB_PAIR_CONST("k3", "0x3CB177BC3CB177BC") SB_PAIR_CONST("k4", "0xBD5CE4F8BD5CE4F8") SB_PAIR_CONST("k5", "0x3E08879A3E08879A") \
+    SB_PAIR_CONST("k6", "0xBEAAAAA7BEAAAAA7") SB_PAIR_CONST("k7", "0x4038AA3B4038AA3B") SB_PAIR_CONST("k8", "0x3325706033257060") \
+    SB_PAIR_CONST("k9", "0x4B4000004B400000") SB_PAIR_CONST("k10", "0x3F8000003F800000") SB_PAIR_CONST("k11", "0x4000000040000000")
+#define SB_TANH_PAIR(A)                                                                                 \
+    "mov.b64 {c2, c3}, " A ";\n and.b32 c2, c2, 0x7fffffff;\n and.b32 c3, c3, 0x7fffffff;\n mov.b64 m, {c2, c3};\n" \
+    "mul.rn.f32x2 z, m, m;\n mov.b32 f0, c2;\n mov.b32 f1, c3;\n min.f32 f0, f0, 0f41200000;\n min.f32 f1, f1, 0f41200000;\n mov.b64 n, {f0, f1};\n" \
+    "fma.rn.f32x2 t, n, k7, k9;\n fma.rn.f32x2 q, k0, z, k1;\n fma.rn.f32x2 r, t, mone, k9;\n fma.rn.f32x2 q, q, z, k2;\n" \
+    "fma.rn.f32x2 r, n, k7, r;\n fma.rn.f32x2 q, q, z, k3;\n fma.rn.f32x2 r, n, k8, r;\n fma.rn.f32x2 q, q, z, k4;\n" \
+    "mov.b64 {f0, f1}, r;\n ex2.approx.ftz.f32 f0, f0;\n ex2.approx.ftz.f32 f1, f1;\n fma.rn.f32x2 q, q, z, k5;\n fma.rn.f32x2 q, q, z, k6;\n" \
+    "mov.b64 {c0, c1}, t;\n shl.b32 c0, c0, 23;\n shl.b32 c1, c1, 23;\n mov.b32 c4, f0;\n mov.b32 c5, f1;\n add.u32 c0, c0, c4;\n add.u32 c1, c1, c5;\n" \
+    "mov.b64 n, {c0, c1};\n add.rn.f32x2 n, n, k10;\n mov.b64 {f0, f1}, n;\n neg.f32 f0, f0;\n neg.f32 f1, f1;\n" \
+    "rcp.approx.ftz.f32 f0, f0;\n rcp.approx.ftz.f32 f1, f1;\n mul.rn.f32x2 z, m, z;\n fma.rn.f32x2 q, z, q, m;\n mov.b64 r, {f0, f1};\n" \
+    "fma.rn.f32x2 t, n, r, k10;\n fma.rn.f32x2 r, r, t, r;\n fma.rn.f32x2 r, r, k11, k10;\n"          \
+    "mov.b64 {c0, c1}, q;\n mov.b64 {c4, c5}, r;\n mov.b32 f0, c2;\n mov.b32 f1, c3;\n"               \
+    "setp.ge.f32 p, f0, 0f3F666666;\n selp.b32 c0, c4, c0, p;\n setp.ge.f32 p, f1, 0f3F666666;\n selp.b32 c1, c5, c1, p;\n" \
+    "mov.b64 {c2, c3}, " A ";\n lop3.b32 c0, c0, c2, 0x7fffffff, 0xE4;\n lop3.b32 c1, c1, c3, 0x7fffffff, 0xE4;\n mov.b64 " A ", {c0, c1};\n"
 /* |b| within [2^-60, 2^60], |a| too or zero (2|a| - 1 in bits: zero wraps to the top): no step leaves the normal range */
 #define SB_LEAST(A) "mov.b64 {c0, c1}, " A ";\n shl.b32 c0, c0, 1;\n shl.b32 c1, c1, 1;\n sub.u32 c0, c0, 1;\n sub.u32 c1, c1, 1;\n min.u32 c2, c2, c0;\n min.u32 c2, c2, c1;\n"
 /* after SB_LEAST over the dividends, SB_TOP over both, SB_LOW_ABS over the divisors (c2 = ~0, top = 0, low = inf before) */

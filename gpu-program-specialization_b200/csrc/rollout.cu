@@ -79,7 +79,7 @@ __device__ __forceinline__ void sts(uint32_t a, const float (&x)[RR]) {
  * integrator's part included.  In a chain of them one takes 75 cycles for an addition with any operand,
  * 110 for an exponential, 200 for a sine or a division (one warp alone on its SM). */
 enum { H_END = 0, H_LOAD = 1, H_STORE = 4, H_STLOAD = 5, H_ADD = 8, H_SUB = 11, H_RSUB = 14, H_MUL = 17, H_DIV = 20, H_RDIV = 23, /* + kind */
-       H_MIN = 26, H_MAX = 29, H_NEG = 32, H_ABS = 33, H_SIN = 34, H_COS, H_EXP, H_LOG, H_UNARY, H_FMA };
+       H_MIN = 26, H_MAX = 29, H_NEG = 32, H_ABS = 33, H_SIN = 34, H_COS, H_EXP, H_LOG, H_TANH, H_UNARY, H_FMA };
 enum { RK_CST = 0, RK_STATE = 1, RK_TEMP = 2 };
 constexpr uint32_t kStoredShift = 18, kStoredUnit = 128;
 
@@ -90,7 +90,9 @@ __constant__ __align__(16) unsigned long long kPairConstants[] = {
     0xB2CD31C1B2CD31C1ull, 0x3638B8243638B824ull, 0xB9500BECB9500BECull, 0x3C0888863C088886ull, 0xBE2AAAABBE2AAAABull, 0ull,
     0x3FB8AA3B3FB8AA3Bull, 0x4B4000004B400000ull, 0x32A5706032A57060ull, 0ull,
     0xCB400000CB400000ull, 0xBD9C5854BD9C5854ull, 0x3E02AC143E02AC14ull, 0xBE06C251BE06C251ull, 0x3E116D423E116D42ull, 0xBE2A392FBE2A392Full,
-    0x3E4CD0023E4CD002ull, 0xBE800113BE800113ull, 0x3EAAAAAA3EAAAAAAull, 0xBF000000BF000000ull, 0x35BFBE8E35BFBE8Eull, 0x3F3172003F317200ull};
+    0x3E4CD0023E4CD002ull, 0xBE800113BE800113ull, 0x3EAAAAAA3EAAAAAAull, 0xBF000000BF000000ull, 0x35BFBE8E35BFBE8Eull, 0x3F3172003F317200ull,
+    0xB9EECA99B9EECA99ull, 0x3B2941E73B2941E7ull, 0xBC0767FDBC0767FDull, 0x3CB177BC3CB177BCull, 0xBD5CE4F8BD5CE4F8ull, 0x3E08879A3E08879Aull,
+    0xBEAAAAA7BEAAAAA7ull, 0x4038AA3B4038AA3Bull, 0x3325706033257060ull, 0x4B4000004B400000ull, 0x3F8000003F800000ull, 0x4000000040000000ull};
 
 /* The block carries a whole observation interval: the instruction that ends a right-hand side goes on with
  * the integrator's part of the stage (E0 to E3: sum += weight * rhs, the next stage's value of this
@@ -146,7 +148,7 @@ __constant__ __align__(16) unsigned long long kPairConstants[] = {
 #define RK_CORE(N)                                                                                      \
     "{\n" SB_PTX_REGISTERS ".reg .b64 x0, x1;\n .reg .pred meet;\n .reg .u32 hb;\n"                                                        \
     "stages: .branchtargets E0, E1, E2, E3;\n targets: .branchtargets EN, LC, LV, LT, ST, KC, KV, KT, AC, AV, AT, SC, SV, STT, RC, RV, RT, MC, MV, MT, DC, DV, DT, QC, QV, QT, " \
-    "NC, NV, NT, XC, XV, XT, NG, AB, SI, CO, EX, LG, LEAVE, LEAVE;\n mov.b64 mone, %14;\n setp.ne.u32 meet, %25, 0;\n"               \
+    "NC, NV, NT, XC, XV, XT, NG, AB, SI, CO, EX, LG, TH, LEAVE, LEAVE;\n mov.b64 mone, %14;\n setp.ne.u32 meet, %25, 0;\n"               \
     "ld.shared.u32 %1, [%0+-8];\n" RK_NEXT RK_GO                                                         \
     RK_THREE(N, "L", RK_MOV) RK_THREE(N, "A", RK_ADD) RK_THREE(N, "R", RK_RSUB)                         \
     "SC:\n" RK_FETCH_##N("%2") RK_NEXT RK_BOTH_##N(RK_SUB) RK_GO                                         \
@@ -165,6 +167,8 @@ __constant__ __align__(16) unsigned long long kPairConstants[] = {
     "LG:\n" RK_K2("k0", "k1", "128") RK_K2("k2", "k3", "144") RK_K2("k4", "k5", "160") RK_K2("k6", "k7", "176") RK_K2("k8", "k9", "192") \
     RK_K2("k10", "k11", "208") "mov.f32 top, 0f00000000;\n mov.f32 low, 0f7F800000;\n" RK_EACH_##N(SB_TOP) RK_EACH_##N(SB_LOW) \
     "setp.lt.f32 p, top, 0f7F800000;\n setp.ge.and.f32 p, low, 0f00800000, p;\n" SB_ALL_OR_LEAVE RK_NEXT RK_EACH_##N(SB_LOG_PAIR) RK_GO \
+    "TH:\n" RK_K2("k0", "k1", "224") RK_K2("k2", "k3", "240") RK_K2("k4", "k5", "256") RK_K2("k6", "k7", "272") RK_K2("k8", "k9", "288") \
+    RK_K2("k10", "k11", "304") RK_NEXT RK_EACH_##N(SB_TANH_PAIR) RK_GO                                   \
     RK_FETCH_THEN(N, "D", "DIV") RK_FETCH_THEN(N, "Q", "RDIV")                                          \
     /* operand / acc; what leaves for an unusual argument takes the accumulator along as it was */      \
     "RDIV:\n mov.u32 c2, 0xffffffff;\n mov.f32 top, 0f00000000;\n mov.f32 low, 0f7F800000;\n" RK_EACHX_##N(SB_LEAST) \
@@ -309,7 +313,7 @@ __device__ __forceinline__ SbInsn rewritten(SbInsn in, uint32_t table, uint32_t 
     if (cs >= SB_CASE_UN && cs < SB_CASE_FMA) {
         const unsigned un = cs - SB_CASE_UN;
         const unsigned h = un == SB_UN_NEG ? H_NEG : un == SB_UN_ABS ? H_ABS : un == SB_UN_SIN ? H_SIN : un == SB_UN_COS ? H_COS
-                         : un == SB_UN_EXP ? H_EXP : un == SB_UN_LOG ? H_LOG : H_UNARY;
+                         : un == SB_UN_EXP ? H_EXP : un == SB_UN_LOG ? H_LOG : un == SB_UN_TANH ? H_TANH : H_UNARY;
         return SbInsn{h, un};
     }
     if (cs == SB_CASE_FMA) return SbInsn{H_FMA, 0u};
