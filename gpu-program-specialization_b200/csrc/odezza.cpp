@@ -107,6 +107,13 @@ TokenShape token_shape(uint8_t opcode) {
 #undef S
 }
 
+const struct TokenShapes {
+    TokenShape of[256];
+    TokenShapes() {
+        for (unsigned opcode = 0; opcode < 256; ++opcode) of[opcode] = token_shape((uint8_t)opcode);
+    }
+} kTokenShapes;
+
 /* Checks one right-hand side by the reference's rules (projects/odezza/core/o_ast.c:81-174: every
  * token inside the byte count, indices in range, finite literals, toggles over direct leaves
  * only, exactly one value left at the single trailing RETURN, at most 2048 tokens and 128 stack
@@ -118,10 +125,13 @@ OdezzaResult translate(const OdezzaAstProgram& program, size_t states, uint32_t 
     bool leaf[SECANT_AST_MAX_STACK_DEPTH];
     size_t depth = 0, tokens = 0, at = 0;
     bool returned = false;
+    const size_t begin = out.size();
+    out.resize(begin + program.byte_count); /* a token keeps its width */
+    uint8_t* to = out.data() + begin;
     while (at < program.byte_count) {
         if (tokens == 2048 || returned) return ODEZZA_ERROR_AST;
         const uint8_t opcode = program.bytes[at++];
-        const TokenShape shape = token_shape(opcode);
+        const TokenShape shape = kTokenShapes.of[opcode];
         if (!shape.secant || shape.payload > program.byte_count - at) return ODEZZA_ERROR_AST;
         const uint8_t* payload = program.bytes + at;
         ++tokens;
@@ -148,8 +158,8 @@ OdezzaResult translate(const OdezzaAstProgram& program, size_t states, uint32_t 
             if (depth == SECANT_AST_MAX_STACK_DEPTH) return ODEZZA_ERROR_AST;
             leaf[depth++] = true;
         }
-        out.push_back(shape.secant);
-        out.insert(out.end(), payload, payload + shape.payload);
+        *to++ = shape.secant;
+        for (unsigned b = 0; b < shape.payload; ++b) *to++ = payload[b];
         at += shape.payload;
     }
     if (!returned || depth != 1) return ODEZZA_ERROR_AST;

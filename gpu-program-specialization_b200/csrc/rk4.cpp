@@ -145,8 +145,8 @@ public:
         std::lock_guard<std::mutex> lock(mutex_);
         job->tickets = std::min(wanted, kMostHelpers);
         if (!job->tickets) return;
-        jobs_.push_back(job);
         try {
+            jobs_.push_back(job);
             while (threads_.size() < job->tickets) threads_.emplace_back([this, now = generation_] { serve(now); });
         } catch (const std::exception&) {
             /* no memory or no thread to be had: fewer helpers, or none */
@@ -317,6 +317,7 @@ extern "C" SecantResult secant_b200_rk4_score(const SecantB200Rk4Run* given) {
     const size_t num_pieces = (run->num_systems + piece_systems - 1) / piece_systems;
     struct Piece {
         EncodedBatch enc;
+        size_t program = 0, insn = 0, patch = 0, affine = 0, lit = 0; /* where its arrays begin in its launch's */
         std::vector<uint32_t> cost; /* per system: its longest main part's instructions, weighted as the rollout machine executes them */
         SecantResult status = SECANT_SUCCESS;
     };
@@ -398,9 +399,10 @@ extern "C" SecantResult secant_b200_rk4_score(const SecantB200Rk4Run* given) {
             scan_one(c);
         }
     };
+    const bool one_launch = num_chunks == 1;
     auto worker = [&]() {
-        scan_pieces();
-        {
+        if (!one_launch) {
+            scan_pieces();
             std::unique_lock<std::mutex> lock(mutex);
             ready.wait(lock, [&] { return encoding_open || stop.load(); });
         }
@@ -428,8 +430,17 @@ extern "C" SecantResult secant_b200_rk4_score(const SecantB200Rk4Run* given) {
     };
     help.job.work = worker;
     helpers().start(&help.job, std::min<size_t>(num_pieces - 1, (hardware ? hardware : 1u) - 1u));
-    scan_pieces();
-    {
+    if (one_launch) { /* encoded as a whole before anything is launched: the scan would only make the encoder's checks again */
+        worker();
+        std::unique_lock<std::mutex> lock(mutex);
+        ready.wait(lock, [&] { return std::find(done.begin(), done.end(), 0) == done.end(); });
+        for (size_t c = 0; c < num_pieces && result == SECANT_SUCCESS; ++c) result = pieces[c].status;
+        if (result != SECANT_SUCCESS) { /* the scan's answer comes first */
+            const SecantResult scan = preflight_all(programs.asts, rules);
+            if (scan != SECANT_SUCCESS) result = scan;
+        }
+    } else {
+        scan_pieces();
         std::unique_lock<std::mutex> lock(mutex);
         ready.wait(lock, [&] { return scanned == num_pieces; });
         for (size_t c = 0; c < num_pieces && result == SECANT_SUCCESS; ++c) result = pieces[c].status; /* the first failing program in order */
@@ -486,6 +497,7 @@ extern "C" SecantResult secant_b200_rk4_score(const SecantB200Rk4Run* given) {
         size_t n_programs = 0, n_insns = 0, n_patches = 0, n_affines = 0, n_lits = 0;
         for (size_t q = piece0; q < piece1; ++q) {
             const EncodedBatch& part = pieces[q].enc;
+            pieces[q].program = n_programs; pieces[q].insn = n_insns; pieces[q].patch = n_patches; pieces[q].affine = n_affines; pieces[q].lit = n_lits;
             n_programs += part.programs.size(); n_insns += part.insns.size(); n_patches += part.patches.size();
             n_affines += part.affines.size(); n_lits += part.lits.size();
             enc.max_insn = std::max(enc.max_insn, part.max_insn); enc.max_extra = std::max(enc.max_extra, part.max_extra);
@@ -514,35 +526,45 @@ extern "C" SecantResult secant_b200_rk4_score(const SecantB200Rk4Run* given) {
         }
         std::memset(host + o_flag, 0, o_order - o_flag); /* the flag and the queue's counter start from zero */
         {
-            size_t at_program = 0, at_insn = 0, at_patch = 0, at_affine = 0, at_lit = 0;
-            for (size_t q = piece0; q < piece1; ++q) {
-                EncodedBatch& part = pieces[q].enc;
-                SbProgram* out = reinterpret_cast<SbProgram*>(host) + at_program;
-                for (size_t i = 0; i < part.programs.size(); ++i) {
-                    SbProgram pr = part.programs[i];
-                    pr.insn_off += (uint32_t)at_insn; pr.patch_off += (uint32_t)at_patch;
-                    pr.affine_off += (uint32_t)at_affine; pr.lit_off += (uint32_t)at_lit;
-                    out[i] = pr;
+            /* every piece is copied by whoever takes it (4,096 systems of three states: 0.95 ms by one thread) */
+            std::atomic<size_t> next_join{piece0};
+            const auto join = [&]() {
+                for (;;) {
+                    const size_t q = next_join.fetch_add(1);
+                    if (q >= piece1) return;
+                    EncodedBatch& part = pieces[q].enc;
+                    const size_t at_insn = pieces[q].insn, at_patch = pieces[q].patch, at_affine = pieces[q].affine, at_lit = pieces[q].lit;
+                    SbProgram* out = reinterpret_cast<SbProgram*>(host) + pieces[q].program;
+                    for (size_t i = 0; i < part.programs.size(); ++i) {
+                        SbProgram pr = part.programs[i];
+                        pr.insn_off += (uint32_t)at_insn; pr.patch_off += (uint32_t)at_patch;
+                        pr.affine_off += (uint32_t)at_affine; pr.lit_off += (uint32_t)at_lit;
+                        out[i] = pr;
+                    }
+                    if (!part.insns.empty()) std::memcpy(host + o_insn + at_insn * sizeof(SbInsn), part.insns.data(), part.insns.size() * sizeof(SbInsn));
+                    if (!part.patches.empty()) std::memcpy(host + o_patch + at_patch * sizeof(SbPatch), part.patches.data(), part.patches.size() * sizeof(SbPatch));
+                    if (!part.affines.empty()) std::memcpy(host + o_aff + at_affine * sizeof(SbAffine), part.affines.data(), part.affines.size() * sizeof(SbAffine));
+                    if (!part.lits.empty()) std::memcpy(host + o_lit + at_lit * sizeof(float), part.lits.data(), part.lits.size() * sizeof(float));
+                    part = EncodedBatch(); /* the piece's own copy is not needed any more */
                 }
-                if (!part.insns.empty()) std::memcpy(host + o_insn + at_insn * sizeof(SbInsn), part.insns.data(), part.insns.size() * sizeof(SbInsn));
-                if (!part.patches.empty()) std::memcpy(host + o_patch + at_patch * sizeof(SbPatch), part.patches.data(), part.patches.size() * sizeof(SbPatch));
-                if (!part.affines.empty()) std::memcpy(host + o_aff + at_affine * sizeof(SbAffine), part.affines.data(), part.affines.size() * sizeof(SbAffine));
-                if (!part.lits.empty()) std::memcpy(host + o_lit + at_lit * sizeof(float), part.lits.data(), part.lits.size() * sizeof(float));
-                at_program += part.programs.size(); at_insn += part.insns.size(); at_patch += part.patches.size();
-                at_affine += part.affines.size(); at_lit += part.lits.size();
-                part = EncodedBatch(); /* the piece's own copy is not needed any more */
-            }
+            };
+            Helpers::Job joining;
+            joining.work = std::ref(join);
+            helpers().start(&joining, piece1 - piece0 - 1);
+            join();
+            helpers().finish(&joining);
             /* Warps take the launch's systems costliest first: a candidate that stays valid runs for its
              * full length, and the long ones should not be the last to start. */
             const size_t n_systems = n_programs / S;
             uint32_t* order = reinterpret_cast<uint32_t*>(host + o_order);
             for (size_t i = 0; i < n_systems; ++i) order[i] = (uint32_t)i;
             try {
-                std::vector<uint32_t> cost;
-                cost.reserve(n_systems);
-                for (size_t q = piece0; q < piece1; ++q) cost.insert(cost.end(), pieces[q].cost.begin(), pieces[q].cost.end());
-                if (cost.size() == n_systems)
-                    std::stable_sort(order, order + n_systems, [&](uint32_t a, uint32_t b) { return cost[a] > cost[b]; });
+                std::vector<uint64_t> keys; /* costliest first, equal costs in their own order */
+                keys.reserve(n_systems);
+                for (size_t q = piece0; q < piece1; ++q)
+                    for (uint32_t cost : pieces[q].cost) keys.push_back((uint64_t)(0xffffffffu - cost) << 32 | keys.size());
+                std::sort(keys.begin(), keys.end());
+                for (size_t i = 0; i < n_systems && i < keys.size(); ++i) order[i] = (uint32_t)keys[i];
             } catch (const std::bad_alloc&) {
                 /* no memory for the sort: the systems are taken in their own order */
             }
