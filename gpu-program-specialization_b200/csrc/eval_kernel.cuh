@@ -222,10 +222,13 @@ __device__ __forceinline__ void put_insn(SbInsn* at, SbInsn ins) {
     "LG:\n mov.f32 top, 0f00000000;\n mov.f32 low, 0f7F800000;\n" SB_EACH(SB_TOP) SB_EACH(SB_LOW)       \
     "setp.lt.f32 p, top, 0f7F800000;\n setp.ge.and.f32 p, low, 0f00800000, p;\n" SB_ALL_OR_LEAVE SB_NEXT \
     SB_LOG_CONSTANTS SB_MINUS_ONE SB_EACH(SB_LOG_PAIR) SB_GO                                            \
-    "DV:\n mov.u32 c2, 0xffffffff;\n" SB_EACH(SB_LEAST) "mov.f32 top, 0f00000000;\n mov.f32 low, 0f7F800000;\n" \
+    "DV:\n mov.f32 top, 0f00000000;\n mov.f32 low, 0f7F800000;\n"                                      \
     SB_EACH(SB_TOP) SB_TOP("%8") SB_TOP("%9") SB_TOP("%10") SB_TOP("%11") SB_TOP("%12") SB_TOP("%13") SB_TOP("%14") SB_TOP("%15") \
+    SB_EACH(SB_LOW_ABS) SB_LOW_ABS("%8") SB_LOW_ABS("%9") SB_LOW_ABS("%10") SB_LOW_ABS("%11") SB_LOW_ABS("%12") SB_LOW_ABS("%13") SB_LOW_ABS("%14") SB_LOW_ABS("%15") \
+    SB_DIV_USUAL "@p bra.uni DW;\n"                                                                     \
+    "mov.u32 c2, 0xffffffff;\n" SB_EACH(SB_LEAST) "mov.f32 low, 0f7F800000;\n"                          \
     SB_LOW_ABS("%8") SB_LOW_ABS("%9") SB_LOW_ABS("%10") SB_LOW_ABS("%11") SB_LOW_ABS("%12") SB_LOW_ABS("%13") SB_LOW_ABS("%14") SB_LOW_ABS("%15") \
-    SB_DIV_RANGE SB_ALL_OR_LEAVE SB_NEXT                                                                \
+    SB_DIV_RANGE SB_ALL_OR_LEAVE "DW:\n" SB_NEXT                                                       \
     SB_DIV_CONSTANTS SB_DIV_PAIR("%0", "%8") SB_DIV_PAIR("%1", "%9") SB_DIV_PAIR("%2", "%10") SB_DIV_PAIR("%3", "%11") \
     SB_DIV_PAIR("%4", "%12") SB_DIV_PAIR("%5", "%13") SB_DIV_PAIR("%6", "%14") SB_DIV_PAIR("%7", "%15") SB_GO
 

@@ -33,7 +33,8 @@
 #define SB_DIV_CONSTANTS \
     SB_PAIR_CONST("k0", "0x3F8000003F800000")
 #define SB_MINUS_ONE "mov.b64 mone, 0xBF800000BF800000;\n"
-/* sin and cos differ in the shift by half a turn, taken off again after the rounding */
+/* (the sign is added: shift and addition are one instruction, shift and xor two)
+ * sin and cos differ in the shift by half a turn, taken off again after the rounding */
 #define SB_SIN_SHIFT "mov.b64 hf, 0;\n mov.b64 nh, 0x8000000080000000;\n"
 #define SB_COS_SHIFT "mov.b64 hf, 0x3F0000003F000000;\n mov.b64 nh, 0xBF000000BF000000;\n"
 #define SB_SIN_PAIR(A)                                                                                  \
@@ -41,17 +42,18 @@
     "fma.rn.f32x2 r, n, k3, " A ";\n fma.rn.f32x2 r, n, k4, r;\n fma.rn.f32x2 r, n, k5, r;\n mul.rn.f32x2 z, r, r;\n" \
     "fma.rn.f32x2 q, k6, z, k7;\n fma.rn.f32x2 q, q, z, k8;\n fma.rn.f32x2 q, q, z, k9;\n fma.rn.f32x2 q, q, z, k10;\n" \
     "mul.rn.f32x2 z, r, z;\n fma.rn.f32x2 r, z, q, r;\n mov.b64 {c0, c1}, t;\n shl.b32 c0, c0, 31;\n shl.b32 c1, c1, 31;\n" \
-    "mov.b64 t, {c0, c1};\n xor.b64 " A ", r, t;\n"
+    "mov.b64 {c2, c3}, r;\n add.u32 c0, c0, c2;\n add.u32 c1, c1, c3;\n mov.b64 " A ", {c0, c1};\n"
 #define SB_EXP_PAIR(A)                                                                                  \
     "fma.rn.f32x2 t, " A ", k0, k1;\n fma.rn.f32x2 n, t, mone, k1;\n fma.rn.f32x2 r, " A ", k0, n;\n fma.rn.f32x2 r, " A ", k2, r;\n" \
     "mov.b64 {f0, f1}, r;\n ex2.approx.ftz.f32 f0, f0;\n ex2.approx.ftz.f32 f1, f1;\n mov.b64 {c0, c1}, t;\n" \
     "shl.b32 c0, c0, 23;\n shl.b32 c1, c1, 23;\n mov.b32 c2, f0;\n mov.b32 c3, f1;\n add.u32 c0, c0, c2;\n add.u32 c1, c1, c3;\n" \
     "mov.b64 " A ", {c0, c1};\n"
-/* the exponent becomes a float through the low bits of 1.5 * 2^23: exact, and off the conversion unit */
+/* the exponent becomes a float through the low bits of 1.5 * 2^23: exact, and off the conversion unit; the
+ * mantissa is what is left when it is taken off the argument's bits (2^23 times the constant is 0 mod 2^32) */
 #define SB_LOG_PAIR(A)                                                                                  \
-    "mov.b64 {c0, c1}, " A ";\n add.u32 c0, c0, 0xC0CAFB0D;\n add.u32 c1, c1, 0xC0CAFB0D;\n"             \
-    "shr.s32 c2, c0, 23;\n shr.s32 c3, c1, 23;\n add.u32 c2, c2, 0x4B400000;\n add.u32 c3, c3, 0x4B400000;\n mov.b64 n, {c2, c3};\n" \
-    "and.b32 c0, c0, 0x7fffff;\n and.b32 c1, c1, 0x7fffff;\n add.u32 c0, c0, 0x3F3504F3;\n add.u32 c1, c1, 0x3F3504F3;\n mov.b64 r, {c0, c1};\n" \
+    "mov.b64 {c0, c1}, " A ";\n add.u32 c2, c0, 0xC0CAFB0D;\n add.u32 c3, c1, 0xC0CAFB0D;\n"             \
+    "shr.s32 c2, c2, 23;\n shr.s32 c3, c3, 23;\n add.u32 c2, c2, 0x4B400000;\n add.u32 c3, c3, 0x4B400000;\n mov.b64 n, {c2, c3};\n" \
+    "mad.lo.u32 c0, c2, 0xFF800000, c0;\n mad.lo.u32 c1, c3, 0xFF800000, c1;\n mov.b64 r, {c0, c1};\n" \
     "add.rn.f32x2 n, n, k0;\n add.rn.f32x2 r, r, mone;\n fma.rn.f32x2 q, k1, r, k2;\n fma.rn.f32x2 q, q, r, k3;\n fma.rn.f32x2 q, q, r, k4;\n" \
     "fma.rn.f32x2 q, q, r, k5;\n fma.rn.f32x2 q, q, r, k6;\n fma.rn.f32x2 q, q, r, k7;\n fma.rn.f32x2 q, q, r, k8;\n mul.rn.f32x2 z, r, r;\n" \
     "mul.rn.f32x2 t, k9, z;\n mul.rn.f32x2 z, r, z;\n fma.rn.f32x2 t, z, q, t;\n fma.rn.f32x2 t, n, k10, t;\n add.rn.f32x2 r, r, t;\n" \
@@ -92,6 +94,8 @@
     "mov.b64 {c2, c3}, " A ";\n lop3.b32 c0, c0, c2, 0x7fffffff, 0xE4;\n lop3.b32 c1, c1, c3, 0x7fffffff, 0xE4;\n mov.b64 " A ", {c0, c1};\n"
 /* |b| within [2^-60, 2^60], |a| too or zero (2|a| - 1 in bits: zero wraps to the top): no step leaves the normal range */
 #define SB_LEAST(A) "mov.b64 {c0, c1}, " A ";\n shl.b32 c0, c0, 1;\n shl.b32 c1, c1, 1;\n sub.u32 c0, c0, 1;\n sub.u32 c1, c1, 1;\n min.u32 c2, c2, c0;\n min.u32 c2, c2, c1;\n"
+/* no zero among the dividends, the usual case: SB_TOP and SB_LOW_ABS over both (top = 0, low = inf before) are enough */
+#define SB_DIV_USUAL "setp.le.f32 p, top, 0f5D800000;\n setp.ge.and.f32 p, low, 0f21800000, p;\n vote.sync.all.pred p, p, 0xffffffff;\n"
 /* after SB_LEAST over the dividends, SB_TOP over both, SB_LOW_ABS over the divisors (c2 = ~0, top = 0, low = inf before) */
 #define SB_DIV_RANGE "setp.le.f32 p, top, 0f5D800000;\n setp.ge.and.f32 p, low, 0f21800000, p;\n setp.ge.and.u32 p, c2, 0x42FFFFFF, p;\n"
 

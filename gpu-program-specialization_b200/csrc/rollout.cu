@@ -171,11 +171,13 @@ __constant__ __align__(16) unsigned long long kPairConstants[] = {
     RK_K2("k10", "k11", "304") RK_NEXT RK_EACH_##N(SB_TANH_PAIR) RK_GO                                   \
     RK_FETCH_THEN(N, "D", "DIV") RK_FETCH_THEN(N, "Q", "RDIV")                                          \
     /* operand / acc; what leaves for an unusual argument takes the accumulator along as it was */      \
-    "RDIV:\n mov.u32 c2, 0xffffffff;\n mov.f32 top, 0f00000000;\n mov.f32 low, 0f7F800000;\n" RK_EACHX_##N(SB_LEAST) \
-    RK_EACH_##N(SB_TOP) RK_EACHX_##N(SB_TOP) RK_EACH_##N(SB_LOW_ABS) SB_DIV_RANGE SB_ALL_OR_LEAVE       \
-    RK_BOTH_##N(RK_SWAP) "bra.uni DW;\n"                                                                \
-    "DIV:\n mov.u32 c2, 0xffffffff;\n mov.f32 top, 0f00000000;\n mov.f32 low, 0f7F800000;\n" RK_EACH_##N(SB_LEAST) \
-    RK_EACH_##N(SB_TOP) RK_EACHX_##N(SB_TOP) RK_EACHX_##N(SB_LOW_ABS) SB_DIV_RANGE SB_ALL_OR_LEAVE      \
+    "RDIV:\n mov.f32 top, 0f00000000;\n mov.f32 low, 0f7F800000;\n" RK_EACH_##N(SB_TOP) RK_EACHX_##N(SB_TOP) \
+    RK_EACH_##N(SB_LOW_ABS) RK_EACHX_##N(SB_LOW_ABS) SB_DIV_USUAL "@p bra.uni RS;\n"                    \
+    "mov.u32 c2, 0xffffffff;\n mov.f32 low, 0f7F800000;\n" RK_EACHX_##N(SB_LEAST) RK_EACH_##N(SB_LOW_ABS) SB_DIV_RANGE SB_ALL_OR_LEAVE \
+    "RS:\n" RK_BOTH_##N(RK_SWAP) "bra.uni DW;\n"                                                       \
+    "DIV:\n mov.f32 top, 0f00000000;\n mov.f32 low, 0f7F800000;\n" RK_EACH_##N(SB_TOP) RK_EACHX_##N(SB_TOP) \
+    RK_EACH_##N(SB_LOW_ABS) RK_EACHX_##N(SB_LOW_ABS) SB_DIV_USUAL "@p bra.uni DW;\n"                    \
+    "mov.u32 c2, 0xffffffff;\n mov.f32 low, 0f7F800000;\n" RK_EACH_##N(SB_LEAST) RK_EACHX_##N(SB_LOW_ABS) SB_DIV_RANGE SB_ALL_OR_LEAVE \
     "DW:\n" RK_NEXT SB_DIV_CONSTANTS RK_BOTH_##N(SB_DIV_PAIR) RK_GO                                      \
     "EN:\n brx.idx.uni %11, stages;\n"                                                                   \
     "E0:\n mov.b64 k0, 0;\n" RK_STAGE_##N(RK_FIRST, "%16", "%17") "bra.uni SWAP;\n"                    \
