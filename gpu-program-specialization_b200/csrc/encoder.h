@@ -32,6 +32,9 @@ struct ProgramRules {
     /* main part: "STORE slot; LOAD x" becomes one instruction (record.h, SB_STORE_THEN_LOAD); only the
      * rollout kernel understands it */
     bool fuse_store_load = false;
+    /* number the toggle bits a program reads 0, 1, ... in its sites and note which they are
+     * (SbProgram::bits, bit_mask): permutations that differ in other bits have the same value */
+    bool number_bits = false;
     /* Records for the population evaluator are split into a bank part, a row prelude and a main
      * part (record.h, SbProgram) and address constants through a per-program table the bank part
      * fills.  Without split_parts (the rollout kernel) a record is one main part that addresses

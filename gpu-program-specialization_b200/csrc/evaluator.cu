@@ -87,13 +87,14 @@ bank_tables_kernel(const DeviceBatch batch, const EvalProblem prob, uint32_t pad
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     float* const tmp = temporaries + (size_t)warp * batch.max_btmp * 32;
     const unsigned long long work = (unsigned long long)batch.num_programs * chunks;
-    const unsigned long long pairs = prob.mode == EVAL_MATERIALIZE ? padded_banks : (unsigned long long)padded_banks << prob.toggle_bits;
+    const unsigned long long pairs = prob.mode == EVAL_MATERIALIZE ? padded_banks : (unsigned long long)padded_banks << batch.max_bits;
     const uint32_t first_cst = batch.programs[0].cst_off;
 #pragma unroll 1
     for (unsigned long long id = (unsigned long long)blockIdx.x * kTableWarps + warp; id < work; id += (unsigned long long)gridDim.x * kTableWarps) {
         const uint32_t lp = (uint32_t)(id / chunks), chunk = (uint32_t)(id - (unsigned long long)lp * chunks);
         const SbProgram* const hp = batch.programs + lp;
-        if (!hp->pre_off) continue;
+        /* nothing to do without a bank part, or beyond the permutations the program tells apart */
+        if (!hp->pre_off || (prob.mode != EVAL_MATERIALIZE && chunk * 32ull >= (unsigned long long)padded_banks << hp->bits)) continue;
         BankSource src;
         src.banks = prob.banks ? prob.banks + (prob.first_program + hp->index) * prob.program_bank_stride : nullptr;
         src.bank_stride = prob.bank_stride;
@@ -107,7 +108,7 @@ bank_tables_kernel(const DeviceBatch batch, const EvalProblem prob, uint32_t pad
         const unsigned long long v = (unsigned long long)chunk * 32u + lane;
         const bool live = v < pairs;
         const uint32_t j = (uint32_t)(v / padded_banks), bank = (uint32_t)(v - (unsigned long long)j * padded_banks);
-        const uint32_t perm = prob.mode == EVAL_MATERIALIZE ? prob.fixed_permutation : j;
+        const uint32_t perm = j; /* numbered by the bits the program reads */
         const bool real = live && bank < src.num_banks;
         float* const mine = tables + (size_t)(hp->cst_off - first_cst) * pairs + ((size_t)j * (padded_banks / RC) + bank / RC) * entries * RC + bank % RC;
         const float* const row = src.banks + (size_t)bank * src.bank_stride;
@@ -177,7 +178,7 @@ __global__ void combine_kernel(const DeviceBatch batch, const EvalProblem prob, 
 template <int RC>
 void launch_tables(const DeviceBatch& batch, const EvalProblem& prob, uint32_t banks, float* tables, cudaStream_t stream) {
     const uint32_t padded = (banks + RC - 1) / RC * RC;
-    const unsigned long long pairs = prob.mode == EVAL_MATERIALIZE ? padded : (unsigned long long)padded << prob.toggle_bits;
+    const unsigned long long pairs = prob.mode == EVAL_MATERIALIZE ? padded : (unsigned long long)padded << batch.max_bits;
     const uint32_t chunks = (uint32_t)((pairs + 31) / 32);
     const unsigned long long work = (unsigned long long)batch.num_programs * chunks;
     const unsigned blocks = (unsigned)std::min<unsigned long long>((work + kTableWarps - 1) / kTableWarps, 148ull * 64ull);
@@ -222,7 +223,9 @@ cudaError_t launch_eval(const DeviceBatch& batch, const EvalProblem& prob, const
     /* a run whose rows are not split has whole sums: they go straight to the caller's grid */
     geom.direct = !materialize && plan.row_splits == 1 ? 1u : 0u;
     float* const sums = geom.direct ? prob.output : partial;
-    const bool span = plan.perms_per_item > 1, one_target = prob.mode == EVAL_SSE && prob.num_targets == 1;
+    /* runs without toggles have a kernel without the permutations' code: with it inside, the population of
+     * 2,048 programs x 64 sets took 34.1 ms instead of 30.0 (registers, not instructions) */
+    const bool span = prob.toggle_bits > 0, one_target = prob.mode == EVAL_SSE && prob.num_targets == 1;
     cudaError_t e = materialize ? launch_materialize(batch, prob, geom, plan, sums, tables, stream)
                     : one_target ? (span ? launch_sse_span : launch_sse)(batch, prob, geom, plan, sums, tables, stream)
                                  : (span ? launch_general_span : launch_general)(batch, prob, geom, plan, sums, tables, stream);

@@ -66,6 +66,8 @@ struct DeviceBatch {
     uint32_t uses_scratch; /* some program needs the scratch spill slot */
     uint64_t total_cst;   /* constant-table entries of all programs (an upper bound will do) */
     uint64_t total_cost;  /* scheduling weights of all programs */
+    double total_perms;   /* permutations with values of their own, of all programs */
+    uint32_t max_bits;    /* most toggle bits a program reads: a program has at most 1 << max_bits of them */
 };
 
 struct EvalProblem {
@@ -83,7 +85,6 @@ struct EvalProblem {
     uint32_t num_constants;
     uint32_t num_banks;       /* >= 1 */
     uint32_t toggle_bits;
-    uint32_t fixed_permutation; /* materialize: the single permutation evaluated */
     uint32_t fast_math;       /* 1: approximate division and transcendental functions (see sbmath.cuh) */
     size_t num_rows;
     float* output;

@@ -11,6 +11,7 @@
 #include "evaluator.cuh"
 
 #include <algorithm>
+#include <cmath>
 
 namespace sb {
 
@@ -55,7 +56,8 @@ namespace {
 size_t smem_needed(const Geom& g, uint32_t warps) { return (size_t)g.tile_bytes * g.tile_buffers + 16 + (size_t)g.warp_bytes * warps; }
 
 /* How a launch is cut into queue items and CTAs when it is small: the sums do not depend on it (they
- * depend on the tiles and the row splits, which stay as they are), so it may follow the machine.
+ * depend on the tiles and the row splits, which stay as they are), so it may follow the machine.  A launch
+ * whose programs read few of the run's toggle bits is small in this sense too.
  *
  * The rules above it aim at large launches, whose grid is many waves deep.  With few programs or rows
  * they gave grids of 150 CTAs on 148 SMs (two waves for one), a dozen items for twenty warps, or half
@@ -66,14 +68,17 @@ size_t smem_needed(const Geom& g, uint32_t warps) { return (size_t)g.tile_bytes 
  * issues 2.6 per cycle at best. */
 struct Cut { uint32_t gpi, ppi; unsigned long long groups; };
 
-double cut_cycles(const LaunchPlan& plan, const Cut& cut, unsigned long long programs, unsigned long long items_per_program, uint32_t passes, size_t tiles,
-                  bool hoists, int sms) {
-    const unsigned long long items = (programs + cut.groups - 1) / cut.groups * items_per_program;
-    const double active = (double)std::min<unsigned long long>(plan.warps, items);
+/* `perms`: the permutations a program has of its own, on the average and at most. */
+double cut_cycles(const LaunchPlan& plan, const Cut& cut, unsigned long long programs, unsigned long long chunks, double perms, double most_perms,
+                  uint32_t passes, size_t tiles, bool hoists, int sms) {
+    const double per_cta = (double)((programs + cut.groups - 1) / cut.groups);
+    const double each = chunks * std::max(1.0, perms / cut.ppi), largest = chunks * std::max(1.0, most_perms / cut.ppi);
+    const double items = std::ceil((per_cta - 1.0) * each + largest), empty = std::max(0.0, per_cta * largest - items);
+    const double active = std::min<double>(plan.warps, items);
     const double rate = std::min(0.14, 2.6 / active);
-    const double item = 900.0 + passes * ((hoists ? 120.0 : 0.0) + 330.0 * cut.gpi * cut.ppi);
-    const double rounds = std::max((double)((items + plan.warps - 1) / plan.warps), (double)items / plan.warps + 0.5);
-    const double cta = 3000.0 + tiles * (1500.0 + rounds * item / rate);
+    const double item = 900.0 + passes * ((hoists ? 120.0 : 0.0) + 330.0 * cut.gpi * std::min<double>(cut.ppi, std::max(1.0, perms)));
+    const double rounds = std::max(std::ceil(items / plan.warps), items / plan.warps + 0.5);
+    const double cta = 3000.0 + tiles * (1500.0 + rounds * item / rate + empty * 400.0 / plan.warps);
     const unsigned long long grid = cut.groups * plan.row_splits;
     return (double)((grid + sms - 1) / sms) * cta;
 }
@@ -90,12 +95,19 @@ void balance_small(LaunchPlan* plan, const DeviceBatch& batch, const EvalProblem
         while (p->warps < 20 && smem_needed(g, p->warps + 1) <= smem_limit) ++p->warps;
         p->smem_bytes = smem_needed(g, p->warps);
     };
+    while (plan->perms_per_item > 1ull << batch.max_bits) plan->perms_per_item /= 2;
     if (plan->tile_buffers == 1) refit(plan);
-    if ((unsigned long long)plan->num_groups * plan->row_splits >= 8ull * (unsigned long long)sms) return; /* deep enough */
+    /* a program has only as many values of its own as it reads toggle bits: the rules above counted all */
+    const bool fewer = !materialize && batch.total_perms < 0.5 * (double)P * (double)(1ull << prob.toggle_bits);
+    if (!fewer && (unsigned long long)plan->num_groups * plan->row_splits >= 8ull * (unsigned long long)sms) return; /* deep enough */
+    const double perms = materialize ? 1.0 : batch.total_perms / (double)P, most_perms = materialize ? 1.0 : (double)(1ull << batch.max_bits);
     const uint32_t passes = (uint32_t)((std::min<size_t>(plan->tile_rows, prob.num_rows) + pass - 1) / pass);
-    const auto items_of = [&](const Cut& c) { return materialize ? 1ull : ((bank_groups / c.gpi) << prob.toggle_bits) / c.ppi; };
+    const auto items_of = [&](const Cut& c) { return materialize ? 1ull : ((bank_groups / c.gpi) << batch.max_bits) / c.ppi; };
+    const auto cycles = [&](const Cut& c) {
+        return cut_cycles(*plan, c, P, bank_groups / c.gpi, perms, most_perms, passes, tiles, batch.max_hoisted != 0, sms);
+    };
     Cut best{plan->groups_per_item, plan->perms_per_item, plan->num_groups};
-    double least = 0.97 * cut_cycles(*plan, best, P, items_of(best), passes, tiles, batch.max_hoisted != 0, sms);
+    double least = 0.97 * cycles(best);
     const Cut widest = best;
     for (uint32_t gpi = widest.gpi; gpi >= 1; --gpi) {
         if (bank_groups % gpi) continue;
@@ -105,7 +117,7 @@ void balance_small(LaunchPlan* plan, const DeviceBatch& batch, const EvalProblem
                 c.groups = std::max<unsigned long long>(1, std::min(c.groups, P));
                 const unsigned long long items = items_of(c);
                 if (items > 0xffffff00ull / ((P + c.groups - 1) / c.groups)) continue;
-                const double t = cut_cycles(*plan, c, P, items, passes, tiles, batch.max_hoisted != 0, sms);
+                const double t = cycles(c);
                 if (t < least) { least = t; best = c; }
             }
     }
@@ -240,7 +252,7 @@ LaunchPlan plan_with_tile(const DeviceBatch& batch, const EvalProblem& prob, int
         plan.partial_elements = (size_t)(n * nq * configs);
     }
     /* constant tables: one float per entry and (padded bank, permutation) */
-    const unsigned long long padded = materialize ? rc : ((unsigned long long)(prob.num_banks + rc - 1) / rc * rc) << prob.toggle_bits;
+    const unsigned long long padded = materialize ? rc : ((unsigned long long)(prob.num_banks + rc - 1) / rc * rc) << batch.max_bits;
     if (batch.total_cst > (~0ull >> 3) / padded) { plan.overflow = true; return plan; }
     plan.table_elements = (size_t)(batch.total_cst * padded);
     plan.table_offset = (plan.partial_elements + 3) / 4 * 4;

@@ -69,7 +69,8 @@ static inline uint32_t sb_w0(unsigned case_id, unsigned aux, unsigned index) {
 /* FMA: aux = kindA | kindB << 2 | kindC << 4 ; w1 = idxA | idxB << 10 | idxC << 20. */
 
 /* One toggle site: instruction `insn` is replaced by alt[choice] for every permutation,
- * choice = bit(bit0) + 2 * bit(bit1); bit1 == 0xff marks a two-way toggle. */
+ * choice = bit(bit0) + 2 * bit(bit1); bit1 == 0xff marks a two-way toggle.  Bits are those of the run's
+ * permutation, or (ProgramRules::number_bits) positions among the bits the program reads. */
 typedef struct SbPatch {
     uint16_t insn;
     uint8_t bit0;
@@ -127,7 +128,8 @@ typedef struct SbProgram {
     uint32_t index;     /* position of the program in the run (output row, bank table) */
     uint32_t cost;      /* scheduling weight: bits 0..15 main part per bank group, bits 16..31 row prelude */
     uint16_t mid_off;
-    uint16_t reserved;
+    uint16_t bits;      /* toggle bits the program reads (0 for the rollout kernel's records) */
+    uint32_t bit_mask;  /* which ones; the sites of its records number them 0 .. bits - 1 in this order */
     uint32_t cst_off;   /* constant-table entries of the programs before this one in launch order (set by the runner) */
 } SbProgram;
 

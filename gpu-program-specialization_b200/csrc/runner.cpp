@@ -323,10 +323,11 @@ constexpr unsigned kLightSlots = 2, kLightTable = 8, kLightHoisted = 4;
 
 bool is_light(const SbProgram& p) { return p.n_slots <= kLightSlots && p.n_cst <= kLightTable && p.n_hoisted <= kLightHoisted; }
 
-/* scheduling weight of a program: one row pass over sixteen bank groups */
+/* scheduling weight of a program: one row pass over sixteen bank groups, for every permutation of its own */
 uint64_t schedule_cost(const SbProgram& p) {
     const uint64_t main_part = p.cost & 0xffffu, prelude = p.cost >> 16;
-    return main_part * ((p.flags & SB_PROG_BANK_INDEPENDENT) ? 1u : 16u) + prelude;
+    const uint64_t once = main_part * ((p.flags & SB_PROG_BANK_INDEPENDENT) ? 1u : 16u) + prelude;
+    return std::min<uint64_t>(once << std::min<unsigned>(p.bits, 32u), 0x1fffffu); /* 21 bits of the order's key */
 }
 
 /* Puts the batch's programs in launch order: light programs first, heavy ones after them; inside each
@@ -440,6 +441,8 @@ SecantResult upload_batch(SecantCubinRunnerImpl* r, Slot& s, std::vector<DeviceB
             db.max_cst = std::max<uint32_t>(db.max_cst, p.n_cst);
             db.total_cst += p.n_cst;
             db.total_cost += schedule_cost(p);
+            db.total_perms += (double)(1ull << p.bits);
+            db.max_bits = std::max<uint32_t>(db.max_bits, p.bits);
             db.max_btmp = std::max<uint32_t>(db.max_btmp, p.n_btmp);
             db.uses_scratch |= (p.flags & SB_PROG_USES_SCRATCH) ? 1u : 0u;
         }
@@ -532,15 +535,16 @@ SecantResult launch_batch(SecantCubinRunnerImpl* r, const DeviceBatch& db, doubl
         /* one launch, unless its constant tables (an entry per program constant and configuration) would
          * take more than the scratch limit: then the programs in as many launches as it takes, and a
          * program at a time at least */
-        const size_t per_program = std::max<size_t>(1, (size_t)db.max_cst * (size_t)((prob.num_banks + 3ull) << prob.toggle_bits));
+        const size_t per_program = std::max<size_t>(1, (size_t)db.max_cst * (size_t)((prob.num_banks + 3ull) << db.max_bits));
         const size_t fit = std::max<size_t>(1, r->scratch_limit / per_program);
-        const size_t step = db.total_cst <= r->scratch_limit / ((prob.num_banks + 3ull) << prob.toggle_bits) ? db.num_programs : fit;
+        const size_t step = db.total_cst <= r->scratch_limit / ((prob.num_banks + 3ull) << db.max_bits) ? db.num_programs : fit;
         for (size_t first = 0; first < db.num_programs && ce == cudaSuccess; first += step) {
             DeviceBatch part = db;
             if (step < db.num_programs) {
                 part.programs += first;
                 part.num_programs = (uint32_t)std::min<size_t>(step, db.num_programs - first);
                 part.total_cst = (uint64_t)part.num_programs * db.max_cst;
+                part.total_perms = db.total_perms * part.num_programs / db.num_programs;
             }
             const LaunchPlan lp = plan_launch(part, prob, r->sm_count, r->smem_limit, r->scratch_limit, share);
             if (!lp.ok) {
@@ -1040,6 +1044,7 @@ SecantResult secant_b200_population_create(SecantCubinRunner r, const SecantAstP
     rules.toggle_bits = rules.banks_allowed ? toggle_bits : 0;
     rules.split_parts = true;
     rules.hoist_bank = true;
+    rules.number_bits = true;
     rules.hoist_row = rules.banks_allowed; /* a population is usually scored against many banks */
     for (size_t i = 0; i < programs->routines.count; ++i) {
         const SecantResult s = preflight(programs->routines.items[i], rules);

@@ -284,7 +284,7 @@ SBT_EXPORT int sbt_plan(uint32_t num_programs, uint32_t max_insn, uint32_t max_s
     DeviceBatch db;
     std::memset(&db, 0, sizeof(db));
     db.num_programs = num_programs; db.max_insn = max_insn; db.max_slots = max_slots; db.max_hoisted = max_hoisted;
-    db.max_cst = max_cst; db.max_btmp = max_btmp;
+    db.max_cst = max_cst; db.max_btmp = max_btmp; db.max_bits = toggle_bits; db.total_perms = (double)num_programs * (double)(1ull << toggle_bits);
     EvalProblem p;
     std::memset(&p, 0, sizeof(p));
     p.mode = mode; p.num_inputs = num_inputs; p.num_targets = num_targets; p.num_banks = num_banks; p.toggle_bits = toggle_bits;

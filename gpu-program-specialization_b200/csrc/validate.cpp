@@ -198,6 +198,7 @@ SecantResult runs_validate(const SecantCubinPlan& plan, const UnpackedRun* runs,
      * the 8 x 2 tile, more are groups of four), and those no toggle reaches as soon as there are
      * toggles (an item then covers several permutations and computes them once) */
     rules.split_parts = true;
+    rules.number_bits = true;
     rules.hoist_bank = true;
     rules.hoist_toggled = false;
     if (rules.banks_allowed)
