@@ -76,11 +76,16 @@ double cut_cycles(const LaunchPlan& plan, const Cut& cut, unsigned long long pro
     const double items = std::ceil((per_cta - 1.0) * each + largest), empty = std::max(0.0, per_cta * largest - items);
     const double active = std::min<double>(plan.warps, items);
     const double rate = std::min(0.14, 2.6 / active);
-    const double item = 900.0 + passes * ((hoists ? 120.0 : 0.0) + 330.0 * cut.gpi * std::min<double>(cut.ppi, std::max(1.0, perms)));
-    const double rounds = std::max(std::ceil(items / plan.warps), items / plan.warps + 0.5);
-    const double cta = 3000.0 + tiles * (1500.0 + rounds * item / rate + empty * 400.0 / plan.warps);
+    const auto slots = [&](double n, double groups) { return 900.0 * n + passes * ((hoists ? 120.0 : 0.0) * n + 330.0 * groups); };
+    const double item = slots(1.0, cut.gpi * std::min<double>(cut.ppi, most_perms));
     const unsigned long long grid = cut.groups * plan.row_splits;
-    return (double)((grid + sms - 1) / sms) * cta;
+    const auto cta = [&](double time) { return 3000.0 + tiles * (1500.0 + time / rate + empty * 400.0 / plan.warps); };
+    if (perms < most_perms) { /* uneven: an average CTA for the work, the one with most permutations for the end */
+        const auto time = [&](double n, double all_perms) { return std::max(item, slots(n, (double)chunks * cut.gpi * all_perms) / plan.warps + 0.5 * item); };
+        const double last = cta(time(items, (per_cta - 1.0) * perms + most_perms));
+        return std::max(last, cta(time(std::ceil(per_cta * each), per_cta * perms)) * (double)grid / sms + 0.5 * last);
+    }
+    return (double)((grid + sms - 1) / sms) * cta(item * std::max(std::ceil(items / plan.warps), items / plan.warps + 0.5));
 }
 
 /* `sms`: the part of the machine this launch has when another runs beside it. */
@@ -112,7 +117,7 @@ void balance_small(LaunchPlan* plan, const DeviceBatch& batch, const EvalProblem
     for (uint32_t gpi = widest.gpi; gpi >= 1; --gpi) {
         if (bank_groups % gpi) continue;
         for (uint32_t ppi = gpi == bank_groups ? widest.ppi : 1u; ppi >= 1; ppi /= 2)
-            for (unsigned waves = 0; waves <= 8; ++waves) {
+            for (unsigned waves = 0; waves <= (fewer ? 32u : 8u); waves += waves < 8 ? 1 : 4) {
                 Cut c{gpi, ppi, waves ? (unsigned long long)waves * sms / plan->row_splits : widest.groups};
                 c.groups = std::max<unsigned long long>(1, std::min(c.groups, P));
                 const unsigned long long items = items_of(c);
