@@ -586,9 +586,11 @@ SecantResult launch_gram_batch(SecantCubinRunnerImpl* r, const std::vector<Devic
         /* rows per range: what the scratch limit leaves for this batch, between 128 and 16,384 */
         const size_t fit = r->scratch_limit / batch_programs;
         const size_t range = std::min<size_t>(run.rows, std::max<size_t>(128, std::min<size_t>(16384, fit)));
-        /* scratch: the range's predictions, then the constant tables of one view at a time (padded to four banks at most) */
+        /* scratch: the range's predictions, then the constant tables of every view (padded to four banks at
+         * most), which the first range makes and the others read again */
         size_t entries = 0;
-        for (const DeviceBatch& db : views) entries = std::max<size_t>(entries, db.total_cst);
+        for (const DeviceBatch& db : views) entries += db.total_cst;
+        std::vector<int> tables_made(views.size(), -1); /* for which register tile */
         const size_t predictions = (batch_programs * range + 3) / 4 * 4;
         float* scratch = nullptr;
         const SecantResult a = stream_scratch(r, k, predictions + 4 * entries, &scratch);
@@ -596,7 +598,9 @@ SecantResult launch_gram_batch(SecantCubinRunnerImpl* r, const std::vector<Devic
         cudaError_t ce = after ? cudaStreamWaitEvent(stream, after, 0) : cudaSuccess;
         for (size_t r0 = 0; r0 < run.rows && ce == cudaSuccess; r0 += range) {
             const size_t rows_now = std::min(range, run.rows - r0);
-            for (const DeviceBatch& db : views) {
+            size_t tables = predictions;
+            for (size_t v = 0; v < views.size(); ++v) {
+                const DeviceBatch& db = views[v];
                 EvalProblem prob = make_problem(plan, run, 0);
                 prob.fast_math = r->fast_math;
                 prob.input += r0;
@@ -604,13 +608,16 @@ SecantResult launch_gram_batch(SecantCubinRunnerImpl* r, const std::vector<Devic
                 /* SbProgram::index is the program's position in the run: shift the base so that the batch's first program lands on row 0 */
                 prob.output = reinterpret_cast<float*>(reinterpret_cast<uintptr_t>(scratch) - first_program * range * sizeof(float));
                 prob.out_program_stride = range;
-                const LaunchPlan lp = plan_launch(db, prob, r->sm_count, r->smem_limit, r->scratch_limit);
+                LaunchPlan lp = plan_launch(db, prob, r->sm_count, r->smem_limit, r->scratch_limit);
                 if (!lp.ok) {
                     r->last_error = "program batch does not fit shared memory";
                     return lp.overflow ? SECANT_ERROR_OVERFLOW : SECANT_ERROR_REGISTER_OVERFLOW;
                 }
+                if (tables_made[v] == lp.variant) lp.table_elements = 0;
+                tables_made[v] = lp.variant;
                 unsigned launches = 0;
-                ce = launch_eval(db, prob, lp, scratch + predictions, stream, &launches);
+                ce = launch_eval(db, prob, lp, scratch + tables, stream, &launches);
+                tables += 4 * db.total_cst;
                 g_kernel_launches.fetch_add(launches);
                 if (ce != cudaSuccess) break;
             }
