@@ -23,7 +23,7 @@ namespace {
  * kernel is the wait for the loads: kAhead rows are loaded before the first is used.  Blocks wholly below
  * the diagonal are left out; their statistics are those of the mirrored ones, bit for bit.
  * 64 cohorts of eight programs, two targets, 16,384 rows, predictions in L2: 51 us with a warp per
- * statistic, 35 this way (2 x 4 blocks 64, eight rows ahead 48). */
+ * statistic, 35 this way (64 with 2 x 4 blocks and six rows ahead). */
 constexpr uint32_t kGramWarps = 4, kLeft = 2, kRight = 2, kAhead = 16;
 
 __device__ __host__ __forceinline__ uint32_t first_right_block(uint32_t left_block) { return left_block * kLeft / kRight; }
