@@ -335,7 +335,9 @@ def toggles_arm(args, w):
                 seconds.append(runner.stats.runtime_seconds + ev0.elapsed_time(ev1) * 1e-3)
         launches = lib.secant_b200_kernel_launch_count() - launches0
     dt = sum(seconds) / len(seconds)
-    lane_ops = float((ops + 2).sum()) * configs * N
+    # one evaluation per permutation that a program tells apart: bits it does not read change nothing
+    distinct = np.array([1 << len(P.toggle_bits_read(a)) for a in pop.asts], dtype=np.float64)
+    lane_ops = float(((ops + 2) * distinct).sum()) * NB * N
     sse, cfg, valid = R.score_fields(best)
     print(json.dumps({"impl": "toggles", "metric": METRIC, "value": float(Pn) * N / dt, "unit": "program-rows/s", "n_gpus": 1,
                       "steps": args.steps, "warmup": args.warmup, "ms_per_step": dt * 1e3, "higher_is_better": True,

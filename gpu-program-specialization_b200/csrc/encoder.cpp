@@ -807,7 +807,7 @@ SecantResult encode_program(const SecantAstInstruction* program, const SecantAst
         em.n_hoisted > 255u)
         return SECANT_ERROR_REGISTER_OVERFLOW;
     out.affines.insert(out.affines.end(), affines.begin(), affines.end());
-    if (rules.number_bits && n_patch) {
+    if (n_patch) {
         const auto each_bit = [&](auto&& f) {
             for (size_t i = rec.patch_off; i < out.patches.size(); ++i) {
                 f(out.patches[i].bit0);
@@ -815,8 +815,8 @@ SecantResult encode_program(const SecantAstInstruction* program, const SecantAst
             }
         };
         each_bit([&](uint8_t& b) { rec.bit_mask |= 1u << b; });
-        each_bit([&](uint8_t& b) { b = (uint8_t)__builtin_popcount(rec.bit_mask & ((1u << b) - 1u)); });
-        rec.bits = (uint16_t)__builtin_popcount(rec.bit_mask);
+        if (rules.number_bits) each_bit([&](uint8_t& b) { b = (uint8_t)__builtin_popcount(rec.bit_mask & ((1u << b) - 1u)); });
+        if (rules.number_bits) rec.bits = (uint16_t)__builtin_popcount(rec.bit_mask);
     }
     rec.n_insn = (uint16_t)total;
     rec.n_patch = (uint16_t)n_patch;

@@ -558,18 +558,6 @@ template <int RC> struct TableWord { typedef float type; };
 template <> struct TableWord<2> { typedef float2 type; };
 template <> struct TableWord<4> { typedef float4 type; };
 
-/* the low bits of v, in order, at the places of mask's bits */
-__device__ __forceinline__ uint32_t deposit(uint32_t v, uint32_t mask) {
-    uint32_t out = 0u;
-#pragma unroll 1
-    for (; mask; v >>= 1) {
-        const uint32_t low = mask & (0u - mask);
-        out |= v & 1u ? low : 0u;
-        mask ^= low;
-    }
-    return out;
-}
-
 /* 16 values per thread: 20 warps per CTA within 96 registers (32-value tiles were measured
  * slower at the 12 warps their 168 registers allow). */
 template <int RR, int RC, bool FAST, bool SPAN, int KIND>

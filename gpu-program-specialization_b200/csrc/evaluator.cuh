@@ -190,6 +190,20 @@ cudaError_t launch_gram(const float* predictions, size_t prediction_ld, uint32_t
 /* One-time per-device kernel attribute setup (dynamic shared memory opt-in). */
 cudaError_t configure_kernels();
 
+#ifdef __CUDACC__
+/* the low bits of v, in order, at the places of mask's bits */
+__device__ __forceinline__ uint32_t deposit(uint32_t v, uint32_t mask) {
+    uint32_t out = 0u;
+#pragma unroll 1
+    for (; mask; v >>= 1) {
+        const uint32_t low = mask & (0u - mask);
+        out |= v & 1u ? low : 0u;
+        mask ^= low;
+    }
+    return out;
+}
+#endif
+
 }  // namespace sb
 
 #endif

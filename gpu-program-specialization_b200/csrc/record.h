@@ -128,8 +128,8 @@ typedef struct SbProgram {
     uint32_t index;     /* position of the program in the run (output row, bank table) */
     uint32_t cost;      /* scheduling weight: bits 0..15 main part per bank group, bits 16..31 row prelude */
     uint16_t mid_off;
-    uint16_t bits;      /* toggle bits the program reads (0 for the rollout kernel's records) */
-    uint32_t bit_mask;  /* which ones; the sites of its records number them 0 .. bits - 1 in this order */
+    uint16_t bits;      /* toggle bits the program reads (0 for the rollout kernel, whose sites name the run's bits) */
+    uint32_t bit_mask;  /* which ones; the evaluator's sites number them 0 .. bits - 1 in this order */
     uint32_t cst_off;   /* constant-table entries of the programs before this one in launch order (set by the runner) */
 } SbProgram;
 

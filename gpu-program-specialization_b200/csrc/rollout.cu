@@ -443,7 +443,6 @@ rk4_kernel(const DeviceBatch batch, const Rk4Problem prob, const RolloutLayout l
     m.temps = shared_address(warea + lay.exec_bytes + lay.table_bytes + lay.source_bytes) + lane * (uint32_t)(RR * 4);
     const unsigned long long configs = (unsigned long long)prob.num_banks << prob.toggle_bits;
     const unsigned long long num_items = configs * prob.num_systems;
-    unsigned int integrated = 0; /* (trajectory, observation interval) pairs this lane carried out */
     /* Items are drawn from a device-wide counter: a group whose candidate went invalid early takes
      * the next one at once, and no warp slot idles behind the longest item of its CTA. */
 #pragma unroll 1
@@ -463,6 +462,16 @@ rk4_kernel(const DeviceBatch batch, const Rk4Problem prob, const RolloutLayout l
     const unsigned long long cfg = item - turn * configs;
     const unsigned long long perm = cfg & ((1ull << prob.toggle_bits) - 1ull);
     const uint32_t bank = (uint32_t)(cfg >> prob.toggle_bits);
+    /* configurations that differ only in toggle bits the system does not read have one score: the one
+     * where those bits are 0 is integrated, and its group writes the others (600 systems of two states,
+     * two bits, three sets: two thirds of the items, 1.31 -> 1.09 ms a call) */
+    uint32_t unread = (uint32_t)((1ull << prob.toggle_bits) - 1ull);
+    for (uint32_t c = 0; c < S; ++c) unread &= ~batch.programs[sys * S + c].bit_mask;
+    if (perm & unread) {
+        group_sync(barrier, threads); /* the item's number has been read */
+        continue;
+    }
+    unsigned int integrated = 0; /* (trajectory, observation interval) pairs this lane carries out */
     const float* bank_ptr = prob.banks ? prob.banks + (size_t)sys * prob.system_bank_stride + (size_t)bank * prob.bank_stride : nullptr;
 
     /* private copy of the right-hand side: toggles resolved, the bank part run once, the main part
@@ -606,14 +615,21 @@ rk4_kernel(const DeviceBatch batch, const Rk4Problem prob, const RolloutLayout l
             residuals += ((unsigned long long)__float_as_uint(other_source[2]) << 32) | __float_as_uint(other_source[1]);
         }
         const bool finite = fabsf(total) <= kFltMax;
-        prob.output[(size_t)sys * prob.output_ld + cfg] = (alive && residuals && finite) ? total / (float)residuals : kFltMax;
+        sq = (alive && residuals && finite) ? total / (float)residuals : kFltMax;
+    }
+    if (s == 0) {
+        sq = __shfl_sync(0xffffffffu, sq, 0);
+        const unsigned long long copies = 1ull << __popc(unread);
+        float* const out = prob.output + (size_t)sys * prob.output_ld + cfg;
+#pragma unroll 1
+        for (unsigned long long x = lane; x < copies; x += 32u) out[deposit((uint32_t)x, unread)] = sq;
+        if (prob.integrated) { /* counted for every configuration that has the score */
+#pragma unroll
+            for (int d = 16; d; d >>= 1) integrated += __shfl_xor_sync(0xffffffffu, integrated, d);
+            if (lane == 0) atomicAdd(prob.integrated, (unsigned long long)integrated * copies);
+        }
     }
     if (S == 1) __syncwarp(); /* a group of several meets again before anything is overwritten */
-    }
-    if (prob.integrated && s == 0) {
-#pragma unroll
-        for (int d = 16; d; d >>= 1) integrated += __shfl_xor_sync(0xffffffffu, integrated, d);
-        if (lane == 0) atomicAdd(prob.integrated, (unsigned long long)integrated);
     }
 }
 

@@ -269,6 +269,18 @@ _WIDTH = {OP["AFFINE"]: 10, OP["LIT"]: 5, OP["TOG4"]: 3, OP["ROUTINE"]: 2, OP["A
           OP["COL"]: 2}
 
 
+def toggle_bits_read(code):
+    """The toggle bits a program selects by (two- and four-way toggles over direct leaves)."""
+    at, bits = 0, set()
+    while code[at] != OP["RET"]:
+        if code[at] == OP["TOG2"]:
+            bits.add(code[at + 1])
+        elif code[at] == OP["TOG4"]:
+            bits |= {code[at + 1], code[at + 2]}
+        at += _WIDTH.get(code[at], 1)
+    return bits
+
+
 def _count_tokens(code, routine_ops):
     at = 0
     n = 0
