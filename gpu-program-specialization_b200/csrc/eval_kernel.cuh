@@ -341,11 +341,10 @@ struct Machine {
         for (int j = 0; j < V / 4; ++j) q[j * 32] = make_ulonglong2(flat[2 * j], flat[2 * j + 1]);
     }
 
-    /* approximate functions: a few instructions per element, unrolled in place */
+    /* approximate functions of what the core leaves (sine, cosine and tanh it never does): a few
+     * instructions per element, unrolled in place */
     __device__ __forceinline__ void fast_unary(unsigned op, f2 (&v)[8]) {
         switch (op) {
-        case SB_UN_SIN: fast_tile<SB_UN_SIN>(v); break;
-        case SB_UN_COS: fast_tile<SB_UN_COS>(v); break;
         case SB_UN_EXP: fast_tile<SB_UN_EXP>(v); break;
         case SB_UN_LOG: fast_tile<SB_UN_LOG>(v); break;
         case SB_UN_EX2: fast_tile<SB_UN_EX2>(v); break;
