@@ -104,9 +104,10 @@ struct LaunchPlan {
     uint32_t row_splits;      /* CTAs sharing one program group, each with a row range */
     size_t rows_per_split;
     size_t smem_bytes;
-    size_t partial_elements;  /* floats of per-split partial sums the launch needs (0: materialize) */
-    size_t table_elements;    /* floats of constant tables, in the same buffer */
-    size_t table_offset;      /* where they begin in it: behind the partial sums, 16-byte aligned */
+    size_t partial_elements;  /* floats of partial sums over all row splits (0: materialize) */
+    size_t table_elements;    /* floats of constant tables */
+    size_t table_offset;      /* where they begin in the launch's scratch, 16-byte aligned: behind the partial sums, or
+                                 at 0 when the rows are not split and the sums go straight to the output */
     uint32_t grid_x;
     bool ok;
     bool overflow;            /* !ok because a count does not fit the kernel's 32-bit indices */
@@ -138,15 +139,17 @@ constexpr int kVariantBanks[kNumVariants] = {4, 2, 1};
 
 Geom make_geom(const DeviceBatch& batch, const EvalProblem& problem, const LaunchPlan& plan);
 
-/* scratch_limit: most floats of per-split partial sums a launch may use (row splits are reduced to fit).
+/* scratch_limit: most floats of scratch a launch may use: the row splits are reduced until their partial sums
+ * fit beside the constant tables (with one split there are none; the tables are not reduced here).
  * share: the part of the machine a small launch should count on (another one runs beside it). */
 LaunchPlan plan_launch(const DeviceBatch& batch, const EvalProblem& problem, int sm_count, size_t smem_limit,
                        size_t scratch_limit, double share = 1.0);
 
 /* Enqueues the evaluation of one batch on `stream`: the evaluator kernel writes per-split partial
  * sums into `partial` (plan.table_offset + plan.table_elements floats, private to the stream until the
- * launch has finished; the programs' constant tables are computed into its end first) and a second kernel adds them in a fixed order into the output, so a result does
- * not depend on the order CTAs ran in.  Returns the CUDA status of the launches. */
+ * launch has finished; the programs' constant tables are computed into its end first) and a second kernel
+ * adds them in a fixed order into the output, so a result does not depend on the order CTAs ran in; with one
+ * row split the sums are whole and go to the output at once.  Returns the CUDA status of the launches. */
 cudaError_t launch_eval(const DeviceBatch& batch, const EvalProblem& problem, const LaunchPlan& plan, float* partial,
                         cudaStream_t stream, unsigned* launches);
 

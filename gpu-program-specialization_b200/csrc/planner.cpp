@@ -235,11 +235,16 @@ LaunchPlan plan_with_tile(const DeviceBatch& batch, const EvalProblem& prob, int
         groups = std::min<unsigned long long>(P, ((unsigned long long)sm_count + splits - 1) / splits);
         plan.num_groups = (uint32_t)groups;
     }
+    /* constant tables: one float per entry and (padded bank, permutation) */
+    const unsigned long long padded = materialize ? rc : ((unsigned long long)(prob.num_banks + rc - 1) / rc * rc) << batch.max_bits;
+    if (batch.total_cst > (~0ull >> 3) / padded) { plan.overflow = true; return plan; }
+    plan.table_elements = (size_t)(batch.total_cst * padded);
     const unsigned long long configs = (unsigned long long)prob.num_banks << prob.toggle_bits;
-    if (!materialize && configs) { /* [split][program][quantity][configuration] floats of scratch */
+    if (!materialize && configs) { /* [split][program][quantity][configuration] floats of scratch, in what the tables leave of it */
         const unsigned long long per_split = (unsigned long long)P * nq;
         if (per_split > (~0ull >> 3) / configs) { plan.overflow = true; return plan; }
-        const unsigned long long fit = std::max<unsigned long long>(1, (unsigned long long)scratch_limit / (per_split * configs));
+        const unsigned long long room = scratch_limit > plan.table_elements ? (scratch_limit - plan.table_elements) / 4 * 4 : 0;
+        const unsigned long long fit = std::max<unsigned long long>(1, room / (per_split * configs));
         splits = (size_t)std::min<unsigned long long>(splits, fit);
     }
     const size_t tiles_per_split = (tiles + splits - 1) / splits;
@@ -256,11 +261,7 @@ LaunchPlan plan_with_tile(const DeviceBatch& batch, const EvalProblem& prob, int
         if (configs && n > (~0ull >> 3) / configs / nq) { plan.overflow = true; return plan; }
         plan.partial_elements = (size_t)(n * nq * configs);
     }
-    /* constant tables: one float per entry and (padded bank, permutation) */
-    const unsigned long long padded = materialize ? rc : ((unsigned long long)(prob.num_banks + rc - 1) / rc * rc) << batch.max_bits;
-    if (batch.total_cst > (~0ull >> 3) / padded) { plan.overflow = true; return plan; }
-    plan.table_elements = (size_t)(batch.total_cst * padded);
-    plan.table_offset = (plan.partial_elements + 3) / 4 * 4;
+    plan.table_offset = plan.row_splits > 1 ? (plan.partial_elements + 3) / 4 * 4 : 0; /* whole sums go to the output */
     balance_small(&plan, batch, prob, std::max(1, (int)(sm_count * share)), smem_limit);
     plan.ok = true;
     return plan;

@@ -99,7 +99,7 @@ struct Slot {
 
 using namespace sb;
 
-constexpr size_t kDefaultScratchFloats = (size_t)1 << 28; /* 1 GiB of per-split partial sums per launch */
+constexpr size_t kDefaultScratchFloats = (size_t)1 << 28; /* 1 GiB of scratch per launch: partial sums or predictions, and constant tables */
 
 struct SecantCubinRunnerImpl {
     SecantCubinPlan owned_plan;     /* used when created straight from a recipe */
@@ -108,7 +108,7 @@ struct SecantCubinRunnerImpl {
     int device = 0, sm_count = 0;
     size_t smem_limit = 0;
     std::vector<cudaStream_t> streams;
-    std::vector<void*> scratch;      /* per compute stream: partial sums of the launch in flight */
+    std::vector<void*> scratch;      /* per compute stream: partial sums (or predictions) and constant tables of the launch in flight */
     std::vector<size_t> scratch_cap;
     cudaStream_t copy_stream = nullptr;
     cudaEvent_t ev_join = nullptr, ev_start = nullptr, ev_stop = nullptr;
@@ -487,9 +487,10 @@ EvalProblem make_problem(const SecantCubinPlan& plan, const UnpackedRun& run, si
     return p;
 }
 
-/* Per-stream scratch for the evaluator's per-split partial sums.  Launches on one stream run in
- * order, so the evaluator and the kernel that folds its partial sums may reuse the buffer of the
- * launch before them; growing it waits for the stream first. */
+/* Per-stream scratch for the evaluator's per-split partial sums and constant tables.  Launches on one stream
+ * run in order, so the evaluator and the kernel that folds its partial sums may reuse the buffer of the
+ * launch before them; growing it waits for the stream first and takes a quarter more than is needed, as far
+ * as the scratch limit allows. */
 SecantResult stream_scratch(SecantCubinRunnerImpl* r, size_t k, size_t elements, float** out) {
     const size_t bytes = elements * sizeof(float);
     if (elements > SIZE_MAX / sizeof(float)) return SECANT_ERROR_OVERFLOW;
@@ -497,10 +498,11 @@ SecantResult stream_scratch(SecantCubinRunnerImpl* r, size_t k, size_t elements,
         SB_CUDA(cudaStreamSynchronize(r->streams[k]), "cudaStreamSynchronize");
         if (r->scratch[k]) SB_CUDA(cudaFree(r->scratch[k]), "cudaFree");
         r->scratch[k] = nullptr; r->scratch_cap[k] = 0;
-        const size_t want = bytes + bytes / 4;
+        const size_t most = std::max(bytes, r->scratch_limit * sizeof(float));
+        const size_t want = std::min(bytes + bytes / 4, most);
         if (cudaMalloc(&r->scratch[k], want) != cudaSuccess) {
             (void)cudaGetLastError();
-            r->last_error = "no device memory for the partial sums of a launch";
+            r->last_error = "no device memory for the scratch of a launch";
             return SECANT_ERROR_ALLOCATION_FAILED;
         }
         r->scratch_cap[k] = want;
@@ -533,11 +535,13 @@ SecantResult launch_batch(SecantCubinRunnerImpl* r, const DeviceBatch& db, doubl
             prob.banks = reinterpret_cast<const float*>(runs[e].banks.address) + runs[e].first_program_index * runs[e].program_bank_stride;
         cudaError_t ce = after ? cudaStreamWaitEvent(stream, after, 0) : cudaSuccess;
         /* one launch, unless its constant tables (an entry per program constant and configuration) would
-         * take more than the scratch limit: then the programs in as many launches as it takes, and a
+         * take more than half of the scratch limit (the rest is for the partial sums of the row splits, without
+         * which few programs would fill few SMs): then the programs in as many launches as it takes, and a
          * program at a time at least */
+        const size_t most_tables = r->scratch_limit / 2;
         const size_t per_program = std::max<size_t>(1, (size_t)db.max_cst * (size_t)((prob.num_banks + 3ull) << db.max_bits));
-        const size_t fit = std::max<size_t>(1, r->scratch_limit / per_program);
-        const size_t step = db.total_cst <= r->scratch_limit / ((prob.num_banks + 3ull) << db.max_bits) ? db.num_programs : fit;
+        const size_t fit = std::max<size_t>(1, most_tables / per_program);
+        const size_t step = db.total_cst <= most_tables / ((prob.num_banks + 3ull) << db.max_bits) ? db.num_programs : fit;
         for (size_t first = 0; first < db.num_programs && ce == cudaSuccess; first += step) {
             DeviceBatch part = db;
             if (step < db.num_programs) {
@@ -552,8 +556,8 @@ SecantResult launch_batch(SecantCubinRunnerImpl* r, const DeviceBatch& db, doubl
                 return lp.overflow ? SECANT_ERROR_OVERFLOW : SECANT_ERROR_REGISTER_OVERFLOW;
             }
             float* partial = nullptr;
-            if (lp.partial_elements || lp.table_elements) {
-                const SecantResult a = stream_scratch(r, k, lp.table_offset + lp.table_elements, &partial);
+            if (const size_t floats = lp.table_offset + lp.table_elements) {
+                const SecantResult a = stream_scratch(r, k, floats, &partial);
                 if (a != SECANT_SUCCESS) return a;
             }
             unsigned launches = 0;
@@ -583,13 +587,14 @@ SecantResult launch_gram_batch(SecantCubinRunnerImpl* r, const std::vector<Devic
         const UnpackedRun& run = runs[e];
         const size_t k = (*stream_cursor)++ % r->streams.size();
         cudaStream_t stream = r->streams[k];
-        /* rows per range: what the scratch limit leaves for this batch, between 128 and 16,384 */
-        const size_t fit = r->scratch_limit / batch_programs;
-        const size_t range = std::min<size_t>(run.rows, std::max<size_t>(128, std::min<size_t>(16384, fit)));
         /* scratch: the range's predictions, then the constant tables of every view (padded to four banks at
          * most), which the first range makes and the others read again */
         size_t entries = 0;
         for (const DeviceBatch& db : views) entries += db.total_cst;
+        /* rows per range: what the scratch limit leaves for this batch's predictions, between 128 and 16,384 */
+        const size_t room = r->scratch_limit > 4 * entries ? (r->scratch_limit - 4 * entries) / 4 * 4 : 0;
+        const size_t fit = room / batch_programs;
+        const size_t range = std::min<size_t>(run.rows, std::max<size_t>(128, std::min<size_t>(16384, fit)));
         std::vector<int> tables_made(views.size(), -1); /* for which register tile */
         const size_t predictions = (batch_programs * range + 3) / 4 * 4;
         float* scratch = nullptr;

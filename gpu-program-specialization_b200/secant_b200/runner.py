@@ -174,7 +174,7 @@ class Runner:
         abi.check(self.lib.secant_b200_runner_set_math(self.handle, 1 if fast else 0), "secant_b200_runner_set_math")
 
     def set_scratch_limit(self, nbytes):
-        """Caps the device scratch one launch may use for per-split partial sums (0 = default)."""
+        """Caps the device scratch one launch may use for partial sums, predictions and constant tables (0 = default)."""
         abi.check(self.lib.secant_b200_runner_set_scratch_limit(self.handle, C.c_size_t(nbytes)), "set_scratch_limit")
 
     def population(self, packed, toggle_bits=0):

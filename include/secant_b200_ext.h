@@ -94,9 +94,12 @@ SECANT_DEC SecantResult secant_b200_runner_set_math(SecantCubinRunner runner, ui
  * (the reference adds with atomics, projects/secant/s_cubin_generate_toggle_sse.c:378-381).  The
  * buffer belongs to the runner (one per launch stream, grown on demand, kept between runs,
  * released by destroy).  More row splits mean more, shorter blocks - better balance when there are
- * few programs - and more scratch.  This call caps the scratch of one launch at `bytes`; 0 restores
- * the default of 1 GiB.  A launch whose single-split scratch alone exceeds the cap still runs, with
- * one split.  Returns INVALID_STATE while a run is in flight.
+ * few programs - and more scratch; with one split the sums go straight to the output.  The programs'
+ * constant tables (one float per entry and configuration) lie in the same buffer, and so do the
+ * predictions of a range of rows in the Gram-statistics shape.  This call caps the scratch of one launch
+ * at `bytes`; 0 restores the default of 1 GiB.  Programs whose tables would take more than half of the cap
+ * are scored in several launches.  What cannot be made smaller still runs: the tables of one program, or
+ * 128 rows of a batch's predictions and its tables.  Returns INVALID_STATE while a run is in flight.
  */
 SECANT_DEC SecantResult secant_b200_runner_set_scratch_limit(SecantCubinRunner runner, size_t bytes);
 

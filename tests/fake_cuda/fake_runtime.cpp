@@ -21,6 +21,7 @@
  */
 #include "evaluator.cuh"
 
+#include <algorithm>
 #include <atomic>
 #include <chrono>
 #include <cstdlib>
@@ -53,6 +54,8 @@ struct World {
     std::map<const void*, Clock> events;    /* live events and the clock they recorded */
     Clock host;                             /* what the host knows to be complete */
     unsigned violations = 0, launches = 0, threads_started = 0;
+    unsigned split_launches = 0;            /* launches whose rows are split */
+    size_t largest_scratch = 0;             /* bytes of the largest scratch allocation a launch was given */
     void* context = reinterpret_cast<void*>(0x1234);
     bool no_context = false;
     std::string last_violation;
@@ -85,6 +88,14 @@ Allocation* owner_of(const void* p) {
         if (p >= base && p < base + kv.second.bytes) return &kv.second;
     }
     return nullptr;
+}
+
+size_t room_behind(const void* p) { /* bytes from p to the end of its allocation */
+    for (auto& kv : world.allocations) {
+        const char* base = static_cast<const char*>(kv.first);
+        if (p >= base && p < base + kv.second.bytes) return (size_t)(base + kv.second.bytes - static_cast<const char*>(p));
+    }
+    return 0;
 }
 
 void violation(const char* what) {
@@ -256,6 +267,9 @@ FAKE_EXPORT void fake_reset(void) {
     world.faults.clear();
     world.violations = 0;
     world.launches = 0;
+    world.threads_started = 0;
+    world.split_launches = 0;
+    world.largest_scratch = 0;
     world.no_context = false;
     world.context = reinterpret_cast<void*>(0x1234);
     world.last_violation.clear();
@@ -292,6 +306,12 @@ FAKE_EXPORT void fake_state(unsigned* what) {
     what[4] = world.launches;
     what[5] = world.threads_started;
 }
+/* since the last reset: bytes of the largest scratch allocation behind a launch, launches whose rows were split */
+FAKE_EXPORT void fake_scratch(uint64_t* what) {
+    std::lock_guard<std::mutex> lock(world.mutex);
+    what[0] = world.largest_scratch;
+    what[1] = world.split_launches;
+}
 FAKE_EXPORT const char* fake_last_violation(void) { return world.last_violation.c_str(); }
 FAKE_EXPORT void fake_set_context(int which) { /* 0: none, n: context n */
     std::lock_guard<std::mutex> lock(world.mutex);
@@ -323,12 +343,14 @@ cudaError_t launch_eval(const DeviceBatch& batch, const EvalProblem&, const Laun
     if (failing("launch_eval")) return cudaErrorUnknown;
     Allocation* records = owner_of(batch.programs);
     if (!records) { violation("launch with program records outside any device allocation"); return cudaErrorInvalidValue; }
-    if (plan.partial_elements) {
+    if (plan.row_splits > 1) ++world.split_launches;
+    if (const size_t needed = (plan.table_offset + plan.table_elements) * sizeof(float)) { /* partial sums, then constant tables */
         Allocation* scratch = owner_of(partial);
-        if (!scratch || scratch->bytes < plan.partial_elements * sizeof(float)) {
-            violation("launch with too little scratch for its partial sums");
+        if (!scratch || room_behind(partial) < needed) {
+            violation("launch with too little scratch for its partial sums and tables");
             return cudaErrorInvalidValue;
         }
+        world.largest_scratch = std::max(world.largest_scratch, scratch->bytes);
         merge(scratch->busy, advance(stream));
     }
     const Clock& now = advance(stream);

@@ -46,8 +46,8 @@ def run_timed_shape(rn, pop, x, y, banks, nb, K):
 def test_population_of_the_timed_shape_over_tiles_and_splits(cuda):
     """320 programs x 64 sets x 1,613 rows: four 512-row tiles, the last one ragged.  Scored three
     ways: with the default plan (every CTA owns one tile, the splits are folded by the second
-    kernel), with the scratch capped so that one CTA walks all tiles (double-buffered staging,
-    accumulation across tiles), and a second time with the default plan (identical bits)."""
+    kernel), with no scratch for partial sums, so that one CTA walks all tiles of its program (double-buffered
+    staging, accumulation across tiles), and a second time with the default plan (identical bits)."""
     pop, x, y, banks, nb, K, F = timed_shape(320, 1613)
     want64, slack = S.sse_reference_parallel(pop, x, y, banks, K, 0, program_bank_stride=nb * K)
     skipped = parity.ill_conditioned_fraction(slack)
@@ -56,7 +56,7 @@ def test_population_of_the_timed_shape_over_tiles_and_splits(cuda):
     with Runner(abi.SHAPE_TOGGLE_SSE, F, 1, K, workers=2, streams=2) as rn:
         split = run_timed_shape(rn, pop, x, y, banks, nb, K)
         again = run_timed_shape(rn, pop, x, y, banks, nb, K)
-        rn.set_scratch_limit(4 * len(pop.asts) * nb)          # room for a single split
+        rn.set_scratch_limit(4)                               # a launch per program, none with split rows
         walked = run_timed_shape(rn, pop, x, y, banks, nb, K)
         rn.set_scratch_limit(0)
     assert np.array_equal(split.view(np.uint32), again.view(np.uint32))      # sums do not depend on scheduling
