@@ -17,21 +17,26 @@
 #define SB_LOW(A) "mov.b64 {f0, f1}, " A ";\n min.NaN.f32 low, low, f0, f1;\n"
 #define SB_LOW_ABS(A) "mov.b64 {f0, f1}, " A ";\n min.NaN.abs.f32 low, low, f0, f1;\n"
 #define SB_ALL_OR_LEAVE "vote.sync.all.pred p, p, 0xffffffff;\n @!p bra.uni LEAVE;\n"
-/* constants of the steps below */
-#define SB_SIN_CONSTANTS \
-    SB_PAIR_CONST("k0", "0x3EA2F9833EA2F983") SB_PAIR_CONST("k1", "0x4B4000004B400000") SB_PAIR_CONST("k2", "0xCB400000CB400000") \
-    SB_PAIR_CONST("k3", "0xC0490FDBC0490FDB") SB_PAIR_CONST("k4", "0x33BBBD2E33BBBD2E") SB_PAIR_CONST("k5", "0x27772CED27772CED") \
-    SB_PAIR_CONST("k6", "0xB2CD31C1B2CD31C1") SB_PAIR_CONST("k7", "0x3638B8243638B824") SB_PAIR_CONST("k8", "0xB9500BECB9500BEC") \
-    SB_PAIR_CONST("k9", "0x3C0888863C088886") SB_PAIR_CONST("k10", "0xBE2AAAABBE2AAAAB")
-#define SB_EXP_CONSTANTS \
-    SB_PAIR_CONST("k0", "0x3FB8AA3B3FB8AA3B") SB_PAIR_CONST("k1", "0x4B4000004B400000") SB_PAIR_CONST("k2", "0x32A5706032A57060")
-#define SB_LOG_CONSTANTS \
-    SB_PAIR_CONST("k0", "0xCB400000CB400000") SB_PAIR_CONST("k1", "0xBD9C5854BD9C5854") SB_PAIR_CONST("k2", "0x3E02AC143E02AC14") \
-    SB_PAIR_CONST("k3", "0xBE06C251BE06C251") SB_PAIR_CONST("k4", "0x3E116D423E116D42") SB_PAIR_CONST("k5", "0xBE2A392FBE2A392F") \
-    SB_PAIR_CONST("k6", "0x3E4CD0023E4CD002") SB_PAIR_CONST("k7", "0xBE800113BE800113") SB_PAIR_CONST("k8", "0x3EAAAAAA3EAAAAAA") \
-    SB_PAIR_CONST("k9", "0xBF000000BF000000") SB_PAIR_CONST("k10", "0x35BFBE8E35BFBE8E") SB_PAIR_CONST("k11", "0x3F3172003F317200")
-#define SB_DIV_CONSTANTS \
-    SB_PAIR_CONST("k0", "0x3F8000003F800000")
+/* Constants of the steps below, each the bits of a float32 and written once: the evaluator's core moves them into
+ * registers (SB_*_CONSTANTS), the rollout core reads them from a table of pairs (SB_PAIR_WORD, rollout.cu) and
+ * the scalar functions name them (sbmath.cuh). */
+#define SB_PAIR_TEXT(I, BITS) "mov.b64 k" #I ", 0x" #BITS #BITS ";\n"
+#define SB_PAIR_WORD(I, BITS) 0x##BITS##BITS##ull,
+#define SB_SIN_LIST(X) \
+    X(0, 3EA2F983) X(1, 4B400000) X(2, CB400000) X(3, C0490FDB) X(4, 33BBBD2E) X(5, 27772CED) \
+    X(6, B2CD31C1) X(7, 3638B824) X(8, B9500BEC) X(9, 3C088886) X(10, BE2AAAAB)
+#define SB_EXP_LIST(X) \
+    X(0, 3FB8AA3B) X(1, 4B400000) X(2, 32A57060)
+#define SB_LOG_LIST(X) \
+    X(0, CB400000) X(1, BD9C5854) X(2, 3E02AC14) X(3, BE06C251) X(4, 3E116D42) X(5, BE2A392F) \
+    X(6, 3E4CD002) X(7, BE800113) X(8, 3EAAAAAA) X(9, BF000000) X(10, 35BFBE8E) X(11, 3F317200)
+#define SB_DIV_LIST(X) \
+    X(0, 3F800000)
+#define SB_SIN_CONSTANTS SB_SIN_LIST(SB_PAIR_TEXT)
+#define SB_EXP_CONSTANTS SB_EXP_LIST(SB_PAIR_TEXT)
+#define SB_LOG_CONSTANTS SB_LOG_LIST(SB_PAIR_TEXT)
+#define SB_DIV_CONSTANTS SB_DIV_LIST(SB_PAIR_TEXT)
+#define SB_TANH_CONSTANTS SB_TANH_LIST(SB_PAIR_TEXT)
 #define SB_MINUS_ONE "mov.b64 mone, 0xBF800000BF800000;\n"
 /* (the sign is added: shift and addition are one instruction, shift and xor two)
  * sin and cos differ in the shift by half a turn, taken off again after the rounding */
@@ -74,11 +79,9 @@
  * least squares), from there on 1 - 2 / (e^2|x| + 1) with the exponential's steps and one Newton step on
  * the reciprocal, |x| cut at 10 where the result is 1; both are computed and one is chosen.  NaN takes the
  * polynomial's side.  At most 1.3 ulp off (all float32 arguments; CUDA's function: 1.8). */
-#define SB_TANH_CONSTANTS \
-    SB_PAIR_CONST("k0", "0xB9EECA99B9EECA99") SB_PAIR_CONST("k1", "0x3B2941E73B2941E7") SB_PAIR_CONST("k2", "0xBC0767FDBC0767FD") \
-    SB_PAIR_CONST("k3", "0x3CB177BC3CB177BC") SB_PAIR_CONST("k4", "0xBD5CE4F8BD5CE4F8") SB_PAIR_CONST("k5", "0x3E08879A3E08879A") \
-    SB_PAIR_CONST("k6", "0xBEAAAAA7BEAAAAA7") SB_PAIR_CONST("k7", "0x4038AA3B4038AA3B") SB_PAIR_CONST("k8", "0x3325706033257060") \
-    SB_PAIR_CONST("k9", "0x4B4000004B400000") SB_PAIR_CONST("k10", "0x3F8000003F800000") SB_PAIR_CONST("k11", "0x4000000040000000")
+#define SB_TANH_LIST(X) \
+    X(0, B9EECA99) X(1, 3B2941E7) X(2, BC0767FD) X(3, 3CB177BC) X(4, BD5CE4F8) X(5, 3E08879A) \
+    X(6, BEAAAAA7) X(7, 4038AA3B) X(8, 33257060) X(9, 4B400000) X(10, 3F800000) X(11, 40000000)
 #define SB_TANH_PAIR(A)                                                                                 \
     "mov.b64 {c2, c3}, " A ";\n and.b32 c2, c2, 0x7fffffff;\n and.b32 c3, c3, 0x7fffffff;\n mov.b64 m, {c2, c3};\n" \
     "mul.rn.f32x2 z, m, m;\n mov.b32 f0, c2;\n mov.b32 f1, c3;\n min.f32 f0, f0, 0f41200000;\n min.f32 f1, f1, 0f41200000;\n mov.b64 n, {f0, f1};\n" \

@@ -84,15 +84,13 @@ enum { RK_CST = 0, RK_STATE = 1, RK_TEMP = 2 };
 constexpr uint32_t kStoredShift = 18, kStoredUnit = 128;
 
 /* the constants of the functions by pairs, read two at a time: moves would cost as much as the
- * arithmetic of a single pair (pairs_ptx.cuh has the same numbers as text) */
+ * arithmetic of a single pair */
 __constant__ __align__(16) unsigned long long kPairConstants[] = {
-    0x3EA2F9833EA2F983ull, 0x4B4000004B400000ull, 0xCB400000CB400000ull, 0xC0490FDBC0490FDBull, 0x33BBBD2E33BBBD2Eull, 0x27772CED27772CEDull,
-    0xB2CD31C1B2CD31C1ull, 0x3638B8243638B824ull, 0xB9500BECB9500BECull, 0x3C0888863C088886ull, 0xBE2AAAABBE2AAAABull, 0ull,
-    0x3FB8AA3B3FB8AA3Bull, 0x4B4000004B400000ull, 0x32A5706032A57060ull, 0ull,
-    0xCB400000CB400000ull, 0xBD9C5854BD9C5854ull, 0x3E02AC143E02AC14ull, 0xBE06C251BE06C251ull, 0x3E116D423E116D42ull, 0xBE2A392FBE2A392Full,
-    0x3E4CD0023E4CD002ull, 0xBE800113BE800113ull, 0x3EAAAAAA3EAAAAAAull, 0xBF000000BF000000ull, 0x35BFBE8E35BFBE8Eull, 0x3F3172003F317200ull,
-    0xB9EECA99B9EECA99ull, 0x3B2941E73B2941E7ull, 0xBC0767FDBC0767FDull, 0x3CB177BC3CB177BCull, 0xBD5CE4F8BD5CE4F8ull, 0x3E08879A3E08879Aull,
-    0xBEAAAAA7BEAAAAA7ull, 0x4038AA3B4038AA3Bull, 0x3325706033257060ull, 0x4B4000004B400000ull, 0x3F8000003F800000ull, 0x4000000040000000ull};
+    SB_SIN_LIST(SB_PAIR_WORD) 0ull, /* 0: eleven and one to fill the last pair of words, as RK_K2's offsets count them */
+    SB_EXP_LIST(SB_PAIR_WORD) 0ull, /* 96 */
+    SB_LOG_LIST(SB_PAIR_WORD)       /* 128 */
+    SB_TANH_LIST(SB_PAIR_WORD)};    /* 224 */
+static_assert(sizeof(kPairConstants) == 320, "the offsets RK_K2 is given count on this layout");
 
 /* The block carries a whole observation interval: the instruction that ends a right-hand side goes on with
  * the integrator's part of the stage (E0 to E3: sum += weight * rhs, the next stage's value of this
