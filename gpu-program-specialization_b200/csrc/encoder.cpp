@@ -651,6 +651,20 @@ struct Emitter {
 
 }  // namespace
 
+ProgramRules rollout_rules(size_t num_states, size_t num_constants, unsigned toggle_bits) {
+    ProgramRules rules;
+    rules.num_columns = num_states;
+    rules.num_constants = num_constants;
+    rules.banks_allowed = true;
+    rules.toggle_bits = toggle_bits;
+    rules.columns_are_slots = true;
+    rules.reserved_slots = (unsigned)num_states;
+    rules.split_parts = true;
+    rules.hoist_bank = true;
+    rules.fuse_store_load = true;
+    return rules;
+}
+
 SecantResult routine_arities(const SecantAstProgramList& routines, uint8_t* arity) {
     if (routines.count > SECANT_AST_MAX_ROUTINES || (routines.count && !routines.items)) return SECANT_ERROR_INVALID_VALUE;
     for (size_t i = 0; i < routines.count; ++i) {

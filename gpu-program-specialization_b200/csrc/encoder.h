@@ -25,8 +25,8 @@ struct ProgramRules {
     bool banks_allowed = false; /* only the toggle shape has banks and toggles */
     unsigned toggle_bits = 0;   /* toggle bit indices must be below this */
     /* Rollout scoring: COLUMN i is not a dataset column but state i of the trajectory being
-     * integrated, which the kernel keeps in spill slot i; the first `reserved_slots` slots
-     * belong to the integrator and program temporaries start after them. */
+     * integrated, which records address as spill slot i; the first `reserved_slots` slots are the
+     * states' and program temporaries start after them. */
     bool columns_are_slots = false;
     unsigned reserved_slots = 0;
     /* main part: "STORE slot; LOAD x" becomes one instruction (record.h, SB_STORE_THEN_LOAD); only the
@@ -53,6 +53,10 @@ struct ProgramRules {
     bool hoist_toggled = true;
     unsigned max_hoisted = 4;
 };
+
+/* The rollout kernel's records: columns are the states, one slot each; what depends on the constants only
+ * is computed in the bank part, once per candidate and not once per stage. */
+ProgramRules rollout_rules(size_t num_states, size_t num_constants, unsigned toggle_bits);
 
 /* Encoded records of a contiguous group of programs, ready to upload as five arrays. */
 struct EncodedBatch {

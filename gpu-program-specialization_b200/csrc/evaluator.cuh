@@ -179,8 +179,8 @@ struct Rk4Problem {
 /* Scans the times and reference values once per call and raises *problem.invalid_flag; every launch_rk4()
  * of the call has to come after it. */
 cudaError_t launch_rk4_validation(const Rk4Problem& problem, cudaStream_t stream);
-/* batch.programs holds num_systems * num_states records, system-major, encoded with
- * columns_are_slots, 4 * num_states reserved slots and a bank part. */
+/* batch.programs holds num_systems * num_states records, system-major, encoded by
+ * rollout_rules(). */
 cudaError_t launch_rk4(const DeviceBatch& batch, const Rk4Problem& problem, size_t smem_limit, cudaStream_t stream);
 
 /* Adds the statistics of the static Gram shape for a batch of cohorts over `rows` rows of

@@ -281,16 +281,7 @@ extern "C" SecantResult secant_b200_rk4_score(const SecantB200Rk4Run* given) {
             return SECANT_ERROR_INSUFFICIENT_BUFFER;
     }
 
-    ProgramRules rules;
-    rules.num_columns = S;
-    rules.num_constants = K;
-    rules.banks_allowed = true;
-    rules.toggle_bits = run->toggle_bits;
-    rules.columns_are_slots = true;
-    rules.reserved_slots = (unsigned)(4 * S); /* stage, next stage, sum, state vectors */
-    rules.split_parts = true;                 /* what depends on the constants only is computed once per candidate, */
-    rules.hoist_bank = true;                  /* not once per stage */
-    rules.fuse_store_load = true;
+    const ProgramRules rules = rollout_rules(S, K, run->toggle_bits);
     for (size_t i = 0; i < programs.routines.count; ++i) {
         const SecantResult r = preflight(programs.routines.items[i], rules);
         if (r != SECANT_SUCCESS) return r;

@@ -436,7 +436,7 @@ rk4_kernel(const DeviceBatch batch, const Rk4Problem prob, const RolloutLayout l
     float* const table = reinterpret_cast<float*>(warea + lay.exec_bytes);
     float* const source = reinterpret_cast<float*>(warea + lay.exec_bytes + lay.table_bytes);
     float* const tmp = source + K + batch.max_extra;
-    const uint32_t table_address = shared_address(table), first_temp = 4u * S; /* the records' reserved slots */
+    const uint32_t table_address = shared_address(table), first_temp = S; /* the states' slots come first */
     Rollout<RR> m;
     m.temps = shared_address(warea + lay.exec_bytes + lay.table_bytes + lay.source_bytes) + lane * (uint32_t)(RR * 4);
     const unsigned long long configs = (unsigned long long)prob.num_banks << prob.toggle_bits;
@@ -658,8 +658,8 @@ cudaError_t launch_width(const DeviceBatch& batch, const Rk4Problem& prob, size_
     lay.exec_bytes = round16(((size_t)batch.max_insn + 1) * sizeof(SbInsn));
     lay.table_bytes = round16(((size_t)batch.max_cst + 1) * RR * 4);
     lay.source_bytes = round16(((size_t)prob.num_constants + batch.max_extra + batch.max_btmp) * 4 + 16);
-    /* max_slots includes the four reserved per state that the records leave before their temporaries */
-    lay.temp_bytes = (batch.max_slots > 4u * S ? batch.max_slots - 4u * S : 0u) * (uint32_t)RR * 128u;
+    /* max_slots counts the states' slots, which the records leave before their temporaries */
+    lay.temp_bytes = (batch.max_slots > S ? batch.max_slots - S : 0u) * (uint32_t)RR * 128u;
     lay.warp_bytes = lay.exec_bytes + lay.table_bytes + lay.source_bytes + lay.temp_bytes;
     lay.group_bytes = 2u * S * (uint32_t)(RR * 128) + 16u + S * lay.warp_bytes;
     /* groups per CTA: the count that puts most warps on an SM (shared memory per SM is the CTA limit

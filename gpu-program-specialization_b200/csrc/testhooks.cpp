@@ -32,8 +32,7 @@ SBT_EXPORT int sbt_encode(const uint8_t* routine_blob, const uint64_t* routine_o
     /* flags: bit 0 run the preflight scan first; bit 1 hoist bank-only and row-only sub-expressions; bit 3 only
      * row-only sub-expressions that no toggle reaches;
      * bit 2 one-part records with direct constant addressing (the rollout kernel's form);
-     * bit 4 the rollout kernel's split form: columns are the first spill slots (four vectors of them are
-     * reserved for the integrator), bank-only sub-expressions move to the bank part, nothing else is hoisted;
+     * bit 4 the rollout kernel's form (rollout_rules(), banks_allowed is ignored);
      * bits 8..15 cap on hoisted row values (0 = default) */
     const bool run_preflight = (flags & 1) != 0, hoist = (flags & 2) != 0, flat = (flags & 4) != 0;
     std::vector<const SecantAstInstruction*> routines(num_routines), asts(num_asts);
@@ -52,14 +51,7 @@ SBT_EXPORT int sbt_encode(const uint8_t* routine_blob, const uint64_t* routine_o
     b->rules.hoist_bank = hoist && !flat;
     b->rules.hoist_row = hoist && !flat;
     b->rules.hoist_toggled = !(flags & 8u);
-    if (flags & 16u) {
-        b->rules.columns_are_slots = true;
-        b->rules.reserved_slots = (unsigned)(4 * num_columns);
-        b->rules.split_parts = true;
-        b->rules.hoist_bank = true;
-        b->rules.hoist_row = false;
-        b->rules.fuse_store_load = true;
-    }
+    if (flags & 16u) b->rules = rollout_rules(num_columns, num_constants, toggle_bits);
     if ((flags >> 8) & 0xff) b->rules.max_hoisted = (unsigned)((flags >> 8) & 0xff);
     SecantResult r = SECANT_SUCCESS;
     if (run_preflight) {
