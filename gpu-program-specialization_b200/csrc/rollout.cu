@@ -706,6 +706,12 @@ cudaError_t launch_rk4_validation(const Rk4Problem& prob, cudaStream_t stream) {
     return cudaGetLastError();
 }
 
+/* Trajectories per lane: the fewest whose pass holds them all, and four beyond 64.  Milliseconds a call with
+ * 1 / 2 / 4 of them, 2,048 systems of three states, 200 steps: 32 trajectories 4.6 / 4.7 / 6.1, 33: 7.7 / 4.9 /
+ * 6.3, 64: 7.6 / 4.6 / 6.4, 65: 10.5 / 7.7 / 6.7, 128: 14.1 / 8.0 / 6.2, 512: 51 / 26 / 19.  The widest form has
+ * 120 registers, so 16 warps per SM instead of 30, and still wins beyond 64 because it walks half the passes;
+ * with eight states the two meet between 129 and 192 trajectories (6.3 against 6.6, 6.7 against 7.1 ms for
+ * 1,024 systems, 100 steps), before that and after it the wider one is ahead there too. */
 cudaError_t launch_rk4(const DeviceBatch& batch, const Rk4Problem& prob, size_t smem_limit, cudaStream_t stream) {
     if (prob.num_trajectories <= 32) return launch_width<1>(batch, prob, smem_limit, stream);
     if (prob.num_trajectories <= 64) return launch_width<2>(batch, prob, smem_limit, stream);
