@@ -43,7 +43,7 @@ for _p in (os.path.join(ROOT, "gpu-program-specialization_b200"), os.path.join(R
 
 from secant_b200 import abi, programs as P  # noqa: E402
 
-WORKLOAD = dict(name="configs[1] Secant-SR population scoring", programs=65536, max_tokens=32, slots=16, banks=64,
+WORKLOAD = dict(name="Secant-SR population scoring", programs=65536, max_tokens=32, slots=16, banks=64,
                 rows=1 << 20, features=8, seed=2)
 METRIC = "scored program·rows/sec"
 
@@ -194,23 +194,24 @@ def reference_arm(args, w):
 
 
 # What the evaluator kernel executes, from one multi-pass profiler capture of a reduced case of this
-# workload (4,096 programs x 131,072 rows, the summary is profiles/eval_kernel_configs1_reduced_ncu_full.md).
+# workload (4,096 programs x 131,072 rows, the summary is profiles/interpreter_cores.md).
 # Not measured in this run: counters of that kind need a profiler and the full size is too large for it.
 EXECUTED_ON_REDUCED_CASE = {
     "source": "profiler capture of a reduced case (4,096 programs x 131,072 rows), not this run",
-    "pipe_fma_pct": 32.8, "pipe_alu_pct": 36.6, "pipe_xu_pct": 13.8, "issue_active_pct": 69.0,
-    "instruction_cache_hit_pct": 97.6, "fp32_share_of_executed_instructions": 0.335,
+    "pipe_fma_pct": 29.7, "pipe_alu_pct": 37.1, "pipe_xu_pct": 15.6, "issue_active_pct": 61.0,
+    "instruction_cache_hit_pct": 99.4, "fp32_share_of_executed_instructions": 0.403,
+    "warp_instructions_per_interpreted_instruction": 56,
 }
 
 
 # ------------------------------------------------------------------------ RK4 arm ----
 
-# The same kind of figures for the rollout kernel: one launch of 2,048 systems of the configs[3]
-# population under a profiler (profiles/rk4_kernel_configs3.md), not this run.
+# The same kind of figures for the rollout kernel: one launch of the first 4,096 systems of the
+# population under a profiler (profiles/interpreter_cores.md), not this run.
 RK4_EXECUTED_ON_REDUCED_CASE = {
-    "source": "profiler capture of one launch of 2,048 systems, not this run",
-    "warp_instructions_per_interpreted_instruction": 50, "fp32_share_of_executed_instructions": 0.138,
-    "issue_active_pct_at_2_warps_per_scheduler": 35.7,
+    "source": "profiler capture of one launch of 4,096 systems, not this run",
+    "warp_instructions_per_interpreted_instruction": 20, "fp32_share_of_executed_instructions": 0.191,
+    "issue_active_pct": 43.8, "instruction_cache_hit_pct": 99.9,
 }
 
 def rk4_arm(args, w):
@@ -271,7 +272,7 @@ def rk4_arm(args, w):
     print(json.dumps({"impl": "rk4", "metric": "candidate systems scored/sec", "value": systems * banks / dt, "unit": "systems/s",
                       "n_gpus": 1, "steps": args.steps, "warmup": args.warmup, "ms_per_step": dt * 1e3, "higher_is_better": True,
                       "dtype": "f32", "data": "synthetic",
-                      "config": {"workload": "configs[3] RK4 rollout scoring", "systems": systems, "coefficient_sets": banks, "states": S, "coefficients": K,
+                      "config": {"workload": "RK4 rollout scoring", "systems": systems, "coefficient_sets": banks, "states": S, "coefficients": K,
                                  "initial_conditions": ics, "rk4_steps": steps, "max_tokens_per_state": 24,
                                  "mean_ops_per_system": float(ops.mean()), "valid_fraction": valid,
                                  "integrated_share": share, "ms_per_call": [round(x * 1e3, 1) for x in seconds],
@@ -475,7 +476,7 @@ def comparator_arm(args, w):
 
 def parity_spot(w, pop, x_h, y_h, banks_h, runner, dev, programs=32, rows=65536):
     """Scores `programs` seeded programs of the timed population on a row prefix with the library and
-    with the CPU checker (float64-accumulated sums, widened by the 2-ulp sensitivity of the math
+    with the CPU oracle (float64-accumulated sums, widened by the 2-ulp sensitivity of the math
     functions as in tests/parity.py) and counts the bins that disagree."""
     import torch
     from concurrent.futures import ThreadPoolExecutor
@@ -505,7 +506,7 @@ def parity_spot(w, pop, x_h, y_h, banks_h, runner, dev, programs=32, rows=65536)
     with ThreadPoolExecutor(max_workers=min(len(pick), os.cpu_count() or 1)) as pool:
         results = list(pool.map(check, range(len(pick))))
     return {"programs": int(len(pick)), "rows": int(rows), "bins": sum(r[2] for r in results), "bad": sum(r[0] for r in results),
-            "skipped": sum(r[1] for r in results), "rule": "1e-4 relative to the float64-accumulated checker sum, widened by 2-ulp sensitivity"}
+            "skipped": sum(r[1] for r in results), "rule": "1e-4 relative to the float64-accumulated oracle sum, widened by 2-ulp sensitivity"}
 
 
 def gpu_arm(args, w):

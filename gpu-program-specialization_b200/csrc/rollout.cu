@@ -75,7 +75,7 @@ __device__ __forceinline__ void sts(uint32_t a, const float (&x)[RR]) {
  * The machine is one block of PTX for the reasons given in eval_kernel.cuh, and here for one more: an
  * item is one chain of dependent instructions, so what an interpreted instruction costs decides how long
  * a call takes (two values per lane share it, where the population evaluator's sixteen do).  With the
- * C++ machine it cost 50 issued instructions, of which dispatch was half; here it costs 22, the
+ * C++ machine it cost 50 issued instructions, of which dispatch was half; here it costs 20, the
  * integrator's part included.  In a chain of them one takes 75 cycles for an addition with any operand,
  * 110 for an exponential, 200 for a sine or a division (one warp alone on its SM). */
 enum { H_END = 0, H_LOAD = 1, H_STORE = 4, H_STLOAD = 5, H_ADD = 8, H_SUB = 11, H_RSUB = 14, H_MUL = 17, H_DIV = 20, H_RDIV = 23, /* + kind */
@@ -417,7 +417,7 @@ __device__ __forceinline__ bool group_all(uint32_t barrier, uint32_t threads, bo
  * sizes in registers; the stage values are in shared memory twice, so one barrier per stage is enough
  * (a warp writes the next stage's value of its state while others still read this stage's).
  * 4,096 systems of three states, 64 trajectories, 1,000 steps: 71.8 ms with one warp per item and the
- * machine in C++, 25.6 now; the warps that are resident (30 of an SM's 64, by their registers) issue in
+ * machine in C++, 25.1 now; the warps that are resident (30 of an SM's 64, by their registers) issue in
  * 44 % of the cycles, and wait for one another at the barriers for a third of their time. */
 template <int RR>
 __global__ void __launch_bounds__(kRolloutMaxWarps * 32, RR == 4 ? 1 : 2)
