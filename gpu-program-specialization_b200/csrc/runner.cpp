@@ -94,6 +94,12 @@ struct Slot {
     std::vector<char> used;         /* which compute streams this batch touched */
 };
 
+/* Programs of an uploaded batch that are launched together: its programs from `first` on, in launch order. */
+struct View {
+    DeviceBatch batch;
+    size_t first;
+};
+
 }  // namespace
 }  // namespace sb
 
@@ -145,7 +151,7 @@ struct SecantB200PopulationImpl {
     std::vector<const uint8_t*> ast_ptrs, routine_ptrs;
     SecantAstProgramSet set{};
     unsigned toggle_bits = 0;
-    struct Resident { void* device = nullptr; std::vector<DeviceBatch> views; size_t first = 0; };
+    struct Resident { void* device = nullptr; std::vector<View> views; std::vector<SbProgram> headers; /* in launch order */ };
     std::vector<Resident> batches;
     uint64_t total_ops = 0;
 };
@@ -362,8 +368,9 @@ void order_programs(Slot& s) {
 
 /* Joins the batch's encoded pieces in the slot's pinned buffer (a program's offsets move by what lies
  * before its piece), grows the device buffer when needed, and enqueues the upload.
- * Layout: programs | insns | patches | affines | lits. */
-SecantResult upload_batch(SecantCubinRunnerImpl* r, Slot& s, std::vector<DeviceBatch>* views) {
+ * Layout: programs | insns | patches | affines | lits.  The pinned buffer keeps the programs' headers, in launch
+ * order, until the slot is used again. */
+SecantResult upload_batch(SecantCubinRunnerImpl* r, Slot& s, std::vector<View>* views) {
     size_t n_programs = 0, n_insns = 0, n_patches = 0, n_affines = 0, n_lits = 0;
     for (size_t q = 0; q < s.used_pieces; ++q) {
         const EncodedBatch& e = s.pieces[q].enc;
@@ -446,7 +453,7 @@ SecantResult upload_batch(SecantCubinRunnerImpl* r, Slot& s, std::vector<DeviceB
             db.max_btmp = std::max<uint32_t>(db.max_btmp, p.n_btmp);
             db.uses_scratch |= (p.flags & SB_PROG_USES_SCRATCH) ? 1u : 0u;
         }
-        views->push_back(db);
+        views->push_back(View{db, bounds[k]});
     }
     return SECANT_SUCCESS;
 }
@@ -513,19 +520,45 @@ SecantResult stream_scratch(SecantCubinRunnerImpl* r, size_t k, size_t elements,
 
 /* The part of the machine a view's launch should count on: with two views of one run entry on two streams
  * both are on the device at a time, and when neither fills it they share it by their work. */
-double view_share(const SecantCubinRunnerImpl* r, const std::vector<DeviceBatch>& views, const DeviceBatch& db, size_t entries) {
+double view_share(const SecantCubinRunnerImpl* r, const std::vector<View>& views, const View& view, size_t entries) {
     if (r->streams.size() < 2 || entries != 1 || views.size() < 2) return 1.0;
     double all = 0.0;
-    for (const DeviceBatch& v : views) all += (double)v.total_cost;
-    return std::min(0.95, std::max(0.05, (double)db.total_cost / std::max(1.0, all)));
+    for (const View& v : views) all += (double)v.batch.total_cost;
+    return std::min(0.95, std::max(0.05, (double)view.batch.total_cost / std::max(1.0, all)));
+}
+
+/* The programs of a view from `first` on whose constant tables take at most `most` floats, one at least.  Every
+ * table of a launch has room for the permutations of the program that reads most bits, so a launch takes its
+ * measure from its own programs: those with most permutations come first in launch order and mostly keep to
+ * themselves (1,024 programs of which one reads 14 bits, 64 sets, 2,000 rows: 466 ms in 105 launches when the
+ * largest program of the view was the measure of all). */
+DeviceBatch tables_that_fit(const View& view, const SbProgram* headers, size_t first, uint32_t banks, size_t most) {
+    DeviceBatch part = view.batch;
+    part.programs += first;
+    part.num_programs = 0;
+    part.total_cst = 0;
+    part.total_perms = 0;
+    part.max_bits = 0;
+    for (size_t i = first; i < view.batch.num_programs; ++i) {
+        const SbProgram& p = headers[view.first + i];
+        const uint64_t entries = part.total_cst + p.n_cst;
+        const uint32_t bits = std::max<uint32_t>(part.max_bits, p.bits);
+        if (part.num_programs && entries > most / ((banks + 3ull) << bits)) break;
+        ++part.num_programs;
+        part.total_cst = entries;
+        part.total_perms += (double)(1ull << p.bits);
+        part.max_bits = bits;
+    }
+    return part;
 }
 
 /* Enqueues the evaluation of one device-resident batch for every run entry, spreading
  * entries over the compute streams.  `after` (optional) is an event each stream waits on
  * first; `done`/`used` (optional) receive one completion event per touched stream. */
-SecantResult launch_batch(SecantCubinRunnerImpl* r, const DeviceBatch& db, double share, const std::vector<UnpackedRun>& runs,
-                          size_t* stream_cursor, cudaEvent_t after, std::vector<cudaEvent_t>* done, std::vector<char>* used) {
+SecantResult launch_batch(SecantCubinRunnerImpl* r, const View& view, const SbProgram* headers, double share,
+                          const std::vector<UnpackedRun>& runs, size_t* stream_cursor, cudaEvent_t after, std::vector<cudaEvent_t>* done, std::vector<char>* used) {
     const SecantCubinPlan& plan = *r->plan;
+    const DeviceBatch& db = view.batch;
     for (size_t e = 0; e < runs.size(); ++e) {
         const size_t k = (*stream_cursor)++ % r->streams.size();
         cudaStream_t stream = r->streams[k];
@@ -539,17 +572,10 @@ SecantResult launch_batch(SecantCubinRunnerImpl* r, const DeviceBatch& db, doubl
          * which few programs would fill few SMs): then the programs in as many launches as it takes, and a
          * program at a time at least */
         const size_t most_tables = r->scratch_limit / 2;
-        const size_t per_program = std::max<size_t>(1, (size_t)db.max_cst * (size_t)((prob.num_banks + 3ull) << db.max_bits));
-        const size_t fit = std::max<size_t>(1, most_tables / per_program);
-        const size_t step = db.total_cst <= most_tables / ((prob.num_banks + 3ull) << db.max_bits) ? db.num_programs : fit;
-        for (size_t first = 0; first < db.num_programs && ce == cudaSuccess; first += step) {
-            DeviceBatch part = db;
-            if (step < db.num_programs) {
-                part.programs += first;
-                part.num_programs = (uint32_t)std::min<size_t>(step, db.num_programs - first);
-                part.total_cst = (uint64_t)part.num_programs * db.max_cst;
-                part.total_perms = db.total_perms * part.num_programs / db.num_programs;
-            }
+        const bool whole = db.total_cst <= most_tables / ((prob.num_banks + 3ull) << db.max_bits);
+        for (size_t first = 0; first < db.num_programs && ce == cudaSuccess;) {
+            const DeviceBatch part = whole ? db : tables_that_fit(view, headers, first, prob.num_banks, most_tables);
+            first += part.num_programs;
             const LaunchPlan lp = plan_launch(part, prob, r->sm_count, r->smem_limit, r->scratch_limit, share);
             if (!lp.ok) {
                 r->last_error = lp.overflow ? "configuration count beyond the evaluator's 32-bit item index" : "program batch does not fit shared memory";
@@ -578,7 +604,7 @@ SecantResult launch_batch(SecantCubinRunnerImpl* r, const DeviceBatch& db, doubl
  * rows into the stream's scratch by the evaluator (every view of the batch), then reduced to the
  * cohorts' statistics, range after range on one stream, so every statistic is added to in row
  * order.  first_program is the batch's first program and a multiple of the cohort size. */
-SecantResult launch_gram_batch(SecantCubinRunnerImpl* r, const std::vector<DeviceBatch>& views, const std::vector<UnpackedRun>& runs,
+SecantResult launch_gram_batch(SecantCubinRunnerImpl* r, const std::vector<View>& views, const std::vector<UnpackedRun>& runs,
                                size_t first_program, size_t batch_programs, size_t* stream_cursor, cudaEvent_t after,
                                std::vector<cudaEvent_t>* done, std::vector<char>* used) {
     const SecantCubinPlan& plan = *r->plan;
@@ -590,7 +616,7 @@ SecantResult launch_gram_batch(SecantCubinRunnerImpl* r, const std::vector<Devic
         /* scratch: the range's predictions, then the constant tables of every view (padded to four banks at
          * most), which the first range makes and the others read again */
         size_t entries = 0;
-        for (const DeviceBatch& db : views) entries += db.total_cst;
+        for (const View& v : views) entries += v.batch.total_cst;
         /* rows per range: what the scratch limit leaves for this batch's predictions, between 128 and 16,384 */
         const size_t room = r->scratch_limit > 4 * entries ? (r->scratch_limit - 4 * entries) / 4 * 4 : 0;
         const size_t fit = room / batch_programs;
@@ -605,7 +631,7 @@ SecantResult launch_gram_batch(SecantCubinRunnerImpl* r, const std::vector<Devic
             const size_t rows_now = std::min(range, run.rows - r0);
             size_t tables = predictions;
             for (size_t v = 0; v < views.size(); ++v) {
-                const DeviceBatch& db = views[v];
+                const DeviceBatch& db = views[v].batch;
                 EvalProblem prob = make_problem(plan, run, 0);
                 prob.fast_math = r->fast_math;
                 prob.input += r0;
@@ -766,7 +792,7 @@ SecantResult execute(SecantCubinRunnerImpl* r, const std::vector<UnpackedRun>& r
     bool unknown = false;
     size_t launched_batches = 0, retired_batches = 0, stream_cursor = 0;
     double upload_seconds = 0, wait_seconds = 0, encode_sum = 0;
-    std::vector<DeviceBatch> views;
+    std::vector<View> views;
     const auto retire = [&]() { /* the oldest batch in flight: wait for it and open its slot for the batch that comes next to it */
         Slot& old = r->slots[retired_batches % r->slots.size()];
         const double t_wait = now_seconds();
@@ -814,8 +840,8 @@ SecantResult execute(SecantCubinRunnerImpl* r, const std::vector<UnpackedRun>& r
             const size_t first = b * batch_size;
             result = launch_gram_batch(r, views, runs, first, std::min(batch_size, P - first), &stream_cursor, slot.uploaded, done, &slot.used);
         } else {
-            for (const DeviceBatch& db : views) {
-                result = launch_batch(r, db, view_share(r, views, db, runs.size()), runs, &stream_cursor, slot.uploaded, done, &slot.used);
+            for (const View& view : views) {
+                result = launch_batch(r, view, static_cast<const SbProgram*>(slot.pinned), view_share(r, views, view, runs.size()), runs, &stream_cursor, slot.uploaded, done, &slot.used);
                 if (result != SECANT_SUCCESS) break;
             }
         }
@@ -1009,8 +1035,8 @@ SecantResult execute_resident(SecantCubinRunnerImpl* r, SecantB200PopulationImpl
     size_t cursor = 0;
     SecantResult result = SECANT_SUCCESS;
     for (auto& b : pop->batches) {
-        for (const DeviceBatch& db : b.views) {
-            result = launch_batch(r, db, view_share(r, b.views, db, runs.size()), runs, &cursor, nullptr, nullptr, nullptr);
+        for (const View& view : b.views) {
+            result = launch_batch(r, view, b.headers.data(), view_share(r, b.views, view, runs.size()), runs, &cursor, nullptr, nullptr, nullptr);
             if (result != SECANT_SUCCESS) break;
         }
         if (result != SECANT_SUCCESS) break;
@@ -1073,6 +1099,7 @@ SecantResult secant_b200_population_create(SecantCubinRunner r, const SecantAstP
     if (!pop) return SECANT_ERROR_ALLOCATION_FAILED;
     pop->runner = r;
     pop->toggle_bits = toggle_bits;
+    Slot staging; /* reuses the upload helper; its device buffers are handed to the population */
     try {
         result = copy_programs(programs->routines, &pop->routine_bytes, &pop->routine_ptrs);
         if (result == SECANT_SUCCESS) result = copy_programs(programs->asts, &pop->ast_bytes, &pop->ast_ptrs);
@@ -1084,7 +1111,6 @@ SecantResult secant_b200_population_create(SecantCubinRunner r, const SecantAstP
         size_t batch_size = (P + 3) / 4;
         if (batch_size < kMinBatch) batch_size = kMinBatch;
         if (batch_size > P) batch_size = P;
-        Slot staging; /* reuses the upload helper; its buffers are handed to the population */
         staging.pieces.resize(1);
         staging.used_pieces = 1;
         for (size_t first = 0; first < P && result == SECANT_SUCCESS; first += batch_size) {
@@ -1105,18 +1131,19 @@ SecantResult secant_b200_population_create(SecantCubinRunner r, const SecantAstP
             result = upload_batch(r, staging, &res.views);
             if (result != SECANT_SUCCESS) break;
             if (cudaStreamSynchronize(r->copy_stream) != cudaSuccess) { result = SECANT_ERROR_DRIVER_FAILED; break; }
+            res.headers.assign(static_cast<const SbProgram*>(staging.pinned), static_cast<const SbProgram*>(staging.pinned) + count);
+            pop->batches.reserve(pop->batches.size() + 1);
             res.device = staging.device; /* keep this allocation; the next batch gets a new one */
-            res.first = first;
             staging.device = nullptr;
             staging.device_cap = 0;
-            pop->batches.push_back(res);
+            pop->batches.push_back(std::move(res));
         }
-        if (staging.pinned) cudaFreeHost(staging.pinned);
-        if (staging.device) cudaFree(staging.device);
-        if (staging.uploaded) cudaEventDestroy(staging.uploaded);
     } catch (const std::bad_alloc&) {
         result = SECANT_ERROR_ALLOCATION_FAILED;
     }
+    if (staging.pinned) cudaFreeHost(staging.pinned);
+    if (staging.device) cudaFree(staging.device);
+    if (staging.uploaded) cudaEventDestroy(staging.uploaded);
     if (result != SECANT_SUCCESS) {
         for (auto& b : pop->batches) cudaFree(b.device);
         delete pop;

@@ -95,6 +95,33 @@ def test_sums_of_unsplit_rows_take_no_scratch(lib):
     assert largest_scratch(lib, h, 0) == (0, 0)
 
 
+@pytest.mark.parametrize("resident", [False, True])
+def test_a_program_with_many_toggle_bits_does_not_size_the_others_tables(lib, resident):
+    """600 programs read two bits at most and one reads twelve.  With room for a few tables of its size the
+    launches stay few: those of the others are as small as they are alone."""
+    class Uneven(Harness):
+        ROWS, BITS = 100, 12
+    h = Uneven(lib, programs=601)
+    asts = list(P.random_population(13, 600, 16, h.F, h.K, 1.0, toggle_bits=2, ops=P.ARITHMETIC_OPS).asts)
+    wide = P.col(0) + b"".join(P.bank(b % h.K) + P.col(b % h.F) + P.tog2(b) + P.op("ADD") for b in range(h.BITS))
+    h.pop = P.PackedPrograms(asts[:300] + [wide + P.RET] + asts[300:])
+    h.pop.fill(h.run.programs)
+    code, r = h.create(workers=1, streams=2)
+    limit = 8 * 4 * (h.K * (h.BANKS + 3) << h.BITS)
+    assert code == 0 and lib.secant_b200_runner_set_scratch_limit(r, limit) == 0
+    pop = C.c_void_p()
+    if resident:
+        assert lib.secant_b200_population_create(r, C.byref(h.run.programs), h.BITS, C.byref(pop)) == 0
+    lib.fake_reset()
+    assert (lib.secant_b200_population_run(pop, C.byref(h.run), C.byref(h.stats)) if resident else h.execute(r)) == 0
+    assert state(lib)["violations"] == 0 and 0 < scratch_of(lib)[0] <= limit
+    assert state(lib)["launches"] <= 6, state(lib)
+    if resident:
+        assert lib.secant_b200_population_destroy(pop) == 0
+    assert lib.secant_cubin_runner_destroy(r) == 0
+    h.release()
+
+
 @pytest.mark.parametrize("limit", [400 * KIB, 1000 * KIB, 4000 * KIB])
 def test_predictions_and_tables_of_the_gram_shape_stay_within_the_limit(lib, limit):
     used, _ = largest_scratch(lib, GramHarness(lib), limit)
