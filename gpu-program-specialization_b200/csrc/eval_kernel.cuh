@@ -65,7 +65,10 @@ __device__ __noinline__ void fma_over_scratch(uint2 ins, const float* rowp, cons
  * Measured on 2,048 programs x 64 sets x 131,072 rows, whole call: 58.6 ms with the scalar C++
  * interpreter; pairs in the C++ switch 69.8 (half the arithmetic, but the code no longer fitted the
  * cache); this core with the functions in C++ 46; with the functions in the block 43; with loops instead
- * of unrolled calls for unusual arguments 31.6.  Warp instructions 37.3e9 -> 18.4e9, cache hit rate of
+ * of unrolled calls for unusual arguments 31.6; sine, cosine and exponential of any argument inside the
+ * block 28.4 (sine and cosine had left it from 4,096 on and for NaN, the exponential beyond 86: 2 % of their tiles,
+ * which took a sixth of the time; 256 programs x 33 sets x 10,007 rows, where such a program is the last to end,
+ * 617 -> 455 us).  Before that, warp instructions 37.3e9 -> 18.4e9, cache hit rate of
  * the fetches 86 -> 98 %. */
 enum Handler : uint32_t {
     H_END = 0,
@@ -132,7 +135,8 @@ __device__ __forceinline__ void put_insn(SbInsn* at, SbInsn ins) {
 /* asm operands: 0..7 the tile, 8..15 the operand, 16 the address of the next instruction, 17 the
  * next handler and 18 word 1 of this instruction (at the end 17 says whether the run is over, 0, or an
  * instruction was left, 1); 19..22 the bases of dataset columns, hoisted
- * values (less kHoistedOffset), constants and slots for this lane; 23 the pair (-1, -1), 24 the pair (-0, -0). */
+ * values (less kHoistedOffset), constants and slots for this lane; 23 the pair (-1, -1), 24 the pair (-0, -0),
+ * 25 the turns of large arguments (sbmath.cuh). */
 #define SB_NEXT "mov.u32 hb, %17;\n ld.shared.v2.u32 {%17, %18}, [%16];\n add.u32 %16, %16, 8;\n"
 #define SB_GO "brx.idx.uni hb, targets;\n"
 #define SB_AT(BASE) "add.u32 ad, %18, " BASE ";\n"
@@ -211,23 +215,27 @@ __device__ __forceinline__ void put_insn(SbInsn* at, SbInsn ins) {
 #define SB_LOADQC_16 "ld.shared.b32 c0, [ad];\n mov.b64 %0, {c0, c0};\n"
 #define SB_MAPQ_CST_16 SB_COPY("%1", "%0") SB_COPY("%2", "%0") SB_COPY("%3", "%0") SB_COPY("%4", "%0") SB_COPY("%5", "%0") SB_COPY("%6", "%0") SB_COPY("%7", "%0")
 /* The accurate functions on all eight pairs (pairs_ptx.cuh). */
+/* what any argument takes is there once, for the pair in the first place: the pairs go round */
+#define SB_ROTATE "mov.b64 m, %0;\n mov.b64 %0, %1;\n mov.b64 %1, %2;\n mov.b64 %2, %3;\n mov.b64 %3, %4;\n mov.b64 %4, %5;\n mov.b64 %5, %6;\n mov.b64 %6, %7;\n mov.b64 %7, m;\n"
 #define SB_EACH(F) F("%0") F("%1") F("%2") F("%3") F("%4") F("%5") F("%6") F("%7")
 #define SB_FUNCTIONS                                                                                    \
     "CO:\n" SB_COS_SHIFT "bra.uni SC0;\n SI:\n" SB_SIN_SHIFT                                            \
-    "SC0:\n mov.f32 top, 0f00000000;\n" SB_EACH(SB_TOP) "setp.lt.f32 p, top, 0f45800000;\n" SB_ALL_OR_LEAVE SB_NEXT \
-    SB_SIN_CONSTANTS SB_EACH(SB_SIN_PAIR) SB_GO                                                         \
-    "EX:\n mov.f32 top, 0f00000000;\n" SB_EACH(SB_TOP) "setp.le.f32 p, top, 0f42AC0000;\n" SB_ALL_OR_LEAVE SB_NEXT \
-    SB_EXP_CONSTANTS SB_MINUS_ONE SB_EACH(SB_EXP_PAIR) SB_GO                                            \
+    "SC0:\n mov.f32 top, 0f00000000;\n" SB_EACH(SB_TOP_NUMBER) "setp.lt.f32 p, top, 0f49800000;\n" SB_VOTE SB_NEXT \
+    SB_SIN_CONSTANTS "@!p bra.uni SA;\n" SB_EACH(SB_SIN_PAIR) SB_GO                                     \
+    "SA:\n mov.u32 c5, 8;\n SL:\n" SB_SIN_ANY("%0", "%25", "SN") SB_ROTATE "sub.u32 c5, c5, 1;\n setp.ne.u32 p, c5, 0;\n @p bra.uni SL;\n" SB_GO \
+    "EX:\n mov.f32 top, 0f00000000;\n" SB_EACH(SB_TOP) "setp.le.f32 p, top, 0f42AC0000;\n" SB_VOTE SB_NEXT \
+    SB_EXP_CONSTANTS SB_MINUS_ONE "@!p bra.uni EA;\n" SB_EACH(SB_EXP_PAIR) SB_GO                        \
+    "EA:\n mov.u32 c5, 8;\n EL:\n" SB_EXP_ANY("%0") SB_ROTATE "sub.u32 c5, c5, 1;\n setp.ne.u32 p, c5, 0;\n @p bra.uni EL;\n" SB_GO \
     "TH:\n" SB_NEXT SB_TANH_CONSTANTS SB_MINUS_ONE SB_EACH(SB_TANH_PAIR) SB_GO                          \
     "LG:\n mov.f32 top, 0f00000000;\n mov.f32 low, 0f7F800000;\n" SB_EACH(SB_TOP) SB_EACH(SB_LOW)       \
     "setp.lt.f32 p, top, 0f7F800000;\n setp.ge.and.f32 p, low, 0f00800000, p;\n" SB_ALL_OR_LEAVE SB_NEXT \
     SB_LOG_CONSTANTS SB_MINUS_ONE SB_EACH(SB_LOG_PAIR) SB_GO                                            \
     "DV:\n mov.f32 top, 0f00000000;\n mov.f32 low, 0f7F800000;\n"                                      \
-    SB_EACH(SB_TOP) SB_TOP("%8") SB_TOP("%9") SB_TOP("%10") SB_TOP("%11") SB_TOP("%12") SB_TOP("%13") SB_TOP("%14") SB_TOP("%15") \
-    SB_EACH(SB_LOW_ABS) SB_LOW_ABS("%8") SB_LOW_ABS("%9") SB_LOW_ABS("%10") SB_LOW_ABS("%11") SB_LOW_ABS("%12") SB_LOW_ABS("%13") SB_LOW_ABS("%14") SB_LOW_ABS("%15") \
+    SB_EACH(SB_TOP_NUMBER) SB_TOP_NUMBER("%8") SB_TOP_NUMBER("%9") SB_TOP_NUMBER("%10") SB_TOP_NUMBER("%11") SB_TOP_NUMBER("%12") SB_TOP_NUMBER("%13") SB_TOP_NUMBER("%14") SB_TOP_NUMBER("%15") \
+    SB_EACH(SB_LOW_NUMBER) SB_LOW_NUMBER("%8") SB_LOW_NUMBER("%9") SB_LOW_NUMBER("%10") SB_LOW_NUMBER("%11") SB_LOW_NUMBER("%12") SB_LOW_NUMBER("%13") SB_LOW_NUMBER("%14") SB_LOW_NUMBER("%15") \
     SB_DIV_USUAL "@p bra.uni DW;\n"                                                                     \
     "mov.u32 c2, 0xffffffff;\n" SB_EACH(SB_LEAST) "mov.f32 low, 0f7F800000;\n"                          \
-    SB_LOW_ABS("%8") SB_LOW_ABS("%9") SB_LOW_ABS("%10") SB_LOW_ABS("%11") SB_LOW_ABS("%12") SB_LOW_ABS("%13") SB_LOW_ABS("%14") SB_LOW_ABS("%15") \
+    SB_LOW_NUMBER("%8") SB_LOW_NUMBER("%9") SB_LOW_NUMBER("%10") SB_LOW_NUMBER("%11") SB_LOW_NUMBER("%12") SB_LOW_NUMBER("%13") SB_LOW_NUMBER("%14") SB_LOW_NUMBER("%15") \
     SB_DIV_RANGE SB_ALL_OR_LEAVE "DW:\n" SB_NEXT                                                       \
     SB_DIV_CONSTANTS SB_DIV_PAIR("%0", "%8") SB_DIV_PAIR("%1", "%9") SB_DIV_PAIR("%2", "%10") SB_DIV_PAIR("%3", "%11") \
     SB_DIV_PAIR("%4", "%12") SB_DIV_PAIR("%5", "%13") SB_DIV_PAIR("%6", "%14") SB_DIV_PAIR("%7", "%15") SB_GO
@@ -253,14 +261,14 @@ __device__ __forceinline__ void put_insn(SbInsn* at, SbInsn ins) {
     "LG:\n mov.f32 low, 0f7F800000;\n" SB_EACH(SB_LOW) "setp.ge.f32 p, low, 0f00800000;\n" SB_ALL_OR_LEAVE SB_NEXT \
     SB_PAIR_CONST("k0", "0x3F3172183F317218") SB_EACH(SB_FAST_LOG) SB_GO                                \
     "DV:\n mov.f32 top, 0f00000000;\n mov.f32 low, 0f7F800000;\n" \
-    SB_TOP("%8") SB_TOP("%9") SB_TOP("%10") SB_TOP("%11") SB_TOP("%12") SB_TOP("%13") SB_TOP("%14") SB_TOP("%15") \
-    SB_LOW_ABS("%8") SB_LOW_ABS("%9") SB_LOW_ABS("%10") SB_LOW_ABS("%11") SB_LOW_ABS("%12") SB_LOW_ABS("%13") SB_LOW_ABS("%14") SB_LOW_ABS("%15") \
+    SB_TOP_NUMBER("%8") SB_TOP_NUMBER("%9") SB_TOP_NUMBER("%10") SB_TOP_NUMBER("%11") SB_TOP_NUMBER("%12") SB_TOP_NUMBER("%13") SB_TOP_NUMBER("%14") SB_TOP_NUMBER("%15") \
+    SB_LOW_NUMBER("%8") SB_LOW_NUMBER("%9") SB_LOW_NUMBER("%10") SB_LOW_NUMBER("%11") SB_LOW_NUMBER("%12") SB_LOW_NUMBER("%13") SB_LOW_NUMBER("%14") SB_LOW_NUMBER("%15") \
     "setp.le.f32 p, top, 0f7E800000;\n setp.ge.and.f32 p, low, 0f00800000, p;\n" SB_ALL_OR_LEAVE SB_NEXT \
     SB_FAST_DIV("%0", "%8") SB_FAST_DIV("%1", "%9") SB_FAST_DIV("%2", "%10") SB_FAST_DIV("%3", "%11")   \
     SB_FAST_DIV("%4", "%12") SB_FAST_DIV("%5", "%13") SB_FAST_DIV("%6", "%14") SB_FAST_DIV("%7", "%15") SB_GO
 
 #define SB_CORE(N, FUNCTIONS)                                                                           \
-    "{\n" SB_PTX_REGISTERS                                                                             \
+    "{\n" SB_PTX_REGISTERS SB_PTX_REGISTERS_ANY                                                        \
     ".reg .u32 hb;\n targets: .branchtargets EN, LR, LC, LS, ST, SH, AR, AC, AS, SR, SC, SS, RR, RC, RS, MR, MC, MS, NG, AB, " \
     "DR, DC, DS, QR, QC, QS, SI, CO, EX, LG, TH, LEAVE, LEAVE;\n"                                           \
     "ld.shared.u32 %17, [%16+-8];\n" SB_NEXT SB_GO                                                       \
@@ -440,7 +448,8 @@ struct Machine {
                      : "+l"(a[0]), "+l"(a[1]), "+l"(a[2]), "+l"(a[3]), "+l"(a[4]), "+l"(a[5]), "+l"(a[6]), "+l"(a[7]), "=&l"(x[0]),    \
                        "=&l"(x[1]), "=&l"(x[2]), "=&l"(x[3]), "=&l"(x[4]), "=&l"(x[5]), "=&l"(x[6]), "=&l"(x[7]), "+r"(ip), "=&r"(h),  \
                        "=&r"(w)                                                                                                       \
-                     : "r"(place.row), "r"(place.hoist - kHoistedOffset), "r"(cst), "r"(place.slots), "l"(minus_one), "l"(minus_zero)                                                    \
+                     : "r"(place.row), "r"(place.hoist - kHoistedOffset), "r"(cst), "r"(place.slots), "l"(minus_one), "l"(minus_zero),                                  \
+                       "l"(__cvta_generic_to_global(&sbm::kTurns))                                                                         \
                      : "memory")
 #pragma unroll 1
         for (;;) {

@@ -12,11 +12,15 @@
 #define SECANT_B200_PAIRS_PTX_CUH
 
 #define SB_PTX_REGISTERS ".reg .u32 ad, c0, c1, c2, c3, c4, c5;\n .reg .f32 f0, f1, top, low;\n .reg .b64 m, t, n, r, z, q, hf, nh, mone, k<12>;\n .reg .pred p;\n"
+#define SB_PTX_REGISTERS_ANY ".reg .b64 v, at, g<10>;\n .reg .f64 d<4>;\n .reg .b32 w0, w1, u0, u1, s0, s1;\n" /* what SB_SIN_ANY takes besides */
 #define SB_PAIR_CONST(R, BITS) "mov.b64 " R ", " BITS ";\n"
 #define SB_TOP(A) "mov.b64 {f0, f1}, " A ";\n max.NaN.abs.f32 top, top, f0, f1;\n"
+/* the same without regard to NaN, which the steps of sine, cosine and division pass on */
+#define SB_TOP_NUMBER(A) "mov.b64 {f0, f1}, " A ";\n max.abs.f32 top, top, f0, f1;\n"
+#define SB_LOW_NUMBER(A) "mov.b64 {f0, f1}, " A ";\n min.abs.f32 low, low, f0, f1;\n"
 #define SB_LOW(A) "mov.b64 {f0, f1}, " A ";\n min.NaN.f32 low, low, f0, f1;\n"
-#define SB_LOW_ABS(A) "mov.b64 {f0, f1}, " A ";\n min.NaN.abs.f32 low, low, f0, f1;\n"
-#define SB_ALL_OR_LEAVE "vote.sync.all.pred p, p, 0xffffffff;\n @!p bra.uni LEAVE;\n"
+#define SB_VOTE "vote.sync.all.pred p, p, 0xffffffff;\n"
+#define SB_ALL_OR_LEAVE SB_VOTE "@!p bra.uni LEAVE;\n"
 /* Constants of the steps below, each the bits of a float32 and written once: the evaluator's core moves them into
  * registers (SB_*_CONSTANTS), the rollout core reads them from a table of pairs (SB_PAIR_WORD, rollout.cu) and
  * the scalar functions name them (sbmath.cuh). */
@@ -25,6 +29,9 @@
 #define SB_SIN_LIST(X) \
     X(0, 3EA2F983) X(1, 4B400000) X(2, CB400000) X(3, C0490FDB) X(4, 33BBBD2E) X(5, 27772CED) \
     X(6, B2CD31C1) X(7, 3638B824) X(8, B9500BEC) X(9, 3C088886) X(10, BE2AAAAB)
+#define SB_TRIG_LIST(X) \
+    X(0, 3FC90FDB) X(1, B94CA22D) X(2, 3C08839E) X(3, BE2AAAA3) X(4, B4920F5C) \
+    X(5, 37D00870) X(6, BAB60B5C) X(7, 3D2AAAAB) X(8, BF000000) X(9, 3F800000)
 #define SB_EXP_LIST(X) \
     X(0, 3FB8AA3B) X(1, 4B400000) X(2, 32A57060)
 #define SB_LOG_LIST(X) \
@@ -48,11 +55,42 @@
     "fma.rn.f32x2 q, k6, z, k7;\n fma.rn.f32x2 q, q, z, k8;\n fma.rn.f32x2 q, q, z, k9;\n fma.rn.f32x2 q, q, z, k10;\n" \
     "mul.rn.f32x2 z, r, z;\n fma.rn.f32x2 r, z, q, r;\n mov.b64 {c0, c1}, t;\n shl.b32 c0, c0, 31;\n shl.b32 c1, c1, 31;\n" \
     "mov.b64 {c2, c3}, r;\n add.u32 c0, c0, c2;\n add.u32 c1, c1, c3;\n mov.b64 " A ", {c0, c1};\n"
+/* sin or cos of any pair (the shift says which, TURNS is the address of the table of sbmath.cuh): the steps above, and for a pair
+ * with a large argument somewhere in the warp those of sincos_large() as well.  Label DONE is the macro's own. */
+#define SB_TRIG_TEXT(I, BITS) "mov.b64 g" #I ", 0x" #BITS #BITS ";\n"
+#define SB_SIN_TURNS(W, F, Q, TURNS)                                                                    \
+    "shr.u32 c0, " W ", 23;\n and.b32 c0, c0, 255;\n max.u32 c0, c0, 147;\n min.u32 c0, c0, 254;\n shl.b32 c0, c0, 4;\n cvt.u64.u32 at, c0;\n" \
+    "add.u64 at, at, " TURNS ";\n ld.global.nc.v2.f64 {d0, d1}, [at+-2352];\n and.b32 c0, " W ", 0x007FFFFF;\n shr.u32 c0, c0, 3;\n" \
+    "and.b32 c1, " W ", 0x80000000;\n or.b32 c0, c0, c1;\n or.b32 c1, c0, 0x3FF00000;\n shl.b32 c0, " W ", 29;\n mov.b64 d2, {c0, c1};\n" \
+    "mul.rn.f64 d0, d2, d0;\n add.rn.f64 d3, d0, 0d4338000000000000;\n mov.b64 {" Q ", c1}, d3;\n add.rn.f64 d3, d3, 0dC338000000000000;\n" \
+    "sub.rn.f64 d0, d0, d3;\n fma.rn.f64 d0, d2, d1, d0;\n cvt.rn.f32.f64 " F ", d0;\n"
+#define SB_SIN_CHOOSE(W, Q, S, C, V) /* the quadrant's function and sign, where the argument is large and finite */ \
+    "add.u32 " Q ", " Q ", c3;\n and.b32 c0, " Q ", 1;\n setp.ne.u32 p, c0, 0;\n selp.b32 c0, " C ", " S ", p;\n and.b32 c1, " Q ", 2;\n" \
+    "shl.b32 c1, c1, 30;\n xor.b32 c0, c0, c1;\n and.b32 c1, " W ", 0x7FFFFFFF;\n sub.u32 c1, c1, 0x49800000;\n setp.lt.u32 p, c1, 0x36000000;\n" \
+    "selp.b32 " V ", c0, " V ", p;\n"
+#define SB_SIN_ANY(A, TURNS, DONE)                                                                      \
+    "mov.b64 v, " A ";\n mov.f32 top, 0f00000000;\n" SB_TOP_NUMBER("v") "setp.lt.f32 p, top, 0f49800000;\n vote.sync.all.pred p, p, 0xffffffff;\n" \
+    SB_SIN_PAIR(A) "@p bra.uni " DONE ";\n mov.b64 {w0, w1}, v;\n" SB_SIN_TURNS("w0", "f0", "u0", TURNS) SB_SIN_TURNS("w1", "f1", "u1", TURNS) \
+    SB_TRIG_LIST(SB_TRIG_TEXT) "mov.b64 r, {f0, f1};\n mul.rn.f32x2 r, r, g0;\n mul.rn.f32x2 z, r, r;\n fma.rn.f32x2 q, g1, z, g2;\n" \
+    "fma.rn.f32x2 q, q, z, g3;\n mul.rn.f32x2 t, r, z;\n fma.rn.f32x2 r, t, q, r;\n fma.rn.f32x2 q, g4, z, g5;\n fma.rn.f32x2 q, q, z, g6;\n" \
+    "fma.rn.f32x2 q, q, z, g7;\n mul.rn.f32x2 t, z, z;\n mul.rn.f32x2 z, z, g8;\n fma.rn.f32x2 q, t, q, z;\n add.rn.f32x2 q, q, g9;\n" \
+    "mov.b64 {c3, c4}, hf;\n shr.u32 c3, c3, 24;\n and.b32 c3, c3, 1;\n"                             \
+    "mov.b64 {f0, f1}, r;\n mov.b64 {top, low}, q;\n mov.b64 {s0, s1}, " A ";\n" SB_SIN_CHOOSE("w0", "u0", "f0", "top", "s0") \
+    SB_SIN_CHOOSE("w1", "u1", "f1", "low", "s1") "mov.b64 " A ", {s0, s1};\n " DONE ":\n"
 #define SB_EXP_PAIR(A)                                                                                  \
     "fma.rn.f32x2 t, " A ", k0, k1;\n fma.rn.f32x2 n, t, mone, k1;\n fma.rn.f32x2 r, " A ", k0, n;\n fma.rn.f32x2 r, " A ", k2, r;\n" \
     "mov.b64 {f0, f1}, r;\n ex2.approx.ftz.f32 f0, f0;\n ex2.approx.ftz.f32 f1, f1;\n mov.b64 {c0, c1}, t;\n" \
     "shl.b32 c0, c0, 23;\n shl.b32 c1, c1, 23;\n mov.b32 c2, f0;\n mov.b32 c3, f1;\n add.u32 c0, c0, c2;\n add.u32 c1, c1, c3;\n" \
     "mov.b64 " A ", {c0, c1};\n"
+/* e^x of any pair: the steps of exp_pair() (sbmath.cuh) */
+#define SB_EXP_ANY(A)                                                                                   \
+    "mov.b64 {f0, f1}, " A ";\n max.NaN.f32 f0, f0, 0fC2D00000;\n max.NaN.f32 f1, f1, 0fC2D00000;\n min.NaN.f32 f0, f0, 0f42B20000;\n" \
+    "min.NaN.f32 f1, f1, 0f42B20000;\n mov.b64 m, {f0, f1};\n fma.rn.f32x2 t, m, k0, k1;\n fma.rn.f32x2 n, t, mone, k1;\n" \
+    "fma.rn.f32x2 r, m, k0, n;\n fma.rn.f32x2 r, m, k2, r;\n mov.b64 {f0, f1}, r;\n ex2.approx.ftz.f32 f0, f0;\n ex2.approx.ftz.f32 f1, f1;\n" \
+    "mov.b64 r, {f0, f1};\n mov.b64 {c0, c1}, t;\n shr.s32 c2, c0, 1;\n shr.s32 c3, c1, 1;\n sub.u32 c0, c0, c2;\n sub.u32 c1, c1, c3;\n" \
+    "shl.b32 c0, c0, 23;\n shl.b32 c1, c1, 23;\n shl.b32 c2, c2, 23;\n shl.b32 c3, c3, 23;\n add.u32 c0, c0, 0x3F800000;\n add.u32 c1, c1, 0x3F800000;\n" \
+    "add.u32 c2, c2, 0x3F800000;\n add.u32 c3, c3, 0x3F800000;\n mov.b64 m, {c2, c3};\n mul.rn.f32x2 r, r, m;\n mov.b64 m, {c0, c1};\n" \
+    "mul.rn.f32x2 " A ", r, m;\n"
 /* the exponent becomes a float through the low bits of 1.5 * 2^23: exact, and off the conversion unit; the
  * mantissa is what is left when it is taken off the argument's bits (2^23 times the constant is 0 mod 2^32) */
 #define SB_LOG_PAIR(A)                                                                                  \
@@ -97,9 +135,9 @@
     "mov.b64 {c2, c3}, " A ";\n lop3.b32 c0, c0, c2, 0x7fffffff, 0xE4;\n lop3.b32 c1, c1, c3, 0x7fffffff, 0xE4;\n mov.b64 " A ", {c0, c1};\n"
 /* |b| within [2^-60, 2^60], |a| too or zero (2|a| - 1 in bits: zero wraps to the top): no step leaves the normal range */
 #define SB_LEAST(A) "mov.b64 {c0, c1}, " A ";\n shl.b32 c0, c0, 1;\n shl.b32 c1, c1, 1;\n sub.u32 c0, c0, 1;\n sub.u32 c1, c1, 1;\n min.u32 c2, c2, c0;\n min.u32 c2, c2, c1;\n"
-/* no zero among the dividends, the usual case: SB_TOP and SB_LOW_ABS over both (top = 0, low = inf before) are enough */
+/* no zero among the dividends, the usual case: SB_TOP_NUMBER and SB_LOW_NUMBER over both (top = 0, low = inf before) are enough */
 #define SB_DIV_USUAL "setp.le.f32 p, top, 0f5D800000;\n setp.ge.and.f32 p, low, 0f21800000, p;\n vote.sync.all.pred p, p, 0xffffffff;\n"
-/* after SB_LEAST over the dividends, SB_TOP over both, SB_LOW_ABS over the divisors (c2 = ~0, top = 0, low = inf before) */
+/* after SB_LEAST over the dividends, SB_TOP_NUMBER over both, SB_LOW_NUMBER over the divisors (c2 = ~0, top = 0, low = inf before) */
 #define SB_DIV_RANGE "setp.le.f32 p, top, 0f5D800000;\n setp.ge.and.f32 p, low, 0f21800000, p;\n setp.ge.and.u32 p, c2, 0x42FFFFFF, p;\n"
 
 #endif

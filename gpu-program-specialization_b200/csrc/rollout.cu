@@ -158,7 +158,7 @@ static_assert(sizeof(kPairConstants) == 320, "the offsets RK_K2 is given count o
     "NG:\n" RK_NEXT RK_EACH_##N(RK_NEG) RK_GO "AB:\n" RK_NEXT RK_EACH_##N(RK_ABS) RK_GO                  \
     "CO:\n" SB_COS_SHIFT "bra.uni SC0;\n SI:\n" SB_SIN_SHIFT                                            \
     "SC0:\n" RK_K2("k0", "k1", "0") RK_K2("k2", "k3", "16") RK_K2("k4", "k5", "32") RK_K2("k6", "k7", "48") RK_K2("k8", "k9", "64") \
-    RK_K2("k10", "m", "80") "mov.f32 top, 0f00000000;\n" RK_EACH_##N(SB_TOP) "setp.lt.f32 p, top, 0f45800000;\n" SB_ALL_OR_LEAVE RK_NEXT \
+    RK_K2("k10", "m", "80") "mov.f32 top, 0f00000000;\n" RK_EACH_##N(SB_TOP) "setp.lt.f32 p, top, 0f49800000;\n" SB_ALL_OR_LEAVE RK_NEXT \
     RK_EACH_##N(SB_SIN_PAIR) RK_GO                                                                      \
     "EX:\n" RK_K2("k0", "k1", "96") RK_K2("k2", "m", "112") "mov.f32 top, 0f00000000;\n" RK_EACH_##N(SB_TOP) \
     "setp.le.f32 p, top, 0f42AC0000;\n" SB_ALL_OR_LEAVE RK_NEXT RK_EACH_##N(SB_EXP_PAIR) RK_GO          \
@@ -170,12 +170,12 @@ static_assert(sizeof(kPairConstants) == 320, "the offsets RK_K2 is given count o
     RK_FETCH_THEN(N, "D", "DIV") RK_FETCH_THEN(N, "Q", "RDIV")                                          \
     /* operand / acc; what leaves for an unusual argument takes the accumulator along as it was */      \
     "RDIV:\n mov.f32 top, 0f00000000;\n mov.f32 low, 0f7F800000;\n" RK_EACH_##N(SB_TOP) RK_EACHX_##N(SB_TOP) \
-    RK_EACH_##N(SB_LOW_ABS) RK_EACHX_##N(SB_LOW_ABS) SB_DIV_USUAL "@p bra.uni RS;\n"                    \
-    "mov.u32 c2, 0xffffffff;\n mov.f32 low, 0f7F800000;\n" RK_EACHX_##N(SB_LEAST) RK_EACH_##N(SB_LOW_ABS) SB_DIV_RANGE SB_ALL_OR_LEAVE \
+    RK_EACH_##N(SB_LOW_NUMBER) RK_EACHX_##N(SB_LOW_NUMBER) SB_DIV_USUAL "@p bra.uni RS;\n"                    \
+    "mov.u32 c2, 0xffffffff;\n mov.f32 low, 0f7F800000;\n" RK_EACHX_##N(SB_LEAST) RK_EACH_##N(SB_LOW_NUMBER) SB_DIV_RANGE SB_ALL_OR_LEAVE \
     "RS:\n" RK_BOTH_##N(RK_SWAP) "bra.uni DW;\n"                                                       \
     "DIV:\n mov.f32 top, 0f00000000;\n mov.f32 low, 0f7F800000;\n" RK_EACH_##N(SB_TOP) RK_EACHX_##N(SB_TOP) \
-    RK_EACH_##N(SB_LOW_ABS) RK_EACHX_##N(SB_LOW_ABS) SB_DIV_USUAL "@p bra.uni DW;\n"                    \
-    "mov.u32 c2, 0xffffffff;\n mov.f32 low, 0f7F800000;\n" RK_EACH_##N(SB_LEAST) RK_EACHX_##N(SB_LOW_ABS) SB_DIV_RANGE SB_ALL_OR_LEAVE \
+    RK_EACH_##N(SB_LOW_NUMBER) RK_EACHX_##N(SB_LOW_NUMBER) SB_DIV_USUAL "@p bra.uni DW;\n"                    \
+    "mov.u32 c2, 0xffffffff;\n mov.f32 low, 0f7F800000;\n" RK_EACH_##N(SB_LEAST) RK_EACHX_##N(SB_LOW_NUMBER) SB_DIV_RANGE SB_ALL_OR_LEAVE \
     "DW:\n" RK_NEXT SB_DIV_CONSTANTS RK_BOTH_##N(SB_DIV_PAIR) RK_GO                                      \
     "EN:\n brx.idx.uni %11, stages;\n"                                                                   \
     "E0:\n mov.b64 k0, 0;\n" RK_STAGE_##N(RK_FIRST, "%16", "%17") "bra.uni SWAP;\n"                    \
