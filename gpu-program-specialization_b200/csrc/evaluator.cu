@@ -193,6 +193,7 @@ void launch_tables(const DeviceBatch& batch, const EvalProblem& prob, uint32_t b
 #define SB_DECLARE(NAME) \
     cudaError_t launch_##NAME(const DeviceBatch&, const EvalProblem&, const Geom&, const LaunchPlan&, float*, const float*, cudaStream_t); \
     cudaError_t configure_##NAME(int smem_limit);
+cudaError_t configure_gram(); /* gram.cu */
 SB_FOR_KINDS(SB_DECLARE) /* eval_*.cu: one file per kind of kernel */
 
 cudaError_t configure_kernels() {
@@ -202,7 +203,7 @@ cudaError_t configure_kernels() {
     if ((e = cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess) return e;
 #define SB_CONFIGURE(NAME) if ((e = configure_##NAME(limit)) != cudaSuccess) return e;
     SB_FOR_KINDS(SB_CONFIGURE)
-    return cudaSuccess;
+    return configure_gram();
 }
 
 cudaError_t launch_eval(const DeviceBatch& batch, const EvalProblem& prob, const LaunchPlan& plan, float* partial,

@@ -72,6 +72,7 @@ size_t align256(size_t v) { return (v + 255) / 256 * 256; }
  * taking it costs as much as encoding it (a program takes about 2 us, a hand-over under 1 us). */
 constexpr size_t kPieceMin = 16, kPieceMax = 128, kPiecesPerThread = 4;
 constexpr size_t kMinBatch = 4096; /* programs of a batch, when the run has as many */
+constexpr size_t kGramFloats = (size_t)1 << 24; /* predictions of a range of rows, see launch_gram_batch() */
 constexpr size_t kSlots = 3; /* batches encoded, uploaded or running at a time */
 
 struct Piece {
@@ -617,12 +618,13 @@ SecantResult launch_gram_batch(SecantCubinRunnerImpl* r, const std::vector<View>
          * most), which the first range makes and the others read again */
         size_t entries = 0;
         for (const View& v : views) entries += v.batch.total_cst;
-        /* rows per range: what the scratch limit leaves for this batch's predictions, between 128 and 16,384 */
+        /* rows per range: what the scratch limit leaves for this batch's predictions, between 128 and as many as stay in
+         * L2 beside the data (64 MB) or 16,384; a multiple of four, which the kernels' loads count on */
         const size_t room = r->scratch_limit > 4 * entries ? (r->scratch_limit - 4 * entries) / 4 * 4 : 0;
-        const size_t fit = room / batch_programs;
-        const size_t range = std::min<size_t>(run.rows, std::max<size_t>(128, std::min<size_t>(16384, fit)));
+        const size_t fit = room / batch_programs / 4 * 4, resident = kGramFloats / batch_programs / 4 * 4;
+        const size_t range = std::min<size_t>((run.rows + 3) / 4 * 4, std::max<size_t>(128, std::min<size_t>(std::max<size_t>(16384, resident), fit)));
         std::vector<int> tables_made(views.size(), -1); /* for which register tile */
-        const size_t predictions = (batch_programs * range + 3) / 4 * 4;
+        const size_t predictions = batch_programs * range;
         float* scratch = nullptr;
         const SecantResult a = stream_scratch(r, k, predictions + 4 * entries, &scratch);
         if (a != SECANT_SUCCESS) return a;
