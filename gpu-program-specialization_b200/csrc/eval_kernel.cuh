@@ -568,7 +568,7 @@ template <> struct TableWord<4> { typedef float4 type; };
 
 /* 16 values per thread: 20 warps per CTA within 96 registers (32-value tiles were measured
  * slower at the 12 warps their 168 registers allow). */
-template <int RR, int RC, bool FAST, bool SPAN, int KIND>
+template <int RR, int RC, bool FAST, bool SPAN, bool PARTS, int KIND>
 __global__ void __launch_bounds__(640, 1)
 eval_kernel(const DeviceBatch batch, const EvalProblem prob, const Geom geom, float* __restrict__ partial,
             const float* __restrict__ tables) {
@@ -610,7 +610,7 @@ eval_kernel(const DeviceBatch batch, const EvalProblem prob, const Geom geom, fl
      * (when one item holds every bank group) one item per block of ppi permutations; the planner keeps
      * items_per_program * prog_count below 2^32 - 256, so item arithmetic is 32-bit */
     const uint32_t chunks = materialize ? 1u : bank_groups / gpi;
-    const uint32_t items_per_program = !SPAN ? chunks : (uint32_t)(((unsigned long long)chunks << batch.max_bits) / ppi);
+    const uint32_t items_per_program = PARTS ? chunks * geom.parts : !SPAN ? chunks : (uint32_t)(((unsigned long long)chunks << batch.max_bits) / ppi);
     const unsigned int num_items = items_per_program * prog_count;
     const unsigned long long configs = (unsigned long long)prob.num_banks << prob.toggle_bits;
     const size_t quantity_stride = geom.direct ? prob.out_target_stride : (size_t)configs;
@@ -656,7 +656,16 @@ eval_kernel(const DeviceBatch batch, const EvalProblem prob, const Geom geom, fl
                 within = item / prog_count;
                 pi = item - within * prog_count;
             }
-            const uint32_t lp = group + pi * geom.num_groups;                        /* index inside the batch */
+            uint32_t pass = 0, end_pass = npass; /* the item's part of the tile */
+            uint32_t lp = group + pi * geom.num_groups; /* index inside the batch */
+            if constexpr (PARTS) {
+                const uint32_t chunk = within / geom.parts;
+                pass = (within - chunk * geom.parts) * geom.passes_per_part;
+                end_pass = min(npass, pass + geom.passes_per_part);
+                within = chunk;
+                lp += batch.first;
+                if (lp >= batch.num_programs) lp -= batch.num_programs;
+            }
             const SbProgram* const hp = batch.programs + lp;
             const uint32_t pre_off = hp->pre_off, n_insn = hp->n_insn - pre_off, mid_off = hp->mid_off - pre_off, main_off = hp->main_off - pre_off;
             const uint32_t n_cst = hp->n_cst, n_patch = hp->n_patch, flags = hp->flags;
@@ -666,6 +675,7 @@ eval_kernel(const DeviceBatch batch, const EvalProblem prob, const Geom geom, fl
             if (SPAN && perm0 >= 1ull << hp->bits) continue;
             const uint32_t perms = !SPAN ? 1u : (uint32_t)min((unsigned long long)ppi, (1ull << hp->bits) - perm0);
             __syncwarp(); /* the previous item's reads of exec, table and psum are done */
+            if (PARTS && lane == 0) exec[-1].w1 = split * geom.parts + pass / geom.passes_per_part; /* which rows the item's sums are of: a word the copy does not use */
             const SbInsn* const code = batch.insns + hp->insn_off + pre_off; /* the row parts; the bank part has run (bank_tables_kernel) */
 #pragma unroll 1
             for (uint32_t i = lane; i < n_insn; i += 32) put_insn(exec + i, rewrite(code[i], strides));
@@ -706,7 +716,7 @@ eval_kernel(const DeviceBatch batch, const EvalProblem prob, const Geom geom, fl
             M m;
             place.code = code;
 #pragma unroll 1
-            for (uint32_t pass = 0; pass < npass; ++pass) {
+            for (; pass < end_pass; ++pass) {
                 place.row = tile32 + (pass * M::PASS + lane * 4) * 4u;
                 const uint32_t row0 = pass * M::PASS + lane * 4; /* first row of this thread in the tile */
                 const bool full = (pass + 1) * M::PASS <= chunk_rows;
@@ -804,7 +814,8 @@ eval_kernel(const DeviceBatch batch, const EvalProblem prob, const Geom geom, fl
                 const bool independent = (flags & SB_PROG_BANK_INDEPENDENT) != 0;
                 const uint32_t width = ngroups * RC, bank0 = first_bg * RC; /* banks of the item, padding included */
                 const uint32_t real = min(width, prob.num_banks - bank0);
-                float* mine = partial + (geom.direct ? gp * prob.out_program_stride : ((size_t)split * batch.num_programs + lp) * nq * configs) +
+                const uint32_t row_share = PARTS ? exec[-1].w1 : split;
+                float* mine = partial + (geom.direct ? gp * prob.out_program_stride : ((size_t)row_share * batch.num_programs + lp) * nq * configs) +
                               ((size_t)bank0 << prob.toggle_bits);
                 float* sums = psum; /* psum is [quantity][permutation][group][bank of the group] */
                 if constexpr (!SPAN) {
@@ -855,12 +866,19 @@ eval_kernel(const DeviceBatch batch, const EvalProblem prob, const Geom geom, fl
 }
 
 
-/* the launches of one kind of kernel, over the tile shapes */
+/* the launches of one kind of kernel, over the tile shapes; PARTS: the launch cuts tiles into parts or does not begin with
+ * its first program (small launches without toggles; what it takes made large ones 1 % slower) */
+template <int KIND, int RR, int RC, bool SPAN, bool PARTS>
+void launch_parts(const DeviceBatch& batch, const EvalProblem& prob, const Geom& geom, const LaunchPlan& plan, float* partial,
+                  const float* tables, cudaStream_t stream) {
+    if (prob.fast_math) eval_kernel<RR, RC, true, SPAN, PARTS, KIND><<<plan.grid_x, plan.warps * 32, plan.smem_bytes, stream>>>(batch, prob, geom, partial, tables);
+    else eval_kernel<RR, RC, false, SPAN, PARTS, KIND><<<plan.grid_x, plan.warps * 32, plan.smem_bytes, stream>>>(batch, prob, geom, partial, tables);
+}
 template <int KIND, int RR, int RC, bool SPAN>
 cudaError_t launch_shape(const DeviceBatch& batch, const EvalProblem& prob, const Geom& geom, const LaunchPlan& plan, float* partial,
                          const float* tables, cudaStream_t stream) {
-    if (prob.fast_math) eval_kernel<RR, RC, true, SPAN, KIND><<<plan.grid_x, plan.warps * 32, plan.smem_bytes, stream>>>(batch, prob, geom, partial, tables);
-    else eval_kernel<RR, RC, false, SPAN, KIND><<<plan.grid_x, plan.warps * 32, plan.smem_bytes, stream>>>(batch, prob, geom, partial, tables);
+    if (!SPAN && (geom.parts > 1u || batch.first)) launch_parts<KIND, RR, RC, SPAN, !SPAN>(batch, prob, geom, plan, partial, tables, stream);
+    else launch_parts<KIND, RR, RC, SPAN, false>(batch, prob, geom, plan, partial, tables, stream);
     return cudaGetLastError();
 }
 template <int KIND, bool SPAN>
@@ -872,16 +890,21 @@ cudaError_t launch_kind(const DeviceBatch& batch, const EvalProblem& prob, const
     default: return launch_shape<KIND, 16, 1, SPAN>(batch, prob, geom, plan, partial, tables, stream);
     }
 }
-template <int KIND, bool SPAN>
-cudaError_t configure_kind(int smem_limit) {
-    const void* kernels[] = {(const void*)eval_kernel<4, 4, false, SPAN, KIND>,  (const void*)eval_kernel<4, 4, true, SPAN, KIND>,
-                             (const void*)eval_kernel<8, 2, false, SPAN, KIND>,  (const void*)eval_kernel<8, 2, true, SPAN, KIND>,
-                             (const void*)eval_kernel<16, 1, false, SPAN, KIND>, (const void*)eval_kernel<16, 1, true, SPAN, KIND>};
+template <int KIND, bool SPAN, bool PARTS>
+cudaError_t configure_parts(int smem_limit) {
+    const void* kernels[] = {(const void*)eval_kernel<4, 4, false, SPAN, PARTS, KIND>,  (const void*)eval_kernel<4, 4, true, SPAN, PARTS, KIND>,
+                             (const void*)eval_kernel<8, 2, false, SPAN, PARTS, KIND>,  (const void*)eval_kernel<8, 2, true, SPAN, PARTS, KIND>,
+                             (const void*)eval_kernel<16, 1, false, SPAN, PARTS, KIND>, (const void*)eval_kernel<16, 1, true, SPAN, PARTS, KIND>};
     for (const void* f : kernels) {
         const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_limit);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
+}
+template <int KIND, bool SPAN>
+cudaError_t configure_kind(int smem_limit) {
+    const cudaError_t e = configure_parts<KIND, SPAN, false>(smem_limit);
+    return e == cudaSuccess && !SPAN ? configure_parts<KIND, SPAN, !SPAN>(smem_limit) : e;
 }
 
 }  // namespace

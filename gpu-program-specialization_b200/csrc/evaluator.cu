@@ -222,7 +222,7 @@ cudaError_t launch_eval(const DeviceBatch& batch, const EvalProblem& prob, const
         ++launched;
     }
     /* a run whose rows are not split has whole sums: they go straight to the caller's grid */
-    geom.direct = !materialize && plan.row_splits == 1 ? 1u : 0u;
+    geom.direct = !materialize && plan.row_splits * plan.parts == 1 ? 1u : 0u;
     float* const sums = geom.direct ? prob.output : partial;
     /* runs without toggles have a kernel without the permutations' code: with it inside, the population of
      * 2,048 programs x 64 sets took 34.1 ms instead of 30.0 (registers, not instructions) */
@@ -237,7 +237,7 @@ cudaError_t launch_eval(const DeviceBatch& batch, const EvalProblem& prob, const
     const unsigned long long configs = (unsigned long long)prob.num_banks << prob.toggle_bits;
     const unsigned long long total = (unsigned long long)nq * configs * batch.num_programs;
     const unsigned blocks = (unsigned)std::min<unsigned long long>((total + 255) / 256, 148ull * 16ull);
-    combine_kernel<<<blocks ? blocks : 1u, 256, 0, stream>>>(batch, prob, partial, plan.row_splits, nq, configs);
+    combine_kernel<<<blocks ? blocks : 1u, 256, 0, stream>>>(batch, prob, partial, plan.row_splits * plan.parts, nq, configs);
     e = cudaGetLastError();
     if (e == cudaSuccess) *launches = ++launched;
     return e;

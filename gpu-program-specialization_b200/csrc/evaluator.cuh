@@ -66,8 +66,10 @@ struct DeviceBatch {
     uint32_t uses_scratch; /* some program needs the scratch spill slot */
     uint64_t total_cst;   /* constant-table entries of all programs (an upper bound will do) */
     uint64_t total_cost;  /* scheduling weights of all programs */
+    uint64_t max_cost;    /* the largest of them */
     double total_perms;   /* permutations with values of their own, of all programs */
     uint32_t max_bits;    /* most toggle bits a program reads: a program has at most 1 << max_bits of them */
+    uint32_t first;       /* the program CTAs begin with; those before it come last */
 };
 
 struct EvalProblem {
@@ -101,10 +103,11 @@ struct LaunchPlan {
     uint32_t num_groups;      /* CTAs along the programs; group g owns programs g, g + num_groups, ... */
     uint32_t groups_per_item; /* bank groups of one permutation a warp handles per queue item */
     uint32_t perms_per_item;  /* consecutive permutations one item covers (a power of two; above 1 only when an item holds every bank group) */
+    uint32_t parts;           /* items that share the rows of a tile, each with a range of its passes and sums of its own */
     uint32_t row_splits;      /* CTAs sharing one program group, each with a row range */
     size_t rows_per_split;
     size_t smem_bytes;
-    size_t partial_elements;  /* floats of partial sums over all row splits (0: materialize) */
+    size_t partial_elements;  /* floats of partial sums over all row splits and parts (0: materialize) */
     size_t table_elements;    /* floats of constant tables */
     size_t table_offset;      /* where they begin in the launch's scratch, 16-byte aligned: behind the partial sums, or
                                  at 0 when the rows are not split and the sums go straight to the output */
@@ -122,6 +125,8 @@ struct Geom {
     uint32_t row_splits;
     uint32_t groups_per_item;
     uint32_t perms_per_item;
+    uint32_t parts;
+    uint32_t passes_per_part;
     uint32_t exec_bytes;      /* per-warp regions, each a multiple of 16 bytes */
     uint32_t table_bytes;
     uint32_t hoist_bytes;
@@ -130,7 +135,7 @@ struct Geom {
     uint32_t warp_bytes;
     uint32_t scratch_slot;    /* spill slot reserved for the element-by-element FMA */
     unsigned long long rows_per_split;
-    uint32_t direct;          /* rows are not split: sums go to the output, not to partial sums */
+    uint32_t direct;          /* neither rows nor tiles are split: sums go to the output, not to partial sums */
 };
 
 constexpr int kNumVariants = 3;
@@ -141,7 +146,9 @@ Geom make_geom(const DeviceBatch& batch, const EvalProblem& problem, const Launc
 
 /* scratch_limit: most floats of scratch a launch may use: the row splits are reduced until their partial sums
  * fit beside the constant tables (with one split there are none; the tables are not reduced here).
- * share: the part of the machine a small launch should count on (another one runs beside it). */
+ * share: the part of the machine a small launch should count on (another one runs beside it); kBehindAnother: all of it, but
+ * only when another launch that fills it leaves SMs one by one, so its CTAs should be short. */
+constexpr double kBehindAnother = -1.0;
 LaunchPlan plan_launch(const DeviceBatch& batch, const EvalProblem& problem, int sm_count, size_t smem_limit,
                        size_t scratch_limit, double share = 1.0);
 

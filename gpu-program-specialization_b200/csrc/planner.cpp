@@ -39,6 +39,8 @@ Geom make_geom(const DeviceBatch& batch, const EvalProblem& prob, const LaunchPl
     g.row_splits = plan.row_splits;
     g.groups_per_item = gpi;
     g.perms_per_item = ppi;
+    g.parts = plan.parts ? plan.parts : 1u;
+    g.passes_per_part = (plan.tile_rows / (32u * rr) + g.parts - 1) / g.parts;
     g.exec_bytes = round16(((size_t)batch.max_insn + 1) * sizeof(SbInsn));
     g.table_bytes = round16((size_t)std::max<uint32_t>(1u, ppi * gpi * batch.max_cst * rc) * 4);
     g.hoist_bytes = round16((size_t)batch.max_hoisted * 32u * rr * 4);
@@ -55,82 +57,125 @@ namespace {
 
 size_t smem_needed(const Geom& g, uint32_t warps) { return (size_t)g.tile_bytes * g.tile_buffers + 16 + (size_t)g.warp_bytes * warps; }
 
-/* How a launch is cut into queue items and CTAs when it is small: the sums do not depend on it (they
- * depend on the tiles and the row splits, which stay as they are), so it may follow the machine.  A launch
- * whose programs read few of the run's toggle bits is small in this sense too.
+/* How a launch is cut into tiles, CTAs and queue items when it is small.
  *
- * The rules above it aim at large launches, whose grid is many waves deep.  With few programs or rows
- * they gave grids of 150 CTAs on 148 SMs (two waves for one), a dozen items for twenty warps, or half
- * the warps because a second tile buffer was reserved that a CTA of one tile does not use.  Here the cut
- * with the shortest estimated time is taken: the grid's waves times a CTA's rounds of items.  The
- * constants are issue slots, measured on the 64-set population: 330 for one pass of the main part with
+ * The rules above it aim at large launches, whose grid is many waves deep.  With few programs or rows they gave
+ * grids of 150 CTAs on 148 SMs (two waves for one), a dozen items for twenty warps, half the warps because a
+ * second tile buffer was reserved that a CTA of one tile does not use, or a CTA with two items on every SM of the
+ * machine.  Here the cut with the shortest estimated time is taken: the grid's waves times a CTA's rounds of items.
+ * The constants are issue slots, measured on the 64-set population: 330 for one pass of the main part with
  * its loss, about 900 to set an item up, and a warp that issues every seventh cycle when alone; an SM
- * issues 2.6 per cycle at best. */
-struct Cut { uint32_t gpi, ppi; unsigned long long groups; };
+ * issues 2.6 per cycle at best.  (A launch whose programs read few of the run's toggle bits is small in this sense
+ * too.)  The order in which rows are added follows the cut, and the cut follows the request and the population.
+ * Tiles of half the rows, CTAs of several tiles and parts of tiles are tried since a CTA of 19 items on 20 warps ends
+ * with its longest program: 124 programs x 8 sets x 47,735 rows 320 -> 197 us a call, 488 x 16 x 5,823 191 -> 145, 124 x
+ * 3 x 19,735 163 -> 155 (all with their few heavy programs in the same launch, see views_to_launch in runner.cpp). */
+struct Cut {
+    uint32_t tile_rows, tiles_per_split, splits, warps; /* tiles_per_split: tiles a CTA walks */
+    uint32_t gpi, ppi, parts; /* parts only without toggles: the permutations are cuts enough, and their kernel has no room for it */
+    unsigned long long groups;
+};
+struct Work { unsigned long long programs, bank_groups; double perms, most_perms; uint32_t passes; bool hoists; int sms; double longest; /* the costliest program over the average */ }; /* perms: of a program, on the average and at most */
 
-/* `perms`: the permutations a program has of its own, on the average and at most. */
-double cut_cycles(const LaunchPlan& plan, const Cut& cut, unsigned long long programs, unsigned long long chunks, double perms, double most_perms,
-                  uint32_t passes, size_t tiles, bool hoists, int sms) {
-    const double per_cta = (double)((programs + cut.groups - 1) / cut.groups);
-    const double each = chunks * std::max(1.0, perms / cut.ppi), largest = chunks * std::max(1.0, most_perms / cut.ppi);
+double cut_cycles(const Cut& cut, const Work& w) {
+    const double per_cta = (double)((w.programs + cut.groups - 1) / cut.groups);
+    const double chunks = (double)(w.bank_groups / cut.gpi * cut.parts); /* items of a permutation, or of cut.ppi of them */
+    const double each = chunks * std::max(1.0, w.perms / cut.ppi), largest = chunks * std::max(1.0, w.most_perms / cut.ppi);
     const double items = std::ceil((per_cta - 1.0) * each + largest), empty = std::max(0.0, per_cta * largest - items);
-    const double active = std::min<double>(plan.warps, items);
+    const double active = std::min<double>(cut.warps, items);
     const double rate = std::min(0.14, 2.6 / active);
-    const auto slots = [&](double n, double groups) { return 900.0 * n + passes * ((hoists ? 120.0 : 0.0) * n + 330.0 * groups); };
-    const double item = slots(1.0, cut.gpi * std::min<double>(cut.ppi, most_perms));
-    const unsigned long long grid = cut.groups * plan.row_splits;
-    const auto cta = [&](double time) { return 3000.0 + tiles * (1500.0 + time / rate + empty * 400.0 / plan.warps); };
-    if (perms < most_perms) { /* uneven: an average CTA for the work, the one with most permutations for the end */
-        const auto time = [&](double n, double all_perms) { return std::max(item, slots(n, (double)chunks * cut.gpi * all_perms) / plan.warps + 0.5 * item); };
-        const double last = cta(time(items, (per_cta - 1.0) * perms + most_perms));
-        return std::max(last, cta(time(std::ceil(per_cta * each), per_cta * perms)) * (double)grid / sms + 0.5 * last);
+    const uint32_t passes = (w.passes + cut.parts - 1) / cut.parts;
+    const auto slots = [&](double n, double groups) { return 900.0 * n + passes * ((w.hoists ? 120.0 : 0.0) * n + 330.0 * groups); };
+    const double item = slots(1.0, cut.gpi * std::min<double>(cut.ppi, w.most_perms));
+    const unsigned long long grid = cut.groups * cut.splits;
+    const auto cta = [&](double time) { return 3000.0 + cut.tiles_per_split * (1500.0 + time / rate + empty * 400.0 / cut.warps); };
+    if (w.perms < w.most_perms) { /* uneven: an average CTA for the work, the one with most permutations for the end */
+        const auto time = [&](double n, double all_perms) { return std::max(item, slots(n, chunks * cut.gpi * all_perms) / cut.warps + 0.5 * item); };
+        const double last = cta(time(items, (per_cta - 1.0) * w.perms + w.most_perms));
+        return std::max(last, cta(time(std::ceil(per_cta * each), per_cta * w.perms)) * (double)grid / w.sms + 0.5 * last);
     }
-    return (double)((grid + sms - 1) / sms) * cta(item * std::max(std::ceil(items / plan.warps), items / plan.warps + 0.5));
+    return (double)((grid + w.sms - 1) / w.sms) * cta(item * std::max({std::ceil(items / cut.warps), items / cut.warps + 0.5, w.longest}));
 }
 
-/* `sms`: the part of the machine this launch has when another runs beside it. */
-void balance_small(LaunchPlan* plan, const DeviceBatch& batch, const EvalProblem& prob, int sms, size_t smem_limit) {
+/* `sms`: the part of the machine (`all`) this launch has when another runs beside it; `room`: floats of scratch for
+ * partial sums. */
+void balance_small(LaunchPlan* plan, const DeviceBatch& batch, const EvalProblem& prob, int sms, int all, bool behind, size_t smem_limit, unsigned long long room) {
     const bool materialize = prob.mode == EVAL_MATERIALIZE;
     const uint32_t rr = (uint32_t)kVariantRows[plan->variant], rc = (uint32_t)kVariantBanks[plan->variant], pass = 32u * rr;
     const unsigned long long P = batch.num_programs, bank_groups = materialize ? 1 : (prob.num_banks + rc - 1) / rc;
-    const size_t tiles = (plan->rows_per_split + plan->tile_rows - 1) / plan->tile_rows;
+    while (plan->perms_per_item > 1ull << batch.max_bits) plan->perms_per_item /= 2;
     /* as many warps as fit beside the tile buffers that are used */
-    const auto refit = [&](LaunchPlan* p) {
+    const auto refit = [&](LaunchPlan* p, uint32_t least) {
         const Geom g = make_geom(batch, prob, *p);
-        while (p->warps < 20 && smem_needed(g, p->warps + 1) <= smem_limit) ++p->warps;
+        const size_t tiles = (size_t)g.tile_bytes * g.tile_buffers + 16;
+        p->warps = tiles < smem_limit ? (uint32_t)std::min<size_t>(20, (smem_limit - tiles) / g.warp_bytes) : 0u;
+        p->warps = std::max(p->warps, least);
         p->smem_bytes = smem_needed(g, p->warps);
     };
-    while (plan->perms_per_item > 1ull << batch.max_bits) plan->perms_per_item /= 2;
-    if (plan->tile_buffers == 1) refit(plan);
+    if (plan->tile_buffers == 1) refit(plan, plan->warps);
     /* a program has only as many values of its own as it reads toggle bits: the rules above counted all */
     const bool fewer = !materialize && batch.total_perms < 0.5 * (double)P * (double)(1ull << prob.toggle_bits);
-    if (!fewer && (unsigned long long)plan->num_groups * plan->row_splits >= 8ull * (unsigned long long)sms) return; /* deep enough */
-    const double perms = materialize ? 1.0 : batch.total_perms / (double)P, most_perms = materialize ? 1.0 : (double)(1ull << batch.max_bits);
-    const uint32_t passes = (uint32_t)((std::min<size_t>(plan->tile_rows, prob.num_rows) + pass - 1) / pass);
-    const auto items_of = [&](const Cut& c) { return materialize ? 1ull : ((bank_groups / c.gpi) << batch.max_bits) / c.ppi; };
-    const auto cycles = [&](const Cut& c) {
-        return cut_cycles(*plan, c, P, bank_groups / c.gpi, perms, most_perms, passes, tiles, batch.max_hoisted != 0, sms);
-    };
-    Cut best{plan->groups_per_item, plan->perms_per_item, plan->num_groups};
-    double least = 0.97 * cycles(best);
-    const Cut widest = best;
-    for (uint32_t gpi = widest.gpi; gpi >= 1; --gpi) {
-        if (bank_groups % gpi) continue;
-        for (uint32_t ppi = gpi == bank_groups ? widest.ppi : 1u; ppi >= 1; ppi /= 2)
-            for (unsigned waves = 0; waves <= (fewer ? 32u : 8u); waves += waves < 8 ? 1 : 4) {
-                Cut c{gpi, ppi, waves ? (unsigned long long)waves * sms / plan->row_splits : widest.groups};
-                c.groups = std::max<unsigned long long>(1, std::min(c.groups, P));
-                const unsigned long long items = items_of(c);
-                if (items > 0xffffff00ull / ((P + c.groups - 1) / c.groups)) continue;
-                const double t = cycles(c);
-                if (t < least) { least = t; best = c; }
+    const unsigned long long rule_items = (P + plan->num_groups - 1) / plan->num_groups * (bank_groups / plan->groups_per_item);
+    const unsigned long long rule_grid = (unsigned long long)plan->num_groups * plan->row_splits;
+    /* deep enough, and its CTAs full enough; what is many waves of the whole machine is not confined to a part of it,
+     * whose size is an estimate (358 programs, 33 sets, 770,512 rows, approximate functions: 6.9 ms, 10.3 when it was) */
+    if (!fewer && rule_grid >= 8ull * (unsigned long long)sms && (rule_items >= 4ull * plan->warps || rule_grid >= 8ull * (unsigned long long)all)) return;
+    Work work{P, bank_groups, materialize ? 1.0 : batch.total_perms / (double)P, materialize ? 1.0 : (double)(1ull << batch.max_bits), 0, batch.max_hoisted != 0, sms,
+              batch.total_cost ? std::min(3.0, std::max(1.0, (double)batch.max_cost * (double)P / (double)batch.total_cost)) : 1.0};
+    const auto passes_of = [&](uint32_t tile_rows) { return (uint32_t)((std::min<size_t>(tile_rows, prob.num_rows) + pass - 1) / pass); };
+    const unsigned long long per_sum = materialize ? 0 : (unsigned long long)P * std::max<uint32_t>(1u, quantities(prob)) * ((unsigned long long)prob.num_banks << prob.toggle_bits);
+    Cut best{plan->tile_rows, (uint32_t)((plan->rows_per_split + plan->tile_rows - 1) / plan->tile_rows), plan->row_splits, plan->warps,
+             plan->groups_per_item, plan->perms_per_item, 1u, plan->num_groups};
+    work.passes = passes_of(plan->tile_rows);
+    double least = 0.97 * cut_cycles(best, work);
+    const Cut rules = best;
+    LaunchPlan trial = *plan;
+    /* (uneven launches keep the tiles and row splits of the rules: their estimate is too coarse for more) */
+    const bool uneven = work.perms < work.most_perms;
+    for (uint32_t half = 0; half < (uneven ? 1u : 2u); ++half) { /* the rules' tile and one of half its rows */
+        trial.tile_rows = half ? (rules.tile_rows / 2 + pass - 1) / pass * pass : rules.tile_rows;
+        if (half && (trial.tile_rows == rules.tile_rows || trial.tile_rows < 256u)) break;
+        work.passes = passes_of(trial.tile_rows);
+        const unsigned long long tiles = (prob.num_rows + trial.tile_rows - 1) / trial.tile_rows;
+        for (trial.tile_buffers = 1; trial.tile_buffers <= (tiles > 1 ? 2u : 1u); ++trial.tile_buffers)
+            for (uint32_t gpi = rules.gpi; gpi >= 1; --gpi) {
+                if (bank_groups % gpi) continue;
+                for (uint32_t ppi = gpi == bank_groups ? rules.ppi : 1u; ppi >= 1; ppi /= 2) {
+                    trial.groups_per_item = gpi;
+                    trial.perms_per_item = ppi;
+                    refit(&trial, 0u);
+                    if (trial.warps < std::min(rules.warps, 12u)) continue;
+                    const unsigned long long items = materialize ? 1ull : ((bank_groups / gpi) << batch.max_bits) / ppi;
+                    for (unsigned waves = uneven ? 0u : 1u; waves <= (fewer ? 32u : 8u); waves += waves < 8 ? 1 : 4) {
+                        const unsigned long long ctas = waves ? (unsigned long long)waves * sms : rules.groups * rules.splits;
+                        Cut c{trial.tile_rows, (uint32_t)((tiles + ctas - 1) / ctas), 0, trial.warps, gpi, ppi, 1u, 0};
+                        if (uneven) { c.tiles_per_split = rules.tiles_per_split; c.warps = rules.warps; }
+                        if ((c.tiles_per_split > 1) != (trial.tile_buffers > 1) || (behind && c.tiles_per_split > rules.tiles_per_split)) continue;
+                        c.splits = (uint32_t)((tiles + c.tiles_per_split - 1) / c.tiles_per_split);
+                        if (per_sum && c.splits > 1 && c.splits > rules.splits && c.splits > room / per_sum) continue;
+                        c.groups = std::max<unsigned long long>(1, std::min(ctas / c.splits, P));
+                        for (c.parts = 1; c.parts <= (prob.toggle_bits ? 1u : work.passes); c.parts *= 2) {
+                            if (c.parts > 1 && per_sum && (unsigned long long)c.splits * c.parts > room / per_sum) break;
+                            if (items * c.parts > 0xffffff00ull / ((P + c.groups - 1) / c.groups)) break;
+                            const double t = cut_cycles(c, work);
+                            if (t < least) { least = t; best = c; }
+                        }
+                        if (waves && c.groups == P && c.tiles_per_split == 1) break; /* more waves are the same cut */
+                    }
+                }
             }
     }
+    if (!plan->tile_rows || best.tile_rows == 0) return;
+    plan->tile_rows = best.tile_rows;
+    plan->tile_buffers = best.tiles_per_split > 1 ? 2u : 1u;
+    plan->row_splits = best.splits;
+    plan->rows_per_split = (size_t)best.tiles_per_split * best.tile_rows;
     plan->groups_per_item = best.gpi;
     plan->perms_per_item = best.ppi;
+    plan->parts = best.parts;
     plan->num_groups = (uint32_t)best.groups;
     plan->grid_x = plan->num_groups * plan->row_splits;
-    refit(plan);
+    refit(plan, 0u);
 }
 
 LaunchPlan plan_with_tile(const DeviceBatch& batch, const EvalProblem& prob, int sm_count, size_t smem_limit, size_t scratch_limit,
@@ -140,6 +185,7 @@ LaunchPlan plan_with_tile(const DeviceBatch& batch, const EvalProblem& prob, int
     plan.overflow = false;
     plan.groups_per_item = 1;
     plan.perms_per_item = 1;
+    plan.parts = 1;
     plan.variant = variant;
     const uint32_t rr = (uint32_t)kVariantRows[variant], rc = (uint32_t)kVariantBanks[variant];
     const uint32_t pass = 32u * rr;
@@ -255,14 +301,16 @@ LaunchPlan plan_with_tile(const DeviceBatch& batch, const EvalProblem& prob, int
     if (grid > 0x7fffffffull) { plan.overflow = true; return plan; }
     plan.grid_x = (uint32_t)grid;
 
+    const unsigned long long room = scratch_limit > plan.table_elements + 3 ? scratch_limit - plan.table_elements - 3 : 0;
+    const bool behind = share == kBehindAnother;
+    balance_small(&plan, batch, prob, behind ? sm_count : std::max(1, (int)(sm_count * share)), sm_count, behind, smem_limit, room);
     plan.partial_elements = 0;
     if (!materialize) {
-        const unsigned long long n = (unsigned long long)plan.row_splits * P;
+        const unsigned long long n = (unsigned long long)plan.row_splits * plan.parts * P;
         if (configs && n > (~0ull >> 3) / configs / nq) { plan.overflow = true; return plan; }
         plan.partial_elements = (size_t)(n * nq * configs);
     }
-    plan.table_offset = plan.row_splits > 1 ? (plan.partial_elements + 3) / 4 * 4 : 0; /* whole sums go to the output */
-    balance_small(&plan, batch, prob, std::max(1, (int)(sm_count * share)), smem_limit);
+    plan.table_offset = plan.row_splits * plan.parts > 1 ? (plan.partial_elements + 3) / 4 * 4 : 0; /* whole sums go to the output */
     plan.ok = true;
     return plan;
 }

@@ -449,6 +449,7 @@ SecantResult upload_batch(SecantCubinRunnerImpl* r, Slot& s, std::vector<View>* 
             db.max_cst = std::max<uint32_t>(db.max_cst, p.n_cst);
             db.total_cst += p.n_cst;
             db.total_cost += schedule_cost(p);
+            db.max_cost = std::max(db.max_cost, schedule_cost(p));
             db.total_perms += (double)(1ull << p.bits);
             db.max_bits = std::max<uint32_t>(db.max_bits, p.bits);
             db.max_btmp = std::max<uint32_t>(db.max_btmp, p.n_btmp);
@@ -537,6 +538,7 @@ DeviceBatch tables_that_fit(const View& view, const SbProgram* headers, size_t f
     DeviceBatch part = view.batch;
     part.programs += first;
     part.num_programs = 0;
+    part.first = 0; /* in launch order: the heavy programs of a joint view come last here */
     part.total_cst = 0;
     part.total_perms = 0;
     part.max_bits = 0;
@@ -553,20 +555,58 @@ DeviceBatch tables_that_fit(const View& view, const SbProgram* headers, size_t f
     return part;
 }
 
+/* The views of a batch as they are launched for a run entry: light and heavy programs in one launch where that keeps
+ * most of the warps, since two launches share the machine badly: the heavy programs are few, and their CTAs take an SM
+ * each for an item or two, or a few SMs for long (256 resident programs, 33 sets, 10,007 rows, 14 of them heavy: 452 us
+ * apart, 288 together).  Heavy programs, which are the costliest, then come first.  A grid of many waves
+ * fills the machine either way, and its light programs are faster with all the warps that fit. */
+std::vector<View> views_to_launch(SecantCubinRunnerImpl* r, const std::vector<View>& views, const EvalProblem& prob) {
+    if (views.size() != 2 || prob.toggle_bits) return views;
+    View all = views[0];
+    const DeviceBatch& heavy = views[1].batch;
+    DeviceBatch& b = all.batch;
+    b.first = b.num_programs;
+    b.num_programs += heavy.num_programs;
+    b.max_insn = std::max(b.max_insn, heavy.max_insn);
+    b.max_extra = std::max(b.max_extra, heavy.max_extra);
+    b.max_slots = std::max(b.max_slots, heavy.max_slots);
+    b.max_hoisted = std::max(b.max_hoisted, heavy.max_hoisted);
+    b.max_cst = std::max(b.max_cst, heavy.max_cst);
+    b.max_btmp = std::max(b.max_btmp, heavy.max_btmp);
+    b.uses_scratch |= heavy.uses_scratch;
+    b.total_cst += heavy.total_cst;
+    b.total_cost += heavy.total_cost;
+    b.max_cost = std::max(b.max_cost, heavy.max_cost);
+    b.total_perms += heavy.total_perms;
+    b.max_bits = std::max(b.max_bits, heavy.max_bits);
+    const LaunchPlan plan = plan_launch(b, prob, r->sm_count, r->smem_limit, r->scratch_limit);
+    if (!plan.ok || plan.warps < 16u || (uint64_t)plan.grid_x >= 8ull * (uint64_t)r->sm_count) return views;
+    /* an item of a pass or two pays for its set-up once more when the heavy programs' memory makes the tile smaller
+     * (3,000 programs without coefficients, 20,011 rows: 1 % of the call) */
+    if (plan.tile_rows / (32u * (uint32_t)kVariantRows[plan.variant]) * plan.groups_per_item < 8u) {
+        const LaunchPlan light = plan_launch(views[0].batch, prob, r->sm_count, r->smem_limit, r->scratch_limit);
+        if (light.ok && light.tile_rows > plan.tile_rows) return views;
+    }
+    return {all};
+}
+
 /* Enqueues the evaluation of one device-resident batch for every run entry, spreading
  * entries over the compute streams.  `after` (optional) is an event each stream waits on
  * first; `done`/`used` (optional) receive one completion event per touched stream. */
-SecantResult launch_batch(SecantCubinRunnerImpl* r, const View& view, const SbProgram* headers, double share,
+SecantResult launch_batch(SecantCubinRunnerImpl* r, const std::vector<View>& batch_views, const SbProgram* headers,
                           const std::vector<UnpackedRun>& runs, size_t* stream_cursor, cudaEvent_t after, std::vector<cudaEvent_t>* done, std::vector<char>* used) {
     const SecantCubinPlan& plan = *r->plan;
-    const DeviceBatch& db = view.batch;
     for (size_t e = 0; e < runs.size(); ++e) {
-        const size_t k = (*stream_cursor)++ % r->streams.size();
-        cudaStream_t stream = r->streams[k];
         EvalProblem prob = make_problem(plan, runs[e], 0); /* SbProgram::index already places every program in the run */
         prob.fast_math = r->fast_math;
         if (runs[e].program_bank_stride)
             prob.banks = reinterpret_cast<const float*>(runs[e].banks.address) + runs[e].first_program_index * runs[e].program_bank_stride;
+        const std::vector<View> views = views_to_launch(r, batch_views, prob);
+        double share = view_share(r, views, views[0], runs.size());
+        for (const View& view : views) {
+        const DeviceBatch& db = view.batch;
+        const size_t k = (*stream_cursor)++ % r->streams.size();
+        cudaStream_t stream = r->streams[k];
         cudaError_t ce = after ? cudaStreamWaitEvent(stream, after, 0) : cudaSuccess;
         /* one launch, unless its constant tables (an entry per program constant and configuration) would
          * take more than half of the scratch limit (the rest is for the partial sums of the row splits, without
@@ -589,6 +629,10 @@ SecantResult launch_batch(SecantCubinRunnerImpl* r, const View& view, const SbPr
             }
             unsigned launches = 0;
             ce = launch_eval(part, prob, lp, partial, stream, &launches);
+            /* the launch beside it has the SMs this one leaves; when it leaves none, the other's CTAs come behind it and are
+             * best spread over all of them (2,938 programs, eleven of them heavy, 227,933 rows: 4.2 ms, 5.0 with those
+             * confined to the SMs their work is worth) */
+            share = lp.grid_x < (uint32_t)r->sm_count ? 1.0 - (double)lp.grid_x / r->sm_count : kBehindAnother;
             g_kernel_launches.fetch_add(launches);
             if (launches)
                 g_row_stream_bytes.fetch_add((uint64_t)lp.num_groups * (prob.num_inputs + (prob.mode == EVAL_MATERIALIZE ? 0u : prob.num_targets)) *
@@ -597,6 +641,7 @@ SecantResult launch_batch(SecantCubinRunnerImpl* r, const View& view, const SbPr
         if (ce == cudaSuccess && done) ce = cudaEventRecord((*done)[k], stream);
         if (ce != cudaSuccess) return cuda_fail(r, ce, "kernel launch");
         if (used) (*used)[k] = 1;
+        }
     }
     return SECANT_SUCCESS;
 }
@@ -605,7 +650,7 @@ SecantResult launch_batch(SecantCubinRunnerImpl* r, const View& view, const SbPr
  * rows into the stream's scratch by the evaluator (every view of the batch), then reduced to the
  * cohorts' statistics, range after range on one stream, so every statistic is added to in row
  * order.  first_program is the batch's first program and a multiple of the cohort size. */
-SecantResult launch_gram_batch(SecantCubinRunnerImpl* r, const std::vector<View>& views, const std::vector<UnpackedRun>& runs,
+SecantResult launch_gram_batch(SecantCubinRunnerImpl* r, const std::vector<View>& batch_views, const std::vector<UnpackedRun>& runs,
                                size_t first_program, size_t batch_programs, size_t* stream_cursor, cudaEvent_t after,
                                std::vector<cudaEvent_t>* done, std::vector<char>* used) {
     const SecantCubinPlan& plan = *r->plan;
@@ -617,12 +662,15 @@ SecantResult launch_gram_batch(SecantCubinRunnerImpl* r, const std::vector<View>
         /* scratch: the range's predictions, then the constant tables of every view (padded to four banks at
          * most), which the first range makes and the others read again */
         size_t entries = 0;
-        for (const View& v : views) entries += v.batch.total_cst;
+        for (const View& v : batch_views) entries += v.batch.total_cst;
         /* rows per range: what the scratch limit leaves for this batch's predictions, between 128 and as many as stay in
          * L2 beside the data (64 MB) or 16,384; a multiple of four, which the kernels' loads count on */
         const size_t room = r->scratch_limit > 4 * entries ? (r->scratch_limit - 4 * entries) / 4 * 4 : 0;
         const size_t fit = room / batch_programs / 4 * 4, resident = kGramFloats / batch_programs / 4 * 4;
         const size_t range = std::min<size_t>((run.rows + 3) / 4 * 4, std::max<size_t>(128, std::min<size_t>(std::max<size_t>(16384, resident), fit)));
+        EvalProblem whole = make_problem(plan, run, 0);
+        whole.num_rows = range;
+        const std::vector<View> views = views_to_launch(r, batch_views, whole);
         std::vector<int> tables_made(views.size(), -1); /* for which register tile */
         const size_t predictions = batch_programs * range;
         float* scratch = nullptr;
@@ -842,10 +890,7 @@ SecantResult execute(SecantCubinRunnerImpl* r, const std::vector<UnpackedRun>& r
             const size_t first = b * batch_size;
             result = launch_gram_batch(r, views, runs, first, std::min(batch_size, P - first), &stream_cursor, slot.uploaded, done, &slot.used);
         } else {
-            for (const View& view : views) {
-                result = launch_batch(r, view, static_cast<const SbProgram*>(slot.pinned), view_share(r, views, view, runs.size()), runs, &stream_cursor, slot.uploaded, done, &slot.used);
-                if (result != SECANT_SUCCESS) break;
-            }
+            result = launch_batch(r, views, static_cast<const SbProgram*>(slot.pinned), runs, &stream_cursor, slot.uploaded, done, &slot.used);
         }
         if (result != SECANT_SUCCESS) break;
         ++launched_batches;
@@ -1037,10 +1082,7 @@ SecantResult execute_resident(SecantCubinRunnerImpl* r, SecantB200PopulationImpl
     size_t cursor = 0;
     SecantResult result = SECANT_SUCCESS;
     for (auto& b : pop->batches) {
-        for (const View& view : b.views) {
-            result = launch_batch(r, view, b.headers.data(), view_share(r, b.views, view, runs.size()), runs, &cursor, nullptr, nullptr, nullptr);
-            if (result != SECANT_SUCCESS) break;
-        }
+        result = launch_batch(r, b.views, b.headers.data(), runs, &cursor, nullptr, nullptr, nullptr);
         if (result != SECANT_SUCCESS) break;
     }
     if (result != SECANT_SUCCESS && plan.shape != SECANT_KERNEL_SHAPE_STATIC_MATERIALIZE_F32 && drain_streams(r)) (void)clear_outputs(r, runs, 0);
