@@ -134,15 +134,10 @@ inline bool direct_leaf(TokenKind k) { return k == TK_COLUMN || k == TK_BANK || 
 /* ---- expression DAG -------------------------------------------------------------------- */
 
 enum NodeType : uint8_t { N_COL, N_BANK, N_AFFINE, N_LIT, N_TOGGLE, N_UN, N_BIN, N_FMA };
-/* What a value depends on.  Joining two classes: a literal adopts the other class, bank and row
- * together make a mixed value. */
-enum ValueClass : int8_t { VC_LITERAL = 0, VC_BANK = 1, VC_ROW = 2, VC_MIXED = 3 };
+/* What a value depends on, as bits: joining two classes is an or. */
+enum ValueClass : uint8_t { VC_LITERAL = 0, VC_BANK = 1, VC_ROW = 2, VC_MIXED = 3 };
 
-ValueClass join(ValueClass a, ValueClass b) {
-    if (a == b || b == VC_LITERAL) return a;
-    if (a == VC_LITERAL) return b;
-    return VC_MIXED;
-}
+inline ValueClass join(ValueClass a, ValueClass b) { return (ValueClass)(a | b); }
 
 struct Node {
     NodeType type = N_LIT;
@@ -164,20 +159,32 @@ struct Node {
     int32_t weight = 0;   /* rough instruction cost of the sub-expression */
 };
 
-unsigned arity_of(const Node& n) { return n.type == N_UN ? 1 : n.type == N_BIN ? 2 : n.type == N_FMA ? 3 : 0; }
+unsigned arity_of(const Node& n) { return n.type > N_TOGGLE ? (unsigned)n.type - N_TOGGLE : 0u; } /* N_UN, N_BIN, N_FMA follow it */
 
 /* rough executed-instruction weights used for scheduling (SbProgram::cost) and for choosing
  * which row-only sub-expressions are worth a hoist slot */
-int unary_weight(unsigned op) {
-    switch (op) {
-    case SB_UN_NEG: case SB_UN_ABS: return 1;
-    case SB_UN_SIN: case SB_UN_COS: return 18;
-    case SB_UN_EXP: case SB_UN_EX2: return 9;
-    case SB_UN_LOG: return 14;
-    default: return 12;
-    }
+constexpr int unary_weight(unsigned op) {
+    return op == SB_UN_NEG || op == SB_UN_ABS ? 1 : op == SB_UN_SIN || op == SB_UN_COS ? 18 : op == SB_UN_EXP || op == SB_UN_EX2 ? 9 : op == SB_UN_LOG ? 14 : 12;
 }
-int binary_weight(unsigned op) { return (op == SB_BIN_DIV || op == SB_BIN_RDIV) ? 11 : 1; }
+constexpr int binary_weight(unsigned op) { return (op == SB_BIN_DIV || op == SB_BIN_RDIV) ? 11 : 1; }
+
+/* What the parser does with a token: one branch decides between the kinds of leaves and operations (programs are
+ * random to the processor, and a branch it guesses wrongly costs as much as the rest of a token). */
+enum Step : uint8_t { STEP_COLUMN, STEP_BANK, STEP_AFFINE, STEP_LITERAL, STEP_TOGGLE, STEP_ARG, STEP_CALL, STEP_RETURN, STEP_UNARY, STEP_BINARY, STEP_FMA, STEP_NONE };
+struct StepTable {
+    struct Row { Step step; uint8_t op, ways, width; uint8_t status; int8_t weight; } row[256];
+    StepTable() {
+        for (unsigned op = 0; op < 256; ++op) {
+            const OpcodeTable::Row& r = kTable.row[op];
+            const Token& t = r.token;
+            const Step operation = t.arity == 1 ? STEP_UNARY : t.arity == 2 ? STEP_BINARY : t.arity == 3 ? STEP_FMA : STEP_NONE;
+            static const Step steps[] = {STEP_COLUMN, STEP_BANK, STEP_AFFINE, STEP_LITERAL, STEP_TOGGLE, STEP_ARG, STEP_CALL, STEP_RETURN};
+            row[op] = Row{t.kind == TK_OPERATION ? operation : steps[t.kind], t.op, t.ways, (uint8_t)t.width, (uint8_t)r.status,
+                          (int8_t)(t.arity == 1 ? unary_weight(t.op) : t.arity == 2 ? binary_weight(t.op) : 4)};
+        }
+    }
+};
+const StepTable kSteps;
 
 struct Parser {
     const SecantAstProgramList& routines;
@@ -186,34 +193,36 @@ struct Parser {
     std::vector<Node>& nodes;
     std::vector<SbAffine>& affines; /* of this program */
     unsigned n_ops = 0;
+    unsigned of_class[4] = {0, 0, 0, 0}; /* operations by what their value depends on */
 
-    Node& make(NodeType type) {
+    int leaf(NodeType type, ValueClass cls, uint32_t index, uint32_t bits) {
         nodes.emplace_back();
-        nodes.back().type = type;
-        return nodes.back();
+        Node& n = nodes.back();
+        n.type = type; n.cls = cls; n.index = index; n.bits = bits;
+        return (int)nodes.size() - 1;
     }
-    /* Labels the node just made with what its value depends on and what it costs, and returns its id.
-     * Children exist before their parents, so one look at them is enough. */
-    int label(Node& n) {
-        switch (n.type) {
-        case N_COL: n.cls = rules.columns_are_slots ? VC_MIXED : VC_ROW; break;
-        case N_BANK: case N_AFFINE: n.cls = VC_BANK; break;
-        case N_LIT: break;
-        case N_TOGGLE:
-            n.toggled = true;
-            for (unsigned i = 0; i < n.ways; ++i) n.cls = join(n.cls, nodes[(size_t)n.child[i]].cls);
-            break;
-        default: {
-            int64_t w = n.type == N_UN ? unary_weight(n.op) : n.type == N_BIN ? binary_weight(n.op) : 4;
-            for (unsigned i = 0; i < arity_of(n); ++i) {
-                const Node& c = nodes[(size_t)n.child[i]];
-                n.cls = join(n.cls, c.cls);
-                n.toggled = n.toggled || c.toggled;
-                w += c.weight;
-            }
-            n.weight = (int32_t)std::min<int64_t>(w, INT32_MAX); /* a shared value counts once per parent */
+    /* An operation over the top of a stack, labelled with what its value depends on and what it costs (a shared value
+     * counts once per parent): children exist before their parents, so one look at them is enough. */
+    template <unsigned ARITY>
+    int operation(NodeType type, const StepTable::Row& row, const int* children) {
+        nodes.emplace_back();
+        Node& n = nodes.back();
+        n.type = type;
+        n.op = row.op;
+        int64_t w = row.weight;
+        unsigned cls = 0, toggled = 0;
+        for (unsigned i = 0; i < ARITY; ++i) {
+            const Node& c = nodes[(size_t)children[i]];
+            n.child[i] = children[i];
+            cls |= c.cls;
+            toggled |= c.toggled ? 1u : 0u;
+            w += c.weight;
         }
-        }
+        n.cls = (ValueClass)cls;
+        n.toggled = toggled != 0;
+        n.weight = (int32_t)std::min<int64_t>(w, INT32_MAX);
+        ++n_ops;
+        ++of_class[cls];
         return (int)nodes.size() - 1;
     }
 
@@ -229,37 +238,63 @@ struct Parser {
     /* One frame of the evaluator: its own value stack, arguments bound to nodes of the caller. */
     SecantResult frame(const SecantAstInstruction* code, const int* args, size_t num_args, unsigned depth, int* result) {
         int stack[SECANT_AST_MAX_STACK_DEPTH];
-        size_t top = 0, leaves_in_a_row = 0, at = 0;
+        size_t top = 0, leaves_in_a_row = 0;
         if (!code) return SECANT_ERROR_BAD_PROGRAM;
-        for (size_t n = 0; n < SECANT_AST_MAX_PROGRAM_INSTRUCTIONS; ++n) {
-            const SecantAstInstruction* ins = code + at;
-            Token t;
-            const SecantResult token_status = read_token(ins, rules, &t);
-            if (token_status != SECANT_SUCCESS) return token_status;
-            const bool pushes = direct_leaf(t.kind) || t.kind == TK_ARG;
-            if (t.kind == TK_ARG && (!args || ins[1] >= num_args)) return SECANT_ERROR_ROUTINE_ARG_IDX_OUT_OF_BOUNDS;
-            if (pushes && top == SECANT_AST_MAX_STACK_DEPTH) return SECANT_ERROR_STACK_OVERFLOW;
-            switch (t.kind) {
-            case TK_COLUMN: { Node& nd = make(N_COL); nd.index = ins[1]; stack[top++] = label(nd); break; }
-            case TK_BANK: { Node& nd = make(N_BANK); nd.index = ins[1]; stack[top++] = label(nd); break; }
-            case TK_AFFINE: {
-                Node& nd = make(N_AFFINE);
-                nd.index = (uint32_t)affine_entry(ins[1], secant_ast_affine_bank_scale_get(ins), secant_ast_affine_bank_offset_get(ins));
-                stack[top++] = label(nd);
+        const SecantAstInstruction* ins = code;
+        const ValueClass column_class = rules.columns_are_slots ? VC_MIXED : VC_ROW;
+        for (size_t n = 0; n < SECANT_AST_MAX_PROGRAM_INSTRUCTIONS; ++n) { /* the checks of read_token() first, in its order */
+            const StepTable::Row row = kSteps.row[ins[0]];
+            if (row.status != SECANT_SUCCESS) return (SecantResult)row.status;
+            size_t leaves = 0;
+            switch (row.step) {
+            case STEP_COLUMN:
+                if (ins[1] >= rules.num_columns) return SECANT_ERROR_BAD_PROGRAM;
+                if (top == SECANT_AST_MAX_STACK_DEPTH) return SECANT_ERROR_STACK_OVERFLOW;
+                stack[top++] = leaf(N_COL, column_class, ins[1], 0);
+                leaves = leaves_in_a_row + 1;
+                break;
+            case STEP_BANK:
+                if (!rules.banks_allowed || ins[1] >= rules.num_constants) return SECANT_ERROR_BAD_PROGRAM;
+                if (top == SECANT_AST_MAX_STACK_DEPTH) return SECANT_ERROR_STACK_OVERFLOW;
+                stack[top++] = leaf(N_BANK, VC_BANK, ins[1], 0);
+                leaves = leaves_in_a_row + 1;
+                break;
+            case STEP_AFFINE: {
+                const float scale = secant_ast_affine_bank_scale_get(ins), offset = secant_ast_affine_bank_offset_get(ins);
+                if (!rules.banks_allowed || ins[1] >= rules.num_constants || !std::isfinite(scale) || !std::isfinite(offset)) return SECANT_ERROR_BAD_PROGRAM;
+                if (top == SECANT_AST_MAX_STACK_DEPTH) return SECANT_ERROR_STACK_OVERFLOW;
+                stack[top++] = leaf(N_AFFINE, VC_BANK, (uint32_t)affine_entry(ins[1], scale, offset), 0);
+                leaves = leaves_in_a_row + 1;
                 break;
             }
-            case TK_LITERAL: { Node& nd = make(N_LIT); nd.bits = secant_ast_constant_bits_get(ins); stack[top++] = label(nd); break; }
-            case TK_ARG: stack[top++] = args[ins[1]]; break;
-            case TK_TOGGLE: {
-                if (leaves_in_a_row < t.ways || top < t.ways) return SECANT_ERROR_BAD_PROGRAM;
-                Node& nd = make(N_TOGGLE);
-                nd.ways = t.ways; nd.bit0 = ins[1]; nd.bit1 = t.ways == 4 ? ins[2] : 0xff;
-                for (size_t i = 0; i < t.ways; ++i) nd.child[i] = stack[top - t.ways + i];
-                top -= t.ways;
-                stack[top++] = label(nd);
+            case STEP_LITERAL:
+                if (top == SECANT_AST_MAX_STACK_DEPTH) return SECANT_ERROR_STACK_OVERFLOW;
+                stack[top++] = leaf(N_LIT, VC_LITERAL, 0, secant_ast_constant_bits_get(ins));
+                leaves = leaves_in_a_row + 1;
+                break;
+            case STEP_ARG:
+                if (!args || ins[1] >= num_args) return SECANT_ERROR_ROUTINE_ARG_IDX_OUT_OF_BOUNDS;
+                if (top == SECANT_AST_MAX_STACK_DEPTH) return SECANT_ERROR_STACK_OVERFLOW;
+                stack[top++] = args[ins[1]];
+                break;
+            case STEP_TOGGLE: {
+                if (!rules.banks_allowed || ins[1] >= rules.toggle_bits || (row.ways == 4 && (ins[2] >= rules.toggle_bits || ins[2] == ins[1])))
+                    return SECANT_ERROR_BAD_PROGRAM;
+                if (leaves_in_a_row < row.ways || top < row.ways) return SECANT_ERROR_BAD_PROGRAM;
+                nodes.emplace_back();
+                Node& nd = nodes.back();
+                nd.type = N_TOGGLE;
+                nd.toggled = true;
+                nd.ways = row.ways; nd.bit0 = ins[1]; nd.bit1 = row.ways == 4 ? ins[2] : 0xff;
+                top -= row.ways;
+                for (size_t i = 0; i < row.ways; ++i) {
+                    nd.child[i] = stack[top + i];
+                    nd.cls = join(nd.cls, nodes[(size_t)stack[top + i]].cls);
+                }
+                stack[top++] = (int)nodes.size() - 1;
                 break;
             }
-            case TK_CALL: {
+            case STEP_CALL: {
                 if (ins[1] >= routines.count || !routines.items[ins[1]]) return SECANT_ERROR_ROUTINE_IDX_OUT_OF_BOUNDS;
                 if (depth >= kRoutineDepth) return SECANT_ERROR_ROUTINE_DEPTH_EXCEEDED;
                 const size_t want = arity[ins[1]];
@@ -271,24 +306,28 @@ struct Parser {
                 stack[top++] = value;
                 break;
             }
-            case TK_RETURN:
+            case STEP_RETURN:
                 if (top != 1u) return SECANT_ERROR_BAD_PROGRAM;
                 *result = stack[0];
                 return SECANT_SUCCESS;
-            case TK_OPERATION: {
-                if (!t.arity) return SECANT_ERROR_BAD_PROGRAM;
-                if (top < t.arity) return SECANT_ERROR_STACK_UNDERFLOW;
-                Node& nd = make(t.node == 1 ? N_UN : t.node == 2 ? N_BIN : N_FMA);
-                nd.op = t.op;
-                for (unsigned i = 0; i < t.arity; ++i) nd.child[i] = stack[top - t.arity + i];
-                top -= t.arity;
-                stack[top++] = label(nd);
-                ++n_ops;
+            case STEP_UNARY:
+                if (top < 1) return SECANT_ERROR_STACK_UNDERFLOW;
+                stack[top - 1] = operation<1>(N_UN, row, stack + top - 1);
                 break;
+            case STEP_BINARY:
+                if (top < 2) return SECANT_ERROR_STACK_UNDERFLOW;
+                --top;
+                stack[top - 1] = operation<2>(N_BIN, row, stack + top - 1);
+                break;
+            case STEP_FMA:
+                if (top < 3) return SECANT_ERROR_STACK_UNDERFLOW;
+                top -= 2;
+                stack[top - 1] = operation<3>(N_FMA, row, stack + top - 1);
+                break;
+            default: return SECANT_ERROR_BAD_PROGRAM;
             }
-            }
-            leaves_in_a_row = direct_leaf(t.kind) ? leaves_in_a_row + 1 : 0;
-            at += t.width;
+            leaves_in_a_row = leaves;
+            ins += row.width;
         }
         return SECANT_ERROR_BAD_PROGRAM;
     }
@@ -303,20 +342,24 @@ struct Operand {
  * which an item that covers several permutations computes once, and values a toggle reaches. */
 enum Run { RUN_BANK = 0, RUN_SHARED = 1, RUN_ROW = 2, RUN_MAIN = 3, NUM_RUNS = 4 };
 
-int insn_weight(const SbInsn& ins) {
-    const unsigned cs = ins.w0 & 0xffu;
-    if (cs >= SB_CASE_BIN && cs < SB_CASE_UN) return 1 + binary_weight((cs - SB_CASE_BIN) / SB_NUM_KINDS);
-    if (cs >= SB_CASE_UN && cs < SB_CASE_FMA) return 1 + unary_weight(cs - SB_CASE_UN);
-    if (cs == SB_CASE_FMA) return 12;
-    return 2;
-}
+struct InsnWeights {
+    uint8_t of[256];
+    constexpr InsnWeights() : of() {
+        for (unsigned cs = 0; cs < 256; ++cs)
+            of[cs] = (uint8_t)(cs >= SB_CASE_BIN && cs < SB_CASE_UN ? 1 + binary_weight((cs - SB_CASE_BIN) / SB_NUM_KINDS)
+                             : cs >= SB_CASE_UN && cs < SB_CASE_FMA ? 1 + unary_weight(cs - SB_CASE_UN) : cs == SB_CASE_FMA ? 12 : 2);
+    }
+};
+constexpr InsnWeights kInsnWeights;
+inline unsigned insn_weight(const SbInsn& ins) { return kInsnWeights.of[ins.w0 & 0xffu]; }
 
 struct LeafEntry { NodeType type; uint32_t key; int entry; };
 
 /* Working storage of one encode_program() call.  Every thread keeps one: a program needs a dozen
  * small arrays, and making them anew for each program cost as much as filling them (5.9 us per
- * program of the 32-token, 16-slot kind on a 2.7 GHz Xeon; 3.7 us with the arrays kept, the nodes
- * labelled as they are parsed and each phase resetting only the nodes it reached). */
+ * program of the 32-token, 16-slot kind on a 2.7 GHz Xeon; 3.0 us with the arrays kept, the nodes
+ * labelled as they are parsed and each phase resetting only the nodes it reached; 2.2 with one branch per token,
+ * classes joined by an or, and leaves counted where they are read). */
 struct Scratch {
     std::vector<Node> nodes;
     std::vector<SbAffine> affines; /* of this program */
@@ -366,8 +409,8 @@ struct Emitter {
 
     static bool leaf_type(const Node& n) { return n.type <= N_TOGGLE; }
     /* a value that can be named as an operand without computing anything */
-    bool ready(int id) const {
-        const Node& n = nodes[id];
+    bool ready(int id) const { return ready(nodes[id]); }
+    bool ready(const Node& n) const {
         return leaf_type(n) || n.slot >= 0 || (run != RUN_BANK && n.hoisted >= 0) || n.entry >= 0;
     }
 
@@ -387,7 +430,8 @@ struct Emitter {
             if (std::find(row_roots.begin(), row_roots.end(), id) == row_roots.end()) row_roots.push_back(id);
             inside_row = true;
         }
-        for (unsigned i = 0; i < arity_of(n); ++i) collect(n.child[i], inside_row, bank_roots, row_roots);
+        const unsigned arity = arity_of(n);
+        for (unsigned i = 0; i < arity; ++i) collect(n.child[i], inside_row, bank_roots, row_roots);
     }
 
     /* maximal computed row-only nodes below `id` that no toggle reaches */
@@ -398,7 +442,8 @@ struct Emitter {
             if (std::find(shared.begin(), shared.end(), id) == shared.end()) shared.push_back(id);
             return;
         }
-        for (unsigned i = 0; i < arity_of(n); ++i) collect_shared(n.child[i], shared);
+        const unsigned arity = arity_of(n);
+        for (unsigned i = 0; i < arity; ++i) collect_shared(n.child[i], shared);
     }
 
     int alloc_slot() {
@@ -428,21 +473,30 @@ struct Emitter {
     /* Counts parent references of every reachable node and computes how many slots each needs
      * while it is being evaluated (Sethi-Ullman numbers, DAG-agnostic estimate). */
     void prepare(int id) {
-        Node& n = nodes[id];
+        Node& n = nodes[id]; /* (no node is made here) */
         if (n.uses++ > 0) return;
         mem.touched.push_back(id);
-        if (ready(id)) { n.su = 0; return; }
-        const unsigned arity = arity_of(n);
-        for (unsigned i = 0; i < arity; ++i) prepare(nodes[id].child[i]);
-        int need[3], cnt = 0;
-        for (unsigned i = 0; i < arity; ++i)
-            if (!ready(nodes[id].child[i])) need[cnt++] = nodes[nodes[id].child[i]].su;
-        for (int i = 0; i < cnt; ++i)
-            for (int j = i + 1; j < cnt; ++j)
-                if (need[j] > need[i]) std::swap(need[i], need[j]);
-        int su = 0; /* the k-th operand evaluated coexists with k parked predecessors */
-        for (int i = 0; i < cnt; ++i) su = std::max(su, need[i] + i);
-        nodes[id].su = su;
+        if (ready(n)) { n.su = 0; return; }
+        const auto need = [&](int child) { /* slots, or -1 where nothing has to be computed */
+            Node& c = nodes[child];
+            if (leaf_type(c)) {
+                if (c.uses++ == 0) mem.touched.push_back(child);
+                return -1;
+            }
+            prepare(child);
+            return ready(c) ? -1 : c.su;
+        };
+        if (n.type == N_UN) {
+            n.su = std::max(0, need(n.child[0]));
+        } else if (n.type == N_BIN) {
+            const int l = need(n.child[0]), r = need(n.child[1]);
+            n.su = std::max(0, std::max(std::max(l, r), std::min(l, r) < 0 ? -1 : std::min(l, r) + 1));
+        } else { /* the k-th operand evaluated, hungriest first, coexists with k parked predecessors */
+            int of[3] = {need(n.child[0]), need(n.child[1]), need(n.child[2])};
+            std::sort(of, of + 3, [](int a, int b) { return a > b; });
+            n.su = 0;
+            for (int i = 0; i < 3 && of[i] >= 0; ++i) n.su = std::max(n.su, of[i] + i);
+        }
     }
 
     void push(uint32_t w0, uint32_t w1) { code[run].push_back(SbInsn{w0, w1}); }
@@ -548,31 +602,33 @@ struct Emitter {
     void gen(int id) {
         if (error != SECANT_SUCCESS) return;
         if (ready(id)) { emit_reading(SB_CASE_LOAD, id); return; }
-        const Node n = nodes[id]; /* copy: the vector may grow below */
-        if (n.type == N_UN) {
-            gen(n.child[0]);
-            push(sb_w0(SB_CASE_UN + n.op, 0, 0), 0);
-            consume(n.child[0]);
-        } else if (n.type == N_BIN) {
-            const int l = n.child[0], r = n.child[1];
+        const NodeType type = nodes[id].type; /* copies: the vector may grow below */
+        const unsigned op = nodes[id].op;
+        if (type == N_UN) {
+            const int child = nodes[id].child[0];
+            gen(child);
+            push(sb_w0(SB_CASE_UN + op, 0, 0), 0);
+            consume(child);
+        } else if (type == N_BIN) {
+            const int l = nodes[id].child[0], r = nodes[id].child[1];
             if (l == r || ready(r)) {          /* acc = l ; acc = acc op r (l == r: gen parks it first) */
                 gen(l);
-                emit_reading(bin_case(n.op), r);
+                emit_reading(bin_case(op), r);
             } else if (ready(l)) {             /* acc = r ; acc = l op acc */
                 gen(r);
-                emit_reading(bin_case(reversed(n.op)), l);
+                emit_reading(bin_case(reversed(op)), l);
             } else {                           /* both computed: the hungrier one goes through a slot */
                 const bool left_first = nodes[l].su >= nodes[r].su;
                 const int first = left_first ? l : r, second = left_first ? r : l;
                 gen(first);
                 if (nodes[first].slot < 0) park(first);
                 gen(second);
-                emit_reading(bin_case(left_first ? reversed(n.op) : n.op), first);
+                emit_reading(bin_case(left_first ? reversed(op) : op), first);
             }
             consume(l);
             consume(r);
         } else {
-            gen_fma(n);
+            gen_fma(Node(nodes[id]));
         }
         if (nodes[id].uses > 1) park(id);
     }
@@ -730,7 +786,8 @@ SecantResult encode_program(const SecantAstInstruction* program, const SecantAst
     em.slots_high = rules.reserved_slots;
     const ValueClass root_class = nodes[root].cls;
     if (rules.split_parts) { /* rollout records (columns_are_slots) have no row-only class: only bank roots turn up */
-        em.collect(root, false, mem.bank_roots, mem.row_roots);
+        if ((rules.hoist_bank && parser.of_class[VC_LITERAL] + parser.of_class[VC_BANK]) || (rules.hoist_row && parser.of_class[VC_ROW]))
+            em.collect(root, false, mem.bank_roots, mem.row_roots); /* otherwise there is nothing to find */
         /* row-only expressions a toggle reaches change with the permutation; what lies below them and
          * does not is worth a value of its own, computed once for all permutations of an item */
         std::vector<int>& chosen = mem.chosen;
@@ -745,7 +802,12 @@ SecantResult encode_program(const SecantAstInstruction* program, const SecantAst
         /* keep the costliest values when there are more than the kernel has room for */
         chosen.insert(chosen.begin(), mem.shared_roots.begin(), mem.shared_roots.end());
         if (chosen.size() > rules.max_hoisted) {
-            std::stable_sort(chosen.begin(), chosen.end(), [&](int a, int b) { return nodes[a].weight > nodes[b].weight; });
+            for (size_t i = 1; i < chosen.size(); ++i) { /* a few values: by insertion, equal weights in their order */
+                const int id = chosen[i];
+                size_t k = i;
+                for (; k && nodes[chosen[k - 1]].weight < nodes[id].weight; --k) chosen[k] = chosen[k - 1];
+                chosen[k] = id;
+            }
             chosen.resize(rules.max_hoisted);
         }
         /* operands before the expressions that use them: children were created first */

@@ -80,9 +80,31 @@ struct Piece {
     SecantResult status = SECANT_SUCCESS;
 };
 
+/* Where the sections of a batch's records begin: programs | insns | patches | affines | lits, in bytes. */
+struct Sections {
+    size_t insn = 0, patch = 0, affine = 0, lit = 0, total = 0;
+    Sections() = default;
+    Sections(size_t programs, size_t insns, size_t patches, size_t affines, size_t lits) {
+        insn = align256(programs * sizeof(SbProgram));
+        patch = align256(insn + insns * sizeof(SbInsn));
+        affine = align256(patch + patches * sizeof(SbPatch));
+        lit = align256(affine + affines * sizeof(SbAffine));
+        total = align256(lit + lits * sizeof(float) + 16);
+    }
+};
+struct Counts { size_t insn = 0, patch = 0, affine = 0, lit = 0; };
+
 struct Slot {
     std::vector<Piece> pieces;
     size_t used_pieces = 0;         /* of the batch held */
+    size_t programs = 0;            /* of the batch held */
+    /* Whoever encodes a piece also puts it where the upload takes it from, while it is in that processor's cache
+     * and the others still encode: the calling thread alone needed 220 us for 3,000 programs.  Sections have room by
+     * what the batch before had (`usual`, per program); where that is not enough the calling thread packs the batch. */
+    bool packing = false;
+    Sections place;
+    Counts room, taken;             /* elements of each section; `taken` is guarded by the runner's mutex */
+    double usual[4] = {0, 0, 0, 0};
     size_t done_pieces = 0;         /* encoded, guarded by the runner's mutex */
     std::vector<uint64_t> order, order_tmp; /* launch order of the batch's programs, see order_programs() */
     std::vector<SbProgram> headers;
@@ -168,6 +190,34 @@ size_t take_piece(SecantCubinRunnerImpl* r) {
     return r->job_next_piece++;
 }
 
+/* Copies a piece's arrays to the slot's pinned buffer, from the elements `at` of its sections on, and its headers (whose
+ * offsets move by that) to the batch's programs from `program` on. */
+void pack_piece(Slot& s, const Sections& place, const EncodedBatch& e, const Counts& at, size_t program) {
+    char* const h = static_cast<char*>(s.pinned);
+    SbProgram* out = s.headers.data() + program;
+    for (SbProgram p : e.programs) {
+        p.insn_off += (uint32_t)at.insn; p.patch_off += (uint32_t)at.patch;
+        p.affine_off += (uint32_t)at.affine; p.lit_off += (uint32_t)at.lit;
+        *out++ = p;
+    }
+    if (!e.insns.empty()) std::memcpy(h + place.insn + at.insn * sizeof(SbInsn), e.insns.data(), e.insns.size() * sizeof(SbInsn));
+    if (!e.patches.empty()) std::memcpy(h + place.patch + at.patch * sizeof(SbPatch), e.patches.data(), e.patches.size() * sizeof(SbPatch));
+    if (!e.affines.empty()) std::memcpy(h + place.affine + at.affine * sizeof(SbAffine), e.affines.data(), e.affines.size() * sizeof(SbAffine));
+    if (!e.lits.empty()) std::memcpy(h + place.lit + at.lit * sizeof(float), e.lits.data(), e.lits.size() * sizeof(float));
+}
+
+/* Makes a slot ready for a batch: room for its headers, and for its records where the slot's buffers are large enough
+ * for what they usually take.  The caller holds the mutex or no job runs on the slot. */
+void prepare_slot(Slot& s, size_t programs) {
+    s.programs = programs;
+    s.headers.resize(programs);
+    s.taken = Counts();
+    const auto room = [&](int k) { return (size_t)(s.usual[k] * 1.15 * (double)programs) + 128; };
+    s.room.insn = room(0); s.room.patch = room(1); s.room.affine = room(2); s.room.lit = room(3);
+    s.place = Sections(programs, s.room.insn, s.room.patch, s.room.affine, s.room.lit);
+    s.packing = s.usual[0] > 0 && s.place.total <= s.pinned_cap && s.place.total <= s.device_cap && s.place.total < (size_t)1 << 32;
+}
+
 /* Encodes piece `index` into its slot; `lock` (held) is released meanwhile. */
 void encode_piece(SecantCubinRunnerImpl* r, std::unique_lock<std::mutex>& lock, size_t index, double* seconds) {
     const SecantAstProgramSet* programs = r->job_programs;
@@ -194,6 +244,17 @@ void encode_piece(SecantCubinRunnerImpl* r, std::unique_lock<std::mutex>& lock, 
         status = SECANT_ERROR_ALLOCATION_FAILED;
     }
     if (SB_FAULT("encode")) status = SECANT_ERROR_BAD_PROGRAM;
+    if (status == SECANT_SUCCESS && slot.packing) {
+        Counts at;
+        const EncodedBatch& e = piece.enc;
+        lock.lock();
+        at = slot.taken;
+        slot.taken.insn += e.insns.size(); slot.taken.patch += e.patches.size(); slot.taken.affine += e.affines.size(); slot.taken.lit += e.lits.size();
+        lock.unlock();
+        if (at.insn + e.insns.size() <= slot.room.insn && at.patch + e.patches.size() <= slot.room.patch &&
+            at.affine + e.affines.size() <= slot.room.affine && at.lit + e.lits.size() <= slot.room.lit)
+            pack_piece(slot, slot.place, e, at, first - batch_first);
+    }
     const double spent = now_seconds() - begin;
 
     lock.lock();
@@ -368,51 +429,47 @@ void order_programs(Slot& s) {
 }
 
 /* Joins the batch's encoded pieces in the slot's pinned buffer (a program's offsets move by what lies
- * before its piece), grows the device buffer when needed, and enqueues the upload.
+ * before its piece) unless that has been done as they were encoded, grows the buffers when needed, and enqueues the upload.
  * Layout: programs | insns | patches | affines | lits.  The pinned buffer keeps the programs' headers, in launch
  * order, until the slot is used again. */
 SecantResult upload_batch(SecantCubinRunnerImpl* r, Slot& s, std::vector<View>* views) {
-    size_t n_programs = 0, n_insns = 0, n_patches = 0, n_affines = 0, n_lits = 0;
+    const size_t n_programs = s.programs;
+    Counts n;
     for (size_t q = 0; q < s.used_pieces; ++q) {
         const EncodedBatch& e = s.pieces[q].enc;
-        n_programs += e.programs.size(); n_insns += e.insns.size(); n_patches += e.patches.size();
-        n_affines += e.affines.size(); n_lits += e.lits.size();
+        n.insn += e.insns.size(); n.patch += e.patches.size(); n.affine += e.affines.size(); n.lit += e.lits.size();
     }
-    if (n_insns > 0xffffffffull || n_patches > 0xffffffffull || n_affines > 0xffffffffull || n_lits > 0xffffffffull) return SECANT_ERROR_OVERFLOW;
-    const size_t o_prog = 0;
-    const size_t o_insn = align256(o_prog + n_programs * sizeof(SbProgram));
-    const size_t o_patch = align256(o_insn + n_insns * sizeof(SbInsn));
-    const size_t o_aff = align256(o_patch + n_patches * sizeof(SbPatch));
-    const size_t o_lit = align256(o_aff + n_affines * sizeof(SbAffine));
-    const size_t total = align256(o_lit + n_lits * sizeof(float) + 16);
-    if (s.pinned_cap < total) {
-        if (s.pinned) SB_CUDA(cudaFreeHost(s.pinned), "cudaFreeHost");
-        s.pinned = nullptr; s.pinned_cap = 0;
-        SB_CUDA(cudaHostAlloc(&s.pinned, total + total / 2, cudaHostAllocDefault), "cudaHostAlloc");
-        s.pinned_cap = total + total / 2;
-    }
-    if (s.device_cap < total) {
-        if (s.device) SB_CUDA(cudaFree(s.device), "cudaFree");
-        s.device = nullptr; s.device_cap = 0;
-        SB_CUDA(cudaMalloc(&s.device, total + total / 2), "cudaMalloc");
-        s.device_cap = total + total / 2;
-    }
-    char* h = static_cast<char*>(s.pinned);
-    s.headers.clear();
-    size_t at_insn = 0, at_patch = 0, at_affine = 0, at_lit = 0;
-    for (size_t q = 0; q < s.used_pieces; ++q) {
-        const EncodedBatch& e = s.pieces[q].enc;
-        for (SbProgram p : e.programs) {
-            p.insn_off += (uint32_t)at_insn; p.patch_off += (uint32_t)at_patch;
-            p.affine_off += (uint32_t)at_affine; p.lit_off += (uint32_t)at_lit;
-            s.headers.push_back(p);
+    if (n.insn > 0xffffffffull || n.patch > 0xffffffffull || n.affine > 0xffffffffull || n.lit > 0xffffffffull) return SECANT_ERROR_OVERFLOW;
+    const bool packed = s.packing && n.insn <= s.room.insn && n.patch <= s.room.patch && n.affine <= s.room.affine && n.lit <= s.room.lit;
+    const Sections at = packed ? s.place : Sections(n_programs, n.insn, n.patch, n.affine, n.lit);
+    s.usual[0] = (double)n.insn / n_programs; s.usual[1] = (double)n.patch / n_programs;
+    s.usual[2] = (double)n.affine / n_programs; s.usual[3] = (double)n.lit / n_programs;
+    if (!packed) {
+        const size_t total = at.total;
+        if (s.pinned_cap < total) {
+            if (s.pinned) SB_CUDA(cudaFreeHost(s.pinned), "cudaFreeHost");
+            s.pinned = nullptr; s.pinned_cap = 0;
+            SB_CUDA(cudaHostAlloc(&s.pinned, total + total / 2, cudaHostAllocDefault), "cudaHostAlloc");
+            s.pinned_cap = total + total / 2;
         }
-        if (!e.insns.empty()) std::memcpy(h + o_insn + at_insn * sizeof(SbInsn), e.insns.data(), e.insns.size() * sizeof(SbInsn));
-        if (!e.patches.empty()) std::memcpy(h + o_patch + at_patch * sizeof(SbPatch), e.patches.data(), e.patches.size() * sizeof(SbPatch));
-        if (!e.affines.empty()) std::memcpy(h + o_aff + at_affine * sizeof(SbAffine), e.affines.data(), e.affines.size() * sizeof(SbAffine));
-        if (!e.lits.empty()) std::memcpy(h + o_lit + at_lit * sizeof(float), e.lits.data(), e.lits.size() * sizeof(float));
-        at_insn += e.insns.size(); at_patch += e.patches.size(); at_affine += e.affines.size(); at_lit += e.lits.size();
+        if (s.device_cap < total) {
+            if (s.device) SB_CUDA(cudaFree(s.device), "cudaFree");
+            s.device = nullptr; s.device_cap = 0;
+            SB_CUDA(cudaMalloc(&s.device, total + total / 2), "cudaMalloc");
+            s.device_cap = total + total / 2;
+        }
+        Counts before;
+        size_t program = 0;
+        for (size_t q = 0; q < s.used_pieces; ++q) {
+            const EncodedBatch& e = s.pieces[q].enc;
+            pack_piece(s, at, e, before, program);
+            before.insn += e.insns.size(); before.patch += e.patches.size(); before.affine += e.affines.size(); before.lit += e.lits.size();
+            program += e.programs.size();
+        }
     }
+    const size_t o_prog = 0, o_insn = at.insn, o_patch = at.patch, o_aff = at.affine, o_lit = at.lit;
+    const size_t total = align256(o_lit + n.lit * sizeof(float) + 16);
+    char* h = static_cast<char*>(s.pinned);
     order_programs(s);
     SbProgram* const out = reinterpret_cast<SbProgram*>(h + o_prog);
     size_t num_light = 0;
@@ -794,6 +851,7 @@ SecantResult execute(SecantCubinRunnerImpl* r, const std::vector<UnpackedRun>& r
     const size_t pieces_per_batch = (batch_size + piece_size - 1) / piece_size;
     auto pieces_of = [&](size_t batch) { return (std::min(batch_size, P - batch * batch_size) + piece_size - 1) / piece_size; };
     auto open_slot = [&](Slot& s, size_t batch) { /* under the mutex; grows the piece list only while no job runs on it */
+        prepare_slot(s, std::min(batch_size, P - batch * batch_size));
         s.used_pieces = pieces_of(batch);
         s.done_pieces = 0;
     };
@@ -1172,6 +1230,8 @@ SecantResult secant_b200_population_create(SecantCubinRunner r, const SecantAstP
                 break;
             }
             SecantB200PopulationImpl::Resident res;
+            prepare_slot(staging, count);
+            staging.packing = false; /* encoded as one piece, before there are buffers */
             result = upload_batch(r, staging, &res.views);
             if (result != SECANT_SUCCESS) break;
             if (cudaStreamSynchronize(r->copy_stream) != cudaSuccess) { result = SECANT_ERROR_DRIVER_FAILED; break; }
