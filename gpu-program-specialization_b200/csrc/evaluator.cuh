@@ -67,6 +67,7 @@ struct DeviceBatch {
     uint64_t total_cst;   /* constant-table entries of all programs (an upper bound will do) */
     uint64_t total_cost;  /* scheduling weights of all programs */
     uint64_t max_cost;    /* the largest of them */
+    uint64_t main_cost, prelude_cost; /* of all programs: one pass of the main part, and of the row preludes */
     double total_perms;   /* permutations with values of their own, of all programs */
     uint32_t max_bits;    /* most toggle bits a program reads: a program has at most 1 << max_bits of them */
     uint32_t first;       /* the program CTAs begin with; those before it come last */
@@ -146,11 +147,15 @@ Geom make_geom(const DeviceBatch& batch, const EvalProblem& problem, const Launc
 
 /* scratch_limit: most floats of scratch a launch may use: the row splits are reduced until their partial sums
  * fit beside the constant tables (with one split there are none; the tables are not reduced here).
- * share: the part of the machine a small launch should count on (another one runs beside it); kBehindAnother: all of it, but
- * only when another launch that fills it leaves SMs one by one, so its CTAs should be short. */
-constexpr double kBehindAnother = -1.0;
+ * neighbour: what a small launch should know of another that runs beside it. */
+struct Neighbour {
+    enum Kind { NONE, SHARES, LEAVES, FILLS } kind; /* SHARES: it takes the rest of the machine.  LEAVES: it comes first and leaves some SMs, and
+                                                       CTAs that do not fit those would hold up its own.  FILLS: it comes first and leaves SMs
+                                                       one by one at its end, so CTAs should be short */
+    double share;                                   /* the part of the machine to count on */
+};
 LaunchPlan plan_launch(const DeviceBatch& batch, const EvalProblem& problem, int sm_count, size_t smem_limit,
-                       size_t scratch_limit, double share = 1.0);
+                       size_t scratch_limit, Neighbour neighbour = Neighbour{Neighbour::NONE, 1.0});
 
 /* Enqueues the evaluation of one batch on `stream`: the evaluator kernel writes per-split partial
  * sums into `partial` (plan.table_offset + plan.table_elements floats, private to the stream until the

@@ -75,7 +75,7 @@ struct Cut {
     uint32_t gpi, ppi, parts; /* parts only without toggles: the permutations are cuts enough, and their kernel has no room for it */
     unsigned long long groups;
 };
-struct Work { unsigned long long programs, bank_groups; double perms, most_perms; uint32_t passes; bool hoists; int sms; double longest; /* the costliest program over the average */ }; /* perms: of a program, on the average and at most */
+struct Work { unsigned long long programs, bank_groups; double perms, most_perms; uint32_t passes; double prelude; /* issue slots of a pass */ int sms; double longest; /* the costliest program over the average */ }; /* perms: of a program, on the average and at most */
 
 double cut_cycles(const Cut& cut, const Work& w) {
     const double per_cta = (double)((w.programs + cut.groups - 1) / cut.groups);
@@ -85,7 +85,7 @@ double cut_cycles(const Cut& cut, const Work& w) {
     const double active = std::min<double>(cut.warps, items);
     const double rate = std::min(0.14, 2.6 / active);
     const uint32_t passes = (w.passes + cut.parts - 1) / cut.parts;
-    const auto slots = [&](double n, double groups) { return 900.0 * n + passes * ((w.hoists ? 120.0 : 0.0) * n + 330.0 * groups); };
+    const auto slots = [&](double n, double groups) { return 900.0 * n + passes * (w.prelude * n + 330.0 * groups); };
     const double item = slots(1.0, cut.gpi * std::min<double>(cut.ppi, w.most_perms));
     const unsigned long long grid = cut.groups * cut.splits;
     const auto cta = [&](double time) { return 3000.0 + cut.tiles_per_split * (1500.0 + time / rate + empty * 400.0 / cut.warps); };
@@ -99,7 +99,9 @@ double cut_cycles(const Cut& cut, const Work& w) {
 
 /* `sms`: the part of the machine (`all`) this launch has when another runs beside it; `room`: floats of scratch for
  * partial sums. */
-void balance_small(LaunchPlan* plan, const DeviceBatch& batch, const EvalProblem& prob, int sms, int all, bool behind, size_t smem_limit, unsigned long long room) {
+void balance_small(LaunchPlan* plan, const DeviceBatch& batch, const EvalProblem& prob, int sms, int all, Neighbour::Kind neighbour, size_t smem_limit,
+                   unsigned long long room) {
+    const bool behind = neighbour == Neighbour::FILLS;
     const bool materialize = prob.mode == EVAL_MATERIALIZE;
     const uint32_t rr = (uint32_t)kVariantRows[plan->variant], rc = (uint32_t)kVariantBanks[plan->variant], pass = 32u * rr;
     const unsigned long long P = batch.num_programs, bank_groups = materialize ? 1 : (prob.num_banks + rc - 1) / rc;
@@ -120,7 +122,10 @@ void balance_small(LaunchPlan* plan, const DeviceBatch& batch, const EvalProblem
     /* deep enough, and its CTAs full enough; what is many waves of the whole machine is not confined to a part of it,
      * whose size is an estimate (358 programs, 33 sets, 770,512 rows, approximate functions: 6.9 ms, 10.3 when it was) */
     if (!fewer && rule_grid >= 8ull * (unsigned long long)sms && (rule_items >= 4ull * plan->warps || rule_grid >= 8ull * (unsigned long long)all)) return;
-    Work work{P, bank_groups, materialize ? 1.0 : batch.total_perms / (double)P, materialize ? 1.0 : (double)(1ull << batch.max_bits), 0, batch.max_hoisted != 0, sms,
+    /* what a pass of the row preludes costs beside one of the main parts; with toggles an item runs the shared prelude once
+     * for all its permutations, and the few slots that leaves on the average serve better */
+    const double prelude = !batch.max_hoisted ? 0.0 : batch.main_cost && !prob.toggle_bits ? 330.0 * (double)batch.prelude_cost / (double)batch.main_cost : 120.0;
+    Work work{P, bank_groups, materialize ? 1.0 : batch.total_perms / (double)P, materialize ? 1.0 : (double)(1ull << batch.max_bits), 0, prelude, sms,
               batch.total_cost ? std::min(3.0, std::max(1.0, (double)batch.max_cost * (double)P / (double)batch.total_cost)) : 1.0};
     const auto passes_of = [&](uint32_t tile_rows) { return (uint32_t)((std::min<size_t>(tile_rows, prob.num_rows) + pass - 1) / pass); };
     const unsigned long long per_sum = materialize ? 0 : (unsigned long long)P * std::max<uint32_t>(1u, quantities(prob)) * ((unsigned long long)prob.num_banks << prob.toggle_bits);
@@ -128,6 +133,7 @@ void balance_small(LaunchPlan* plan, const DeviceBatch& batch, const EvalProblem
              plan->groups_per_item, plan->perms_per_item, 1u, plan->num_groups};
     work.passes = passes_of(plan->tile_rows);
     double least = 0.97 * cut_cycles(best, work);
+    if (neighbour == Neighbour::LEAVES && rule_grid > (unsigned long long)sms) least = 1e300; /* any cut of one wave instead */
     const Cut rules = best;
     LaunchPlan trial = *plan;
     /* (uneven launches keep the tiles and row splits of the rules: their estimate is too coarse for more) */
@@ -146,7 +152,8 @@ void balance_small(LaunchPlan* plan, const DeviceBatch& batch, const EvalProblem
                     refit(&trial, 0u);
                     if (trial.warps < std::min(rules.warps, 12u)) continue;
                     const unsigned long long items = materialize ? 1ull : ((bank_groups / gpi) << batch.max_bits) / ppi;
-                    for (unsigned waves = uneven ? 0u : 1u; waves <= (fewer ? 32u : 8u); waves += waves < 8 ? 1 : 4) {
+                    const unsigned most_waves = neighbour == Neighbour::LEAVES && !uneven ? 1u : fewer ? 32u : 8u;
+                    for (unsigned waves = uneven ? 0u : 1u; waves <= most_waves; waves += waves < 8 ? 1 : 4) {
                         const unsigned long long ctas = waves ? (unsigned long long)waves * sms : rules.groups * rules.splits;
                         Cut c{trial.tile_rows, (uint32_t)((tiles + ctas - 1) / ctas), 0, trial.warps, gpi, ppi, 1u, 0};
                         if (uneven) { c.tiles_per_split = rules.tiles_per_split; c.warps = rules.warps; }
@@ -179,7 +186,7 @@ void balance_small(LaunchPlan* plan, const DeviceBatch& batch, const EvalProblem
 }
 
 LaunchPlan plan_with_tile(const DeviceBatch& batch, const EvalProblem& prob, int sm_count, size_t smem_limit, size_t scratch_limit,
-                          int variant, double share) {
+                          int variant, const Neighbour& neighbour) {
     LaunchPlan plan{};
     plan.ok = false;
     plan.overflow = false;
@@ -302,8 +309,7 @@ LaunchPlan plan_with_tile(const DeviceBatch& batch, const EvalProblem& prob, int
     plan.grid_x = (uint32_t)grid;
 
     const unsigned long long room = scratch_limit > plan.table_elements + 3 ? scratch_limit - plan.table_elements - 3 : 0;
-    const bool behind = share == kBehindAnother;
-    balance_small(&plan, batch, prob, behind ? sm_count : std::max(1, (int)(sm_count * share)), sm_count, behind, smem_limit, room);
+    balance_small(&plan, batch, prob, std::max(1, (int)(sm_count * neighbour.share)), sm_count, neighbour.kind, smem_limit, room);
     plan.partial_elements = 0;
     if (!materialize) {
         const unsigned long long n = (unsigned long long)plan.row_splits * plan.parts * P;
@@ -317,7 +323,7 @@ LaunchPlan plan_with_tile(const DeviceBatch& batch, const EvalProblem& prob, int
 
 }  // namespace
 
-LaunchPlan plan_launch(const DeviceBatch& batch, const EvalProblem& prob, int sm_count, size_t smem_limit, size_t scratch_limit, double share) {
+LaunchPlan plan_launch(const DeviceBatch& batch, const EvalProblem& prob, int sm_count, size_t smem_limit, size_t scratch_limit, Neighbour neighbour) {
     /* register tile: 4 rows x 4 banks per thread, or 8 x 2 / 16 x 1 when there are fewer banks.  Up
      * to four banks take the 8 x 2 tile: three or four banks are then two bank groups, so the row
      * prelude serves two runs of the main part and computes each row's value twice instead of four
@@ -329,7 +335,7 @@ LaunchPlan plan_launch(const DeviceBatch& batch, const EvalProblem& prob, int sm
     if (prob.mode == EVAL_MATERIALIZE) variant = 2;
     LaunchPlan plan{};
     for (; variant >= 0; --variant) {
-        plan = plan_with_tile(batch, prob, sm_count, smem_limit, scratch_limit, variant, share);
+        plan = plan_with_tile(batch, prob, sm_count, smem_limit, scratch_limit, variant, neighbour);
         if (plan.ok || plan.overflow) break;
     }
     return plan;

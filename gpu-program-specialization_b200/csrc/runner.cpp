@@ -507,6 +507,8 @@ SecantResult upload_batch(SecantCubinRunnerImpl* r, Slot& s, std::vector<View>* 
             db.total_cst += p.n_cst;
             db.total_cost += schedule_cost(p);
             db.max_cost = std::max(db.max_cost, schedule_cost(p));
+            db.main_cost += p.cost & 0xffffu;
+            db.prelude_cost += p.cost >> 16;
             db.total_perms += (double)(1ull << p.bits);
             db.max_bits = std::max<uint32_t>(db.max_bits, p.bits);
             db.max_btmp = std::max<uint32_t>(db.max_btmp, p.n_btmp);
@@ -579,11 +581,11 @@ SecantResult stream_scratch(SecantCubinRunnerImpl* r, size_t k, size_t elements,
 
 /* The part of the machine a view's launch should count on: with two views of one run entry on two streams
  * both are on the device at a time, and when neither fills it they share it by their work. */
-double view_share(const SecantCubinRunnerImpl* r, const std::vector<View>& views, const View& view, size_t entries) {
-    if (r->streams.size() < 2 || entries != 1 || views.size() < 2) return 1.0;
+Neighbour view_share(const SecantCubinRunnerImpl* r, const std::vector<View>& views, const View& view, size_t entries) {
+    if (r->streams.size() < 2 || entries != 1 || views.size() < 2) return Neighbour{Neighbour::NONE, 1.0};
     double all = 0.0;
     for (const View& v : views) all += (double)v.batch.total_cost;
-    return std::min(0.95, std::max(0.05, (double)view.batch.total_cost / std::max(1.0, all)));
+    return Neighbour{Neighbour::SHARES, std::min(0.95, std::max(0.05, (double)view.batch.total_cost / std::max(1.0, all)))};
 }
 
 /* The programs of a view from `first` on whose constant tables take at most `most` floats, one at least.  Every
@@ -634,6 +636,8 @@ std::vector<View> views_to_launch(SecantCubinRunnerImpl* r, const std::vector<Vi
     b.total_cst += heavy.total_cst;
     b.total_cost += heavy.total_cost;
     b.max_cost = std::max(b.max_cost, heavy.max_cost);
+    b.main_cost += heavy.main_cost;
+    b.prelude_cost += heavy.prelude_cost;
     b.total_perms += heavy.total_perms;
     b.max_bits = std::max(b.max_bits, heavy.max_bits);
     const LaunchPlan plan = plan_launch(b, prob, r->sm_count, r->smem_limit, r->scratch_limit);
@@ -659,7 +663,7 @@ SecantResult launch_batch(SecantCubinRunnerImpl* r, const std::vector<View>& bat
         if (runs[e].program_bank_stride)
             prob.banks = reinterpret_cast<const float*>(runs[e].banks.address) + runs[e].first_program_index * runs[e].program_bank_stride;
         const std::vector<View> views = views_to_launch(r, batch_views, prob);
-        double share = view_share(r, views, views[0], runs.size());
+        Neighbour neighbour = view_share(r, views, views[0], runs.size());
         for (const View& view : views) {
         const DeviceBatch& db = view.batch;
         const size_t k = (*stream_cursor)++ % r->streams.size();
@@ -674,7 +678,7 @@ SecantResult launch_batch(SecantCubinRunnerImpl* r, const std::vector<View>& bat
         for (size_t first = 0; first < db.num_programs && ce == cudaSuccess;) {
             const DeviceBatch part = whole ? db : tables_that_fit(view, headers, first, prob.num_banks, most_tables);
             first += part.num_programs;
-            const LaunchPlan lp = plan_launch(part, prob, r->sm_count, r->smem_limit, r->scratch_limit, share);
+            const LaunchPlan lp = plan_launch(part, prob, r->sm_count, r->smem_limit, r->scratch_limit, neighbour);
             if (!lp.ok) {
                 r->last_error = lp.overflow ? "configuration count beyond the evaluator's 32-bit item index" : "program batch does not fit shared memory";
                 return lp.overflow ? SECANT_ERROR_OVERFLOW : SECANT_ERROR_REGISTER_OVERFLOW;
@@ -689,7 +693,8 @@ SecantResult launch_batch(SecantCubinRunnerImpl* r, const std::vector<View>& bat
             /* the launch beside it has the SMs this one leaves; when it leaves none, the other's CTAs come behind it and are
              * best spread over all of them (2,938 programs, eleven of them heavy, 227,933 rows: 4.2 ms, 5.0 with those
              * confined to the SMs their work is worth) */
-            share = lp.grid_x < (uint32_t)r->sm_count ? 1.0 - (double)lp.grid_x / r->sm_count : kBehindAnother;
+            if (neighbour.kind != Neighbour::NONE)
+                neighbour = lp.grid_x < (uint32_t)r->sm_count ? Neighbour{Neighbour::LEAVES, 1.0 - (double)lp.grid_x / r->sm_count} : Neighbour{Neighbour::FILLS, 1.0};
             g_kernel_launches.fetch_add(launches);
             if (launches)
                 g_row_stream_bytes.fetch_add((uint64_t)lp.num_groups * (prob.num_inputs + (prob.mode == EVAL_MATERIALIZE ? 0u : prob.num_targets)) *
