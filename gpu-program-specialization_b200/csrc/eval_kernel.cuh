@@ -81,7 +81,7 @@ enum Handler : uint32_t {
     H_SIN = 26, H_COS, H_EXP, H_LOG, H_TANH,       /* unusual arguments leave the block; word 1 = SB_UN_* */
     H_UNARY,                                       /* any other function, word 1 = SB_UN_* */
     H_RARE,                                        /* word 1 = the record's word 0 */
-    H_COUNT
+    H_NARROW                                       /* + what follows H_DIV, up to H_TANH: the same for the first bank column only */
 };
 /* Operand kinds are the record's; the offset of a hoisted row value has this bit set, and the handlers
  * of row operands choose between the two bases by it (four handlers less each, one select more). */
@@ -117,8 +117,13 @@ struct HandlerTable {
 };
 __constant__ HandlerTable kHandlers = HandlerTable();
 
-__device__ __forceinline__ SbInsn rewrite(SbInsn ins, const OperandStrides& st) {
-    const uint32_t e = kHandlers.entry[ins.w0 & 0xffu], idx = ins.w0 >> 16, h = e & 0xffu;
+/* `narrow`: the instruction's values are the same in all bank columns (it belongs to a row prelude, or to a program that
+ * does not depend on the coefficients), and only the first column is read in the end: those that have such a form (`all`:
+ * divisions and logarithms as well) leave the others as they are. */
+__device__ __forceinline__ SbInsn rewrite(SbInsn ins, const OperandStrides& st, bool narrow, bool all) {
+    const uint32_t e = kHandlers.entry[ins.w0 & 0xffu], idx = ins.w0 >> 16;
+    uint32_t h = e & 0xffu;
+    if (narrow && h >= H_DIV && h <= H_TANH && (all || (h >= H_SIN && h <= H_EXP))) h += H_NARROW - H_DIV;
     if (!(e & 1u << 10)) return SbInsn{h, h == H_RARE ? ins.w0 : e >> 16};
     const uint32_t kind = (e >> 8) & 3u;
     if (kind == SB_KIND_ROW && (idx & SB_ROW_HOISTED)) return SbInsn{h, kHoistedOffset | (idx - SB_ROW_HOISTED) * st.of[3]};
@@ -215,17 +220,23 @@ __device__ __forceinline__ void put_insn(SbInsn* at, SbInsn ins) {
 #define SB_LOADQC_16 "ld.shared.b32 c0, [ad];\n mov.b64 %0, {c0, c0};\n"
 #define SB_MAPQ_CST_16 SB_COPY("%1", "%0") SB_COPY("%2", "%0") SB_COPY("%3", "%0") SB_COPY("%4", "%0") SB_COPY("%5", "%0") SB_COPY("%6", "%0") SB_COPY("%7", "%0")
 /* The accurate functions on all eight pairs (pairs_ptx.cuh). */
-/* what any argument takes is there once, for the pair in the first place: the pairs go round */
+/* What any argument takes is there once, for the pair in the first place: the pairs go round, c5 of them, or (top bit of c5,
+ * only in the 4 x 4 tile) those of its first column change places. */
 #define SB_ROTATE "mov.b64 m, %0;\n mov.b64 %0, %1;\n mov.b64 %1, %2;\n mov.b64 %2, %3;\n mov.b64 %3, %4;\n mov.b64 %4, %5;\n mov.b64 %5, %6;\n mov.b64 %6, %7;\n mov.b64 %7, m;\n"
+#define SB_AROUND(NAME) SB_ROTATE "sub.u32 c5, c5, 1;\n setp.ne.u32 p, c5, 0;\n @p bra.uni " NAME "L;\n" SB_GO
+#define SB_AROUND_4(NAME)                                                                               \
+    "setp.lt.s32 p, c5, 0;\n @p bra.uni " NAME "WAP;\n" SB_ROTATE "bra.uni " NAME "ROUND;\n"            \
+    NAME "WAP:\n mov.b64 m, %0;\n mov.b64 %0, %4;\n mov.b64 %4, m;\n" NAME "ROUND:\n sub.u32 c5, c5, 1;\n and.b32 c4, c5, 15;\n" \
+    "setp.ne.u32 p, c4, 0;\n @p bra.uni " NAME "L;\n" SB_GO
 #define SB_EACH(F) F("%0") F("%1") F("%2") F("%3") F("%4") F("%5") F("%6") F("%7")
-#define SB_FUNCTIONS                                                                                    \
+#define SB_FUNCTIONS(AROUND)                                                                                    \
     "CO:\n" SB_COS_SHIFT "bra.uni SC0;\n SI:\n" SB_SIN_SHIFT                                            \
     "SC0:\n mov.f32 top, 0f00000000;\n" SB_EACH(SB_TOP_NUMBER) "setp.lt.f32 p, top, 0f49800000;\n" SB_VOTE SB_NEXT \
     SB_SIN_CONSTANTS "@!p bra.uni SA;\n" SB_EACH(SB_SIN_PAIR) SB_GO                                     \
-    "SA:\n mov.u32 c5, 8;\n SL:\n" SB_SIN_ANY("%0", "%25", "SN") SB_ROTATE "sub.u32 c5, c5, 1;\n setp.ne.u32 p, c5, 0;\n @p bra.uni SL;\n" SB_GO \
+    "SA:\n mov.u32 c5, 8;\n SL:\n" SB_SIN_ANY("%0", "%25", "SN") AROUND("S")                           \
     "EX:\n mov.f32 top, 0f00000000;\n" SB_EACH(SB_TOP) "setp.le.f32 p, top, 0f42AC0000;\n" SB_VOTE SB_NEXT \
     SB_EXP_CONSTANTS SB_MINUS_ONE "@!p bra.uni EA;\n" SB_EACH(SB_EXP_PAIR) SB_GO                        \
-    "EA:\n mov.u32 c5, 8;\n EL:\n" SB_EXP_ANY("%0") SB_ROTATE "sub.u32 c5, c5, 1;\n setp.ne.u32 p, c5, 0;\n @p bra.uni EL;\n" SB_GO \
+    "EA:\n mov.u32 c5, 8;\n EL:\n" SB_EXP_ANY("%0") AROUND("E")                                       \
     "TH:\n" SB_NEXT SB_TANH_CONSTANTS SB_MINUS_ONE SB_EACH(SB_TANH_PAIR) SB_GO                          \
     "LG:\n mov.f32 top, 0f00000000;\n mov.f32 low, 0f7F800000;\n" SB_EACH(SB_TOP) SB_EACH(SB_LOW)       \
     "setp.lt.f32 p, top, 0f7F800000;\n setp.ge.and.f32 p, low, 0f00800000, p;\n" SB_ALL_OR_LEAVE SB_NEXT \
@@ -267,10 +278,43 @@ __device__ __forceinline__ void put_insn(SbInsn* at, SbInsn ins) {
     SB_FAST_DIV("%0", "%8") SB_FAST_DIV("%1", "%9") SB_FAST_DIV("%2", "%10") SB_FAST_DIV("%3", "%11")   \
     SB_FAST_DIV("%4", "%12") SB_FAST_DIV("%5", "%13") SB_FAST_DIV("%6", "%14") SB_FAST_DIV("%7", "%15") SB_GO
 
+/* Functions (and, approximate, divisions) of the first bank column of the 4 x 4 tile, pairs 0 and 4: a quarter of the
+ * arithmetic for what is the same in all columns.  Of 64 sets' work the row preludes and the programs without
+ * coefficients are a tenth, of 16 sets' almost a third: 169 programs x 20 sets x 1,042,866 rows 4.38 -> 4.29 ms, 1,024 x 16
+ * x 1,048,583 with approximate functions 21.9 -> 21.3, 470 x 8 x 18,277 168 -> 163 us.  What bounds it is the
+ * instruction cache, which the accurate functions fill: with narrow forms of all of them the first took 10 % fewer
+ * instructions and 4.62 ms, so sine, cosine and exponential go through the loops that arguments of any size take, and
+ * the others stay as they are.  Launches with toggles, whose kernel is the largest, go without (2.77 ms against 2.84). */
+#define SB_FIRST(F) F("%0") F("%4")
+#define SB_NARROW_TARGETS_4 ", NDR, NDC, NDS, NQR, NQC, NQS, NSI, NCO, NEX, NLG, NTH"
+#define SB_NARROW_TARGETS_8 ""
+#define SB_NARROW_TARGETS_16 ""
+#define SB_NARROW_DIVISIONS                                                                             \
+    "NDR:\n" SB_AT_ROW SB_LD2("%8", "%12", "0") "bra.uni NDV;\n"                                       \
+    "NDC:\n" SB_AT("%21") "ld.shared.b32 c0, [ad];\n mov.b64 %8, {c0, c0};\n mov.b64 %12, {c0, c0};\n bra.uni NDV;\n" \
+    "NDS:\n" SB_AT("%22") "ld.shared.b64 %8, [ad];\n ld.shared.b64 %12, [ad+1024];\n bra.uni NDV;\n"   \
+    "NQR:\n" SB_AT_ROW SB_COPY("%8", "%0") SB_COPY("%12", "%4") SB_LD2("%0", "%4", "0") "bra.uni NDV;\n" \
+    "NQC:\n" SB_AT("%21") SB_COPY("%8", "%0") SB_COPY("%12", "%4") "ld.shared.b32 c0, [ad];\n mov.b64 %0, {c0, c0};\n mov.b64 %4, {c0, c0};\n bra.uni NDV;\n" \
+    "NQS:\n" SB_AT("%22") SB_COPY("%8", "%0") SB_COPY("%12", "%4") "ld.shared.b64 %0, [ad];\n ld.shared.b64 %4, [ad+1024];\n bra.uni NDV;\n"
+#define SB_NARROW_ACCURATE                                                                              \
+    "NCO:\n" SB_COS_SHIFT "bra.uni NS0;\n NSI:\n" SB_SIN_SHIFT "NS0:\n" SB_NEXT SB_SIN_CONSTANTS "mov.u32 c5, 0x80000002;\n bra.uni SL;\n" \
+    "NEX:\n" SB_NEXT SB_EXP_CONSTANTS SB_MINUS_ONE "mov.u32 c5, 0x80000002;\n bra.uni EL;\n"            \
+    "NDR: NDC: NDS: NQR: NQC: NQS: NLG: NTH: bra.uni LEAVE;\n"
+#define SB_NARROW_FAST                                                                                  \
+    SB_NARROW_DIVISIONS                                                                                 \
+    "NCO:\n" SB_NEXT SB_FIRST(SB_FAST_COS) SB_GO "NTH:\n" SB_NEXT SB_FIRST(SB_FAST_TANH) SB_GO "NSI:\n" SB_NEXT SB_FIRST(SB_FAST_SIN) SB_GO \
+    "NEX:\n mov.f32 top, 0f00000000;\n" SB_FIRST(SB_TOP) "setp.le.f32 p, top, 0f42AE0000;\n" SB_ALL_OR_LEAVE SB_NEXT \
+    SB_PAIR_CONST("k0", "0x3FB8AA3B3FB8AA3B") SB_FIRST(SB_FAST_EXP) SB_GO                               \
+    "NLG:\n mov.f32 low, 0f7F800000;\n" SB_FIRST(SB_LOW) "setp.ge.f32 p, low, 0f00800000;\n" SB_ALL_OR_LEAVE SB_NEXT \
+    SB_PAIR_CONST("k0", "0x3F3172183F317218") SB_FIRST(SB_FAST_LOG) SB_GO                               \
+    "NDV:\n mov.f32 top, 0f00000000;\n mov.f32 low, 0f7F800000;\n" SB_TOP_NUMBER("%8") SB_TOP_NUMBER("%12") SB_LOW_NUMBER("%8") SB_LOW_NUMBER("%12") \
+    "setp.le.f32 p, top, 0f7E800000;\n setp.ge.and.f32 p, low, 0f00800000, p;\n" SB_ALL_OR_LEAVE SB_NEXT \
+    SB_FAST_DIV("%0", "%8") SB_FAST_DIV("%4", "%12") SB_GO
+
 #define SB_CORE(N, FUNCTIONS)                                                                           \
     "{\n" SB_PTX_REGISTERS SB_PTX_REGISTERS_ANY                                                        \
     ".reg .u32 hb;\n targets: .branchtargets EN, LR, LC, LS, ST, SH, AR, AC, AS, SR, SC, SS, RR, RC, RS, MR, MC, MS, NG, AB, " \
-    "DR, DC, DS, QR, QC, QS, SI, CO, EX, LG, TH, LEAVE, LEAVE;\n"                                           \
+    "DR, DC, DS, QR, QC, QS, SI, CO, EX, LG, TH, LEAVE, LEAVE" SB_NARROW_TARGETS_##N ";\n"                                           \
     "ld.shared.u32 %17, [%16+-8];\n" SB_NEXT SB_GO                                                       \
     SB_THREE(N, "L", SB_MOV8) SB_THREE(N, "A", SB_ADD8) SB_THREE(N, "S", SB_SUB8) SB_THREE(N, "R", SB_RSUB8) \
     SB_THREE(N, "M", SB_MUL8) SB_DIVISIONS(N)                                                           \
@@ -453,14 +497,15 @@ struct Machine {
                      : "memory")
 #pragma unroll 1
         for (;;) {
-            if constexpr (RR == 4 && FAST) SB_RUN_CORE(4, SB_FAST_FUNCTIONS);
-            else if constexpr (RR == 4) SB_RUN_CORE(4, SB_FUNCTIONS);
+            if constexpr (RR == 4 && FAST) SB_RUN_CORE(4, SB_FAST_FUNCTIONS SB_NARROW_FAST);
+            else if constexpr (RR == 4) SB_RUN_CORE(4, SB_FUNCTIONS(SB_AROUND_4) SB_NARROW_ACCURATE);
             else if constexpr (RR == 8 && FAST) SB_RUN_CORE(8, SB_FAST_FUNCTIONS);
-            else if constexpr (RR == 8) SB_RUN_CORE(8, SB_FUNCTIONS);
+            else if constexpr (RR == 8) SB_RUN_CORE(8, SB_FUNCTIONS(SB_AROUND));
             else if constexpr (FAST) SB_RUN_CORE(16, SB_FAST_FUNCTIONS);
-            else SB_RUN_CORE(16, SB_FUNCTIONS);
+            else SB_RUN_CORE(16, SB_FUNCTIONS(SB_AROUND));
             if (h == 0u) return;
             asm volatile("ld.shared.u32 %0, [%1+-16];" : "=r"(h) : "r"(ip) : "memory"); /* of the instruction the core stopped at */
+            if (RR == 4 && h >= H_NARROW) h -= H_NARROW - H_DIV; /* in all columns: what the others hold is not read */
             if (FAST && h < H_SIN) {
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
@@ -674,11 +719,12 @@ eval_kernel(const DeviceBatch batch, const EvalProblem prob, const Geom geom, fl
             const uint32_t perm0 = SPAN ? block * ppi : 0u;
             if (SPAN && perm0 >= 1ull << hp->bits) continue;
             const uint32_t perms = !SPAN ? 1u : (uint32_t)min((unsigned long long)ppi, (1ull << hp->bits) - perm0);
+            const auto narrow = [&](uint32_t i) { return RR == 4 && !SPAN && (i < main_off || (flags & SB_PROG_BANK_INDEPENDENT)); };
             __syncwarp(); /* the previous item's reads of exec, table and psum are done */
             if (PARTS && lane == 0) exec[-1].w1 = split * geom.parts + pass / geom.passes_per_part; /* which rows the item's sums are of: a word the copy does not use */
             const SbInsn* const code = batch.insns + hp->insn_off + pre_off; /* the row parts; the bank part has run (bank_tables_kernel) */
 #pragma unroll 1
-            for (uint32_t i = lane; i < n_insn; i += 32) put_insn(exec + i, rewrite(code[i], strides));
+            for (uint32_t i = lane; i < n_insn; i += 32) put_insn(exec + i, rewrite(code[i], strides, narrow(i), FAST));
             const uint32_t first_bg = materialize ? 0u : (within - block * chunks) * gpi;
             const uint32_t ngroups = materialize ? 1u : min(gpi, bank_groups - first_bg);
             const SbPatch* const patches = batch.patches + hp->patch_off;
@@ -690,7 +736,7 @@ eval_kernel(const DeviceBatch batch, const EvalProblem prob, const Geom geom, fl
                     const SbPatch* p = patches + i;
                     unsigned choice = (perm >> p->bit0) & 1u;
                     if (p->bit1 != 0xffu) choice |= ((perm >> p->bit1) & 1u) << 1;
-                    if (p->insn >= pre_off) put_insn(exec + (p->insn - pre_off), rewrite(p->alt[choice], strides));
+                    if (p->insn >= pre_off) put_insn(exec + (p->insn - pre_off), rewrite(p->alt[choice], strides, narrow(p->insn - pre_off), FAST));
                 }
                 __syncwarp();
             };
