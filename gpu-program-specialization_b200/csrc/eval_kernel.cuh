@@ -778,13 +778,16 @@ eval_kernel(const DeviceBatch batch, const EvalProblem prob, const Geom geom, fl
                 const int first = SPAN ? (has_shared ? -1 : 0) : (has_shared ? -2 : has_prelude ? -1 : 0);
                 const int last = SPAN ? (int)perms * per_perm : (int)eval_groups;
 #pragma unroll 1
-                for (int s = first; s < last; ++s) {
+                for (int s = first, permutation = 0, step = 0; s < last; ++s) {
+                    /* SPAN: step `step` of permutation `permutation`, counted on: a division per step cost 384 gated programs
+                     * 3.15 ms instead of 2.99 */
+                    if (SPAN && s > 0 && ++step == per_perm) { step = 0; ++permutation; }
                     int j = 0, g = s < 0 ? 0 : s;
                     bool prelude = s < 0;
                     uint32_t start = s == first && has_shared ? 0u : s < 0 ? mid_off : main_off;
                     if (SPAN) {
-                        j = s < 0 ? 0 : s / per_perm;
-                        const int w = s - j * per_perm; /* step inside the permutation */
+                        j = permutation;
+                        const int w = step;
                         prelude = s < 0 || (has_prelude && w == 0);
                         g = prelude ? 0 : w - (has_prelude ? 1 : 0);
                         start = prelude ? (s < 0 ? 0u : mid_off) : main_off;
