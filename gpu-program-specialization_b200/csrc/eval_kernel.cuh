@@ -231,7 +231,7 @@ __device__ __forceinline__ void put_insn(SbInsn* at, SbInsn ins) {
 #define SB_EACH(F) F("%0") F("%1") F("%2") F("%3") F("%4") F("%5") F("%6") F("%7")
 #define SB_FUNCTIONS(AROUND)                                                                                    \
     "CO:\n" SB_COS_SHIFT "bra.uni SC0;\n SI:\n" SB_SIN_SHIFT                                            \
-    "SC0:\n mov.f32 top, 0f00000000;\n" SB_EACH(SB_TOP_NUMBER) "setp.lt.f32 p, top, 0f49800000;\n" SB_VOTE SB_NEXT \
+    "SC0:\n mov.f32 top, 0f00000000;\n" SB_EACH(SB_TOP_NUMBER) "setp.lt.f32 p, top, 0f45800000;\n" SB_VOTE SB_NEXT \
     SB_SIN_CONSTANTS "@!p bra.uni SA;\n" SB_EACH(SB_SIN_PAIR) SB_GO                                     \
     "SA:\n mov.u32 c5, 8;\n SL:\n" SB_SIN_ANY("%0", "%25", "SN") AROUND("S")                           \
     "EX:\n mov.f32 top, 0f00000000;\n" SB_EACH(SB_TOP) "setp.le.f32 p, top, 0f42AC0000;\n" SB_VOTE SB_NEXT \

@@ -59,17 +59,17 @@
  * with a large argument somewhere in the warp those of sincos_large() as well.  Label DONE is the macro's own. */
 #define SB_TRIG_TEXT(I, BITS) "mov.b64 g" #I ", 0x" #BITS #BITS ";\n"
 #define SB_SIN_TURNS(W, F, Q, TURNS)                                                                    \
-    "shr.u32 c0, " W ", 23;\n and.b32 c0, c0, 255;\n max.u32 c0, c0, 147;\n min.u32 c0, c0, 254;\n shl.b32 c0, c0, 4;\n cvt.u64.u32 at, c0;\n" \
-    "add.u64 at, at, " TURNS ";\n ld.global.nc.v2.f64 {d0, d1}, [at+-2352];\n and.b32 c0, " W ", 0x007FFFFF;\n shr.u32 c0, c0, 3;\n" \
+    "shr.u32 c0, " W ", 23;\n and.b32 c0, c0, 255;\n max.u32 c0, c0, 139;\n min.u32 c0, c0, 254;\n shl.b32 c0, c0, 4;\n cvt.u64.u32 at, c0;\n" \
+    "add.u64 at, at, " TURNS ";\n ld.global.nc.v2.f64 {d0, d1}, [at+-2224];\n and.b32 c0, " W ", 0x007FFFFF;\n shr.u32 c0, c0, 3;\n" \
     "and.b32 c1, " W ", 0x80000000;\n or.b32 c0, c0, c1;\n or.b32 c1, c0, 0x3FF00000;\n shl.b32 c0, " W ", 29;\n mov.b64 d2, {c0, c1};\n" \
-    "mul.rn.f64 d0, d2, d0;\n add.rn.f64 d3, d0, 0d4338000000000000;\n mov.b64 {" Q ", c1}, d3;\n add.rn.f64 d3, d3, 0dC338000000000000;\n" \
+    "mul.rn.f64 d0, d2, d0;\n fma.rn.f64 d3, d2, d1, d0;\n add.rn.f64 d3, d3, 0d4338000000000000;\n mov.b64 {" Q ", c1}, d3;\n add.rn.f64 d3, d3, 0dC338000000000000;\n" \
     "sub.rn.f64 d0, d0, d3;\n fma.rn.f64 d0, d2, d1, d0;\n cvt.rn.f32.f64 " F ", d0;\n"
 #define SB_SIN_CHOOSE(W, Q, S, C, V) /* the quadrant's function and sign, where the argument is large and finite */ \
     "add.u32 " Q ", " Q ", c3;\n and.b32 c0, " Q ", 1;\n setp.ne.u32 p, c0, 0;\n selp.b32 c0, " C ", " S ", p;\n and.b32 c1, " Q ", 2;\n" \
-    "shl.b32 c1, c1, 30;\n xor.b32 c0, c0, c1;\n and.b32 c1, " W ", 0x7FFFFFFF;\n sub.u32 c1, c1, 0x49800000;\n setp.lt.u32 p, c1, 0x36000000;\n" \
+    "shl.b32 c1, c1, 30;\n xor.b32 c0, c0, c1;\n and.b32 c1, " W ", 0x7FFFFFFF;\n sub.u32 c1, c1, 0x45800000;\n setp.lt.u32 p, c1, 0x3A000000;\n" \
     "selp.b32 " V ", c0, " V ", p;\n"
 #define SB_SIN_ANY(A, TURNS, DONE)                                                                      \
-    "mov.b64 v, " A ";\n mov.f32 top, 0f00000000;\n" SB_TOP_NUMBER("v") "setp.lt.f32 p, top, 0f49800000;\n vote.sync.all.pred p, p, 0xffffffff;\n" \
+    "mov.b64 v, " A ";\n mov.f32 top, 0f00000000;\n" SB_TOP_NUMBER("v") "setp.lt.f32 p, top, 0f45800000;\n vote.sync.all.pred p, p, 0xffffffff;\n" \
     SB_SIN_PAIR(A) "@p bra.uni " DONE ";\n mov.b64 {w0, w1}, v;\n" SB_SIN_TURNS("w0", "f0", "u0", TURNS) SB_SIN_TURNS("w1", "f1", "u1", TURNS) \
     SB_TRIG_LIST(SB_TRIG_TEXT) "mov.b64 r, {f0, f1};\n mul.rn.f32x2 r, r, g0;\n mul.rn.f32x2 z, r, r;\n fma.rn.f32x2 q, g1, z, g2;\n" \
     "fma.rn.f32x2 q, q, z, g3;\n mul.rn.f32x2 t, r, z;\n fma.rn.f32x2 r, t, q, r;\n fma.rn.f32x2 q, g4, z, g5;\n fma.rn.f32x2 q, q, z, g6;\n" \

@@ -165,7 +165,7 @@ static_assert(sizeof(kPairConstants) == 320, "the offsets RK_K2 is given count o
     "NG:\n" RK_NEXT RK_EACH_##N(RK_NEG) RK_GO "AB:\n" RK_NEXT RK_EACH_##N(RK_ABS) RK_GO                  \
     "CO:\n" SB_COS_SHIFT "bra.uni SC0;\n SI:\n" SB_SIN_SHIFT                                            \
     "SC0:\n" RK_K2("k0", "k1", "0") RK_K2("k2", "k3", "16") RK_K2("k4", "k5", "32") RK_K2("k6", "k7", "48") RK_K2("k8", "k9", "64") \
-    RK_K2("k10", "m", "80") "mov.f32 top, 0f00000000;\n" RK_EACH_##N(SB_TOP) "setp.lt.f32 p, top, 0f49800000;\n" SB_ALL_OR_LEAVE RK_NEXT \
+    RK_K2("k10", "m", "80") "mov.f32 top, 0f00000000;\n" RK_EACH_##N(SB_TOP) "setp.lt.f32 p, top, 0f45800000;\n" SB_ALL_OR_LEAVE RK_NEXT \
     RK_EACH_##N(SB_SIN_PAIR) RK_GO                                                                      \
     "EX:\n" RK_K2("k0", "k1", "96") RK_K2("k2", "m", "112") "mov.f32 top, 0f00000000;\n" RK_EACH_##N(SB_TOP) \
     "setp.le.f32 p, top, 0f42AC0000;\n" SB_ALL_OR_LEAVE RK_NEXT RK_EACH_##N(SB_EXP_PAIR) RK_GO          \
