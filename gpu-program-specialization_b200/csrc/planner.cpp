@@ -136,9 +136,12 @@ void balance_small(LaunchPlan* plan, const DeviceBatch& batch, const EvalProblem
     if (neighbour == Neighbour::LEAVES && rule_grid > (unsigned long long)sms) least = 1e300; /* any cut of one wave instead */
     const Cut rules = best;
     LaunchPlan trial = *plan;
-    /* (uneven launches keep the tiles and row splits of the rules: their estimate is too coarse for more) */
-    const bool uneven = work.perms < work.most_perms;
-    for (uint32_t half = 0; half < (uneven ? 1u : 2u); ++half) { /* the rules' tile and one of half its rows */
+    /* Two kinds of launches keep the tiles and row splits of the rules.  Uneven ones, whose estimate is too coarse for more,
+     * and those behind a launch that fills the machine, which follows the rules too: in a large population the order in
+     * which rows are added then does not hang on the cut of its few heavy programs, so programs of nearly equal scores do not
+     * change their ranks with it (2,048 programs x 64 sets: up to 2 % of the first 1,024 ranks otherwise). */
+    const bool uneven = work.perms < work.most_perms, same_rows = uneven || behind;
+    for (uint32_t half = 0; half < (same_rows ? 1u : 2u); ++half) { /* the rules' tile and one of half its rows */
         trial.tile_rows = half ? (rules.tile_rows / 2 + pass - 1) / pass * pass : rules.tile_rows;
         if (half && (trial.tile_rows == rules.tile_rows || trial.tile_rows < 256u)) break;
         work.passes = passes_of(trial.tile_rows);
@@ -156,12 +159,13 @@ void balance_small(LaunchPlan* plan, const DeviceBatch& batch, const EvalProblem
                     for (unsigned waves = uneven ? 0u : 1u; waves <= most_waves; waves += waves < 8 ? 1 : 4) {
                         const unsigned long long ctas = waves ? (unsigned long long)waves * sms : rules.groups * rules.splits;
                         Cut c{trial.tile_rows, (uint32_t)((tiles + ctas - 1) / ctas), 0, trial.warps, gpi, ppi, 1u, 0};
-                        if (uneven) { c.tiles_per_split = rules.tiles_per_split; c.warps = rules.warps; }
-                        if ((c.tiles_per_split > 1) != (trial.tile_buffers > 1) || (behind && c.tiles_per_split > rules.tiles_per_split)) continue;
+                        if (same_rows) c.tiles_per_split = rules.tiles_per_split;
+                        if (uneven) c.warps = rules.warps;
+                        if ((c.tiles_per_split > 1) != (trial.tile_buffers > 1)) continue;
                         c.splits = (uint32_t)((tiles + c.tiles_per_split - 1) / c.tiles_per_split);
                         if (per_sum && c.splits > 1 && c.splits > rules.splits && c.splits > room / per_sum) continue;
                         c.groups = std::max<unsigned long long>(1, std::min(ctas / c.splits, P));
-                        for (c.parts = 1; c.parts <= (prob.toggle_bits ? 1u : work.passes); c.parts *= 2) {
+                        for (c.parts = 1; c.parts <= (prob.toggle_bits || same_rows ? 1u : work.passes); c.parts *= 2) {
                             if (c.parts > 1 && per_sum && (unsigned long long)c.splits * c.parts > room / per_sum) break;
                             if (items * c.parts > 0xffffff00ull / ((P + c.groups - 1) / c.groups)) break;
                             const double t = cut_cycles(c, work);
