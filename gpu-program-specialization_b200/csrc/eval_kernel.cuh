@@ -66,7 +66,7 @@ __device__ __noinline__ void fma_over_scratch(uint2 ins, const float* rowp, cons
  * interpreter; pairs in the C++ switch 69.8 (half the arithmetic, but the code no longer fitted the
  * cache); this core with the functions in C++ 46; with the functions in the block 43; with loops instead
  * of unrolled calls for unusual arguments 31.6; sine, cosine and exponential of any argument inside the
- * block 28.4 (sine and cosine had left it from 4,096 on and for NaN, the exponential beyond 86: 2 % of their tiles,
+ * block 29.3 (sine and cosine had left it from 4,096 on and for NaN, the exponential beyond 86: 2 % of their tiles,
  * which took a sixth of the time; 256 programs x 33 sets x 10,007 rows, where such a program is the last to end,
  * 617 -> 455 us).  Before that, warp instructions 37.3e9 -> 18.4e9, cache hit rate of
  * the fetches 86 -> 98 %. */

@@ -56,21 +56,29 @@
     "mul.rn.f32x2 z, r, z;\n fma.rn.f32x2 r, z, q, r;\n mov.b64 {c0, c1}, t;\n shl.b32 c0, c0, 31;\n shl.b32 c1, c1, 31;\n" \
     "mov.b64 {c2, c3}, r;\n add.u32 c0, c0, c2;\n add.u32 c1, c1, c3;\n mov.b64 " A ", {c0, c1};\n"
 /* sin or cos of any pair (the shift says which, TURNS is the address of the table of sbmath.cuh): the steps above, and for a pair
- * with a large argument somewhere in the warp those of sincos_large() as well.  Label DONE is the macro's own. */
+ * with a large argument somewhere in the warp those of sincos_large() as well.  Labels DONE and DONE"D" are the macro's own. */
 #define SB_TRIG_TEXT(I, BITS) "mov.b64 g" #I ", 0x" #BITS #BITS ";\n"
 #define SB_SIN_TURNS(W, F, Q, TURNS)                                                                    \
-    "shr.u32 c0, " W ", 23;\n and.b32 c0, c0, 255;\n max.u32 c0, c0, 139;\n min.u32 c0, c0, 254;\n shl.b32 c0, c0, 4;\n cvt.u64.u32 at, c0;\n" \
-    "add.u64 at, at, " TURNS ";\n ld.global.nc.v2.f64 {d0, d1}, [at+-2224];\n and.b32 c0, " W ", 0x007FFFFF;\n shr.u32 c0, c0, 3;\n" \
+    "shr.u32 c0, " W ", 23;\n and.b32 c0, c0, 255;\n max.u32 c0, c0, 177;\n min.u32 c0, c0, 254;\n shl.b32 c0, c0, 4;\n cvt.u64.u32 at, c0;\n" \
+    "add.u64 at, at, " TURNS ";\n ld.global.nc.v2.f64 {d0, d1}, [at+-2832];\n and.b32 c0, " W ", 0x007FFFFF;\n shr.u32 c0, c0, 3;\n" \
     "and.b32 c1, " W ", 0x80000000;\n or.b32 c0, c0, c1;\n or.b32 c1, c0, 0x3FF00000;\n shl.b32 c0, " W ", 29;\n mov.b64 d2, {c0, c1};\n" \
     "mul.rn.f64 d0, d2, d0;\n fma.rn.f64 d3, d2, d1, d0;\n add.rn.f64 d3, d3, 0d4338000000000000;\n mov.b64 {" Q ", c1}, d3;\n add.rn.f64 d3, d3, 0dC338000000000000;\n" \
     "sub.rn.f64 d0, d0, d3;\n fma.rn.f64 d0, d2, d1, d0;\n cvt.rn.f32.f64 " F ", d0;\n"
+#define SB_SIN_DOUBLE(W, F, Q) /* the same below 2^50, with 2/pi in two parts */                           \
+    "mov.b32 " F ", " W ";\n cvt.f64.f32 d2, " F ";\n mul.rn.f64 d0, d2, 0d3FE45F306DC9C883;\n neg.f64 d1, d0;\n" \
+    "fma.rn.f64 d1, d2, 0d3FE45F306DC9C883, d1;\n fma.rn.f64 d1, d2, 0dBC86B01EC5417056, d1;\n add.rn.f64 d3, d0, 0d4338000000000000;\n" \
+    "mov.b64 {" Q ", c1}, d3;\n add.rn.f64 d3, d3, 0dC338000000000000;\n sub.rn.f64 d0, d0, d3;\n add.rn.f64 d0, d0, d1;\n cvt.rn.f32.f64 " F ", d0;\n"
+#define SB_SIN_BEYOND(W, F, Q, TURNS) /* takes it from the table at 2^50 and beyond */                     \
+    SB_SIN_TURNS(W, "low", "s1", TURNS) "and.b32 c0, " W ", 0x7FFFFFFF;\n setp.ge.u32 p, c0, 0x58800000;\n" \
+    "selp.f32 " F ", low, " F ", p;\n selp.b32 " Q ", s1, " Q ", p;\n"
 #define SB_SIN_CHOOSE(W, Q, S, C, V) /* the quadrant's function and sign, where the argument is large and finite */ \
     "add.u32 " Q ", " Q ", c3;\n and.b32 c0, " Q ", 1;\n setp.ne.u32 p, c0, 0;\n selp.b32 c0, " C ", " S ", p;\n and.b32 c1, " Q ", 2;\n" \
     "shl.b32 c1, c1, 30;\n xor.b32 c0, c0, c1;\n and.b32 c1, " W ", 0x7FFFFFFF;\n sub.u32 c1, c1, 0x45800000;\n setp.lt.u32 p, c1, 0x3A000000;\n" \
     "selp.b32 " V ", c0, " V ", p;\n"
 #define SB_SIN_ANY(A, TURNS, DONE)                                                                      \
     "mov.b64 v, " A ";\n mov.f32 top, 0f00000000;\n" SB_TOP_NUMBER("v") "setp.lt.f32 p, top, 0f45800000;\n vote.sync.all.pred p, p, 0xffffffff;\n" \
-    SB_SIN_PAIR(A) "@p bra.uni " DONE ";\n mov.b64 {w0, w1}, v;\n" SB_SIN_TURNS("w0", "f0", "u0", TURNS) SB_SIN_TURNS("w1", "f1", "u1", TURNS) \
+    SB_SIN_PAIR(A) "@p bra.uni " DONE ";\n mov.b64 {w0, w1}, v;\n" SB_SIN_DOUBLE("w0", "f0", "u0") SB_SIN_DOUBLE("w1", "f1", "u1") \
+    "setp.lt.f32 p, top, 0f58800000;\n" SB_VOTE "@p bra.uni " DONE "D;\n" SB_SIN_BEYOND("w0", "f0", "u0", TURNS) SB_SIN_BEYOND("w1", "f1", "u1", TURNS) DONE "D:\n" \
     SB_TRIG_LIST(SB_TRIG_TEXT) "mov.b64 r, {f0, f1};\n mul.rn.f32x2 r, r, g0;\n mul.rn.f32x2 z, r, r;\n fma.rn.f32x2 q, g1, z, g2;\n" \
     "fma.rn.f32x2 q, q, z, g3;\n mul.rn.f32x2 t, r, z;\n fma.rn.f32x2 r, t, q, r;\n fma.rn.f32x2 q, g4, z, g5;\n fma.rn.f32x2 q, q, z, g6;\n" \
     "fma.rn.f32x2 q, q, z, g7;\n mul.rn.f32x2 t, z, z;\n mul.rn.f32x2 z, z, g8;\n fma.rn.f32x2 q, t, q, z;\n add.rn.f32x2 q, q, g9;\n" \

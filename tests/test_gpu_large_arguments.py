@@ -19,10 +19,11 @@ def arguments(name, spread):
     n = x[at].size
     if name == "EXP":
         special = rng.uniform(-110, 95, n)
-    else:                                                            # every exponent from 2^11 on, and both sides of 4,096 and of 2^20
+    else:                                                            # every exponent from 2^11 on, and both sides of 4,096, 2^20 and 2^50
         special = np.exp2(11 + np.arange(n) * (116.99 / max(1, n - 1))) * rng.choice([-1, 1], n)
         special[1::5] = 2.0 ** 20 * (1 + (np.arange(special[1::5].size) - 8) * 2.0 ** -23)
         special[2::5] = 4096.0 * (1 + (np.arange(special[2::5].size) - 8) * 2.0 ** -23)
+        special[3::5] = 2.0 ** 50 * (1 + (np.arange(special[3::5].size) - 8) * 2.0 ** -23)
     x[at] = special.astype(np.float32)
     return x
 
