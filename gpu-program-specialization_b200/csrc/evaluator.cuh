@@ -151,7 +151,7 @@ Geom make_geom(const DeviceBatch& batch, const EvalProblem& problem, const Launc
 struct Neighbour {
     enum Kind { NONE, SHARES, LEAVES, FILLS } kind; /* SHARES: it takes the rest of the machine.  LEAVES: it comes first and leaves some SMs, and
                                                        CTAs that do not fit those would hold up its own.  FILLS: it comes first and leaves SMs
-                                                       one by one at its end, so CTAs should be short */
+                                                       one by one at its end: rows are cut by the rules */
     double share;                                   /* the part of the machine to count on */
 };
 LaunchPlan plan_launch(const DeviceBatch& batch, const EvalProblem& problem, int sm_count, size_t smem_limit,
