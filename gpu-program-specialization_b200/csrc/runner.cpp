@@ -398,6 +398,16 @@ uint64_t schedule_cost(const SbProgram& p) {
     return std::min<uint64_t>(once << std::min<unsigned>(p.bits, 32u), 0x1fffffu); /* 21 bits of the order's key */
 }
 
+/* adds what the planner weighs of a program to its batch's */
+void add_weights(DeviceBatch& batch, const SbProgram& p) {
+    const uint64_t cost = schedule_cost(p);
+    batch.total_cost += cost;
+    batch.max_cost = std::max(batch.max_cost, cost);
+    batch.main_cost += p.cost & 0xffffu;
+    batch.prelude_cost += p.cost >> 16;
+    batch.total_perms += (double)(1ull << p.bits);
+}
+
 /* Puts the batch's programs in launch order: light programs first, heavy ones after them; inside each
  * group the costly ones first, so that every CTA, which takes a strided subset, has a queue from its
  * costliest item to its cheapest and its warps finish a tile close together; ties keep the run's order.
@@ -505,11 +515,7 @@ SecantResult upload_batch(SecantCubinRunnerImpl* r, Slot& s, std::vector<View>* 
             db.max_hoisted = std::max<uint32_t>(db.max_hoisted, p.n_hoisted);
             db.max_cst = std::max<uint32_t>(db.max_cst, p.n_cst);
             db.total_cst += p.n_cst;
-            db.total_cost += schedule_cost(p);
-            db.max_cost = std::max(db.max_cost, schedule_cost(p));
-            db.main_cost += p.cost & 0xffffu;
-            db.prelude_cost += p.cost >> 16;
-            db.total_perms += (double)(1ull << p.bits);
+            add_weights(db, p);
             db.max_bits = std::max<uint32_t>(db.max_bits, p.bits);
             db.max_btmp = std::max<uint32_t>(db.max_btmp, p.n_btmp);
             db.uses_scratch |= (p.flags & SB_PROG_USES_SCRATCH) ? 1u : 0u;
@@ -599,6 +605,7 @@ DeviceBatch tables_that_fit(const View& view, const SbProgram* headers, size_t f
     part.num_programs = 0;
     part.first = 0; /* in launch order: the heavy programs of a joint view come last here */
     part.total_cst = 0;
+    part.total_cost = part.max_cost = part.main_cost = part.prelude_cost = 0; /* what the planner weighs against its number of programs */
     part.total_perms = 0;
     part.max_bits = 0;
     for (size_t i = first; i < view.batch.num_programs; ++i) {
@@ -608,8 +615,8 @@ DeviceBatch tables_that_fit(const View& view, const SbProgram* headers, size_t f
         if (part.num_programs && entries > most / ((banks + 3ull) << bits)) break;
         ++part.num_programs;
         part.total_cst = entries;
-        part.total_perms += (double)(1ull << p.bits);
         part.max_bits = bits;
+        add_weights(part, p);
     }
     return part;
 }

@@ -46,6 +46,8 @@ struct Allocation { size_t bytes; bool pinned; Clock busy; Clock written; };
 
 struct Fault { unsigned calls = 0, fail_at = 0; bool sticky = false; };
 
+constexpr size_t kCutWords = 12;
+
 struct World {
     std::mutex mutex;
     std::map<std::string, Fault> faults;
@@ -56,6 +58,7 @@ struct World {
     unsigned violations = 0, launches = 0, threads_started = 0;
     unsigned split_launches = 0;            /* launches whose rows are split */
     size_t largest_scratch = 0;             /* bytes of the largest scratch allocation a launch was given */
+    std::vector<uint64_t> cuts;             /* per evaluator launch: kCutWords words, see fake_cuts() */
     void* context = reinterpret_cast<void*>(0x1234);
     bool no_context = false;
     std::string last_violation;
@@ -270,6 +273,7 @@ FAKE_EXPORT void fake_reset(void) {
     world.threads_started = 0;
     world.split_launches = 0;
     world.largest_scratch = 0;
+    world.cuts.clear();
     world.no_context = false;
     world.context = reinterpret_cast<void*>(0x1234);
     world.last_violation.clear();
@@ -311,6 +315,14 @@ FAKE_EXPORT void fake_scratch(uint64_t* what) {
     std::lock_guard<std::mutex> lock(world.mutex);
     what[0] = world.largest_scratch;
     what[1] = world.split_launches;
+}
+/* The evaluator launches since the last reset, twelve words each: stream, programs, grid, rows of a tile, row splits, rows of
+ * a split, parts of a tile, then the programs' total and largest scheduling weight and their passes' weights (main part,
+ * prelude), and the program CTAs begin with.  Returns how many launches there were. */
+FAKE_EXPORT size_t fake_cuts(uint64_t* out, size_t capacity) {
+    std::lock_guard<std::mutex> lock(world.mutex);
+    for (size_t i = 0; i < world.cuts.size() && i < capacity * kCutWords; ++i) out[i] = world.cuts[i];
+    return world.cuts.size() / kCutWords;
 }
 FAKE_EXPORT const char* fake_last_violation(void) { return world.last_violation.c_str(); }
 FAKE_EXPORT void fake_set_context(int which) { /* 0: none, n: context n */
@@ -363,6 +375,9 @@ cudaError_t launch_eval(const DeviceBatch& batch, const EvalProblem&, const Laun
     }
     merge(records->busy, now);
     ++world.launches;
+    const uint64_t cut[kCutWords] = {(uint64_t)(uintptr_t)stream, batch.num_programs, plan.grid_x, plan.tile_rows, plan.row_splits, plan.rows_per_split,
+                                     plan.parts, batch.total_cost, batch.max_cost, batch.main_cost, batch.prelude_cost, batch.first};
+    world.cuts.insert(world.cuts.end(), cut, cut + kCutWords);
     *launches = 2;
     return cudaSuccess;
 }
