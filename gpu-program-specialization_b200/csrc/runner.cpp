@@ -670,9 +670,12 @@ SecantResult launch_batch(SecantCubinRunnerImpl* r, const std::vector<View>& bat
         if (runs[e].program_bank_stride)
             prob.banks = reinterpret_cast<const float*>(runs[e].banks.address) + runs[e].first_program_index * runs[e].program_bank_stride;
         const std::vector<View> views = views_to_launch(r, batch_views, prob);
+        /* what a view's launches should know of the last launch of the view before, on another stream; a view's own
+         * launches come one after the other */
         Neighbour neighbour = view_share(r, views, views[0], runs.size());
         for (const View& view : views) {
         const DeviceBatch& db = view.batch;
+        Neighbour next = neighbour;
         const size_t k = (*stream_cursor)++ % r->streams.size();
         cudaStream_t stream = r->streams[k];
         cudaError_t ce = after ? cudaStreamWaitEvent(stream, after, 0) : cudaSuccess;
@@ -701,12 +704,13 @@ SecantResult launch_batch(SecantCubinRunnerImpl* r, const std::vector<View>& bat
              * best spread over all of them (2,938 programs, eleven of them heavy, 227,933 rows: 4.2 ms, 5.0 with those
              * confined to the SMs their work is worth) */
             if (neighbour.kind != Neighbour::NONE)
-                neighbour = lp.grid_x < (uint32_t)r->sm_count ? Neighbour{Neighbour::LEAVES, 1.0 - (double)lp.grid_x / r->sm_count} : Neighbour{Neighbour::FILLS, 1.0};
+                next = lp.grid_x < (uint32_t)r->sm_count ? Neighbour{Neighbour::LEAVES, 1.0 - (double)lp.grid_x / r->sm_count} : Neighbour{Neighbour::FILLS, 1.0};
             g_kernel_launches.fetch_add(launches);
             if (launches)
                 g_row_stream_bytes.fetch_add((uint64_t)lp.num_groups * (prob.num_inputs + (prob.mode == EVAL_MATERIALIZE ? 0u : prob.num_targets)) *
                                              (uint64_t)prob.num_rows * sizeof(float));
         }
+        neighbour = next;
         if (ce == cudaSuccess && done) ce = cudaEventRecord((*done)[k], stream);
         if (ce != cudaSuccess) return cuda_fail(r, ce, "kernel launch");
         if (used) (*used)[k] = 1;

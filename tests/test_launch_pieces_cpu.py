@@ -70,3 +70,17 @@ def test_a_piece_has_the_weights_of_its_own_programs(lib, heavy):
     for key in ("programs", "total_cost", "main_cost", "prelude_cost"):
         assert sum(p[key] for p in pieces) == sum(w[key] for w in whole), key
     assert all(p["max_cost"] <= p["total_cost"] <= p["programs"] * p["max_cost"] for p in pieces)
+
+
+@pytest.mark.parametrize("light,heavy", [(300, 3), (300, 60), (80, 3)])
+def test_pieces_on_one_stream_do_not_make_room_for_one_another(lib, light, heavy):
+    """A launch leaves room for one on another stream; the pieces of one kind of programs follow each other on theirs, so
+    pieces of the same weights are cut alike."""
+    h = Pieces(lib, light, heavy)
+    pieces = run(lib, h, 2, 2 * 4 * 10 * 8 * ((h.BANKS + 3) << h.BITS))
+    h.release()
+    assert len({p["stream"] for p in pieces}) == 2
+    alike = {}
+    for p in pieces:
+        alike.setdefault((p["stream"], p["programs"], p["total_cost"]), set()).add((p["grid"], p["splits"], p["tile"], p["rows"], p["parts"]))
+    assert len(pieces) > len(alike) and all(len(c) == 1 for c in alike.values()), alike
