@@ -721,7 +721,6 @@ eval_kernel(const DeviceBatch batch, const EvalProblem prob, const Geom geom, fl
             const uint32_t perms = !SPAN ? 1u : (uint32_t)min((unsigned long long)ppi, (1ull << hp->bits) - perm0);
             const auto narrow = [&](uint32_t i) { return RR == 4 && !SPAN && (i < main_off || (flags & SB_PROG_BANK_INDEPENDENT)); };
             __syncwarp(); /* the previous item's reads of exec, table and psum are done */
-            if (PARTS && lane == 0) exec[-1].w1 = split * geom.parts + pass / geom.passes_per_part; /* which rows the item's sums are of: a word the copy does not use */
             const SbInsn* const code = batch.insns + hp->insn_off + pre_off; /* the row parts; the bank part has run (bank_tables_kernel) */
 #pragma unroll 1
             for (uint32_t i = lane; i < n_insn; i += 32) put_insn(exec + i, rewrite(code[i], strides, narrow(i), FAST));
@@ -740,7 +739,7 @@ eval_kernel(const DeviceBatch batch, const EvalProblem prob, const Geom geom, fl
                 }
                 __syncwarp();
             };
-            if (!materialize) {
+            if (!materialize && !PARTS) {
 #pragma unroll 1
                 for (uint32_t e = lane; e < nq * wide * RC; e += 32) psum[e] = 0.0f;
             }
@@ -758,6 +757,12 @@ eval_kernel(const DeviceBatch batch, const EvalProblem prob, const Geom geom, fl
             __syncwarp();
             const bool has_shared = mid_off > 0u, has_prelude = main_off > mid_off;
             const uint32_t eval_groups = (flags & SB_PROG_BANK_INDEPENDENT) ? 1u : ngroups;
+
+            /* PARTS: where this lane's totals of a pass go, [pass][program][quantity][bank]; of the last group's
+             * columns only those below `banks` are banks */
+            const uint32_t my_bank = first_bg * RC + lane / (32 / RC), banks = lane_sums ? prob.num_banks : 0u;
+            float* totals = partial;
+            if constexpr (PARTS && !materialize) totals += ((c0 / M::PASS + pass) * batch.num_programs + lp) * nq * configs + my_bank;
 
             M m;
             place.code = code;
@@ -826,7 +831,9 @@ eval_kernel(const DeviceBatch batch, const EvalProblem prob, const Geom geom, fl
                                 part[c] = __fmaf_rn(sbm::hi2(e), sbm::hi2(e), part[c]);
                             }
                         }
-                        add_shared(psum32 + gi * (RC * 4u), column_totals<RC>(part, lane), lane_sums);
+                        const float total = column_totals<RC>(part, lane);
+                        if constexpr (!PARTS) add_shared(psum32 + gi * (RC * 4u), total, lane_sums);
+                        else if (my_bank + g * RC < banks) totals[g * RC] = total;
                     } else {
                         /* several targets, or affine statistics: quantity q of pair gi lives in psum[(q * wide + gi) * RC + c] */
 #pragma unroll 1
@@ -850,12 +857,15 @@ eval_kernel(const DeviceBatch batch, const EvalProblem prob, const Geom geom, fl
                                     s[c] = __fadd_rn(__fadd_rn(s[c], sbm::lo2(term)), sbm::hi2(term));
                                 }
                             }
-                            add_shared(psum32 + (qn * wide + gi) * (RC * 4u), column_totals<RC>(s, lane), lane_sums);
+                            const float total = column_totals<RC>(s, lane);
+                            if constexpr (!PARTS) add_shared(psum32 + (qn * wide + gi) * (RC * 4u), total, lane_sums);
+                            else if (my_bank + g * RC < banks) totals[qn * configs + g * RC] = total;
                         }
                     }
                 }
+                if constexpr (PARTS && !materialize) totals += (size_t)batch.num_programs * nq * configs;
             }
-            if (materialize) continue;
+            if (materialize || PARTS) continue;
             __syncwarp();
             /* this CTA's partial sums of the item: stored on its first tile, added to afterwards (only this
              * CTA touches them, and a barrier separates its tiles) */
@@ -863,8 +873,7 @@ eval_kernel(const DeviceBatch batch, const EvalProblem prob, const Geom geom, fl
                 const bool independent = (flags & SB_PROG_BANK_INDEPENDENT) != 0;
                 const uint32_t width = ngroups * RC, bank0 = first_bg * RC; /* banks of the item, padding included */
                 const uint32_t real = min(width, prob.num_banks - bank0);
-                const uint32_t row_share = PARTS ? exec[-1].w1 : split;
-                float* mine = partial + (geom.direct ? gp * prob.out_program_stride : ((size_t)row_share * batch.num_programs + lp) * nq * configs) +
+                float* mine = partial + (geom.direct ? gp * prob.out_program_stride : ((size_t)split * batch.num_programs + lp) * nq * configs) +
                               ((size_t)bank0 << prob.toggle_bits);
                 float* sums = psum; /* psum is [quantity][permutation][group][bank of the group] */
                 if constexpr (!SPAN) {
@@ -915,8 +924,9 @@ eval_kernel(const DeviceBatch batch, const EvalProblem prob, const Geom geom, fl
 }
 
 
-/* the launches of one kind of kernel, over the tile shapes; PARTS: the launch cuts tiles into parts or does not begin with
- * its first program (small launches without toggles; what it takes made large ones 1 % slower) */
+/* the launches of one kind of kernel, over the tile shapes; PARTS: the launch keeps the totals of passes (in place of sums in
+ * shared memory), cuts tiles into parts or does not begin with its first program (small launches without toggles; what it
+ * takes made large ones 1 % slower) */
 template <int KIND, int RR, int RC, bool SPAN, bool PARTS>
 void launch_parts(const DeviceBatch& batch, const EvalProblem& prob, const Geom& geom, const LaunchPlan& plan, float* partial,
                   const float* tables, cudaStream_t stream) {
@@ -926,7 +936,7 @@ void launch_parts(const DeviceBatch& batch, const EvalProblem& prob, const Geom&
 template <int KIND, int RR, int RC, bool SPAN>
 cudaError_t launch_shape(const DeviceBatch& batch, const EvalProblem& prob, const Geom& geom, const LaunchPlan& plan, float* partial,
                          const float* tables, cudaStream_t stream) {
-    if (!SPAN && (geom.parts > 1u || batch.first)) launch_parts<KIND, RR, RC, SPAN, !SPAN>(batch, prob, geom, plan, partial, tables, stream);
+    if (!SPAN && (plan.pass_sums || geom.parts > 1u || batch.first)) launch_parts<KIND, RR, RC, SPAN, !SPAN>(batch, prob, geom, plan, partial, tables, stream);
     else launch_parts<KIND, RR, RC, SPAN, false>(batch, prob, geom, plan, partial, tables, stream);
     return cudaGetLastError();
 }

@@ -175,6 +175,68 @@ __global__ void combine_kernel(const DeviceBatch batch, const EvalProblem prob, 
     }
 }
 
+/* The same for a launch that kept the total of every pass ([pass][program][quantity][configuration]): adds them as the rules'
+ * cut of the rows would have, the passes of a tile from zero, the tiles of a split, the splits, so the sum has the bits of a
+ * launch cut by the rules.  `slots` threads share an output, each with a tile at a time; the thread of slot 0 folds the tiles in
+ * order while the others fetch the next ones (two buffers of tile sums, one barrier for every `slots` tiles).  Bound by the
+ * latency of its loads, of which a tile has up to eight: they are all started before the first is added, and there are as many
+ * slots as the machine has room for threads (128,000 outputs x 157 passes, four slots: 36 us, 52 with loads that wait for
+ * each other).  There are fewer totals than 2^32 (planner.cpp). */
+struct PassNest { uint32_t tile, split; }; /* passes of a tile, tiles of a split */
+constexpr uint32_t kFoldThreads = 256;
+
+__global__ void __launch_bounds__(kFoldThreads)
+combine_passes_kernel(const DeviceBatch batch, const EvalProblem prob, const float* __restrict__ partial, uint32_t passes, PassNest before,
+                      PassNest others, uint32_t per_program, uint32_t slots) {
+    __shared__ float sums[2][kFoldThreads];
+    const uint32_t outputs = kFoldThreads / slots, slot = threadIdx.x / outputs;
+    const uint32_t total = per_program * batch.num_programs, i = blockIdx.x * outputs + threadIdx.x % outputs;
+    const bool live = i < total;
+    const uint32_t lp = live ? i / per_program : 0u, within = i - lp * per_program;
+    const uint32_t qn = within / prob.num_banks, cfg = within - qn * prob.num_banks;
+    /* of a program that reads no coefficient only the first bank group is evaluated, and its first total is every bank's */
+    const bool independent = (batch.programs[lp].flags & SB_PROG_BANK_INDEPENDENT) != 0;
+    const PassNest nest = lp < batch.first ? before : others;
+    const uint32_t tiles = (passes + nest.tile - 1) / nest.tile;
+    const uint32_t most = max((passes + before.tile - 1) / before.tile, (passes + others.tile - 1) / others.tile);
+    const float* const from = partial + (i - (independent ? cfg : 0u));
+    float split = 0.0f, sum = 0.0f;
+    uint32_t buffer = 0, in_split = 0;
+#pragma unroll 1
+    for (uint32_t first = 0; first < most; first += slots, buffer ^= 1u) {
+        const uint32_t tile = first + slot;
+        if (live && tile < tiles) {
+            const uint32_t begin = tile * nest.tile, end = min(passes, begin + nest.tile);
+            float v = 0.0f;
+#pragma unroll 1
+            for (uint32_t p = begin; p < end; p += 8u) {
+                float x[8];
+#pragma unroll
+                for (uint32_t j = 0; j < 8u; ++j)
+                    if (p + j < end) x[j] = __ldg(from + (size_t)(p + j) * total);
+#pragma unroll
+                for (uint32_t j = 0; j < 8u; ++j)
+                    if (p + j < end) v = __fadd_rn(v, x[j]);
+            }
+            sums[buffer][threadIdx.x] = v;
+        }
+        __syncthreads();
+        if (slot == 0 && live) {
+            const uint32_t n = first < tiles ? min(slots, tiles - first) : 0u;
+#pragma unroll 4
+            for (uint32_t s = 0; s < n; ++s) {
+                const float v = sums[buffer][s * outputs + threadIdx.x];
+                split = in_split ? __fadd_rn(split, v) : v;
+                if (++in_split == nest.split || first + s + 1 == tiles) {
+                    sum = first + s < nest.split ? split : __fadd_rn(sum, split);
+                    in_split = 0;
+                }
+            }
+        }
+    }
+    if (slot == 0 && live) prob.output[(prob.first_program + batch.programs[lp].index) * prob.out_program_stride + (size_t)qn * prob.out_target_stride + cfg] = sum;
+}
+
 template <int RC>
 void launch_tables(const DeviceBatch& batch, const EvalProblem& prob, uint32_t banks, float* tables, cudaStream_t stream) {
     const uint32_t padded = (banks + RC - 1) / RC * RC;
@@ -222,7 +284,7 @@ cudaError_t launch_eval(const DeviceBatch& batch, const EvalProblem& prob, const
         ++launched;
     }
     /* a run whose rows are not split has whole sums: they go straight to the caller's grid */
-    geom.direct = !materialize && plan.row_splits * plan.parts == 1 ? 1u : 0u;
+    geom.direct = !materialize && !plan.pass_sums && plan.row_splits == 1 ? 1u : 0u;
     float* const sums = geom.direct ? prob.output : partial;
     /* runs without toggles have a kernel without the permutations' code: with it inside, the population of
      * 2,048 programs x 64 sets took 34.1 ms instead of 30.0 (registers, not instructions) */
@@ -236,8 +298,22 @@ cudaError_t launch_eval(const DeviceBatch& batch, const EvalProblem& prob, const
     const uint32_t nq = prob.mode == EVAL_AFFINE_STATS ? prob.num_targets + 2u : prob.num_targets;
     const unsigned long long configs = (unsigned long long)prob.num_banks << prob.toggle_bits;
     const unsigned long long total = (unsigned long long)nq * configs * batch.num_programs;
-    const unsigned blocks = (unsigned)std::min<unsigned long long>((total + 255) / 256, 148ull * 16ull);
-    combine_kernel<<<blocks ? blocks : 1u, 256, 0, stream>>>(batch, prob, partial, plan.row_splits * plan.parts, nq, configs);
+    if (plan.pass_sums) {
+        const uint32_t pass = 32u * (uint32_t)kVariantRows[plan.variant], passes = (uint32_t)((prob.num_rows + pass - 1) / pass);
+        PassNest nest[2];
+        uint32_t most = 1, slots = 1;
+        for (int k = 0; k < 2; ++k) {
+            nest[k] = PassNest{plan.rules[k].tile_rows / pass, (uint32_t)(plan.rules[k].rows_per_split / plan.rules[k].tile_rows)};
+            most = std::max(most, (passes + nest[k].tile - 1) / nest[k].tile);
+        }
+        while (slots < most && slots < 32u && total * slots < 148ull * 2048ull) slots *= 2;
+        const unsigned long long outputs = kFoldThreads / slots;
+        combine_passes_kernel<<<(unsigned)((total + outputs - 1) / outputs), kFoldThreads, 0, stream>>>(batch, prob, partial, passes, nest[0], nest[1],
+                                                                                                       nq * prob.num_banks, slots);
+    } else {
+        const unsigned blocks = (unsigned)std::min<unsigned long long>((total + 255) / 256, 148ull * 16ull);
+        combine_kernel<<<blocks ? blocks : 1u, 256, 0, stream>>>(batch, prob, partial, plan.row_splits, nq, configs);
+    }
     e = cudaGetLastError();
     if (e == cudaSuccess) *launches = ++launched;
     return e;

@@ -95,6 +95,13 @@ struct EvalProblem {
     size_t out_target_stride;  /* elements between consecutive targets  */
 };
 
+/* How the planner's rules cut the rows of a launch into tiles and row splits, and with that the order in which rows are added:
+ * the passes of a tile from zero, the tiles of a split, the splits. */
+struct RowCut {
+    uint32_t tile_rows;
+    size_t rows_per_split;
+};
+
 /* Launch geometry chosen by plan_launch(). */
 struct LaunchPlan {
     int variant;              /* rows x banks per thread: 0: 4x4, 1: 8x2, 2: 16x1 */
@@ -104,11 +111,13 @@ struct LaunchPlan {
     uint32_t num_groups;      /* CTAs along the programs; group g owns programs g, g + num_groups, ... */
     uint32_t groups_per_item; /* bank groups of one permutation a warp handles per queue item */
     uint32_t perms_per_item;  /* consecutive permutations one item covers (a power of two; above 1 only when an item holds every bank group) */
-    uint32_t parts;           /* items that share the rows of a tile, each with a range of its passes and sums of its own */
+    uint32_t parts;           /* items that share the rows of a tile, each with a range of its passes */
     uint32_t row_splits;      /* CTAs sharing one program group, each with a row range */
     size_t rows_per_split;
+    RowCut rules[2];          /* of the programs before DeviceBatch::first, and of the others */
+    bool pass_sums;           /* rows are not cut by the rules: the total of every pass is kept, and added in the rules' order afterwards */
     size_t smem_bytes;
-    size_t partial_elements;  /* floats of partial sums over all row splits and parts (0: materialize) */
+    size_t partial_elements;  /* floats of partial sums over all row splits, or passes (0: materialize) */
     size_t table_elements;    /* floats of constant tables */
     size_t table_offset;      /* where they begin in the launch's scratch, 16-byte aligned: behind the partial sums, or
                                  at 0 when the rows are not split and the sums go straight to the output */
@@ -136,7 +145,7 @@ struct Geom {
     uint32_t warp_bytes;
     uint32_t scratch_slot;    /* spill slot reserved for the element-by-element FMA */
     unsigned long long rows_per_split;
-    uint32_t direct;          /* neither rows nor tiles are split: sums go to the output, not to partial sums */
+    uint32_t direct;          /* rows are not split: sums go to the output, not to partial sums */
 };
 
 constexpr int kNumVariants = 3;
@@ -147,21 +156,26 @@ Geom make_geom(const DeviceBatch& batch, const EvalProblem& problem, const Launc
 
 /* scratch_limit: most floats of scratch a launch may use: the row splits are reduced until their partial sums
  * fit beside the constant tables (with one split there are none; the tables are not reduced here).
- * neighbour: what a small launch should know of another that runs beside it. */
+ * neighbour: what a small launch should know of another that runs beside it; it decides about time, never about the order in
+ * which rows are added.
+ * rules: of a batch of two kinds of programs (DeviceBatch::first), how each kind's rows are cut when it is launched by itself. */
 struct Neighbour {
     enum Kind { NONE, SHARES, LEAVES, FILLS } kind; /* SHARES: it takes the rest of the machine.  LEAVES: it comes first and leaves some SMs, and
                                                        CTAs that do not fit those would hold up its own.  FILLS: it comes first and leaves SMs
-                                                       one by one at its end: rows are cut by the rules */
+                                                       one by one at its end */
     double share;                                   /* the part of the machine to count on */
 };
 LaunchPlan plan_launch(const DeviceBatch& batch, const EvalProblem& problem, int sm_count, size_t smem_limit,
-                       size_t scratch_limit, Neighbour neighbour = Neighbour{Neighbour::NONE, 1.0});
+                       size_t scratch_limit, Neighbour neighbour = Neighbour{Neighbour::NONE, 1.0}, const RowCut* rules = nullptr);
+/* The same by the rules alone, without the cut of small launches: its register tile and rules[0] are what a launch adds by. */
+LaunchPlan plan_rules(const DeviceBatch& batch, const EvalProblem& problem, int sm_count, size_t smem_limit, size_t scratch_limit);
 
 /* Enqueues the evaluation of one batch on `stream`: the evaluator kernel writes per-split partial
  * sums into `partial` (plan.table_offset + plan.table_elements floats, private to the stream until the
  * launch has finished; the programs' constant tables are computed into its end first) and a second kernel
  * adds them in a fixed order into the output, so a result does not depend on the order CTAs ran in; with one
- * row split the sums are whole and go to the output at once.  Returns the CUDA status of the launches. */
+ * row split the sums are whole and go to the output at once.  With plan.pass_sums the partial sums are those of
+ * every pass, and the second kernel adds them as the rules' cut would.  Returns the CUDA status of the launches. */
 cudaError_t launch_eval(const DeviceBatch& batch, const EvalProblem& problem, const LaunchPlan& plan, float* partial,
                         cudaStream_t stream, unsigned* launches);
 

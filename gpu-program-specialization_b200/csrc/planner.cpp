@@ -66,7 +66,10 @@ size_t smem_needed(const Geom& g, uint32_t warps) { return (size_t)g.tile_bytes 
  * The constants are issue slots, measured on the 64-set population: 330 for one pass of the main part with
  * its loss, about 900 to set an item up, and a warp that issues every seventh cycle when alone; an SM
  * issues 2.6 per cycle at best.  (A launch whose programs read few of the run's toggle bits is small in this sense
- * too.)  The order in which rows are added follows the cut, and the cut follows the request and the population.
+ * too.)  The order in which rows are added does not follow the cut: where its rows are not the rules', the launch keeps the
+ * total of every pass, which is the same number in any cut, and they are added as the rules' tiles and splits would add them
+ * (combine_passes_kernel in evaluator.cu).  With toggles, whose kernel keeps no such totals, and where there is no room for
+ * them, the rows stay the rules'.
  * Tiles of half the rows, CTAs of several tiles and parts of tiles are tried since a CTA of 19 items on 20 warps ends
  * with its longest program: 124 programs x 8 sets x 47,735 rows 320 -> 197 us a call, 488 x 16 x 5,823 191 -> 145, 124 x
  * 3 x 19,735 163 -> 155 (all with their few heavy programs in the same launch, see views_to_launch in runner.cpp). */
@@ -97,11 +100,10 @@ double cut_cycles(const Cut& cut, const Work& w) {
     return (double)((grid + w.sms - 1) / w.sms) * cta(item * std::max({std::ceil(items / cut.warps), items / cut.warps + 0.5, w.longest}));
 }
 
-/* `sms`: the part of the machine (`all`) this launch has when another runs beside it; `room`: floats of scratch for
- * partial sums. */
+/* `sms`: the part of the machine (`all`) this launch has when another runs beside it; `free_rows`: other rows than the rules'
+ * may be tried. */
 void balance_small(LaunchPlan* plan, const DeviceBatch& batch, const EvalProblem& prob, int sms, int all, Neighbour::Kind neighbour, size_t smem_limit,
-                   unsigned long long room) {
-    const bool behind = neighbour == Neighbour::FILLS;
+                   bool free_rows) {
     const bool materialize = prob.mode == EVAL_MATERIALIZE;
     const uint32_t rr = (uint32_t)kVariantRows[plan->variant], rc = (uint32_t)kVariantBanks[plan->variant], pass = 32u * rr;
     const unsigned long long P = batch.num_programs, bank_groups = materialize ? 1 : (prob.num_banks + rc - 1) / rc;
@@ -128,7 +130,6 @@ void balance_small(LaunchPlan* plan, const DeviceBatch& batch, const EvalProblem
     Work work{P, bank_groups, materialize ? 1.0 : batch.total_perms / (double)P, materialize ? 1.0 : (double)(1ull << batch.max_bits), 0, prelude, sms,
               batch.total_cost ? std::min(3.0, std::max(1.0, (double)batch.max_cost * (double)P / (double)batch.total_cost)) : 1.0};
     const auto passes_of = [&](uint32_t tile_rows) { return (uint32_t)((std::min<size_t>(tile_rows, prob.num_rows) + pass - 1) / pass); };
-    const unsigned long long per_sum = materialize ? 0 : (unsigned long long)P * std::max<uint32_t>(1u, quantities(prob)) * ((unsigned long long)prob.num_banks << prob.toggle_bits);
     Cut best{plan->tile_rows, (uint32_t)((plan->rows_per_split + plan->tile_rows - 1) / plan->tile_rows), plan->row_splits, plan->warps,
              plan->groups_per_item, plan->perms_per_item, 1u, plan->num_groups};
     work.passes = passes_of(plan->tile_rows);
@@ -136,12 +137,8 @@ void balance_small(LaunchPlan* plan, const DeviceBatch& batch, const EvalProblem
     if (neighbour == Neighbour::LEAVES && rule_grid > (unsigned long long)sms) least = 1e300; /* any cut of one wave instead */
     const Cut rules = best;
     LaunchPlan trial = *plan;
-    /* Two kinds of launches keep the tiles and row splits of the rules.  Uneven ones, whose estimate is too coarse for more,
-     * and those behind a launch that fills the machine, which follows the rules too: in a large population the order in
-     * which rows are added then does not hang on the cut of its few heavy programs, so programs of nearly equal scores do not
-     * change their ranks with it (2,048 programs x 64 sets: up to 2 % of the first 1,024 ranks otherwise). */
-    const bool uneven = work.perms < work.most_perms, same_rows = uneven || behind;
-    for (uint32_t half = 0; half < (same_rows ? 1u : 2u); ++half) { /* the rules' tile and one of half its rows */
+    const bool uneven = work.perms < work.most_perms;
+    for (uint32_t half = 0; half < (free_rows ? 2u : 1u); ++half) { /* the rules' tile and one of half its rows */
         trial.tile_rows = half ? (rules.tile_rows / 2 + pass - 1) / pass * pass : rules.tile_rows;
         if (half && (trial.tile_rows == rules.tile_rows || trial.tile_rows < 256u)) break;
         work.passes = passes_of(trial.tile_rows);
@@ -159,14 +156,12 @@ void balance_small(LaunchPlan* plan, const DeviceBatch& batch, const EvalProblem
                     for (unsigned waves = uneven ? 0u : 1u; waves <= most_waves; waves += waves < 8 ? 1 : 4) {
                         const unsigned long long ctas = waves ? (unsigned long long)waves * sms : rules.groups * rules.splits;
                         Cut c{trial.tile_rows, (uint32_t)((tiles + ctas - 1) / ctas), 0, trial.warps, gpi, ppi, 1u, 0};
-                        if (same_rows) c.tiles_per_split = rules.tiles_per_split;
+                        if (!free_rows) c.tiles_per_split = rules.tiles_per_split;
                         if (uneven) c.warps = rules.warps;
                         if ((c.tiles_per_split > 1) != (trial.tile_buffers > 1)) continue;
                         c.splits = (uint32_t)((tiles + c.tiles_per_split - 1) / c.tiles_per_split);
-                        if (per_sum && c.splits > 1 && c.splits > rules.splits && c.splits > room / per_sum) continue;
                         c.groups = std::max<unsigned long long>(1, std::min(ctas / c.splits, P));
-                        for (c.parts = 1; c.parts <= (prob.toggle_bits || same_rows ? 1u : work.passes); c.parts *= 2) {
-                            if (c.parts > 1 && per_sum && (unsigned long long)c.splits * c.parts > room / per_sum) break;
+                        for (c.parts = 1; c.parts <= (free_rows ? work.passes : 1u); c.parts *= 2) {
                             if (items * c.parts > 0xffffff00ull / ((P + c.groups - 1) / c.groups)) break;
                             const double t = cut_cycles(c, work);
                             if (t < least) { least = t; best = c; }
@@ -176,7 +171,6 @@ void balance_small(LaunchPlan* plan, const DeviceBatch& batch, const EvalProblem
                 }
             }
     }
-    if (!plan->tile_rows || best.tile_rows == 0) return;
     plan->tile_rows = best.tile_rows;
     plan->tile_buffers = best.tiles_per_split > 1 ? 2u : 1u;
     plan->row_splits = best.splits;
@@ -189,8 +183,13 @@ void balance_small(LaunchPlan* plan, const DeviceBatch& batch, const EvalProblem
     refit(plan, 0u);
 }
 
+/* Most floats for the totals of passes (256 MB).  A launch that needs more has 8.6e9 values of rows to compute, 13 ms at least,
+ * and is of many waves by the rules unless its programs are few; below, the totals pay (1,000 programs x 64 sets x 60,000 rows,
+ * 30 million of them: 6.6 ms, 7.0 with the rules' rows). */
+constexpr unsigned long long kMostPassSums = 1ull << 26;
+
 LaunchPlan plan_with_tile(const DeviceBatch& batch, const EvalProblem& prob, int sm_count, size_t smem_limit, size_t scratch_limit,
-                          int variant, const Neighbour& neighbour) {
+                          int variant, bool balance, const Neighbour& neighbour, const RowCut* joint) {
     LaunchPlan plan{};
     plan.ok = false;
     plan.overflow = false;
@@ -312,22 +311,36 @@ LaunchPlan plan_with_tile(const DeviceBatch& batch, const EvalProblem& prob, int
     if (grid > 0x7fffffffull) { plan.overflow = true; return plan; }
     plan.grid_x = (uint32_t)grid;
 
+    const RowCut own{plan.tile_rows, plan.rows_per_split};
+    plan.rules[0] = joint ? joint[0] : own;
+    plan.rules[1] = joint ? joint[1] : own;
     const unsigned long long room = scratch_limit > plan.table_elements + 3 ? scratch_limit - plan.table_elements - 3 : 0;
-    balance_small(&plan, batch, prob, std::max(1, (int)(sm_count * neighbour.share)), sm_count, neighbour.kind, smem_limit, room);
+    const unsigned long long passes = (prob.num_rows + pass - 1) / pass;
+    const bool keeps_passes = !prob.toggle_bits && (materialize || passes <= std::min(room, kMostPassSums) / std::max(1ull, configs) / nq / P);
+    if (joint && !keeps_passes) return plan;
+    /* behind a launch that fills the machine the rules' rows stay as well: the estimate knows nothing of the SMs that become
+     * free one by one (4,000 programs x 16 sets x 30,000 rows, 188 of them heavy: 3.89 ms with them, 4.39 with the cut it
+     * prefers; 2,048 x 64 x 131,072: 28.6 and 28.1) */
+    if (balance)
+        balance_small(&plan, batch, prob, std::max(1, (int)(sm_count * neighbour.share)), sm_count, neighbour.kind, smem_limit,
+                      keeps_passes && neighbour.kind != Neighbour::FILLS);
+    plan.pass_sums = !materialize && (joint || plan.parts > 1 || plan.tile_rows != own.tile_rows || plan.rows_per_split != own.rows_per_split);
     plan.partial_elements = 0;
     if (!materialize) {
-        const unsigned long long n = (unsigned long long)plan.row_splits * plan.parts * P;
+        const unsigned long long n = (plan.pass_sums ? passes : plan.row_splits) * P;
         if (configs && n > (~0ull >> 3) / configs / nq) { plan.overflow = true; return plan; }
         plan.partial_elements = (size_t)(n * nq * configs);
     }
-    plan.table_offset = plan.row_splits * plan.parts > 1 ? (plan.partial_elements + 3) / 4 * 4 : 0; /* whole sums go to the output */
+    plan.table_offset = plan.pass_sums || plan.row_splits > 1 ? (plan.partial_elements + 3) / 4 * 4 : 0; /* whole sums go to the output */
     plan.ok = true;
     return plan;
 }
 
 }  // namespace
 
-LaunchPlan plan_launch(const DeviceBatch& batch, const EvalProblem& prob, int sm_count, size_t smem_limit, size_t scratch_limit, Neighbour neighbour) {
+namespace {
+LaunchPlan plan_any_tile(const DeviceBatch& batch, const EvalProblem& prob, int sm_count, size_t smem_limit, size_t scratch_limit, bool balance,
+                         const Neighbour& neighbour, const RowCut* rules) {
     /* register tile: 4 rows x 4 banks per thread, or 8 x 2 / 16 x 1 when there are fewer banks.  Up
      * to four banks take the 8 x 2 tile: three or four banks are then two bank groups, so the row
      * prelude serves two runs of the main part and computes each row's value twice instead of four
@@ -339,10 +352,19 @@ LaunchPlan plan_launch(const DeviceBatch& batch, const EvalProblem& prob, int sm
     if (prob.mode == EVAL_MATERIALIZE) variant = 2;
     LaunchPlan plan{};
     for (; variant >= 0; --variant) {
-        plan = plan_with_tile(batch, prob, sm_count, smem_limit, scratch_limit, variant, neighbour);
+        plan = plan_with_tile(batch, prob, sm_count, smem_limit, scratch_limit, variant, balance, neighbour, rules);
         if (plan.ok || plan.overflow) break;
     }
     return plan;
+}
+}  // namespace
+
+LaunchPlan plan_launch(const DeviceBatch& batch, const EvalProblem& prob, int sm_count, size_t smem_limit, size_t scratch_limit, Neighbour neighbour,
+                       const RowCut* rules) {
+    return plan_any_tile(batch, prob, sm_count, smem_limit, scratch_limit, true, neighbour, rules);
+}
+LaunchPlan plan_rules(const DeviceBatch& batch, const EvalProblem& prob, int sm_count, size_t smem_limit, size_t scratch_limit) {
+    return plan_any_tile(batch, prob, sm_count, smem_limit, scratch_limit, false, Neighbour{Neighbour::NONE, 1.0}, nullptr);
 }
 
 }  // namespace sb

@@ -121,6 +121,7 @@ struct Slot {
 struct View {
     DeviceBatch batch;
     size_t first;
+    RowCut rules[2] = {}; /* of a joint view: how its two kinds' rows are cut when they are launched apart */
 };
 
 }  // namespace
@@ -520,7 +521,7 @@ SecantResult upload_batch(SecantCubinRunnerImpl* r, Slot& s, std::vector<View>* 
             db.max_btmp = std::max<uint32_t>(db.max_btmp, p.n_btmp);
             db.uses_scratch |= (p.flags & SB_PROG_USES_SCRATCH) ? 1u : 0u;
         }
-        views->push_back(View{db, bounds[k]});
+        views->push_back(View{db, bounds[k], {}});
     }
     return SECANT_SUCCESS;
 }
@@ -594,6 +595,12 @@ Neighbour view_share(const SecantCubinRunnerImpl* r, const std::vector<View>& vi
     return Neighbour{Neighbour::SHARES, std::min(0.95, std::max(0.05, (double)view.batch.total_cost / std::max(1.0, all)))};
 }
 
+/* Half of the scratch limit is for constant tables (an entry per program constant and configuration), the rest for the
+ * partial sums of the row splits, without which few programs would fill few SMs. */
+bool tables_fit(const SecantCubinRunnerImpl* r, const DeviceBatch& batch, uint32_t banks) {
+    return batch.total_cst <= r->scratch_limit / 2 / ((banks + 3ull) << batch.max_bits);
+}
+
 /* The programs of a view from `first` on whose constant tables take at most `most` floats, one at least.  Every
  * table of a launch has room for the permutations of the program that reads most bits, so a launch takes its
  * measure from its own programs: those with most permutations come first in launch order and mostly keep to
@@ -603,7 +610,6 @@ DeviceBatch tables_that_fit(const View& view, const SbProgram* headers, size_t f
     DeviceBatch part = view.batch;
     part.programs += first;
     part.num_programs = 0;
-    part.first = 0; /* in launch order: the heavy programs of a joint view come last here */
     part.total_cst = 0;
     part.total_cost = part.max_cost = part.main_cost = part.prelude_cost = 0; /* what the planner weighs against its number of programs */
     part.total_perms = 0;
@@ -647,8 +653,16 @@ std::vector<View> views_to_launch(SecantCubinRunnerImpl* r, const std::vector<Vi
     b.prelude_cost += heavy.prelude_cost;
     b.total_perms += heavy.total_perms;
     b.max_bits = std::max(b.max_bits, heavy.max_bits);
-    const LaunchPlan plan = plan_launch(b, prob, r->sm_count, r->smem_limit, r->scratch_limit);
-    if (!plan.ok || plan.warps < 16u || (uint64_t)plan.grid_x >= 8ull * (uint64_t)r->sm_count) return views;
+    if (!tables_fit(r, b, prob.num_banks)) return views;
+    int variant = -1; /* each program's rows are added in the order of the launch its kind would have */
+    for (int k = 0; k < 2; ++k) {
+        const LaunchPlan alone = plan_rules(views[k].batch, prob, r->sm_count, r->smem_limit, r->scratch_limit);
+        if (!alone.ok || (k && alone.variant != variant)) return views;
+        variant = alone.variant;
+        all.rules[k] = alone.rules[0];
+    }
+    const LaunchPlan plan = plan_launch(b, prob, r->sm_count, r->smem_limit, r->scratch_limit, Neighbour{Neighbour::NONE, 1.0}, all.rules);
+    if (!plan.ok || plan.variant != variant || plan.warps < 16u || (uint64_t)plan.grid_x >= 8ull * (uint64_t)r->sm_count) return views;
     /* an item of a pass or two pays for its set-up once more when the heavy programs' memory makes the tile smaller
      * (3,000 programs without coefficients, 20,011 rows: 1 % of the call) */
     if (plan.tile_rows / (32u * (uint32_t)kVariantRows[plan.variant]) * plan.groups_per_item < 8u) {
@@ -673,22 +687,20 @@ SecantResult launch_batch(SecantCubinRunnerImpl* r, const std::vector<View>& bat
         /* what a view's launches should know of the last launch of the view before, on another stream; a view's own
          * launches come one after the other */
         Neighbour neighbour = view_share(r, views, views[0], runs.size());
+        const bool beside = neighbour.kind != Neighbour::NONE;
         for (const View& view : views) {
         const DeviceBatch& db = view.batch;
         Neighbour next = neighbour;
         const size_t k = (*stream_cursor)++ % r->streams.size();
         cudaStream_t stream = r->streams[k];
         cudaError_t ce = after ? cudaStreamWaitEvent(stream, after, 0) : cudaSuccess;
-        /* one launch, unless its constant tables (an entry per program constant and configuration) would
-         * take more than half of the scratch limit (the rest is for the partial sums of the row splits, without
-         * which few programs would fill few SMs): then the programs in as many launches as it takes, and a
-         * program at a time at least */
-        const size_t most_tables = r->scratch_limit / 2;
-        const bool whole = db.total_cst <= most_tables / ((prob.num_banks + 3ull) << db.max_bits);
+        /* one launch, unless its constant tables would take too much: then the programs in as many launches as it
+         * takes, and a program at a time at least */
+        const bool whole = tables_fit(r, db, prob.num_banks);
         for (size_t first = 0; first < db.num_programs && ce == cudaSuccess;) {
-            const DeviceBatch part = whole ? db : tables_that_fit(view, headers, first, prob.num_banks, most_tables);
+            const DeviceBatch part = whole ? db : tables_that_fit(view, headers, first, prob.num_banks, r->scratch_limit / 2);
             first += part.num_programs;
-            const LaunchPlan lp = plan_launch(part, prob, r->sm_count, r->smem_limit, r->scratch_limit, neighbour);
+            const LaunchPlan lp = plan_launch(part, prob, r->sm_count, r->smem_limit, r->scratch_limit, neighbour, part.first ? view.rules : nullptr);
             if (!lp.ok) {
                 r->last_error = lp.overflow ? "configuration count beyond the evaluator's 32-bit item index" : "program batch does not fit shared memory";
                 return lp.overflow ? SECANT_ERROR_OVERFLOW : SECANT_ERROR_REGISTER_OVERFLOW;
@@ -703,8 +715,7 @@ SecantResult launch_batch(SecantCubinRunnerImpl* r, const std::vector<View>& bat
             /* the launch beside it has the SMs this one leaves; when it leaves none, the other's CTAs come behind it and are
              * best spread over all of them (2,938 programs, eleven of them heavy, 227,933 rows: 4.2 ms, 5.0 with those
              * confined to the SMs their work is worth) */
-            if (neighbour.kind != Neighbour::NONE)
-                next = lp.grid_x < (uint32_t)r->sm_count ? Neighbour{Neighbour::LEAVES, 1.0 - (double)lp.grid_x / r->sm_count} : Neighbour{Neighbour::FILLS, 1.0};
+            if (beside) next = lp.grid_x < (uint32_t)r->sm_count ? Neighbour{Neighbour::LEAVES, 1.0 - (double)lp.grid_x / r->sm_count} : Neighbour{Neighbour::FILLS, 1.0};
             g_kernel_launches.fetch_add(launches);
             if (launches)
                 g_row_stream_bytes.fetch_add((uint64_t)lp.num_groups * (prob.num_inputs + (prob.mode == EVAL_MATERIALIZE ? 0u : prob.num_targets)) *

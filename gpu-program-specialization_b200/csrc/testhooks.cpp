@@ -267,31 +267,39 @@ SBT_EXPORT int sbt_validate_runs(const SecantCubinRecipeHeader* recipe, const Se
 /* Launch geometry the runner would pick for a batch with the given maxima (planner.cpp), so its
  * bounds can be checked without a device.  Returns 1 when a plan exists, 0 when the batch does not
  * fit shared memory, -1 when a count does not fit the kernel's 32-bit indices.
- * out[0..13] = variant, warps, tile_rows, tile_buffers, num_groups, groups_per_item, row_splits,
- * rows_per_split, smem_bytes, partial_elements, grid_x, warp_bytes, items per CTA and tile, perms_per_item. */
+ * weights: total and largest scheduling weight, main parts' and preludes', or null.  neighbour, share: see Neighbour.  joint:
+ * the program CTAs begin with, then tile rows and rows of a split by the rules for the programs before and from it, or null.
+ * out[0..17] = variant, warps, tile_rows, tile_buffers, num_groups, groups_per_item, row_splits,
+ * rows_per_split, smem_bytes, partial_elements, grid_x, warp_bytes, items per CTA and tile, perms_per_item,
+ * parts, pass_sums, tile rows and rows of a split by the rules. */
 #include "evaluator.cuh"
 SBT_EXPORT int sbt_plan(uint32_t num_programs, uint32_t max_insn, uint32_t max_slots, uint32_t max_hoisted, uint32_t max_cst,
                         uint32_t max_btmp, int mode, uint32_t num_inputs, uint32_t num_targets, uint32_t num_banks,
-                        uint32_t toggle_bits, uint64_t rows, int sm_count, uint64_t smem_limit, uint64_t scratch_floats, uint64_t* out) {
+                        uint32_t toggle_bits, uint64_t rows, int sm_count, uint64_t smem_limit, uint64_t scratch_floats,
+                        const uint64_t* weights, int neighbour, double share, const uint64_t* joint, uint64_t* out) {
     DeviceBatch db;
     std::memset(&db, 0, sizeof(db));
     db.num_programs = num_programs; db.max_insn = max_insn; db.max_slots = max_slots; db.max_hoisted = max_hoisted;
     db.max_cst = max_cst; db.max_btmp = max_btmp; db.max_bits = toggle_bits; db.total_perms = (double)num_programs * (double)(1ull << toggle_bits);
+    if (weights) { db.total_cost = weights[0]; db.max_cost = weights[1]; db.main_cost = weights[2]; db.prelude_cost = weights[3]; }
+    if (joint) db.first = (uint32_t)joint[0];
     EvalProblem p;
     std::memset(&p, 0, sizeof(p));
     p.mode = mode; p.num_inputs = num_inputs; p.num_targets = num_targets; p.num_banks = num_banks; p.toggle_bits = toggle_bits;
     p.num_rows = rows;
-    const LaunchPlan plan = plan_launch(db, p, sm_count, smem_limit, scratch_floats);
+    const RowCut rules[2] = {{joint ? (uint32_t)joint[1] : 0u, joint ? (size_t)joint[2] : 0u}, {joint ? (uint32_t)joint[3] : 0u, joint ? (size_t)joint[4] : 0u}};
+    const LaunchPlan plan = plan_launch(db, p, sm_count, smem_limit, scratch_floats, Neighbour{(Neighbour::Kind)neighbour, share}, joint ? rules : nullptr);
     if (!plan.ok) return plan.overflow ? -1 : 0;
     const Geom g = make_geom(db, p, plan);
     const uint64_t rc = (uint64_t)kVariantBanks[plan.variant];
     const uint64_t bank_groups = mode == EVAL_MATERIALIZE ? 1 : (num_banks + rc - 1) / rc;
-    const uint64_t items_per_program = mode == EVAL_MATERIALIZE ? 1 : ((bank_groups / plan.groups_per_item) << toggle_bits) / plan.perms_per_item;
+    const uint64_t items_per_program = (mode == EVAL_MATERIALIZE ? 1 : ((bank_groups / plan.groups_per_item) << toggle_bits) / plan.perms_per_item) * plan.parts;
     const uint64_t per_cta = (num_programs + plan.num_groups - 1) / plan.num_groups;
-    const uint64_t v[14] = {(uint64_t)plan.variant, plan.warps, plan.tile_rows, plan.tile_buffers, plan.num_groups, plan.groups_per_item,
+    const uint64_t v[18] = {(uint64_t)plan.variant, plan.warps, plan.tile_rows, plan.tile_buffers, plan.num_groups, plan.groups_per_item,
                             plan.row_splits, plan.rows_per_split, plan.smem_bytes, plan.partial_elements, plan.grid_x, g.warp_bytes,
-                            per_cta * items_per_program, plan.perms_per_item};
-    for (int i = 0; i < 14; ++i) out[i] = v[i];
+                            per_cta * items_per_program, plan.perms_per_item, plan.parts, plan.pass_sums ? 1u : 0u,
+                            plan.rules[0].tile_rows, plan.rules[0].rows_per_split};
+    for (int i = 0; i < 18; ++i) out[i] = v[i];
     return 1;
 }
 

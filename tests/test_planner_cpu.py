@@ -8,15 +8,17 @@ import pytest
 import support as S
 
 SMEM = 232448          # opt-in shared memory per block of a B200, bytes
-FIELDS = "variant warps tile_rows buffers groups gpi splits rows_per_split smem partial grid warp_bytes items ppi".split()
+FIELDS = "variant warps tile_rows buffers groups gpi splits rows_per_split smem partial grid warp_bytes items ppi parts pass_sums rule_tile rule_rows".split()
 SSE, MATERIALIZE, AFFINE = 0, 1, 2
+NONE, SHARES, LEAVES = 0, 1, 2
 
 
 def plan(programs, rows, banks=64, bits=0, inputs=8, targets=1, mode=SSE, insn=80, slots=2, hoisted=4, table=8, btmp=3,
-         sms=148, smem=SMEM, scratch=1 << 28):
-    out = (C.c_uint64 * 14)()
+         sms=148, smem=SMEM, scratch=1 << 28, weights=None, neighbour=NONE, share=1.0, joint=None):
+    out = (C.c_uint64 * 18)()
     code = S.hooks().sbt_plan(programs, insn, slots, hoisted, table, btmp, mode, inputs, targets, banks, bits, C.c_uint64(rows), sms,
-                              C.c_uint64(smem), C.c_uint64(scratch), out)
+                              C.c_uint64(smem), C.c_uint64(scratch), weights and (C.c_uint64 * 4)(*weights), neighbour,
+                              C.c_double(share), joint and (C.c_uint64 * 5)(*joint), out)
     return code, dict(zip(FIELDS, list(out)))
 
 
