@@ -198,9 +198,8 @@ def reference_arm(args, w):
 # Not measured in this run: counters of that kind need a profiler and the full size is too large for it.
 EXECUTED_ON_REDUCED_CASE = {
     "source": "profiler capture of a reduced case (4,096 programs x 131,072 rows), not this run",
-    "pipe_fma_pct": 29.7, "pipe_alu_pct": 37.1, "pipe_xu_pct": 15.6, "issue_active_pct": 61.0,
-    "instruction_cache_hit_pct": 99.4, "fp32_share_of_executed_instructions": 0.403,
-    "warp_instructions_per_interpreted_instruction": 56,
+    "pipe_fma_pct": 33.3, "pipe_fma_cycles_pct": 56.1, "pipe_alu_pct": 39.3, "pipe_xu_pct": 16.6, "issue_active_pct": 65.0,
+    "instruction_cache_hit_pct": 99.1,
 }
 
 
@@ -210,8 +209,8 @@ EXECUTED_ON_REDUCED_CASE = {
 # population under a profiler (profiles/interpreter_cores.md), not this run.
 RK4_EXECUTED_ON_REDUCED_CASE = {
     "source": "profiler capture of one launch of 4,096 systems, not this run",
-    "warp_instructions_per_interpreted_instruction": 20, "fp32_share_of_executed_instructions": 0.191,
-    "issue_active_pct": 43.8, "instruction_cache_hit_pct": 99.9,
+    "pipe_fma_pct": 16.6, "pipe_fma_cycles_pct": 23.5, "pipe_alu_pct": 23.4, "pipe_xu_pct": 5.3, "issue_active_pct": 45.0,
+    "instruction_cache_hit_pct": 99.9,
 }
 
 def rk4_arm(args, w):
