@@ -99,8 +99,9 @@ static_assert(sizeof(kPairConstants) == 320, "the offsets RK_K2 is given count o
  * nearly all cases: the end of the stage does that itself (MEET), with one branch for both kinds, and only what
  * begins otherwise (REST: a fused multiply-add) starts from its first instruction.  That, and a stage chosen by
  * selects instead of an indexed branch, is two indexed branches less per stage: 1,846 systems of one state, 130
- * trajectories, 527 steps 12.1 -> 11.45 ms; 600 engine systems of two states, 184 stages 1.09 -> 1.04 ms a call; 4,096 of three
- * states, 1,000 steps 23.4 -> 23.2.
+ * trajectories, 527 steps 16.6 -> 16.3 ms (three populations); 600 engine systems of two states, 184 stages 1.05 -> 1.00 ms a
+ * call; of 4,096 of three states, 1,000 steps, whose stages wait for the longest right-hand side, it does not show (six
+ * populations: 23.9 -> 23.8, which differ by 0.1 between runs).
  * (The functions on a copy while the warp votes on their arguments, so that the vote is no link of the chain, and
  * the copy taken over behind it: 23.2 -> 24.7 ms.  It is instructions that cost here as well.)
  *
@@ -425,8 +426,8 @@ __device__ __forceinline__ bool group_all(uint32_t barrier, uint32_t threads, bo
  * sizes in registers; the stage values are in shared memory twice, so one barrier per stage is enough
  * (a warp writes the next stage's value of its state while others still read this stage's).
  * 4,096 systems of three states, 64 trajectories, 1,000 steps: 71.8 ms with one warp per item and the
- * machine in C++, 23.2 now; the warps that are resident (30 of an SM's 64, by their registers) issue in
- * 44 % of the cycles, and wait for one another at the barriers for a third of their time. */
+ * machine in C++, 23.8 now; the warps that are resident (30 of an SM's 64, by their registers) issue in
+ * 45 % of the cycles, and wait for one another at the barriers for a third of their time. */
 template <int RR>
 __global__ void __launch_bounds__(kRolloutMaxWarps * 32, RR == 4 ? 1 : 2)
 rk4_kernel(const DeviceBatch batch, const Rk4Problem prob, const RolloutLayout lay) {
