@@ -654,15 +654,15 @@ std::vector<View> views_to_launch(SecantCubinRunnerImpl* r, const std::vector<Vi
     b.total_perms += heavy.total_perms;
     b.max_bits = std::max(b.max_bits, heavy.max_bits);
     if (!tables_fit(r, b, prob.num_banks)) return views;
-    int variant = -1; /* each program's rows are added in the order of the launch its kind would have */
-    for (int k = 0; k < 2; ++k) {
+    int variant = -1; /* each program's rows are added in the order of the launch its kind would have; predictions are not added */
+    for (int k = 0; k < 2 && prob.mode != EVAL_MATERIALIZE; ++k) {
         const LaunchPlan alone = plan_rules(views[k].batch, prob, r->sm_count, r->smem_limit, r->scratch_limit);
         if (!alone.ok || (k && alone.variant != variant)) return views;
         variant = alone.variant;
         all.rules[k] = alone.rules[0];
     }
     const LaunchPlan plan = plan_launch(b, prob, r->sm_count, r->smem_limit, r->scratch_limit, Neighbour{Neighbour::NONE, 1.0}, all.rules);
-    if (!plan.ok || plan.variant != variant || plan.warps < 16u || (uint64_t)plan.grid_x >= 8ull * (uint64_t)r->sm_count) return views;
+    if (!plan.ok || (variant >= 0 && plan.variant != variant) || plan.warps < 16u || (uint64_t)plan.grid_x >= 8ull * (uint64_t)r->sm_count) return views;
     /* an item of a pass or two pays for its set-up once more when the heavy programs' memory makes the tile smaller
      * (3,000 programs without coefficients, 20,011 rows: 1 % of the call) */
     if (plan.tile_rows / (32u * (uint32_t)kVariantRows[plan.variant]) * plan.groups_per_item < 8u) {
